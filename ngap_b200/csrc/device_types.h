@@ -53,6 +53,28 @@ __host__ __device__ inline uint32_t prefix_hash(uint32_t key) {
   return (key * 0x9E3779B1u) ^ (key >> 15);
 }
 
+// Look-ahead filter of a tile: a bitmap over a hash of the next `len` class ids.
+// The bit of a position is set when some state the tile injects there leads
+// to a path that is alive after `len` symbols or reports within them, so a
+// position whose bit is clear needs no injection at all (hash collisions only
+// set bits). hash = sum of c_i * mul^(len - 1 - i) over the class ids c_i,
+// modulo 2^32; bit (hash * scale) >> shift of `bits`. With mul = live classes
+// and scale = 1 << shift the bitmap is indexed by the exact key. A position
+// with fewer than len symbols left in its unit needs injection when at least
+// min_rep are left (the shortest path to a report). len = 0: no filter.
+constexpr int kMaxFilter = 16;       // most symbols a filter looks ahead
+constexpr uint32_t kFilterMul = 0x9E3779B1u;    // odd multipliers of the hashed form
+constexpr uint32_t kFilterScale = 0x85EBCA6Bu;
+
+struct FilterDev {
+  int32_t len = 0;
+  int32_t min_rep = 1;
+  int32_t shift = 0;
+  uint32_t mul = 0, scale = 0;
+  uint32_t drop = 0;                // mul^len: weight of the symbol that leaves a rolling hash
+  const uint32_t* bits = nullptr;
+};
+
 // A tile: a set of whole CCs (of one group, or of several for a global tile),
 // matched by one warp per unit. Its hot tables form one contiguous image,
 // staged into shared memory by the CTA that works on the tile when it fits
@@ -91,6 +113,7 @@ struct TileDev {
   const uint32_t* sid = nullptr;    // [nstates] local -> report id (sid | group << 22)
   const uint32_t* aas = nullptr;    // [naas] local ids
   const uint32_t* start = nullptr;  // [nstart] local ids
+  FilterDev filt;
   PrefixTableDev pt[kMaxDepth];
 };
 

@@ -255,6 +255,7 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
   CUDA_TRY(cudaSetDevice(device));
   rc = build_tiles(g->gs, to, t->tiles);
   if (rc != NGAP_OK) return rc;
+  build_filters(t->tiles);
   t->num_groups = (int)g->gs.groups.size();
   for (auto& th : t->tiles) {
     if (th.nstates >= kMaxTileStates - 1) {
@@ -297,6 +298,13 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
     if ((rc = t->upload(th.sid, &d.sid)) != NGAP_OK) return rc;
     if ((rc = t->upload(th.aas, &d.aas)) != NGAP_OK) return rc;
     if ((rc = t->upload(th.start, &d.start)) != NGAP_OK) return rc;
+    d.filt.len = th.filt.len;
+    d.filt.min_rep = th.filt.min_rep;
+    d.filt.shift = th.filt.shift;
+    d.filt.mul = th.filt.mul;
+    d.filt.scale = th.filt.scale;
+    d.filt.drop = th.filt.drop;
+    if ((rc = t->upload(th.filt.bits, &d.filt.bits)) != NGAP_OK) return rc;
     for (int k = 0; k < kMaxDepth; k++) {
       const PrefixTableHost& ph = th.pt[k];
       PrefixTableDev& pd = d.pt[k];

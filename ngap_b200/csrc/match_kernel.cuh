@@ -43,6 +43,10 @@ constexpr int kReportBuf = 64;    // reports per warp buffered in shared memory
 constexpr int kInjectLow = 256;   // inject new positions while the stack holds fewer entries
 constexpr int kStickyCap = 64;    // sticky states tracked per warp (more fall back to entries)
 constexpr int kPendCap = 16;      // sticky states met while copying one injection batch
+constexpr int kScanLane = 8;      // consecutive positions a lane tests per filter scan step
+constexpr int kScanStep = 32 * kScanLane;
+constexpr int kCandLow = 64;      // the filter scans on while fewer candidates are queued
+constexpr int kCandCap = kCandLow + kScanStep;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr uint32_t kNoEntry = 0xffffffffu;  // never a valid entry: offsets stay < 8191
 constexpr uint32_t kIdMask = 0x7fffffffu;
@@ -98,13 +102,16 @@ constexpr int32_t kWaitRounds = 1 << 24;  // default bound of an mbarrier wait
 constexpr uint32_t kNoAct = 0xffffffffu;
 
 // A window buffer: up to kMaxDepth - 1 look-behind bytes, 15 bytes of
-// alignment, W window bytes and one look-ahead byte.
-__host__ __device__ inline int window_buf_bytes(int W) { return ((W + 48) + 15) & ~15; }
-static_assert(kMaxDepth - 1 + 15 + 1 + 15 <= 48, "window buffer slack");
+// alignment, W window bytes and the look-ahead bytes (one, or the filter's).
+__host__ __device__ inline int window_buf_bytes(int W) { return ((W + 64) + 15) & ~15; }
+static_assert(kMaxDepth - 1 + 15 + kMaxFilter + 15 <= 64, "window buffer slack");
+// a filter scan step may read (and ignore) up to a step and a filter past the
+// window's bytes: those are the next buffer, the reports and the scratch
+static_assert(kScanStep + kMaxFilter + 8 <= kReportBuf * 8, "filter scan over-read");
 
 __host__ __device__ inline int warp_smem_bytes(int W) {
   return kStackCap * 4 + 2 * window_buf_bytes(W) + kReportBuf * 8 + 3 * 32 * 4 + 16 +
-         kStickyCap * 8 + kPendCap * 8 + 16;
+         kStickyCap * 8 + kPendCap * 8 + 16 + kCandCap * 2;
 }
 
 __host__ __device__ inline int cta_smem_bytes(int W, int image_region) {
@@ -122,6 +129,7 @@ struct WarpSmem {
   uint32_t* pend_s;          // kPendCap sticky states met while copying a batch
   uint32_t* pend_q;
   uint32_t* pend_n;          // count (one word)
+  int16_t* cand;             // kCandCap window offsets that passed the filter
 };
 
 // Per-warp state kept in registers (uniform across the warp).
@@ -508,12 +516,14 @@ __device__ __forceinline__ bool register_each(const MatchParams& p, WarpSmem& ws
   return mine;
 }
 
-// Always-active states for window offsets [r0, r0 + batch) (one per lane).
+// Always-active states for window offsets [r0, r0 + batch) (one per lane), or
+// with CAND for the `batch` filter candidates ws.cand[r0 ...].
+template <bool CAND>
 __device__ __forceinline__ void inject_aas(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                            const TileView& tv, const UnitCtx& c, int lane, int r0,
                                            int batch, int depth, unsigned long long& n_injected) {
   const TileDev& t = *tv.t;
-  const int r = r0 + lane;
+  const int r = CAND ? (int)ws.cand[r0 + min(lane, batch - 1)] : r0 + lane;
   const bool valid = lane < batch && r < c.iend;
   const int64_t q = c.wb + r;
   if (depth == 0) {  // scan the always-active list
@@ -616,7 +626,7 @@ __device__ __forceinline__ void inject_aas(const MatchParams& p, WarpSmem& ws, W
     const int kk = (int)(kraw & 0xffu);
     const uint32_t v = (kraw & 0x100u) ? ws.inj[32 + l0]
                                        : __ldg(tv.pt[kk - 1].vlist + ws.inj[32 + l0] + (idx - before));
-    const uint32_t off = (uint32_t)(r0 + l0 + kk - 1);
+    const uint32_t off = (uint32_t)((CAND ? (int)ws.cand[r0 + l0] : r0 + l0) + kk - 1);
     uint32_t e = (v << kEntryPosBits) | off;
     if (tv.sticky && is_sticky(tv, v)) {  // registered after the copy instead
       const uint32_t slot = atomicAdd(ws.pend_n, 1u);
@@ -645,14 +655,11 @@ struct InjAhead {
   uint32_t kf[2];
 };
 
-// The lane's position h of the batch at r0: k (live classes of the next
-// symbols, a dead class or the window end stop it), whether the whole key is
-// live (use), and the key.
-__device__ __forceinline__ void inject_key(const TileView& tv, const UnitCtx& c, int lane, int r0,
-                                           int batch, int depth, int h, int& k, bool& use,
-                                           uint32_t& key) {
-  const int r = r0 + 32 * h + lane;
-  const bool valid = 32 * h + lane < batch && r < c.iend;
+// Window offset r: k (live classes of the next symbols, a dead class or the
+// window end stop it), whether the whole key is live (use), and the key.
+__device__ __forceinline__ void inject_key(const TileView& tv, const UnitCtx& c, int r, bool in_batch,
+                                           int depth, int& k, bool& use, uint32_t& key) {
+  const bool valid = in_batch && r < c.iend;
   const int kmax = valid ? min(depth, c.wlen - r) : 0;
   k = kmax;
   key = 0u;
@@ -673,7 +680,8 @@ __device__ __forceinline__ void inject_key(const TileView& tv, const UnitCtx& c,
 // flight per lane. Same entries and reports as inject_aas over the two halves.
 // AHEAD (the lean PRIV 0 instances): after this batch's lookups, the lane's inline
 // table words of the next batch are read too, and the next call uses them.
-template <bool AHEAD>
+// CAND: the positions are the filter candidates ws.cand[r0 .. r0 + batch).
+template <bool AHEAD, bool CAND>
 __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                             const TileView& tv, const UnitCtx& c, int lane, int r0,
                                             int batch, int depth, unsigned long long& n_injected,
@@ -685,7 +693,7 @@ __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, 
   const bool read_ahead = AHEAD && ahead.r0 == r0;  // read during the last batch's expansions
 #pragma unroll
   for (int h = 0; h < 2; h++) {
-    r[h] = r0 + 32 * h + lane;
+    r[h] = CAND ? (int)ws.cand[r0 + min(32 * h + lane, batch - 1)] : r0 + 32 * h + lane;
     vb[h] = ve[h] = 0u;
     one[h] = kNoEntry;
     uint32_t key = 0u;
@@ -695,7 +703,7 @@ __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, 
       use[h] = (ahead.kf[h] >> 8) & 1u;
       word = (ahead.kf[h] >> 9) & 1u;
     }
-    if (!read_ahead || (use[h] && !word)) inject_key(tv, c, lane, r0, batch, depth, h, k[h], use[h], key);
+    if (!read_ahead || (use[h] && !word)) inject_key(tv, c, r[h], 32 * h + lane < batch, depth, k[h], use[h], key);
     if (!use[h]) continue;
     if (word) {  // decode the inline1 word read ahead
       const uint32_t x = ahead.x[h];
@@ -714,7 +722,7 @@ __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, 
   }
   // read the next batch's table words now: their DRAM round trip overlaps
   // this batch's list copies and the expansions that follow
-  ahead.r0 = -1 << 30;
+  if (AHEAD) ahead.r0 = -1 << 30;
   const int r1 = r0 + batch;
   // (only for inline tables, where the word read ahead is the whole lookup;
   // for the others it would cost a second key computation and no load)
@@ -724,7 +732,7 @@ __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, 
       int kn;
       bool un;
       uint32_t key;
-      inject_key(tv, c, lane, r1, batch, depth, h, kn, un, key);
+      inject_key(tv, c, r1 + 32 * h + lane, 32 * h + lane < batch, depth, kn, un, key);
       bool word = false;
       if (un) {
         const PrefixTableDev& pt = tv.pt[kn - 1];
@@ -821,7 +829,8 @@ __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, 
       const uint32_t v = (kraw & 0x100u)
                              ? ws.inj[32 + l0]
                              : __ldg(tv.pt[kk - 1].vlist + ws.inj[32 + l0] + (idx - before));
-      const uint32_t off = (uint32_t)(r0 + 32 * h + l0 + kk - 1);
+      const uint32_t off =
+          (uint32_t)((CAND ? (int)ws.cand[r0 + 32 * h + l0] : r0 + 32 * h + l0) + kk - 1);
       store_entry(p, ws, w, base + (int)idx, (v << kEntryPosBits) | off);
     }
     base += (int)ht;
@@ -831,13 +840,59 @@ __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, 
   __syncwarp();
 }
 
+// One step of the look-ahead filter (FilterDev): tests window offsets [s0, s0 +
+// kScanStep), kScanLane consecutive ones per lane, and appends those that
+// pass to the candidate queue (n entries so far); returns the new count. s0
+// is a multiple of 8 as a shared-memory address, so positions below r0 (the
+// first to test) are masked off here.
+// What bounds it is one bitmap read per position (L2, or L1 for the small
+// bitmaps), none of which depends on another: a lane's eight are issued before
+// any is used. Measured on a B200, whole calls: 1000 25-mers on 16 MiB 691 ->
+// 308 us (kernel 598 -> 217: 4 % of the positions pass), 200 25-mers with
+// three table levels on 3 MB 79.5 -> 2.65 ms, 50 edit-distance 20-mers with
+// one level on 1 MB 20.6 -> 0.46 ms, the 32 MiB mix 3.90 -> 2.41 ms.
+__device__ __forceinline__ int filter_scan(WarpSmem& ws, const TileView& tv, const UnitCtx& c,
+                                           int lane, int s0, int r0, int n) {
+  const FilterDev& f = tv.t->filt;
+  const int len = f.len, min_rep = f.min_rep, shift = f.shift;
+  const uint32_t mul = f.mul, scale = f.scale, drop = f.drop;
+  const uint32_t* __restrict__ bits = f.bits;
+  const int o = s0 + kScanLane * lane;
+  const uint8_t* in = c.in + o;
+  uint32_t h = 0u;
+  for (int i = 0; i < len - 1; i++) h = h * mul + in[i];
+  const uint2 old = *reinterpret_cast<const uint2*>(in);  // the lane's own symbols (8-aligned)
+  uint32_t idx[kScanLane], word[kScanLane];
+  unsigned pass = 0u, test = 0u;
+#pragma unroll
+  for (int j = 0; j < kScanLane; j++) {
+    h = h * mul + in[len - 1 + j];  // a symbol enters, and the one before the lane's j-th leaves
+    if (j > 0) h -= __byte_perm(j <= 4 ? old.x : old.y, 0, 0x4440 | ((j - 1) & 3)) * drop;
+    idx[j] = (h * scale) >> shift;
+    const int r = o + j;
+    const int left = c.lim - r;  // symbols left in the unit
+    const bool in_range = r >= r0 && r < c.iend;
+    if (in_range && left >= len) test |= 1u << j;
+    else if (in_range && left >= min_rep) pass |= 1u << j;
+  }
+#pragma unroll
+  for (int j = 0; j < kScanLane; j++) word[j] = (test >> j) & 1u ? __ldg(bits + (idx[j] >> 5)) : 0u;
+#pragma unroll
+  for (int j = 0; j < kScanLane; j++) pass |= ((word[j] >> (idx[j] & 31)) & 1u) << j;
+  int total;
+  int pos = n + warp_excl<4>(__popc(pass), lane, total);
+  for (; pass; pass &= pass - 1u) ws.cand[pos++] = (int16_t)(o + __ffs(pass) - 1);
+  __syncwarp();
+  return n + total;
+}
+
 // Injection of a batch of positions: always-active states, then the sticky
 // states met while copying, then the work of every active sticky state at
 // these positions. Layered tiles (phase 2) do their sticky work separately.
 __device__ __forceinline__ void inject(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                        const TileView& tv, const UnitCtx& c, int lane, int r0,
                                        int batch, int depth, unsigned long long& n_injected) {
-  inject_aas(p, ws, w, tv, c, lane, r0, batch, depth, n_injected);
+  inject_aas<false>(p, ws, w, tv, c, lane, r0, batch, depth, n_injected);
   if (!tv.sticky || tv.t->phase == 2) return;
   __syncwarp();
   const int np = min((int)*ws.pend_n, kPendCap);
@@ -1254,8 +1309,8 @@ __device__ __forceinline__ void expand_step2(const MatchParams& p, WarpSmem& ws,
 // A warp's view of one tile and the knobs derived from it.
 struct TileRun {
   TileView tv;
-  int depth, batch, defer;
-  bool layered, wide_inject;
+  int depth, batch, defer, look;
+  bool layered, wide_inject, filtered;
 };
 
 // Builds the view of tile t whose image is at ib (shared-memory copy or the
@@ -1289,6 +1344,8 @@ __device__ __forceinline__ void tile_run(const MatchParams& p, const TileDev* t,
   // that every position but the unit's last ones gets the full table depth.
   tr.layered = !LEAN && t->phase == 2;
   tr.defer = (tr.depth > 1 && (!tv.sticky || tr.layered)) ? tr.depth - 1 : 0;
+  tr.filtered = t->filt.len > 0;
+  tr.look = max(1, t->filt.len);
 }
 
 // Two kinds of work per launch:
@@ -1324,6 +1381,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   ws.pend_s = ws.stk_q + kStickyCap;
   ws.pend_q = ws.pend_s + kPendCap;
   ws.pend_n = ws.pend_q + kPendCap;
+  ws.cand = reinterpret_cast<int16_t*>(ws.pend_n + 4);
   if (lane == 0) *ws.pend_n = 0u;
   const int slot = blockIdx.x * kWarpsPerCta + warp;
   WarpRun w;
@@ -1349,12 +1407,12 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   unsigned long long n_expanded = 0, n_injected = 0;
   int staged = -1;  // tile whose image is in shared memory
 
-  // loads window [wb, min(wb + W, hi)) plus one look-ahead byte and `lb`
+  // loads window [wb, min(wb + W, hi)) plus `look` look-ahead bytes and `lb`
   // look-behind bytes into buffer buf; returns the byte count, and in `skip`
   // the offset of wb's byte in the buffer
-  auto issue = [&](int buf, int64_t wb, int64_t hi, int lb, uint32_t& skip) {
+  auto issue = [&](int buf, int64_t wb, int64_t hi, int lb, int look, uint32_t& skip) {
     const int64_t we = min(wb + (int64_t)W, hi);
-    const int64_t end = min(we + 1, hi);
+    const int64_t end = min(we + look, hi);
     const int64_t a0 = (wb - lb) & ~(int64_t)15;
     const uint32_t bytes = (uint32_t)(((end - a0) + 15) & ~(int64_t)15);
     skip = (uint32_t)(wb - a0);
@@ -1385,7 +1443,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   auto run_unit = [&](unsigned uid, const TileDev* t, const TileRun& tr) {
     const TileView& tv = tr.tv;
     const int depth = tr.depth, batch = tr.batch, defer = tr.defer;
-    const bool layered = tr.layered, wide_inject = tr.wide_inject;
+    const bool layered = tr.layered, wide_inject = tr.wide_inject, filtered = tr.filtered;
     const UnitDev un = p.units[uid];
     const unsigned long long work0 = n_expanded + n_injected;  // per-unit trace
     if (p.unit_work && lane == 0) p.unit_cycles[uid] = clock64();  // start; the end subtracts
@@ -1438,7 +1496,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
     int cur = 0;
     uint32_t nbytes[2], skip[2];
     if (c.hi > un.lo && (int32_t)uid != p.skip_copy_unit) {
-      nbytes[0] = issue(0, un.lo, c.hi, 0, skip[0]);
+      nbytes[0] = issue(0, un.lo, c.hi, 0, tr.look, skip[0]);
     } else {  // idle, or the test hook: nothing is in flight (the hook's first wait gives up)
       nbytes[0] = 0u;
       skip[0] = 0u;
@@ -1471,7 +1529,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
       live = __any_sync(kFull, live);
       __syncwarp();
       if (we < c.hi)
-        nbytes[cur ^ 1] = issue(cur ^ 1, we, c.hi, (int)min((int64_t)defer, we - un.lo), skip[cur ^ 1]);
+        nbytes[cur ^ 1] = issue(cur ^ 1, we, c.hi, (int)min((int64_t)defer, we - un.lo), tr.look,
+                                skip[cur ^ 1]);
       c.in = ws.in[cur] + skip[cur];
       // carried states: matched at wb
       w.top = 0;
@@ -1511,6 +1570,11 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
       int cursor = !live || (t->naas == 0 && (LEAN || layered || !tv.sticky))
                        ? c.iend
                        : (int)(inj_pos - wb);
+      // filtered tiles: `cursor` is where the filter scans next (moved down to a
+      // multiple of 8 in shared memory), `first` the first position to test
+      const int first = cursor;
+      int ncand = 0;
+      if (filtered && cursor < c.iend) cursor -= (int)(smem_u32(c.in + cursor) & 7u);
       InjAhead ahead;  // table words of the next batch, read ahead (this window only)
       // layered tiles: next window offset of the sticky states' work
       int scur = live && layered && w.nstk > 0 ? 0 : c.wlen;
@@ -1518,13 +1582,28 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
         // inject only when the overflow stack is empty, so that it holds at
         // most one batch's excess
         if (w.top < kInjectLow && w.ovf_n == 0) {
-          if (cursor < c.iend) {
+          if (filtered) {
+            if (ncand < kCandLow && cursor < c.iend) {
+              ncand = filter_scan(ws, tv, c, lane, cursor, first, ncand);
+              cursor += kScanStep;
+              continue;
+            }
+            if (ncand > 0) {
+              const int m = min(ncand, wide_inject ? 2 * batch : batch);
+              ncand -= m;
+              if (wide_inject)
+                inject_aas2<false, true>(p, ws, w, tv, c, lane, ncand, m, depth, n_injected, ahead);
+              else
+                inject_aas<true>(p, ws, w, tv, c, lane, ncand, m, depth, n_injected);
+              continue;
+            }
+          } else if (cursor < c.iend) {
             if (wide_inject) {
-              inject_aas2<LEAN && PRIV == 0>(p, ws, w, tv, c, lane, cursor, 2 * batch, depth,
+              inject_aas2<LEAN && PRIV == 0, false>(p, ws, w, tv, c, lane, cursor, 2 * batch, depth,
                                              n_injected, ahead);
               cursor += 2 * batch;
             } else if (LEAN) {
-              inject_aas(p, ws, w, tv, c, lane, cursor, batch, depth, n_injected);
+              inject_aas<false>(p, ws, w, tv, c, lane, cursor, batch, depth, n_injected);
               cursor += batch;
             } else {
               inject(p, ws, w, tv, c, lane, cursor, batch, depth, n_injected);
@@ -1547,7 +1626,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
             __syncwarp();
             continue;
           }
-          if (cursor < c.iend || (!LEAN && scur < c.wlen)) continue;
+          if (cursor < c.iend || ncand > 0 || (!LEAN && scur < c.wlen)) continue;
           break;
         }
         // (layered tiles have no edge into a sticky state: no successor to register)

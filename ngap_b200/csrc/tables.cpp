@@ -31,7 +31,9 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
+#include <cmath>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <numeric>
 #include <thread>
@@ -814,7 +816,163 @@ std::vector<std::vector<int>> global_sets_of(const GroupSet& gs, const std::vect
   return sets;
 }
 
+// ---- look-ahead filters -------------------------------------------------------
+
+// The states a tile injects at a position: its always-active states, or for a
+// layered tile the successors of its sticky states. Empty when the tile gets
+// no filter: plain tiles that register sticky states while they run.
+std::vector<uint32_t> filter_sources(const TileHost& t) {
+  if (t.phase == kPlain && t.nsticky > 0) return {};
+  if (t.phase == kLayered) return {};
+  return t.aas;
+}
+
+struct FilterPlan {
+  int len = 0, fbits = 0, min_rep = 0;
+  bool exact = false;
+};
+
+// Chooses how many symbols the filter looks ahead and its size from the
+// number of paths (with their class choices) that are alive after d symbols,
+// counted level by level. A path that reports after d < len symbols sets the
+// bits of every continuation, so such paths count ncls^(len - d) times.
+// The estimate of the share of positions that pass takes classes as equally
+// likely in small alphabets; over text (more than 8 classes) symbol laws are
+// skewed, and a symbol is taken to agree with probability L^-0.6 (a Zipf law
+// over 95 symbols agrees with itself with probability 0.07 = 95^-0.6).
+// Bounds: 2^28 bits (32 MB: the bitmap stays in the 126 MB L2), 32 bits per
+// key (3 % false positives), more while it fits L1 beside the kernel's shared
+// memory (kCachedBits), and kVisits steps of the walk that sets the bits.
+FilterPlan plan_filter(const TileHost& t, const std::vector<uint32_t>& src) {
+  constexpr double kVisits = 48e6, kFills = 4e6;
+  constexpr int kMaxBits = 28, kCachedBits = 18, kMinBits = 15;
+  FilterPlan best;
+  double best_est = 0.5;  // a filter that half of the positions pass saves too little
+  const double L = std::max(1, t.nlive);
+  const double pe = t.nlive <= 8 ? 1.0 / L : std::pow(L, -0.6);
+  auto classes_of = [&](uint32_t v) {
+    int n = 0;
+    for (int c = 0; c < t.nlive; c++) n += accepts_cls(t, v, c) ? 1 : 0;
+    return (double)n;
+  };
+  std::vector<double> ncl(t.nstates, -1.0), cur(t.nstates, 0.0), nxt(t.nstates, 0.0);
+  auto width = [&](uint32_t v) {
+    if (ncl[v] < 0) ncl[v] = classes_of(v);
+    return ncl[v];
+  };
+  for (uint32_t v : src) cur[v] = width(v);
+  double visits = 0, pass_rep = 0;
+  std::vector<double> reps;  // paths that first report after d + 1 symbols
+  int min_rep = 0;
+  for (int d = 1; d <= kMaxFilter; d++) {
+    double alive = 0, rep = 0;
+    for (int32_t v = 0; v < t.nstates; v++) {
+      if (cur[v] <= 0) continue;
+      (is_report(t, v) ? rep : alive) += cur[v];
+    }
+    if (rep > 0 && min_rep == 0) min_rep = d;
+    visits += alive + rep;
+    double fills = 0, f = 1;
+    for (int k = (int)reps.size() - 1; k >= 0; k--) {
+      f *= std::max(1, t.ncls);
+      fills += reps[k] * f;
+    }
+    if (visits > kVisits || fills > kFills) break;
+    pass_rep += rep * std::pow(pe, d);
+    const double keys = fills + alive + rep;
+    const double space = std::pow(L, d);
+    const bool exact = space <= (double)(1u << kMaxBits) && space <= 32 * std::max(keys, 1024.0);
+    int fbits = kMinBits;
+    while (fbits < kMaxBits && std::pow(2.0, fbits) < (exact ? space : 32 * keys)) fbits++;
+    while (!exact && fbits < kCachedBits && std::pow(2.0, fbits) < 512 * keys) fbits++;
+    const double fp = exact ? 0.0 : keys / std::pow(2.0, fbits);
+    const double est = pass_rep + alive * std::pow(pe, d) + fp;
+    // a longer filter has to gain: its bits cost time to set and room in L2
+    if (est < 0.8 * best_est - 2e-3) {
+      best_est = est;
+      best.len = d;
+      best.fbits = fbits;
+      best.exact = exact;
+    }
+    if (alive <= 0) break;  // every path has reported or ended
+    // next level: paths that have reported stand for all their continuations
+    std::fill(nxt.begin(), nxt.end(), 0.0);
+    for (int32_t v = 0; v < t.nstates; v++) {
+      if (cur[v] <= 0 || is_report(t, v)) continue;
+      for (int k = 0; k < 4; k++) {
+        const uint32_t u = t.succ[(size_t)v * 4 + k];
+        if (u != kNoSucc) nxt[u & 0x7fffffffu] += cur[v] * width(u & 0x7fffffffu);
+      }
+    }
+    reps.push_back(rep);
+    cur.swap(nxt);
+  }
+  best.min_rep = min_rep;
+  return best;
+}
+
+void build_filter(TileHost& t) {
+  const std::vector<uint32_t> src = filter_sources(t);
+  if (src.empty()) return;
+  const FilterPlan pl = plan_filter(t, src);
+  if (pl.len == 0) return;
+  FilterHost& f = t.filt;
+  f.len = pl.len;
+  // no report within kMaxFilter symbols: more are needed than a filter looks ahead
+  f.min_rep = pl.min_rep > 0 ? pl.min_rep : kMaxFilter + 1;
+  f.shift = 32 - pl.fbits;
+  f.mul = pl.exact ? (uint32_t)t.nlive : kFilterMul;
+  f.scale = pl.exact ? 1u << f.shift : kFilterScale;
+  f.drop = 1;
+  for (int i = 0; i < f.len; i++) f.drop *= f.mul;
+  f.bits.assign((size_t)1 << (pl.fbits > 5 ? pl.fbits - 5 : 0), 0);
+  auto set = [&](uint32_t h) {
+    const uint32_t b = (h * f.scale) >> f.shift;
+    uint32_t* w = &f.bits[b >> 5];
+    const uint32_t m = 1u << (b & 31);
+    if (!(__atomic_load_n(w, __ATOMIC_RELAXED) & m)) __atomic_fetch_or(w, m, __ATOMIC_RELAXED);
+  };
+  // class ids each state accepts, as a flat list
+  std::vector<uint32_t> coff(t.nstates + 1, 0);
+  std::vector<uint8_t> clist;
+  for (int32_t v = 0; v < t.nstates; v++) {
+    for (int c = 0; c < t.nlive; c++)
+      if (accepts_cls(t, v, c)) clist.push_back((uint8_t)c);
+    coff[v + 1] = (uint32_t)clist.size();
+  }
+  // every continuation (the dead class included) of a path that has reported
+  std::function<void(int, uint32_t)> fill = [&](int d, uint32_t h) {
+    if (d == f.len) return set(h);
+    for (int c = 0; c < t.ncls; c++) fill(d + 1, h * f.mul + (uint32_t)c);
+  };
+  // h: hash of the d symbols read, the last of which v matched
+  std::function<void(uint32_t, int, uint32_t)> walk = [&](uint32_t v, int d, uint32_t h) {
+    if (d == f.len || is_report(t, v)) return fill(d, h);
+    for (int k = 0; k < 4; k++) {
+      uint32_t u = t.succ[(size_t)v * 4 + k];
+      if (u == kNoSucc) continue;
+      u &= 0x7fffffffu;
+      for (uint32_t i = coff[u]; i < coff[u + 1]; i++) walk(u, d + 1, h * f.mul + clist[i]);
+    }
+  };
+  std::atomic<size_t> next{0};
+  auto work = [&]() {
+    for (size_t i; (i = next.fetch_add(1)) < src.size();)
+      for (uint32_t k = coff[src[i]]; k < coff[src[i] + 1]; k++) walk(src[i], 1, clist[k]);
+  };
+  const int nth = (int)std::min<size_t>(std::min(std::max(1u, std::thread::hardware_concurrency()), 32u),
+                                        src.size() / 8 + 1);
+  std::vector<std::thread> th;
+  for (int i = 1; i < nth; i++) th.emplace_back(work);
+  work();
+  for (auto& x : th) x.join();
+}
+
 }  // namespace
+
+void build_filters(std::vector<TileHost>& tiles) {
+  for (TileHost& t : tiles) build_filter(t);
+}
 
 int build_tiles(const GroupSet& gs, const TableOpts& opts, std::vector<TileHost>& tiles) {
   tiles.clear();

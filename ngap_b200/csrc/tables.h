@@ -21,6 +21,13 @@ struct PrefixTableHost {
   int32_t max_len = 0;                // longest state list
 };
 
+// Host form of FilterDev.
+struct FilterHost {
+  int32_t len = 0, min_rep = 1, shift = 0;
+  uint32_t mul = 0, scale = 0, drop = 0;
+  std::vector<uint32_t> bits;
+};
+
 struct TileHost {
   int32_t group = 0;
   int32_t nstates = 0;
@@ -54,6 +61,7 @@ struct TileHost {
   std::vector<uint8_t> image;        // succ | cmask | rep | sticky | cls, 16-byte aligned parts
   int32_t off_cmask = 0, off_rep = 0, off_sticky = 0, off_cls = 0;
   PrefixTableHost pt[kMaxDepth];
+  FilterHost filt;
 };
 
 struct TableOpts {
@@ -85,6 +93,9 @@ inline int64_t image_bytes(int64_t n, int cw) {
 
 // Splits every group into tiles and builds each tile's tables.
 int build_tiles(const GroupSet& gs, const TableOpts& opts, std::vector<TileHost>& tiles);
+
+// Builds the look-ahead filter of every tile that gains from one.
+void build_filters(std::vector<TileHost>& tiles);
 
 // Checks the public table options (NULL = the defaults) and converts them;
 // `fn` names the entry point in the error message. *device gets the device.
