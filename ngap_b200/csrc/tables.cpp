@@ -820,11 +820,25 @@ std::vector<std::vector<int>> global_sets_of(const GroupSet& gs, const std::vect
 
 // The states a tile injects at a position: its always-active states, or for a
 // layered tile the successors of its sticky states. Empty when the tile gets
-// no filter: plain tiles that register sticky states while they run.
+// no filter: plain tiles that register sticky states while they run, layered
+// tiles whose sticky states report (at every position) or that have
+// always-active states beside them.
 std::vector<uint32_t> filter_sources(const TileHost& t) {
   if (t.phase == kPlain && t.nsticky > 0) return {};
-  if (t.phase == kLayered) return {};
-  return t.aas;
+  if (t.phase != kLayered) return t.aas;
+  if (!t.aas.empty()) return {};
+  std::vector<uint32_t> src;
+  for (uint32_t a : t.act_local) {
+    const uint32_t s = a & kActIdMask;
+    if (is_report(t, s)) return {};
+    for (int k = 0; k < 4; k++) {
+      const uint32_t u = t.succ[(size_t)s * 4 + k];
+      if (u != kNoSucc) src.push_back(u & 0x7fffffffu);
+    }
+  }
+  std::sort(src.begin(), src.end());
+  src.erase(std::unique(src.begin(), src.end()), src.end());
+  return src;
 }
 
 struct FilterPlan {
@@ -888,7 +902,9 @@ FilterPlan plan_filter(const TileHost& t, const std::vector<uint32_t>& src) {
     const double fp = exact ? 0.0 : keys / std::pow(2.0, fbits);
     const double est = pass_rep + alive * std::pow(pe, d) + fp;
     // a longer filter has to gain: its bits cost time to set and room in L2
-    if (est < 0.8 * best_est - 2e-3) {
+    // (a candidate of a layered tile is dear: it is tested against every
+    // active sticky state)
+    if (est < 0.8 * best_est - (t.phase == kLayered ? 2e-4 : 2e-3)) {
       best_est = est;
       best.len = d;
       best.fbits = fbits;

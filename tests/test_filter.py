@@ -142,6 +142,26 @@ def short_rules(rng, n, lo, hi, alpha):
     return w.text()
 
 
+BYTES = np.arange(20, 220, dtype=np.uint8)
+BYTES_LAW = np.arange(1, 201) ** -1.3 / np.sum(np.arange(1, 201) ** -1.3)
+
+
+def wide_dotstar(rng, n):
+    """a{2,4} .* b{2,5} over a large alphabet (more than three class words)."""
+    w = W.AnmlWriter("wide")
+    for p in range(n):
+        a, b = int(rng.integers(2, 5)), int(rng.integers(2, 6))
+        for i in range(a):
+            w.ste(f"w{p}a{i}", [int(rng.choice(BYTES, p=BYTES_LAW))],
+                  [f"w{p}a{i + 1}"] if i + 1 < a else [f"w{p}s", f"w{p}b0"],
+                  start="all-input" if i == 0 else None)
+        w.ste(f"w{p}s", None, [f"w{p}s", f"w{p}b0"], symbol_set="*")
+        for i in range(b):
+            w.ste(f"w{p}b{i}", [int(rng.choice(BYTES, p=BYTES_LAW))], [f"w{p}b{i + 1}"] if i + 1 < b else [],
+                  report=(i == b - 1))
+    return w.text()
+
+
 def rule_sets():
     rng = np.random.default_rng(31)
     kw = dict(input_len=1 << 12, plant_every=1 << 8)
@@ -154,6 +174,7 @@ def rule_sets():
         "short": short_rules(rng, 12, 2, 9, W.PRINTABLE),
         "dense": short_rules(rng, 30, 1, 4, W.PRINTABLE[:20]),
         "one": short_rules(rng, 3, 1, 1, W.PRINTABLE),
+        "wide": wide_dotstar(np.random.default_rng(32), 400),
         "mixed": short_rules(rng, 60, 3, 20, W.PRINTABLE[:20]),
     }
 
@@ -172,7 +193,7 @@ def test_filter_covers_every_path(checker, tmp_path, name, groups, mode):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("name", ["hamming", "motif", "dotstar", "dense", "mixed"])
+@pytest.mark.parametrize("name", ["hamming", "motif", "dotstar", "dense", "mixed", "wide"])
 def test_filtered_matches(engine, name):
     anml = rule_sets()[name]
     groups = nb.Groups(nb.Nfa.from_string(anml), group_num=2)
@@ -183,6 +204,8 @@ def test_filtered_matches(engine, name):
                                           plant_every=61)[1],
            "dotstar": lambda: W.dotstar_set(seed=6, n_patterns=60, input_len=6000, plant_every=97)[1]}
     data = gen[name]() if name in gen else rng.choice(W.PRINTABLE[:20], size=6000).astype(np.uint8)
+    if name == "wide":
+        data = rng.choice(BYTES, size=6000, p=BYTES_LAW).astype(np.uint8)
     data = data.copy()
     data[rng.integers(0, len(data), 40)] = rng.choice(alpha, size=40)
     data[1000:1040] = 0  # bytes no state accepts
