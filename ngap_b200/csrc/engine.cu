@@ -122,6 +122,7 @@ struct ngap_engine {
   UnitDev* d_units = nullptr;
   size_t units_cap = 0;
   int32_t nunits = 0;
+  int64_t longest_unit = 0;  // positions of the plan's longest unit
   TaskDev* d_tasks = nullptr;
   size_t tasks_cap = 0;
   int32_t ntasks = 0;
@@ -500,7 +501,8 @@ int ensure_slots(ngap_engine* e, size_t slots, int max_states, int max_nact, int
 }
 
 // Splits the work into units: unbounded tiles get one unit per segment;
-// bounded tiles are cut into chunks of `chunk` emitted positions, each with
+// bounded tiles are cut into chunks of `chunk` emitted positions (AutoChunk when the caller
+// gives none), each with
 // max_path - 1 positions of warm-up (clamped at the segment start). Units of
 // one tile are then cut into CTA tasks: the long per-segment units of
 // unbounded tiles one per warp of a task and first, the chunks after them in
@@ -514,7 +516,38 @@ struct SegSpec {
   int32_t index;    // segment or stream index
 };
 
-void add_units(const TileHost& th, int tile, const SegSpec& s, int window, int chunk_opt,
+// The launch that runs a tile (make_tasks): 0 activation tiles, 1 plain tiles
+// without sticky states, 2 the rest.
+int launch_of(const TileHost& th) {
+  return th.phase == 1 ? 0 : (th.phase == 0 && th.nsticky == 0 ? 1 : 2);
+}
+
+// Chunk length of bounded tiles when the caller gives none. Long inputs: the
+// window's length less the warm-up (a unit is then one window), which is best
+// while it gives every warp several units. Shorter ones (positions: those of
+// the launch's bounded tiles) are cut to one unit per warp, because a warp
+// walks its unit serially and idle warps gain nothing; below 128 positions the
+// warm-up and a unit's start cost more than the shorter walk gains. Match times
+// on a B200 by chunk length (128, 384, 1024, 2048): 64 literals on 1 MiB 61, 43,
+// 47, 61 us; 200 25-mers on 3 MB 1769, 1617, 1516, 2646 us; a server's burst
+// of four batches 748, 809, 1090, 1484 us; 1000 25-mers on 16 MiB (more units
+// than warps at any of them) 895, 405, 258, 260 us.
+struct AutoChunk {
+  int64_t positions[3] = {0, 0, 0};  // of bounded tiles, per launch
+  int64_t warps = 1;
+  void add(const TileHost& th, int64_t len) {
+    if (th.max_path >= 0) positions[launch_of(th)] += len;
+  }
+  int64_t chunk(const TileHost& th, int window) const {
+    const int64_t warm = th.max_path > 0 ? th.max_path - 1 : 0;
+    const int64_t base = std::max<int64_t>(window, 2048);
+    const int64_t longest = std::max<int64_t>(base - warm, base / 2);
+    const int64_t share = (positions[launch_of(th)] + warps - 1) / warps;
+    return std::min(longest, std::max<int64_t>({(share + 63) & ~(int64_t)63, 128, warm}));
+  }
+};
+
+void add_units(const TileHost& th, int tile, const SegSpec& s, int64_t chunk,
                std::pair<int64_t, int32_t> act, std::vector<UnitDev>& pass1,
                std::vector<UnitDev>& unbounded, std::vector<UnitDev>& bounded) {
   UnitDev u{};
@@ -535,11 +568,6 @@ void add_units(const TileHost& th, int tile, const SegSpec& s, int window, int c
     return;
   }
   const int64_t warm = th.max_path > 0 ? th.max_path - 1 : 0;
-  // chunk length is independent of the window (whole windows for every
-  // algorithm); a chunk should span at least its warm-up
-  const int64_t base = std::max<int64_t>(window, 2048);
-  int64_t chunk = chunk_opt > 0 ? chunk_opt : std::max<int64_t>(base - warm, base / 2);
-  chunk = std::max<int64_t>(chunk, 1);
   for (int64_t em = s.lo; em < s.hi; em += chunk) {
     u.lo = std::max(s.lo, em - warm);
     u.hi = std::min(em + chunk, s.hi);
@@ -684,12 +712,16 @@ ActRows plan_units(const ngap_tables* t, const UnitPlanKey& k, int grid,
                    int32_t* ntasks2, int32_t free_range[6], int32_t free_tile[3]) {
   std::vector<UnitDev> pass1, unbounded, bounded;
   ActRows rows({t}, k.num_seg);
+  AutoChunk ac;
+  ac.warps = (int64_t)grid * kWarpsPerCta;
+  for (const TileHost& th : t->tiles) ac.add(th, k.num_seg * k.seg_len);
   for (int ti = 0; ti < (int)t->tiles.size(); ti++) {
+    const int64_t chunk = k.chunk > 0 ? k.chunk : ac.chunk(t->tiles[ti], k.window);
     for (int64_t s = 0; s < k.num_seg; s++) {
       SegSpec sp{s * k.seg_len, (s + 1) * k.seg_len, k.first_seg + s == 0 || k.is_dup != 0, 0ull,
                  0, (int32_t)s};
-      add_units(t->tiles[ti], ti, sp, k.window, k.chunk, rows.row(0, t->tiles[ti], s), pass1,
-                unbounded, bounded);
+      add_units(t->tiles[ti], ti, sp, chunk, rows.row(0, t->tiles[ti], s), pass1, unbounded,
+                bounded);
     }
   }
   const int32_t region = t->image_region;
@@ -698,6 +730,20 @@ ActRows plan_units(const ngap_tables* t, const UnitPlanKey& k, int grid,
   make_tasks(units, pass1, unbounded, bounded, grid, is_free, is_lean, tasks, ntasks1, ntasks2,
              free_range, free_tile);
   return rows;
+}
+
+int64_t longest_unit(const std::vector<UnitDev>& units) {
+  int64_t n = 0;
+  for (const UnitDev& u : units) n = std::max(n, u.hi - u.lo);
+  return n;
+}
+
+// An automatic window no longer than the plan's longest unit: the shared
+// memory that longer windows would take is left to L1, which holds small
+// filters and tables (64 literals on 1 MiB, chunks of 384: 43 us with windows of
+// 2048 positions, 37 us with 1024).
+int fit_window(int window, int64_t longest) {
+  return (int)std::min<int64_t>(window, std::max<int64_t>(64, (longest + 63) & ~(int64_t)63));
 }
 
 // Per-unit work counters when tracing (zeroed on st); null otherwise.
@@ -1172,7 +1218,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   // shared memory: the largest tile image that fits the budget, plus the warps
   // (a window too large for what is left is shortened)
   while (window > 64 && cta_smem_bytes(window, t->image_region) > 227 * 1024 - 1024) window /= 2;
-  const int smem = cta_smem_bytes(window, t->image_region);
+  int smem = cta_smem_bytes(window, t->image_region);
   if ((rc = set_smem(e, smem)) != NGAP_OK) return rc;
   int bps = 0;
   rc = cached_blocks_per_sm(e, priv, smem, &bps);
@@ -1210,11 +1256,16 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
     if (!tasks.empty()) ups.push_back({e->d_tasks, tasks.data(), tasks.size() * sizeof(TaskDev)});
     if ((rc = upload_plan(e, st, ups)) != NGAP_OK) return rc;
     e->nunits = (int32_t)units.size();
+    e->longest_unit = longest_unit(units);
     e->h_units = units;
     e->ntasks = (int32_t)tasks.size();
     e->plan_tables = t->serial;
     e->plan_key = key;
     e->batch_ts = 0;  // the batched plan cache no longer describes the buffers
+  }
+  if (p->window <= 0) {
+    window = fit_window(window, e->longest_unit);
+    smem = cta_smem_bytes(window, t->image_region);
   }
   const int grid = plan_grid(e, full_grid);
   e->grid = grid;
@@ -1593,7 +1644,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   if (rc != NGAP_OK) return rc;
   window = std::min(window, kMaxWindow);
   while (window > 64 && cta_smem_bytes(window, ts->image_region) > 227 * 1024 - 1024) window /= 2;
-  const int smem = cta_smem_bytes(window, ts->image_region);
+  int smem = cta_smem_bytes(window, ts->image_region);
   if ((rc = set_smem(e, smem)) != NGAP_OK) return rc;
   int bps = 0;
   rc = cached_blocks_per_sm(e, priv, smem, &bps);
@@ -1635,18 +1686,24 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     std::vector<UnitDev> pass1, unbounded, bounded, units;
     std::vector<TaskDev> tasks;
     const ActRows rows(ts->tables, nstreams);
+    AutoChunk ac;
+    ac.warps = (int64_t)full_grid * kWarpsPerCta;
+    for (const ngap_batch_stream& s : sv)
+      for (const TileHost& th : ts->tables[s.nfa]->tiles) ac.add(th, (int64_t)s.length);
     for (size_t n = 0; n < ts->tables.size(); n++) {
       const ngap_tables* t = ts->tables[n];
-      for (int ti = 0; ti < (int)t->tiles.size(); ti++)
+      for (int ti = 0; ti < (int)t->tiles.size(); ti++) {
+        const int64_t auto_chunk = ac.chunk(t->tiles[ti], window);
         for (int si : by_nfa[n]) {
           const ngap_batch_stream& s = sv[si];
           if (s.length == 0) continue;
           SegSpec sp{(int64_t)s.offset, (int64_t)(s.offset + s.length), true,
                      (uint64_t)si << sshift, (int64_t)s.offset, si};
-          add_units(t->tiles[ti], ts->tile_base[n] + ti, sp, window,
-                    s.chunk > 0 ? s.chunk : p->chunk, rows.row((int)n, t->tiles[ti], si), pass1,
-                    unbounded, bounded);
+          add_units(t->tiles[ti], ts->tile_base[n] + ti, sp,
+                    s.chunk > 0 ? s.chunk : (p->chunk > 0 ? p->chunk : auto_chunk),
+                    rows.row((int)n, t->tiles[ti], si), pass1, unbounded, bounded);
         }
+      }
     }
     const int32_t region = ts->image_region;
     auto is_free = [&](int tile) { return ts->plan_bytes[tile] > region; };
@@ -1675,6 +1732,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     if (!tasks.empty()) ups.push_back({e->d_tasks, tasks.data(), tasks.size() * sizeof(TaskDev)});
     if ((rc = upload_plan(e, st, ups)) != NGAP_OK) return rc;
     e->nunits = (int32_t)units.size();
+    e->longest_unit = longest_unit(units);
     e->h_units = units;
     e->ntasks = (int32_t)tasks.size();
     e->plan_tables = 0;  // the plain plan cache no longer describes the buffers
@@ -1684,6 +1742,10 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     e->batch_window = window;
     e->batch_chunk = p->chunk;
     replanned = true;
+  }
+  if (p->window <= 0) {
+    window = fit_window(window, e->longest_unit);
+    smem = cta_smem_bytes(window, ts->image_region);
   }
   const int grid = plan_grid(e, full_grid);
   e->grid = grid;
