@@ -167,7 +167,7 @@ struct ngap_engine {
   size_t slots = 0;
   int carry_cap = 0, mark_words = 0, ovf_cap = 0;
   int max_smem_set = -1;
-  int bps_smem[3] = {-1, -1, -1}, bps_val[3] = {0, 0, 0};  // resident CTAs per SM, per PRIV
+  int bps_smem = -1, bps_val = 0;  // resident CTAs per SM at the last shared-memory size
   // pinned staging of plan uploads (grow-only) and the event of the last one
   uint8_t* h_plan = nullptr;
   size_t h_plan_cap = 0;
@@ -841,7 +841,6 @@ int plan_grid(const ngap_engine* e, int full_grid) {
 // tiles without sticky states in the lean kernel instance; then the rest
 // (the layered tiles read what the first launch recorded). Each launch takes
 // its tasks first, then its free units.
-template <int PRIV>
 int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
   mp.free_cursor = e->d_unit_counter + 1;
   const TaskDev* const tasks0 = mp.tasks;
@@ -858,9 +857,9 @@ int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
     CUDA_TRY(cudaMemsetAsync(e->d_unit_counter, 0, 2 * sizeof(unsigned int), st));
     const int grid = launch_grid(e, ntasks, nfree);
     if (lean)
-      match_kernel<PRIV, true><<<grid, kCtaThreads, smem, st>>>(mp);
+      match_kernel<true><<<grid, kCtaThreads, smem, st>>>(mp);
     else
-      match_kernel<PRIV, false><<<grid, kCtaThreads, smem, st>>>(mp);
+      match_kernel<false><<<grid, kCtaThreads, smem, st>>>(mp);
     CUDA_TRY(cudaGetLastError());
     e->launches++;
     return NGAP_OK;
@@ -875,11 +874,6 @@ int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
     e->launches++;
   }
   return run(false, e->ntasks1 + e->ntasks2, e->ntasks - e->ntasks1 - e->ntasks2, 2);
-}
-
-int launch_any(ngap_engine* e, const MatchParams& mp, int smem, cudaStream_t st, int priv) {
-  return priv == 0 ? launch_plan<0>(e, mp, smem, st)
-                   : priv == 1 ? launch_plan<1>(e, mp, smem, st) : launch_plan<2>(e, mp, smem, st);
 }
 
 __global__ void swap_halves(uint64_t* a, uint64_t n) {
@@ -903,11 +897,9 @@ int set_smem(ngap_engine* e, int smem) {
     e->max_smem_set = g_smem_set[dev];
     return NGAP_OK;
   }
-  const void* kernels[6] = {(const void*)match_kernel<0, false>, (const void*)match_kernel<1, false>,
-                            (const void*)match_kernel<2, false>, (const void*)match_kernel<0, true>,
-                            (const void*)match_kernel<1, true>, (const void*)match_kernel<2, true>};
+  const void* kernels[2] = {(const void*)match_kernel<false>, (const void*)match_kernel<true>};
   cudaError_t ce = cudaSuccess;
-  for (int k = 0; k < 6 && ce == cudaSuccess; k++)
+  for (int k = 0; k < 2 && ce == cudaSuccess; k++)
     ce = cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (ce != cudaSuccess) {
     set_error("shared memory request of %d bytes rejected: %s", smem, cudaGetErrorString(ce));
@@ -918,31 +910,21 @@ int set_smem(ngap_engine* e, int smem) {
   return NGAP_OK;
 }
 
-template <int PRIV>
-int blocks_per_sm(int smem, int* out) {
-  CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, match_kernel<PRIV, false>, kCtaThreads,
-                                                         smem));
-  if (*out < 1) {
-    set_error("the matching kernel does not fit on an SM with %d bytes of shared memory", smem);
-    return NGAP_E_CUDA;
-  }
-  return NGAP_OK;
-}
-
-// blocks_per_sm of the engine's last shared-memory size per algorithm (the
+// Resident CTAs per SM, cached for the engine's last shared-memory size (the
 // occupancy query costs a driver call on every match otherwise).
-int cached_blocks_per_sm(ngap_engine* e, int priv, int smem, int* out) {
-  if (e->bps_smem[priv] == smem) {
-    *out = e->bps_val[priv];
-    return NGAP_OK;
+int blocks_per_sm(ngap_engine* e, int smem, int* out) {
+  if (e->bps_smem != smem) {
+    int n = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, match_kernel<false>, kCtaThreads, smem));
+    if (n < 1) {
+      set_error("the matching kernel does not fit on an SM with %d bytes of shared memory", smem);
+      return NGAP_E_CUDA;
+    }
+    e->bps_smem = smem;
+    e->bps_val = n;
   }
-  const int rc = priv == 0 ? blocks_per_sm<0>(smem, out)
-                 : priv == 1 ? blocks_per_sm<1>(smem, out) : blocks_per_sm<2>(smem, out);
-  if (rc == NGAP_OK) {
-    e->bps_smem[priv] = smem;
-    e->bps_val[priv] = *out;
-  }
-  return rc;
+  *out = e->bps_val;
+  return NGAP_OK;
 }
 
 // One sort of report keys: d_in[0 .. *d_n) (clamped to cap) into unique
@@ -1126,19 +1108,20 @@ int sort_unique_fields(ngap_engine* e, const unsigned long long* d_n, uint64_t c
   return sort_reports(e, j, st);
 }
 
-// --algorithm -> prefix depth, privatization and window. The blocking
-// algorithm scans the always-active list like NAP, over whole windows: windows
-// of one position cost a TMA copy and a wait per position and tile (64
-// literals in ten groups on 1 MiB: 9466 us on a B200, 85 us with windows of 2048).
-int algo_config(int algo, int table_depth, int* depth, int* priv, int* window) {
+// --algorithm -> prefix depth. The blocking algorithm scans the always-active
+// list like NAP, over whole windows: windows of one position cost a TMA copy
+// and a wait per position and tile (64 literals in ten groups on 1 MiB: 9466 us
+// on a B200, 85 us with windows of 2048). R1, R2 and all ask for
+// privatization, which the kernel does for every algorithm (walk_paths).
+int algo_config(int algo, int table_depth, int* depth) {
   switch (algo) {
-    case NGAP_ALGO_BLOCKING: *depth = 0; break;
+    case NGAP_ALGO_BLOCKING:
     case NGAP_ALGO_NAP: *depth = 0; break;
-    case NGAP_ALGO_NONBLOCKING: *depth = 1; break;
-    case NGAP_ALGO_NONBLOCKING_R1: *depth = 1; *priv = 1; break;
-    case NGAP_ALGO_NONBLOCKING_R2: *depth = 1; *priv = 2; break;
-    case NGAP_ALGO_NONBLOCKING_PC: *depth = std::max(1, table_depth); break;
-    case NGAP_ALGO_NONBLOCKING_ALL: *depth = std::max(1, table_depth); *priv = 1; break;
+    case NGAP_ALGO_NONBLOCKING:
+    case NGAP_ALGO_NONBLOCKING_R1:
+    case NGAP_ALGO_NONBLOCKING_R2: *depth = 1; break;
+    case NGAP_ALGO_NONBLOCKING_PC:
+    case NGAP_ALGO_NONBLOCKING_ALL: *depth = std::max(1, table_depth); break;
     default:
       set_error("not supported algoritm %d", algo);
       return NGAP_E_INVALID;
@@ -1183,25 +1166,14 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   e->launches = 0;
   e->sort_chain_pending = 0;
   e->ran = false;
-  int algo = p->algorithm;
   // automatic window: 2048 positions (against 1024: Hamming set 0.654 ->
   // 0.624 ms, high_frontier and the literal set 1-2 % faster; shortened
   // below when the shared memory of the warps and a staged image does not fit)
-  int depth = 1, priv = 0, window = p->window > 0 ? p->window : 2048;
+  int depth = 1, window = p->window > 0 ? p->window : 2048;
   int table_depth = 0;
   for (auto& th : t->tiles) table_depth = std::max(table_depth, th.depth);
-  switch (algo) {
-    case NGAP_ALGO_BLOCKING: depth = 0; break;
-    case NGAP_ALGO_NAP: depth = 0; break;
-    case NGAP_ALGO_NONBLOCKING: depth = 1; break;
-    case NGAP_ALGO_NONBLOCKING_R1: depth = 1; priv = 1; break;
-    case NGAP_ALGO_NONBLOCKING_R2: depth = 1; priv = 2; break;
-    case NGAP_ALGO_NONBLOCKING_PC: depth = std::max(1, table_depth); break;
-    case NGAP_ALGO_NONBLOCKING_ALL: depth = std::max(1, table_depth); priv = 1; break;
-    default:
-      set_error("not supported algoritm %d", algo);
-      return NGAP_E_INVALID;
-  }
+  int rc = algo_config(p->algorithm, table_depth, &depth);
+  if (rc != NGAP_OK) return rc;
   window = std::min(window, kMaxWindow);
   // input: own 16-byte-aligned, padded copy
   size_t need = ((total + 15) & ~(uint64_t)15) + 64;
@@ -1213,15 +1185,14 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
     e->input_cap = need;
   }
   uint64_t cap = p->result_capacity > 0 ? p->result_capacity : 54619400ull;
-  int rc = ensure_reports(e, cap);
-  if (rc != NGAP_OK) return rc;
+  if ((rc = ensure_reports(e, cap)) != NGAP_OK) return rc;
   // shared memory: the largest tile image that fits the budget, plus the warps
   // (a window too large for what is left is shortened)
   while (window > 64 && cta_smem_bytes(window, t->image_region) > 227 * 1024 - 1024) window /= 2;
   int smem = cta_smem_bytes(window, t->image_region);
   if ((rc = set_smem(e, smem)) != NGAP_OK) return rc;
   int bps = 0;
-  rc = cached_blocks_per_sm(e, priv, smem, &bps);
+  rc = blocks_per_sm(e, smem, &bps);
   if (rc != NGAP_OK) return rc;
   const int full_grid = e->num_sms * bps;
   // units and tasks
@@ -1291,7 +1262,6 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   mp.input = e->d_input;
   mp.window = window;
   mp.depth = depth;
-  mp.active_threshold = p->active_threshold;
   mp.unique = p->unique;
   mp.report_off = p->report_off;
   mp.off_shift = 32;
@@ -1320,7 +1290,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   e->trace_seg_len = p->seg_len;
   CUDA_TRY(cudaEventRecord(e->ev[1], st));
   if (e->ntasks > 0 || e->free_range[1] > 0 || e->free_range[3] > 0 || e->free_range[5] > 0) {
-    rc = launch_any(e, mp, smem, st, priv);
+    rc = launch_plan(e, mp, smem, st);
     if (rc != NGAP_OK) return rc;
   }
   CUDA_TRY(cudaEventRecord(e->ev[2], st));
@@ -1639,15 +1609,15 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   // automatic window: 2048 positions (against 1024: Hamming set 0.654 ->
   // 0.624 ms, high_frontier and the literal set 1-2 % faster; shortened
   // below when the shared memory of the warps and a staged image does not fit)
-  int depth = 1, priv = 0, window = p->window > 0 ? p->window : 2048;
-  int rc = algo_config(p->algorithm, ts->max_depth, &depth, &priv, &window);
+  int depth = 1, window = p->window > 0 ? p->window : 2048;
+  int rc = algo_config(p->algorithm, ts->max_depth, &depth);
   if (rc != NGAP_OK) return rc;
   window = std::min(window, kMaxWindow);
   while (window > 64 && cta_smem_bytes(window, ts->image_region) > 227 * 1024 - 1024) window /= 2;
   int smem = cta_smem_bytes(window, ts->image_region);
   if ((rc = set_smem(e, smem)) != NGAP_OK) return rc;
   int bps = 0;
-  rc = cached_blocks_per_sm(e, priv, smem, &bps);
+  rc = blocks_per_sm(e, smem, &bps);
   if (rc != NGAP_OK) return rc;
   const int full_grid = e->num_sms * bps;
   // buffers (before any capture)
@@ -1762,7 +1732,6 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   mp.input = e->d_input;
   mp.window = window;
   mp.depth = depth;
-  mp.active_threshold = p->active_threshold;
   mp.unique = p->unique;
   mp.report_off = p->report_off;
   mp.off_shift = oshift;
@@ -1801,7 +1770,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     CUDA_TRY(cudaMemsetAsync(e->d_err, 0, sizeof(int), qs));
     int r = NGAP_OK;
     if (e->ntasks > 0 || e->free_range[1] > 0 || e->free_range[3] > 0 || e->free_range[5] > 0) {
-      r = launch_any(e, mp, smem, qs, priv);
+      r = launch_plan(e, mp, smem, qs);
       if (r != NGAP_OK) return r;
     }
     if (!p->report_off) {

@@ -66,7 +66,6 @@ struct MatchParams {
   const uint8_t* input;     // 16-byte aligned, readable up to round_up(len, 16)
   int32_t window;           // W <= kMaxWindow
   int32_t depth;            // 0: scan the AAS list; >= 1: tables up to min(depth, tile.depth)
-  int32_t active_threshold; // privatize when more lanes than this expand
   int32_t unique;
   int32_t report_off;
   int32_t off_shift;        // bit position of the offset in report keys (32 when not batched)
@@ -678,7 +677,7 @@ __device__ __forceinline__ void inject_key(const TileView& tv, const UnitCtx& c,
 // r0 + 32 + lane), for tiles without sticky states: both table lookups of a
 // lane are issued before either list is read, so a warp has two lookups in
 // flight per lane. Same entries and reports as inject_aas over the two halves.
-// AHEAD (the lean PRIV 0 instances): after this batch's lookups, the lane's inline
+// AHEAD (the lean kernel): after this batch's lookups, the lane's inline
 // table words of the next batch are read too, and the next call uses them.
 // CAND: the positions are the filter candidates ws.cand[r0 .. r0 + batch).
 template <bool AHEAD, bool CAND>
@@ -1139,7 +1138,8 @@ __device__ __forceinline__ void layered_candidates(const MatchParams& p, WarpSme
 }
 
 // Expands the up-to-32 entries on top of the stack: one step of the worklist.
-template <int PRIV>
+// For tiles that register sticky states, and for --unique; the others follow
+// their paths in registers (walk_paths).
 __device__ __forceinline__ void expand_step(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                             const TileView& tv, const UnitCtx& c, int lane,
                                             int cursor, unsigned long long& n_expanded) {
@@ -1192,178 +1192,109 @@ __device__ __forceinline__ void expand_step(const MatchParams& p, WarpSmem& ws, 
 #pragma unroll
     for (int j = 0; j < 4; j++) carry_state(p, w, lane, need && at_end && ok[j], u[j] & kIdMask);
   }
-  const bool privatize = PRIV > 0 && !tv.sticky &&
-                         __popc(__ballot_sync(kFull, go)) > p.active_threshold;
-  if (!privatize) {
-    const int pc = (need && !at_end) ? cnt : 0;
-    int total;
-    const int ex = warp_excl<3>(pc, lane, total);
-    if (pc) {
-      int pos = w.top + ex;
-      const uint32_t tag = (uint32_t)(r + 1);
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (ok[j]) store_entry(p, ws, w, pos++, ((u[j] & kIdMask) << kEntryPosBits) | tag);
-    }
-    grow_stack(p, w, total);
-    __syncwarp();
-    return;
-  }
-  // privatization (kernel_ngap_OA.cu:96-138): expand the matched successors in
-  // registers one more level instead of pushing them
-  const bool inner = need && !at_end;  // successors' successors read in[r + 2] <= window end
-  const uint32_t s2 = inner ? c.in[r + 2] : 0u;
-  uint32_t u2[4][4];
-  bool ok2[4][4];
-  int cnt2 = 0;
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    uint4 sc2 = make_uint4(kNoSucc, kNoSucc, kNoSucc, kNoSucc);
-    uint4 sm2 = make_uint4(0u, 0u, 0u, 0u);
-    if (inner && ok[j]) {
-      sc2 = load_succ(tv, u[j] & kIdMask);
-      if (tv.fused) sm2 = load_smask(tv, u[j] & kIdMask);
-    }
-    u2[j][0] = sc2.x;
-    u2[j][1] = sc2.y;
-    u2[j][2] = sc2.z;
-    u2[j][3] = sc2.w;
-    const uint32_t um2[4] = {sm2.x, sm2.y, sm2.z, sm2.w};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      ok2[j][k] = succ_accepts(tv, u2[j][k], um2[k], s2);
-      cnt2 += ok2[j][k];
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 4; j++) report4(p, ws, w, tv, lane, ok2[j], u2[j], q + 2, q + 2 >= c.emit_lo);
-  const bool need2 = inner && q + 3 < c.hi;
-  const bool at_end2 = r + 2 == c.wlen;
-  if (__any_sync(kFull, need2 && at_end2)) {
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-#pragma unroll
-      for (int k = 0; k < 4; k++)
-        carry_state(p, w, lane, need2 && at_end2 && ok2[j][k], u2[j][k] & kIdMask);
-  }
-  const int pc = (need2 && !at_end2) ? cnt2 : 0;
+  const int pc = (need && !at_end) ? cnt : 0;
   int total;
-  const int ex = warp_excl<5>(pc, lane, total);
+  const int ex = warp_excl<3>(pc, lane, total);
   if (pc) {
     int pos = w.top + ex;
-    const uint32_t tag = (uint32_t)(r + 2);
+    const uint32_t tag = (uint32_t)(r + 1);
 #pragma unroll
     for (int j = 0; j < 4; j++)
-#pragma unroll
-      for (int k = 0; k < 4; k++)
-        if (ok2[j][k]) store_entry(p, ws, w, pos++, ((u2[j][k] & kIdMask) << kEntryPosBits) | tag);
+      if (ok[j]) store_entry(p, ws, w, pos++, ((u[j] & kIdMask) << kEntryPosBits) | tag);
   }
   grow_stack(p, w, total);
   __syncwarp();
 }
 
-// One worklist step over up to 64 entries, two per lane, for tiles without
-// sticky states and without privatization: both entries' successor records
-// are requested before either is used, so a warp keeps two L2 round trips in
-// flight per lane instead of one. Same results as two expand_step calls.
-// FUSED: the tile's records carry the successors' class masks (one 32-byte
-// record per state); the window arithmetic is 32-bit (UnitCtx::lim, elo)
-// and the rare report and carry paths are entered on one vote each.
-template <bool FUSED>
-__device__ __forceinline__ void expand_step2(const MatchParams& p, WarpSmem& ws, WarpRun& w,
-                                             const TileView& tv, const UnitCtx& c, int lane,
-                                             unsigned long long& n_expanded) {
-  const int n = min(w.top, 64);
-  uint32_t e[2];
-  e[0] = lane < n ? ws.stack[w.top - 1 - lane] : kNoEntry;
-  e[1] = lane + 32 < n ? ws.stack[w.top - 33 - lane] : kNoEntry;
-  w.top -= n;
-  __syncwarp();
-  if (p.unique) {  // identical entries in one half-step are expanded once (--unique)
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const unsigned peers = __match_any_sync(kFull, e[k]);
-      if ((__ffs(peers) - 1) != lane) e[k] = kNoEntry;
-    }
-  }
-  uint4 sc[2], sm[2];
-  uint32_t s[2];
-  int r[2];
-  bool go[2];
-#pragma unroll
-  for (int k = 0; k < 2; k++) {
-    r[k] = (int)(e[k] & ((1u << kEntryPosBits) - 1));
-    go[k] = e[k] != kNoEntry && r[k] + 1 < c.lim;
-    sc[k] = make_uint4(kNoSucc, kNoSucc, kNoSucc, kNoSucc);
-    sm[k] = make_uint4(0u, 0u, 0u, 0u);
-    s[k] = 0u;
-    if (go[k]) {
-      const uint32_t v = e[k] >> kEntryPosBits;
-      if (FUSED) {
-        sc[k] = tv.succ[(size_t)v * 2];
-        sm[k] = tv.succ[(size_t)v * 2 + 1];
-      } else {
-        sc[k] = load_succ(tv, v);
+// The worklist of tiles that register no sticky states: every lane takes an
+// entry and follows its path through the window in registers, pushing only
+// the successors beyond the first, and lanes whose path ended take new entries
+// while half the lanes are idle. This is the reference's privatization
+// (code/src/ngap/kernel_ngap_OA.cu:96-138: a matched successor expanded in
+// registers) without its limit of one extra level, and for every algorithm:
+// most paths have one matching successor, so the push, the prefix sum and the
+// pop per level were most of a step. One vote per position covers the rare
+// events (a report, a state for the next window, a second successor).
+// What bounds it is the length of a step's instruction chain and one record
+// read per step. Measured on a B200 against steps that popped 32 or 64
+// entries and pushed their successors (match times): 200 25-mers with three
+// table levels 1516 -> 699 us, 50 edit-distance 20-mers with one 391 -> 226,
+// 512 streams 10.3 -> 9.1 ms, 1000 25-mers 215 -> 206 us, one 81-byte line 29.4
+// -> 25.3 us.
+__device__ __forceinline__ void walk_paths(const MatchParams& p, WarpSmem& ws, WarpRun& w,
+                                           const TileView& tv, const UnitCtx& c, int lane,
+                                           unsigned long long& n_expanded) {
+  uint32_t v = 0;
+  int r = 0;
+  bool act = false;
+  unsigned live = 0u;
+  while (true) {
+    if (w.top > 0 && __popc(live) <= 16) {  // idle lanes take the entries on top of the stack
+      const int n = min(w.top, 32 - __popc(live));
+      const int k = __popc(~live & lanemask_lt(lane));
+      if (!act && k < n) {
+        const uint32_t e = ws.stack[w.top - 1 - k];
+        v = e >> kEntryPosBits;
+        r = (int)(e & ((1u << kEntryPosBits) - 1));
+        act = r + 1 < c.lim;
       }
-      s[k] = c.in[r[k] + 1];
+      w.top -= n;
+      __syncwarp();
     }
+    uint4 sc = make_uint4(kNoSucc, kNoSucc, kNoSucc, kNoSucc);
+    uint4 sm = make_uint4(0u, 0u, 0u, 0u);
+    uint32_t s = 0u;
+    if (act) {
+      sc = load_succ(tv, v);
+      if (tv.fused) sm = load_smask(tv, v);
+      s = c.in[r + 1];
+    }
+    n_expanded += act;
+    const uint32_t u[4] = {sc.x, sc.y, sc.z, sc.w};
+    const uint32_t um[4] = {sm.x, sm.y, sm.z, sm.w};
+    bool ok[4], rep = false;
+    int cnt = 0;
+    uint32_t follow = 0u;
+#pragma unroll
+    for (int j = 3; j >= 0; j--) {
+      ok[j] = act && succ_accepts(tv, u[j], um[j], s);
+      rep |= ok[j] && (u[j] >> 31);
+      cnt += ok[j];
+      if (ok[j]) follow = u[j] & kIdMask;
+    }
+    const bool need = act && r + 2 < c.lim && cnt > 0;  // the successors have a next symbol
+    const bool at_end = r + 1 == c.wlen;                // and sit at the next window's start
+    const unsigned events = __reduce_or_sync(
+        kFull, (rep && r + 1 >= c.elo ? 1u : 0u) | (need && at_end ? 2u : 0u) |
+                   (need && !at_end && cnt > 1 ? 4u : 0u));
+    if (events) {
+      if (events & 1u) report4(p, ws, w, tv, lane, ok, u, c.wb + r + 1, r + 1 >= c.elo);
+      if (events & 2u) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          carry_state(p, w, lane, need && at_end && ok[j], u[j] & kIdMask);
+      }
+      if (events & 4u) {  // successors beyond the first
+        const int more = need && !at_end ? cnt - 1 : 0;
+        int total;
+        int pos = w.top + warp_excl<2>(more, lane, total);
+        bool first = true;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (more && ok[j] && !first)
+            store_entry(p, ws, w, pos++, ((u[j] & kIdMask) << kEntryPosBits) | (uint32_t)(r + 1));
+          first = first && !ok[j];
+        }
+        grow_stack(p, w, total);
+        __syncwarp();
+      }
+    }
+    act = need && !at_end;
+    v = follow;
+    r++;
+    live = __ballot_sync(kFull, act);
+    if (live == 0u && w.top == 0) return;
   }
-  n_expanded += (unsigned)go[0] + (unsigned)go[1];
-  bool ok[2][4], need[2], at_end[2];
-  bool rep = false, carry = false;
-  int cnt = 0;
-#pragma unroll
-  for (int k = 0; k < 2; k++) {
-    const uint32_t u[4] = {sc[k].x, sc[k].y, sc[k].z, sc[k].w};
-    const uint32_t um[4] = {sm[k].x, sm[k].y, sm[k].z, sm[k].w};
-    bool rk = false;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      ok[k][j] = go[k] && (FUSED ? ((um[j] >> s[k]) & 1u) != 0u : succ_accepts(tv, u[j], um[j], s[k]));
-      rk |= ok[k][j] && (u[j] >> 31);
-    }
-    rep |= rk && r[k] + 1 >= c.elo;
-    need[k] = go[k] && r[k] + 2 < c.lim;
-    at_end[k] = r[k] + 1 == c.wlen;
-    carry |= need[k] && at_end[k];
-    if (need[k] && !at_end[k]) {
-#pragma unroll
-      for (int j = 0; j < 4; j++) cnt += ok[k][j];
-    }
-  }
-  if (__any_sync(kFull, rep)) {  // reports (rare): the warp-collective path per half
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const uint32_t u[4] = {sc[k].x, sc[k].y, sc[k].z, sc[k].w};
-      const int64_t q = c.wb + r[k];
-      report4(p, ws, w, tv, lane, ok[k], u, q + 1, r[k] + 1 >= c.elo);
-    }
-  }
-  if (__any_sync(kFull, carry)) {  // states landing on the next window's first position
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const uint32_t u[4] = {sc[k].x, sc[k].y, sc[k].z, sc[k].w};
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        carry_state(p, w, lane, need[k] && at_end[k] && ok[k][j], u[j] & kIdMask);
-    }
-  }
-  int total;
-  const int ex = warp_excl<4>(cnt, lane, total);
-  if (cnt) {
-    int pos = w.top + ex;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      if (!(need[k] && !at_end[k])) continue;
-      const uint32_t u[4] = {sc[k].x, sc[k].y, sc[k].z, sc[k].w};
-      const uint32_t tag = (uint32_t)(r[k] + 1);
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (ok[k][j]) store_entry(p, ws, w, pos++, ((u[j] & kIdMask) << kEntryPosBits) | tag);
-    }
-  }
-  grow_stack(p, w, total);
-  __syncwarp();
 }
 
 // A warp's view of one tile and the knobs derived from it.
@@ -1418,7 +1349,7 @@ __device__ __forceinline__ void tile_run(const MatchParams& p, const TileDev* t,
 // CTAs take tasks until none is left, then free units. LEAN kernels serve
 // launches whose tiles have no sticky states and are plain (no activation or
 // layered pass): that code is compiled out, for a smaller hot loop.
-template <int PRIV, bool LEAN>
+template <bool LEAN>
 __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   __shared__ int s_task;
@@ -1663,7 +1594,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
             }
           } else if (cursor < c.iend) {
             if (wide_inject) {
-              inject_aas2<LEAN && PRIV == 0, false>(p, ws, w, tv, c, lane, cursor, 2 * batch, depth,
+              inject_aas2<LEAN, false>(p, ws, w, tv, c, lane, cursor, 2 * batch, depth,
                                              n_injected, ahead);
               cursor += 2 * batch;
             } else if (LEAN) {
@@ -1694,14 +1625,10 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
           break;
         }
         // (layered tiles have no edge into a sticky state: no successor to register)
-        if (PRIV == 0 && (LEAN || !tv.sticky || layered)) {
-          if (tv.fused)
-            expand_step2<true>(p, ws, w, tv, c, lane, n_expanded);
-          else
-            expand_step2<false>(p, ws, w, tv, c, lane, n_expanded);
-        } else {
-          expand_step<PRIV>(p, ws, w, tv, c, lane, cursor, n_expanded);
-        }
+        if ((LEAN || !tv.sticky || layered) && !p.unique)
+          walk_paths(p, ws, w, tv, c, lane, n_expanded);
+        else
+          expand_step(p, ws, w, tv, c, lane, cursor, n_expanded);
       }
       inj_pos = max(inj_pos, wb + c.iend);  // a batch may end past iend
       cur ^= 1;
