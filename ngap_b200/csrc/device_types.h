@@ -76,9 +76,8 @@ struct FilterDev {
 };
 
 // A tile: a set of whole CCs (of one group, or of several for a global tile),
-// matched by one warp per unit. Its hot tables form one contiguous image,
-// staged into shared memory by the CTA that works on the tile when it fits
-// (global tiles are read in place, through L2):
+// matched by one warp per unit. Its hot tables form one contiguous image, read
+// in place through L1 and L2:
 //   [succ][cmask: nstates x cw x u32][rep: ceil(nstates/32) x u32][cls: 256 B]
 // succ: up to 4 tile-local successors per state; narrow tiles (< 32767
 // states) store 4 x u16 (bit 15 = report successor, 0xffff = none), wide
@@ -133,13 +132,6 @@ struct UnitDev {
   int64_t act_row;   // phase 1 and 2 tiles: first activation slot of the unit's segment
   int32_t act_rowid; // its row (pair, segment) in the compacted activation lists
   int32_t stream;    // segment (plain matching) or stream (batched matching) index
-};
-
-// A CTA-level task: consecutive units [ubegin, uend) of one tile.
-struct TaskDev {
-  int32_t tile;
-  int32_t ubegin, uend;
-  int32_t pad;
 };
 
 }  // namespace ngap

@@ -6,7 +6,6 @@
 #include <atomic>
 #include <cstring>
 #include <map>
-#include <functional>
 #include <mutex>
 #include <memory>
 #include <tuple>
@@ -75,8 +74,6 @@ struct ngap_tables {
   std::vector<void*> allocs;
   int64_t bytes = 0;
   int32_t max_states = 0;
-  int32_t image_region = 0;  // shared-memory bytes reserved for tile images
-  std::vector<int32_t> plan_bytes;  // per tile: image size of the planning rule (TileHost)
   std::vector<char> tile_lean;      // per tile: plain, no sticky states (the lean kernel runs it)
   std::vector<int32_t> pair_nact;  // activation slots of each (activation, layered) tile pair
   int32_t max_nact = 0;            // largest pair
@@ -109,6 +106,12 @@ struct UnitPlanKey {
   }
 };
 
+// Units of the three launches of a plan (make_units).
+struct UnitRanges {
+  int32_t begin[3] = {0, 0, 0}, count[3] = {0, 0, 0};
+  int32_t one_tile[3] = {-1, -1, -1};  // the one tile of a launch's units, or -1
+};
+
 struct ngap_engine {
   int device = 0;
   int num_sms = 0;
@@ -123,13 +126,7 @@ struct ngap_engine {
   size_t units_cap = 0;
   int32_t nunits = 0;
   int64_t longest_unit = 0;  // positions of the plan's longest unit
-  TaskDev* d_tasks = nullptr;
-  size_t tasks_cap = 0;
-  int32_t ntasks = 0;
-  int32_t ntasks1 = 0;       // tasks of activation tiles, launched first
-  int32_t ntasks2 = 0;       // tasks of plain tiles without sticky states (the lean launch)
-  int32_t free_range[6] = {0, 0, 0, 0, 0, 0};  // free units: [begin, count) of each launch
-  int32_t free_tile[3] = {-1, -1, -1};  // the one tile of each launch's free units, or -1
+  UnitRanges ranges;
   // worklist traces
   bool trace = false;
   unsigned long long* d_unit_work = nullptr;
@@ -205,7 +202,6 @@ struct ngap_engine {
   ~ngap_engine() {
     cudaFree(d_input);
     cudaFree(d_units);
-    cudaFree(d_tasks);
     cudaFree(d_reports);
     cudaFree(d_tmp);
     cudaFree(d_unique);
@@ -323,11 +319,7 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
       if ((rc = t->upload(ph.rlist, &pd.rlist)) != NGAP_OK) return rc;
     }
     t->dev_desc.push_back(d);
-    t->plan_bytes.push_back((int32_t)th.plan_bytes);
-    if (th.plan_bytes <= to.image_budget)
-      t->image_region = std::max(t->image_region, (int32_t)th.plan_bytes);
   }
-  t->image_region = (t->image_region + 127) & ~127;
   const TileDev* dt = nullptr;
   if ((rc = t->upload(t->dev_desc, &dt)) != NGAP_OK) return rc;
   t->d_tiles = const_cast<TileDev*>(dt);
@@ -361,7 +353,7 @@ int ngap_engine_create(int device, ngap_engine** out) {
   CUDA_TRY(cudaFuncSetAttribute(small_sort_unique<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSmallSortSmem));
   CUDA_TRY(cudaMalloc(&e->d_err, sizeof(int)));
-  CUDA_TRY(cudaMalloc(&e->d_unit_counter, 2 * sizeof(unsigned int)));  // tasks, free units
+  CUDA_TRY(cudaMalloc(&e->d_unit_counter, sizeof(unsigned int)));
   CUDA_TRY(cudaMallocHost(&e->h_counters, kNumCounters * sizeof(unsigned long long)));
   for (auto& ev : e->ev) CUDA_TRY(cudaEventCreate(&ev));
   *out = e.release();
@@ -501,12 +493,9 @@ int ensure_slots(ngap_engine* e, size_t slots, int max_states, int max_nact, int
 }
 
 // Splits the work into units: unbounded tiles get one unit per segment;
-// bounded tiles are cut into chunks of `chunk` emitted positions (AutoChunk when the caller
-// gives none), each with
-// max_path - 1 positions of warm-up (clamped at the segment start). Units of
-// one tile are then cut into CTA tasks: the long per-segment units of
-// unbounded tiles one per warp of a task and first, the chunks after them in
-// tasks sized to give every CTA several tasks.
+// bounded tiles are cut into chunks of emitted positions (AutoChunk when the
+// caller gives no length), each with max_path - 1 positions of warm-up (clamped
+// at the segment start).
 // One independent input range (a segment, or a whole stream in batched mode).
 struct SegSpec {
   int64_t lo, hi;
@@ -516,7 +505,7 @@ struct SegSpec {
   int32_t index;    // segment or stream index
 };
 
-// The launch that runs a tile (make_tasks): 0 activation tiles, 1 plain tiles
+// The launch that runs a tile (make_units): 0 activation tiles, 1 plain tiles
 // without sticky states, 2 the rest.
 int launch_of(const TileHost& th) {
   return th.phase == 1 ? 0 : (th.phase == 0 && th.nsticky == 0 ? 1 : 2);
@@ -607,109 +596,39 @@ struct ActRows {
   }
 };
 
-// Units (already grouped by tile) -> work of the launches. Units of tiles
-// whose image is staged in shared memory become CTA tasks: the long units of
-// cyclic tiles first, one per warp of a task; chunks after them in tasks sized
-// to give every CTA several tasks. Units of tiles read in place (is_free)
-// are taken one by one by warps (free units), after the tasks of their
-// launch. Three launches: the activation tiles; the plain tiles without
-// sticky states (is_lean: the lean kernel instance, with fewer registers
-// spilled and a smaller code path); the rest. Layout of `units`, per launch
-// in that order: [cyclic tasks][chunk tasks][cyclic free][chunk free];
-// ntasks1 / ntasks2 count the tasks of the first two launches, free_range
-// holds (begin, count) of each launch's free units.
-void make_tasks(std::vector<UnitDev>& units, const std::vector<UnitDev>& pass1,
-                const std::vector<UnitDev>& unbounded, const std::vector<UnitDev>& bounded,
-                int grid, const std::function<bool(int)>& is_free,
-                const std::function<bool(int)>& is_lean, std::vector<TaskDev>& tasks,
-                int32_t* ntasks1, int32_t* ntasks2, int32_t free_range[6], int32_t free_tile[3]) {
+// Units (already grouped by tile) in launch order: the activation tiles; the
+// plain tiles without sticky states (is_lean: the lean kernel instance, with
+// fewer registers spilled and a smaller code path); the rest. Within a launch the long
+// units of cyclic tiles come first. A launch whose units all belong to one
+// tile has its CTAs stage that tile's descriptors in shared memory.
+UnitRanges make_units(std::vector<UnitDev>& units, const std::vector<UnitDev>& pass1,
+                      const std::vector<UnitDev>& unbounded, const std::vector<UnitDev>& bounded,
+                      const std::vector<char>& lean) {
+  UnitRanges r;
   units.clear();
-  tasks.clear();
-  auto split = [&](const std::vector<UnitDev>& src, std::vector<UnitDev>& st,
-                   std::vector<UnitDev>& fr) {
-    for (const UnitDev& u : src) (is_free(u.tile) ? fr : st).push_back(u);
+  auto append = [&](const std::vector<UnitDev>& v, int which) {
+    for (const UnitDev& u : v)
+      if (which == 0 || (lean[u.tile] != 0) == (which == 1)) units.push_back(u);
   };
-  std::vector<UnitDev> p1s, p1f, ubs, ubf, bs, bf, lubs, lubf, lbs, lbf;
-  split(pass1, p1s, p1f);
-  std::vector<UnitDev> lean_ub, lean_b, rest_ub, rest_b;
-  for (const UnitDev& u : unbounded) (is_lean(u.tile) ? lean_ub : rest_ub).push_back(u);
-  for (const UnitDev& u : bounded) (is_lean(u.tile) ? lean_b : rest_b).push_back(u);
-  split(lean_ub, lubs, lubf);
-  split(lean_b, lbs, lbf);
-  split(rest_ub, ubs, ubf);
-  split(rest_b, bs, bf);
-  // a launch whose free units all belong to one tile: its CTAs stage that
-  // tile's descriptors in shared memory once
-  auto one_tile = [](const std::vector<UnitDev>& a, const std::vector<UnitDev>& b) {
-    int tile = -1;
-    for (const auto* v : {&a, &b})
-      for (const UnitDev& u : *v) {
-        if (tile >= 0 && u.tile != tile) return -1;
-        tile = u.tile;
-      }
-    return tile;
-  };
-  free_tile[0] = one_tile(p1f, {});
-  free_tile[1] = one_tile(lubf, lbf);
-  free_tile[2] = one_tile(ubf, bf);
-  auto per = [&](size_t n) {
-    return std::max<int64_t>(kWarpsPerCta,
-                             std::min<int64_t>(512, (int64_t)n / std::max(1, 4 * grid)));
-  };
-  // a task holds at most `per` units and, past its first unit, about a
-  // 16 * grid-th of the range's positions (at least 64 KiB), so that long
-  // chunks do not make long tasks
-  auto cut = [&](size_t b, size_t e, int64_t per) {
-    int64_t total = 0;
-    for (size_t k = b; k < e; k++) total += units[k].hi - units[k].lo;
-    const int64_t cap = std::max<int64_t>(1 << 16, total / std::max(1, 16 * grid));
-    size_t i = b;
-    while (i < e) {
-      size_t j = i;
-      int64_t bytes = 0;
-      while (j < e && units[j].tile == units[i].tile && (int64_t)(j - i) < per &&
-             (j == i || bytes + (units[j].hi - units[j].lo) <= cap)) {
-        bytes += units[j].hi - units[j].lo;
-        j++;
-      }
-      TaskDev tk;
-      tk.tile = units[i].tile;
-      tk.ubegin = (int32_t)i;
-      tk.uend = (int32_t)j;
-      tk.pad = 0;
-      tasks.push_back(tk);
-      i = j;
+  for (int which = 0; which < 3; which++) {
+    r.begin[which] = (int32_t)units.size();
+    if (which == 0) {
+      append(pass1, 0);
+    } else {
+      append(unbounded, which);
+      append(bounded, which);
     }
-  };
-  auto append = [&](const std::vector<UnitDev>& v) {
-    const size_t b = units.size();
-    units.insert(units.end(), v.begin(), v.end());
-    return b;
-  };
-  size_t b = append(p1s);
-  cut(b, units.size(), per(p1s.size()));
-  *ntasks1 = (int32_t)tasks.size();
-  free_range[0] = (int32_t)append(p1f);
-  free_range[1] = (int32_t)p1f.size();
-  auto launch = [&](const std::vector<UnitDev>& cs, const std::vector<UnitDev>& chs,
-                    const std::vector<UnitDev>& cf, const std::vector<UnitDev>& chf,
-                    int32_t* fr) {
-    size_t bb = append(cs);
-    cut(bb, units.size(), kWarpsPerCta);
-    bb = append(chs);
-    cut(bb, units.size(), per(chs.size()));
-    fr[0] = (int32_t)append(cf);
-    append(chf);
-    fr[1] = (int32_t)(cf.size() + chf.size());
-  };
-  launch(lubs, lbs, lubf, lbf, free_range + 2);
-  *ntasks2 = (int32_t)tasks.size() - *ntasks1;
-  launch(ubs, bs, ubf, bf, free_range + 4);
+    r.count[which] = (int32_t)units.size() - r.begin[which];
+    for (int32_t i = r.begin[which]; i < (int32_t)units.size(); i++) {
+      if (i == r.begin[which]) r.one_tile[which] = units[i].tile;
+      else if (units[i].tile != r.one_tile[which]) r.one_tile[which] = -1;
+    }
+  }
+  return r;
 }
 
 ActRows plan_units(const ngap_tables* t, const UnitPlanKey& k, int grid,
-                   std::vector<UnitDev>& units, std::vector<TaskDev>& tasks, int32_t* ntasks1,
-                   int32_t* ntasks2, int32_t free_range[6], int32_t free_tile[3]) {
+                   std::vector<UnitDev>& units, UnitRanges& ranges) {
   std::vector<UnitDev> pass1, unbounded, bounded;
   ActRows rows({t}, k.num_seg);
   AutoChunk ac;
@@ -724,11 +643,7 @@ ActRows plan_units(const ngap_tables* t, const UnitPlanKey& k, int grid,
                 bounded);
     }
   }
-  const int32_t region = t->image_region;
-  auto is_free = [&](int tile) { return t->plan_bytes[tile] > region; };
-  auto is_lean = [&](int tile) { return t->tile_lean[tile] != 0; };
-  make_tasks(units, pass1, unbounded, bounded, grid, is_free, is_lean, tasks, ntasks1, ntasks2,
-             free_range, free_tile);
+  ranges = make_units(units, pass1, unbounded, bounded, t->tile_lean);
   return rows;
 }
 
@@ -821,41 +736,26 @@ __global__ void act_compact(const int64_t* __restrict__ row_off, const int32_t* 
   if (lane == 0) cnt[row] = c;
 }
 
-// The matching launches of a plan: the activation tiles' tasks, then the rest
-// (the layered tiles read what the first launch recorded).
-// CTAs one launch needs: one per task, plus one per kWarpsPerCta free units,
-// at most the grid.
-int launch_grid(const ngap_engine* e, int ntasks, int nfree) {
-  const int64_t want = (int64_t)ntasks + ((int64_t)nfree + kWarpsPerCta - 1) / kWarpsPerCta;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(e->grid, want));
-}
-
-int plan_grid(const ngap_engine* e, int full_grid) {
-  const int64_t want = (int64_t)e->ntasks +
-                       ((int64_t)e->free_range[1] + e->free_range[3] + e->free_range[5] +
-                        kWarpsPerCta - 1) / kWarpsPerCta;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(full_grid, want));
+// CTAs of a launch: one per unit up to the whole grid, so that few units spread
+// over as many SMs.
+int launch_grid(int64_t nunits, int grid) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(grid, nunits));
 }
 
 // The matching launches of a plan: the activation tiles' work; the plain
 // tiles without sticky states in the lean kernel instance; then the rest
-// (the layered tiles read what the first launch recorded). Each launch takes
-// its tasks first, then its free units.
+// (the layered tiles read what the first launch recorded).
 int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
-  mp.free_cursor = e->d_unit_counter + 1;
-  const TaskDev* const tasks0 = mp.tasks;
+  mp.unit_cursor = e->d_unit_counter;
   if (e->act_entries > 0)
     CUDA_TRY(cudaMemsetAsync(e->d_act, 0xff, (size_t)e->act_entries * sizeof(uint32_t), st));
-  auto run = [&](bool lean, int32_t tbegin, int32_t ntasks, int which) -> int {
-    const int32_t nfree = e->free_range[2 * which + 1];
-    if (ntasks == 0 && nfree == 0) return NGAP_OK;
-    mp.tasks = tasks0 + tbegin;
-    mp.ntasks = ntasks;
-    mp.free_begin = e->free_range[2 * which];
-    mp.nfree = nfree;
-    mp.free_tile = e->free_tile[which];
-    CUDA_TRY(cudaMemsetAsync(e->d_unit_counter, 0, 2 * sizeof(unsigned int), st));
-    const int grid = launch_grid(e, ntasks, nfree);
+  auto run = [&](bool lean, int which) -> int {
+    if (e->ranges.count[which] == 0) return NGAP_OK;
+    mp.unit_begin = e->ranges.begin[which];
+    mp.nunits = e->ranges.count[which];
+    mp.one_tile = e->ranges.one_tile[which];
+    CUDA_TRY(cudaMemsetAsync(e->d_unit_counter, 0, sizeof(unsigned int), st));
+    const int grid = launch_grid(mp.nunits, e->grid);
     if (lean)
       match_kernel<true><<<grid, kCtaThreads, smem, st>>>(mp);
     else
@@ -864,8 +764,8 @@ int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
     e->launches++;
     return NGAP_OK;
   };
-  int rc = run(false, 0, e->ntasks1, 0);
-  if (rc == NGAP_OK) rc = run(true, e->ntasks1, e->ntasks2, 1);
+  int rc = run(false, 0);
+  if (rc == NGAP_OK) rc = run(true, 1);
   if (rc != NGAP_OK) return rc;
   if (e->act_rows > 0) {
     act_compact<<<(e->act_rows + 7) / 8, 256, 0, st>>>(e->d_row_off, e->d_row_n, e->act_rows,
@@ -873,7 +773,7 @@ int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
     CUDA_TRY(cudaGetLastError());
     e->launches++;
   }
-  return run(false, e->ntasks1 + e->ntasks2, e->ntasks - e->ntasks1 - e->ntasks2, 2);
+  return run(false, 2);
 }
 
 __global__ void swap_halves(uint64_t* a, uint64_t n) {
@@ -1167,8 +1067,8 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   e->sort_chain_pending = 0;
   e->ran = false;
   // automatic window: 2048 positions (against 1024: Hamming set 0.654 ->
-  // 0.624 ms, high_frontier and the literal set 1-2 % faster; shortened
-  // below when the shared memory of the warps and a staged image does not fit)
+  // 0.624 ms, high_frontier and the literal set 1-2 % faster; fit_window
+  // shortens it below)
   int depth = 1, window = p->window > 0 ? p->window : 2048;
   int table_depth = 0;
   for (auto& th : t->tiles) table_depth = std::max(table_depth, th.depth);
@@ -1186,25 +1086,19 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   }
   uint64_t cap = p->result_capacity > 0 ? p->result_capacity : 54619400ull;
   if ((rc = ensure_reports(e, cap)) != NGAP_OK) return rc;
-  // shared memory: the largest tile image that fits the budget, plus the warps
-  // (a window too large for what is left is shortened)
-  while (window > 64 && cta_smem_bytes(window, t->image_region) > 227 * 1024 - 1024) window /= 2;
-  int smem = cta_smem_bytes(window, t->image_region);
+  // shared memory: the warps' (a window too large for it is shortened)
+  while (window > 64 && cta_smem_bytes(window) > 227 * 1024 - 1024) window /= 2;
+  int smem = cta_smem_bytes(window);
   if ((rc = set_smem(e, smem)) != NGAP_OK) return rc;
   int bps = 0;
   rc = blocks_per_sm(e, smem, &bps);
   if (rc != NGAP_OK) return rc;
   const int full_grid = e->num_sms * bps;
-  // units and tasks
+  // units
   UnitPlanKey key{p->num_seg, p->seg_len, p->is_dup ? 1 : 0, window, p->chunk, p->first_segment};
   if (e->plan_tables != t->serial || key < e->plan_key || e->plan_key < key) {
     std::vector<UnitDev> units;
-    std::vector<TaskDev> tasks;
-    int32_t ntasks1 = 0, ntasks2 = 0;
-    const ActRows rows = plan_units(t, key, full_grid, units, tasks, &ntasks1, &ntasks2,
-                                    e->free_range, e->free_tile);
-    e->ntasks1 = ntasks1;
-    e->ntasks2 = ntasks2;
+    const ActRows rows = plan_units(t, key, full_grid, units, e->ranges);
     std::vector<Upload> ups;
     if ((rc = set_act_rows(e, rows, ups)) != NGAP_OK) return rc;
     if (units.size() > e->units_cap) {
@@ -1215,31 +1109,20 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
       CUDA_TRY(cudaMalloc(&e->d_units, cap * sizeof(UnitDev)));
       e->units_cap = cap;
     }
-    if (tasks.size() > e->tasks_cap) {
-      const size_t cap = grown(e->tasks_cap, tasks.size());
-      cudaFree(e->d_tasks);
-      e->d_tasks = nullptr;
-      e->tasks_cap = 0;
-      CUDA_TRY(cudaMalloc(&e->d_tasks, cap * sizeof(TaskDev)));
-      e->tasks_cap = cap;
-    }
     if (!units.empty()) ups.push_back({e->d_units, units.data(), units.size() * sizeof(UnitDev)});
-    if (!tasks.empty()) ups.push_back({e->d_tasks, tasks.data(), tasks.size() * sizeof(TaskDev)});
     if ((rc = upload_plan(e, st, ups)) != NGAP_OK) return rc;
     e->nunits = (int32_t)units.size();
     e->longest_unit = longest_unit(units);
     e->h_units = units;
-    e->ntasks = (int32_t)tasks.size();
     e->plan_tables = t->serial;
     e->plan_key = key;
     e->batch_ts = 0;  // the batched plan cache no longer describes the buffers
   }
   if (p->window <= 0) {
     window = fit_window(window, e->longest_unit);
-    smem = cta_smem_bytes(window, t->image_region);
+    smem = cta_smem_bytes(window);
   }
-  const int grid = plan_grid(e, full_grid);
-  e->grid = grid;
+  e->grid = full_grid;
   // per-warp scratch for the full grid, whatever this plan uses: a later
   // larger plan then never reallocates (cudaMalloc waits for the device)
   rc = ensure_slots(e, (size_t)full_grid * kWarpsPerCta, t->max_states, t->max_nact, kDefaultQueue);
@@ -1256,9 +1139,6 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   MatchParams mp;
   mp.tiles = t->d_tiles;
   mp.units = e->d_units;
-  mp.tasks = e->d_tasks;
-  mp.ntasks = e->ntasks;
-  mp.image_region = t->image_region;
   mp.input = e->d_input;
   mp.window = window;
   mp.depth = depth;
@@ -1269,7 +1149,6 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   mp.reports = e->d_reports;
   mp.rep_cap = cap;
   mp.err = e->d_err;
-  mp.task_counter = e->d_unit_counter;
   mp.carry = e->d_carry;
   mp.marks = e->d_marks;
   mp.ovf = e->d_ovf;
@@ -1289,7 +1168,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   if ((rc = trace_buffer(e, st, &mp.unit_work, &mp.unit_cycles)) != NGAP_OK) return rc;
   e->trace_seg_len = p->seg_len;
   CUDA_TRY(cudaEventRecord(e->ev[1], st));
-  if (e->ntasks > 0 || e->free_range[1] > 0 || e->free_range[3] > 0 || e->free_range[5] > 0) {
+  if (e->nunits > 0) {
     rc = launch_plan(e, mp, smem, st);
     if (rc != NGAP_OK) return rc;
   }
@@ -1388,8 +1267,7 @@ int ngap_engine_memory(const ngap_engine* e, ngap_engine_mem* out) {
   out->scratch =
       (int64_t)e->slots * 4 * ((int64_t)e->carry_cap + e->mark_words + e->ovf_cap + 2 * e->stk_cap);
   out->plan = 8 * (int64_t)e->act_cap + 16 * (int64_t)e->rows_cap + 16 * (int64_t)e->unit_work_cap +
-              (int64_t)sizeof(UnitDev) * (int64_t)e->units_cap +
-              (int64_t)sizeof(TaskDev) * (int64_t)e->tasks_cap;
+              (int64_t)sizeof(UnitDev) * (int64_t)e->units_cap;
   return NGAP_OK;
 }
 
@@ -1516,9 +1394,8 @@ struct ngap_tableset {
   std::vector<const ngap_tables*> tables;
   std::vector<int> tile_base;  // first tile of each NFA in the combined descriptor array
   TileDev* d_tiles = nullptr;
-  int ntiles = 0, image_region = 0, max_states = 0, max_groups = 1, max_depth = 1, device = 0;
+  int ntiles = 0, max_states = 0, max_groups = 1, max_depth = 1, device = 0;
   int max_nact = 0;
-  std::vector<int32_t> plan_bytes;  // per tile of the combined array (planning size)
   std::vector<char> tile_lean;      // per tile of the combined array (ngap_tables::tile_lean)
   ~ngap_tableset() { cudaFree(d_tiles); }
 };
@@ -1542,9 +1419,7 @@ int ngap_tableset_create(const ngap_tables* const* tables, int n, ngap_tableset*
     ts->tables.push_back(t);
     ts->tile_base.push_back((int)all.size());
     all.insert(all.end(), t->dev_desc.begin(), t->dev_desc.end());
-    ts->plan_bytes.insert(ts->plan_bytes.end(), t->plan_bytes.begin(), t->plan_bytes.end());
     ts->tile_lean.insert(ts->tile_lean.end(), t->tile_lean.begin(), t->tile_lean.end());
-    ts->image_region = std::max(ts->image_region, t->image_region);
     ts->max_states = std::max(ts->max_states, t->max_states);
     ts->max_groups = std::max(ts->max_groups, t->num_groups);
     ts->max_nact = std::max(ts->max_nact, t->max_nact);
@@ -1607,14 +1482,14 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   e->stream = st;
   e->ran = false;
   // automatic window: 2048 positions (against 1024: Hamming set 0.654 ->
-  // 0.624 ms, high_frontier and the literal set 1-2 % faster; shortened
-  // below when the shared memory of the warps and a staged image does not fit)
+  // 0.624 ms, high_frontier and the literal set 1-2 % faster; fit_window
+  // shortens it below)
   int depth = 1, window = p->window > 0 ? p->window : 2048;
   int rc = algo_config(p->algorithm, ts->max_depth, &depth);
   if (rc != NGAP_OK) return rc;
   window = std::min(window, kMaxWindow);
-  while (window > 64 && cta_smem_bytes(window, ts->image_region) > 227 * 1024 - 1024) window /= 2;
-  int smem = cta_smem_bytes(window, ts->image_region);
+  while (window > 64 && cta_smem_bytes(window) > 227 * 1024 - 1024) window /= 2;
+  int smem = cta_smem_bytes(window);
   if ((rc = set_smem(e, smem)) != NGAP_OK) return rc;
   int bps = 0;
   rc = blocks_per_sm(e, smem, &bps);
@@ -1638,7 +1513,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     CUDA_TRY(cudaMalloc(&e->d_stream_ids, cap * sizeof(uint32_t)));
     e->stream_ids_cap = cap;
   }
-  // plan: tiles outer (tasks share a staged image), streams of the tile's NFA inner
+  // plan: tiles outer, streams of the tile's NFA inner
   const std::vector<ngap_batch_stream> sv(streams, streams + nstreams);
   auto same_streams = [&]() {
     if (e->batch_streams.size() != sv.size()) return false;
@@ -1654,7 +1529,6 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     std::vector<std::vector<int>> by_nfa(ts->tables.size());
     for (int i = 0; i < nstreams; i++) by_nfa[sv[i].nfa].push_back(i);
     std::vector<UnitDev> pass1, unbounded, bounded, units;
-    std::vector<TaskDev> tasks;
     const ActRows rows(ts->tables, nstreams);
     AutoChunk ac;
     ac.warps = (int64_t)full_grid * kWarpsPerCta;
@@ -1675,11 +1549,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
         }
       }
     }
-    const int32_t region = ts->image_region;
-    auto is_free = [&](int tile) { return ts->plan_bytes[tile] > region; };
-    auto is_lean = [&](int tile) { return ts->tile_lean[tile] != 0; };
-    make_tasks(units, pass1, unbounded, bounded, full_grid, is_free, is_lean, tasks, &e->ntasks1,
-               &e->ntasks2, e->free_range, e->free_tile);
+    e->ranges = make_units(units, pass1, unbounded, bounded, ts->tile_lean);
     std::vector<Upload> ups;
     if ((rc = set_act_rows(e, rows, ups)) != NGAP_OK) return rc;
     if (units.size() > e->units_cap) {
@@ -1690,21 +1560,11 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
       CUDA_TRY(cudaMalloc(&e->d_units, cap * sizeof(UnitDev)));
       e->units_cap = cap;
     }
-    if (tasks.size() > e->tasks_cap) {
-      const size_t cap = grown(e->tasks_cap, tasks.size());
-      cudaFree(e->d_tasks);
-      e->d_tasks = nullptr;
-      e->tasks_cap = 0;
-      CUDA_TRY(cudaMalloc(&e->d_tasks, cap * sizeof(TaskDev)));
-      e->tasks_cap = cap;
-    }
     if (!units.empty()) ups.push_back({e->d_units, units.data(), units.size() * sizeof(UnitDev)});
-    if (!tasks.empty()) ups.push_back({e->d_tasks, tasks.data(), tasks.size() * sizeof(TaskDev)});
     if ((rc = upload_plan(e, st, ups)) != NGAP_OK) return rc;
     e->nunits = (int32_t)units.size();
     e->longest_unit = longest_unit(units);
     e->h_units = units;
-    e->ntasks = (int32_t)tasks.size();
     e->plan_tables = 0;  // the plain plan cache no longer describes the buffers
     e->plan_key = UnitPlanKey{-1, -1, -1, -1, -1, -1};
     e->batch_ts = ts->serial;
@@ -1715,10 +1575,9 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   }
   if (p->window <= 0) {
     window = fit_window(window, e->longest_unit);
-    smem = cta_smem_bytes(window, ts->image_region);
+    smem = cta_smem_bytes(window);
   }
-  const int grid = plan_grid(e, full_grid);
-  e->grid = grid;
+  e->grid = full_grid;
   if ((rc = ensure_slots(e, (size_t)full_grid * kWarpsPerCta, ts->max_states, ts->max_nact,
                          p->queue_capacity > 0 ? std::max(p->queue_capacity, 1024) : kDefaultQueue)) != NGAP_OK)
     return rc;
@@ -1726,9 +1585,6 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   MatchParams mp;
   mp.tiles = ts->d_tiles;
   mp.units = e->d_units;
-  mp.tasks = e->d_tasks;
-  mp.ntasks = e->ntasks;
-  mp.image_region = ts->image_region;
   mp.input = e->d_input;
   mp.window = window;
   mp.depth = depth;
@@ -1739,7 +1595,6 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   mp.reports = e->d_reports;
   mp.rep_cap = cap;
   mp.err = e->d_err;
-  mp.task_counter = e->d_unit_counter;
   mp.carry = e->d_carry;
   mp.marks = e->d_marks;
   mp.ovf = e->d_ovf;
@@ -1769,7 +1624,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     CUDA_TRY(cudaMemsetAsync(e->d_counters, 0, 8 * sizeof(unsigned long long), qs));
     CUDA_TRY(cudaMemsetAsync(e->d_err, 0, sizeof(int), qs));
     int r = NGAP_OK;
-    if (e->ntasks > 0 || e->free_range[1] > 0 || e->free_range[3] > 0 || e->free_range[5] > 0) {
+    if (e->nunits > 0) {
       r = launch_plan(e, mp, smem, qs);
       if (r != NGAP_OK) return r;
     }

@@ -13,15 +13,14 @@
 // kernel_ngap_OA.cu:242-311).
 //
 // B200 organisation (not the reference's):
-//  * a CTA takes a task (a tile and a range of its units) and stages the
-//    tile's table image (successors, byte-class masks, report bits, byte ->
-//    class map) into shared memory once; its warps (kWarpsPerCta) then take units of that
-//    task, one warp per unit, with no block-wide barrier in the hot loop;
+//  * one warp per unit (a tile and a range of positions), taken from a global
+//    cursor, with no block-wide barrier after the start; tiles are read in
+//    place, through L1 and L2;
+//  * a look-ahead filter (FilterDev) picks the positions that need injection;
 //  * per warp, in shared memory: a LIFO worklist of packed entries
-//    (state << 13 | offset in the window); one expansion step pops up to 32
-//    entries, evaluates all their successors, and pushes the survivors with a
-//    single bit-sliced ballot prefix sum; entries past the shared capacity
-//    spill to a per-warp global overflow stack;
+//    (state << 13 | offset in the window) whose paths are followed in
+//    registers; entries past the shared capacity spill to a per-warp global
+//    overflow stack;
 //  * input windows are fetched by cp.async.bulk (1-D TMA, completion on an
 //    mbarrier, bounded wait), double-buffered, and translated to class ids in
 //    place;
@@ -36,11 +35,21 @@
 
 namespace ngap {
 
-constexpr int kWarpsPerCta = 20;
+// 16 warps of 128 registers per SM, and as little shared memory as they need:
+// what shared memory does not take is L1, which holds the hot parts of tables,
+// filters and images. Measured on a B200 (match times): 20 warps of 96
+// registers with tile images staged in shared memory and worklists of 512
+// entries, then 16 warps, then 384 entries and images read in place: 512
+// streams 8.96, 6.22, 3.25 ms; 1000 25-mers 205, 192, 184 us; motifs with 1.5 M
+// reports 328, 264, 156 us; 300 dot-star regexes 216, 179, 140 us; 64 literals
+// 33, 27, 27 us; 200 25-mers with three table levels (many live paths) 699,
+// 746, 765 us (256 entries: 817). Other counts for the 25-mers: 12 warps of 168
+// registers 214 us, 18 of 112 191 us, 24 of 80 (spilled) 335 us.
+constexpr int kWarpsPerCta = 16;
 constexpr int kCtaThreads = kWarpsPerCta * 32;
-constexpr int kStackCap = 512;    // entries per warp in shared memory
+constexpr int kStackCap = 384;    // entries per warp in shared memory
 constexpr int kReportBuf = 64;    // reports per warp buffered in shared memory
-constexpr int kInjectLow = 256;   // inject new positions while the stack holds fewer entries
+constexpr int kInjectLow = 192;   // inject new positions while the stack holds fewer entries
 constexpr int kStickyCap = 64;    // sticky states tracked per warp (more fall back to entries)
 constexpr int kPendCap = 16;      // sticky states met while copying one injection batch
 constexpr int kScanLane = 8;      // consecutive positions a lane tests per filter scan step
@@ -60,9 +69,6 @@ constexpr int kErrCarry = 8;      // carry buffer full
 struct MatchParams {
   const TileDev* tiles;
   const UnitDev* units;
-  const TaskDev* tasks;
-  int32_t ntasks;
-  int32_t image_region;     // shared-memory bytes reserved for a tile image
   const uint8_t* input;     // 16-byte aligned, readable up to round_up(len, 16)
   int32_t window;           // W <= kMaxWindow
   int32_t depth;            // 0: scan the AAS list; >= 1: tables up to min(depth, tile.depth)
@@ -73,7 +79,6 @@ struct MatchParams {
   uint64_t* reports;        // key = offset << 32 | id
   uint64_t rep_cap;
   int* err;
-  unsigned int* task_counter;
   uint32_t* carry;          // [slots][carry_cap]
   uint32_t* marks;          // [slots][mark_words]
   uint32_t* ovf;            // [slots][ovf_cap]
@@ -87,10 +92,10 @@ struct MatchParams {
   int32_t stk_g_cap;        // kStickyCap
   unsigned long long* unit_work;  // [units]: entries expanded + injected per unit (tracing), or null
   unsigned long long* unit_cycles;  // [units]: SM clock cycles per unit (tracing), or null
-  int32_t free_begin;       // units [free_begin, free_begin + nfree) are taken warp by warp
-  int32_t nfree;
-  int32_t free_tile;        // the one tile of all free units (descriptors staged per CTA), or -1
-  unsigned int* free_cursor;  // next free unit (zeroed before the launch)
+  int32_t unit_begin;       // units [unit_begin, unit_begin + nunits) of this launch
+  int32_t nunits;
+  int32_t one_tile;         // the one tile of the launch's units (descriptors staged per CTA), or -1
+  unsigned int* unit_cursor;  // next unit (zeroed before the launch)
   int32_t wait_rounds;      // try_wait rounds before an mbarrier wait gives up
   int32_t skip_copy_unit;   // test hook: this unit's first window copy is not issued (-1: none),
                             // so its wait runs out and the launch reports kErrTimeout
@@ -113,9 +118,7 @@ __host__ __device__ inline int warp_smem_bytes(int W) {
          kStickyCap * 8 + kPendCap * 8 + 16 + kCandCap * 2;
 }
 
-__host__ __device__ inline int cta_smem_bytes(int W, int image_region) {
-  return image_region + kWarpsPerCta * warp_smem_bytes(W);
-}
+__host__ __device__ inline int cta_smem_bytes(int W) { return kWarpsPerCta * warp_smem_bytes(W); }
 
 struct WarpSmem {
   uint32_t* stack;           // kStackCap
@@ -148,8 +151,7 @@ struct WarpRun {
   bool stk_rep;    // layered units: some registered sticky state is a report state
 };
 
-// The tile a warp works on: hot tables in shared memory (or global memory
-// when the image does not fit) and the cold ones in global memory.
+// The tile a warp works on.
 struct TileView {
   const uint4* succ;    // wide tiles
   const uint32_t* cmask;
@@ -167,8 +169,8 @@ struct TileView {
 
 // Successors of v in the 32-bit convention (bit 31 = report, kNoSucc = none).
 __device__ __forceinline__ uint4 load_succ(const TileView& tv, uint32_t v) {
-  if (!tv.narrow) return tv.succ[(size_t)v << tv.fused];
-  const uint2 x = reinterpret_cast<const uint2*>(tv.succ)[v];  // narrow tiles: 4 x u16
+  if (!tv.narrow) return __ldg(tv.succ + ((size_t)v << tv.fused));
+  const uint2 x = __ldg(reinterpret_cast<const uint2*>(tv.succ) + v);  // narrow tiles: 4 x u16
   auto wide = [](uint32_t h) {
     return h == 0xffffu ? kNoSucc : ((h & 0x7fffu) | ((h & 0x8000u) << 16));
   };
@@ -178,7 +180,7 @@ __device__ __forceinline__ uint4 load_succ(const TileView& tv, uint32_t v) {
 // Fused tiles: the class masks of v's four successors (0 where none), the
 // second half of v's 32-byte record.
 __device__ __forceinline__ uint4 load_smask(const TileView& tv, uint32_t v) {
-  return tv.succ[((size_t)v << 1) + 1];
+  return __ldg(tv.succ + ((size_t)v << 1) + 1);
 }
 
 // Successor j of a state accepts class c: from the record's masks (fused
@@ -236,7 +238,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int32_
 }
 
 __device__ __forceinline__ bool accepts(const TileView& tv, uint32_t v, uint32_t c) {
-  return (tv.cmask[(size_t)v * tv.cw + (c >> 5)] >> (c & 31)) & 1u;
+  return (__ldg(tv.cmask + (size_t)v * tv.cw + (c >> 5)) >> (c & 31)) & 1u;
 }
 
 __device__ __forceinline__ bool succ_accepts(const TileView& tv, uint32_t u, uint32_t m, uint32_t c) {
@@ -245,7 +247,7 @@ __device__ __forceinline__ bool succ_accepts(const TileView& tv, uint32_t u, uin
 }
 
 __device__ __forceinline__ bool is_report(const TileView& tv, uint32_t v) {
-  return (tv.rep[v >> 5] >> (v & 31)) & 1u;
+  return (__ldg(tv.rep + (v >> 5)) >> (v & 31)) & 1u;
 }
 
 __device__ __forceinline__ unsigned lanemask_lt(int lane) { return (1u << lane) - 1u; }
@@ -425,7 +427,7 @@ __device__ __forceinline__ void report4(const MatchParams& p, WarpSmem& ws, Warp
 // catches up the positions already injected.
 
 __device__ __forceinline__ bool is_sticky(const TileView& tv, uint32_t v) {
-  return (tv.sticky[v >> 5] >> (v & 31)) & 1u;
+  return (__ldg(tv.sticky + (v >> 5)) >> (v & 31)) & 1u;
 }
 
 // Work of active sticky state s at stream position t (act: s matched at t - 1):
@@ -1304,13 +1306,14 @@ struct TileRun {
   bool layered, wide_inject, filtered;
 };
 
-// Builds the view of tile t whose image is at ib (shared-memory copy or the
-// global image), prefix-table descriptors at pt and byte classes at cls.
+// Builds the view of tile t, prefix-table descriptors at pt and byte classes at
+// cls (copies in shared memory where one tile serves the whole launch).
 template <bool LEAN>
-__device__ __forceinline__ void tile_run(const MatchParams& p, const TileDev* t, const uint8_t* ib,
+__device__ __forceinline__ void tile_run(const MatchParams& p, const TileDev* t,
                                          const PrefixTableDev* pt, const uint8_t* cls,
                                          TileRun& tr) {
   TileView& tv = tr.tv;
+  const uint8_t* ib = t->image;
   tv.succ = reinterpret_cast<const uint4*>(ib);
   tv.cmask = reinterpret_cast<const uint32_t*>(ib + t->off_cmask);
   tv.rep = reinterpret_cast<const uint32_t*>(ib + t->off_rep);
@@ -1339,27 +1342,18 @@ __device__ __forceinline__ void tile_run(const MatchParams& p, const TileDev* t,
   tr.look = max(1, t->filt.len);
 }
 
-// Two kinds of work per launch:
-//  * tasks (consecutive units of one tile whose image fits shared memory):
-//    a CTA stages the image once and its warps take the task's units; the
-//    CTA waits for all of them before the next task replaces the image;
-//  * free units (tiles read in place through L2): every warp takes the next
-//    unit from a global cursor on its own and reads the tile's descriptors
-//    from global memory, so no warp waits for another.
-// CTAs take tasks until none is left, then free units. LEAN kernels serve
-// launches whose tiles have no sticky states and are plain (no activation or
-// layered pass): that code is compiled out, for a smaller hot loop.
+// Every warp takes the launch's units one by one from a global cursor, so no
+// warp waits for another. LEAN kernels serve launches whose tiles have no
+// sticky states and are plain (no activation or layered pass): that code is
+// compiled out, for a smaller hot loop.
 template <bool LEAN>
 __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  __shared__ int s_task;
-  __shared__ unsigned s_next;
   __shared__ __align__(16) PrefixTableDev s_pt[kMaxDepth];
   __shared__ __align__(16) uint8_t s_cls[256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int W = p.window;
-  uint8_t* image = smem_raw;
-  uint8_t* base = smem_raw + p.image_region + (size_t)warp * warp_smem_bytes(W);
+  uint8_t* base = smem_raw + (size_t)warp * warp_smem_bytes(W);
   WarpSmem ws;
   ws.stack = reinterpret_cast<uint32_t*>(base);
   ws.in[0] = base + kStackCap * 4;
@@ -1396,7 +1390,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   bool pending[2] = {false, false};
   bool dead = false;
   unsigned long long n_expanded = 0, n_injected = 0;
-  int staged = -1;  // tile whose image is in shared memory
 
   // loads window [wb, min(wb + W, hi)) plus `look` look-ahead bytes and `lb`
   // look-behind bytes into buffer buf; returns the byte count, and in `skip`
@@ -1655,97 +1648,29 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
     }
   };
 
-  // One loop, one call of run_unit: the next unit comes from the CTA's
-  // current task (staged tiles; a new task after a CTA barrier once the
-  // current one is exhausted) until no task is left, then from the free
-  // units, warp by warp. Every warp of a CTA takes the same barriers: a warp
-  // that gave up (dead) still waits for its CTA's tasks to end.
-  bool tasks_left = p.ntasks > 0;
-  bool free_ready = false;
-  bool need_task = true;
-  bool task_fits = false;
-  int task_end = 0;
-  const TileDev* task_tile = nullptr;
-  while (true) {
-    unsigned uid = 0;
-    const TileDev* t = nullptr;
-    if (tasks_left) {
-      if (need_task) {
-        __syncthreads();  // every warp is done with the last task before its image is replaced
-        if (threadIdx.x == 0) s_task = (int)atomicAdd(p.task_counter, 1u);
-        __syncthreads();
-        const int task = s_task;
-        if (task >= p.ntasks) {
-          tasks_left = false;
-          continue;
-        }
-        const TaskDev tk = p.tasks[task];
-        t = &p.tiles[tk.tile];
-        const bool fits = t->image_bytes <= p.image_region;
-        if (fits && staged != tk.tile) {  // stage the tile image
-          const uint4* src = reinterpret_cast<const uint4*>(t->image);
-          uint4* dst = reinterpret_cast<uint4*>(image);
-          for (int i = threadIdx.x; i < t->image_bytes / 16; i += kCtaThreads) dst[i] = __ldg(src + i);
-          staged = tk.tile;
-        }
-        {  // the tile's prefix-table descriptors, read at every injection, and its byte classes
-          const uint32_t* src = reinterpret_cast<const uint32_t*>(t->pt);
-          uint32_t* dst = reinterpret_cast<uint32_t*>(s_pt);
-          for (int i = threadIdx.x; i < (int)(sizeof(s_pt) / 4); i += kCtaThreads) dst[i] = src[i];
-          if (threadIdx.x < 64)
-            reinterpret_cast<uint32_t*>(s_cls)[threadIdx.x] =
-                __ldg(reinterpret_cast<const uint32_t*>(t->image + t->off_cls) + threadIdx.x);
-        }
-        if (threadIdx.x == 0) s_next = (unsigned)tk.ubegin;
-        __syncthreads();
-        task_tile = t;
-        task_fits = fits;
-        task_end = tk.uend;
-        need_task = false;
-      }
-      if (dead) {
-        need_task = true;
-        continue;
-      }
-      if (lane == 0) uid = atomicAdd(&s_next, 1u);
-      uid = __shfl_sync(kFull, uid, 0);
-      if (uid >= (unsigned)task_end) {
-        need_task = true;
-        continue;
-      }
-      t = task_tile;
-    } else {
-      if (!free_ready) {  // CTA-uniform: every warp of the CTA has left the tasks
-        if (p.free_tile >= 0) {  // one tile for all free units: its descriptors in shared memory
-          const TileDev* ft = &p.tiles[p.free_tile];
-          const uint32_t* src = reinterpret_cast<const uint32_t*>(ft->pt);
-          uint32_t* dst = reinterpret_cast<uint32_t*>(s_pt);
-          for (int i = threadIdx.x; i < (int)(sizeof(s_pt) / 4); i += kCtaThreads) dst[i] = src[i];
-          if (threadIdx.x < 64)
-            reinterpret_cast<uint32_t*>(s_cls)[threadIdx.x] =
-                __ldg(reinterpret_cast<const uint32_t*>(ft->image + ft->off_cls) + threadIdx.x);
-          __syncthreads();
-        }
-        free_ready = true;
-      }
-      if (dead || p.nfree <= 0) break;
-      unsigned k = 0;
-      if (lane == 0) k = atomicAdd(p.free_cursor, 1u);
-      k = __shfl_sync(kFull, k, 0);
-      if (k >= (unsigned)p.nfree) break;
-      uid = (unsigned)p.free_begin + k;
-      t = &p.tiles[p.units[uid].tile];
-    }
-    // the unit's view of its tile (rebuilt per unit, so that it is not live
-    // across units): the staged image and shared descriptors of the task, or
-    // for free units the global image and descriptors, read in place
+  if (p.one_tile >= 0) {  // one tile for all units: its descriptors in shared memory
+    const TileDev* ot = &p.tiles[p.one_tile];
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(ot->pt);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(s_pt);
+    for (int i = threadIdx.x; i < (int)(sizeof(s_pt) / 4); i += kCtaThreads) dst[i] = src[i];
+    if (threadIdx.x < 64)
+      reinterpret_cast<uint32_t*>(s_cls)[threadIdx.x] =
+          __ldg(reinterpret_cast<const uint32_t*>(ot->image + ot->off_cls) + threadIdx.x);
+    __syncthreads();
+  }
+  while (!dead) {
+    unsigned k = 0;
+    if (lane == 0) k = atomicAdd(p.unit_cursor, 1u);
+    k = __shfl_sync(kFull, k, 0);
+    if (k >= (unsigned)p.nunits) break;
+    const unsigned uid = (unsigned)p.unit_begin + k;
+    const TileDev* t = &p.tiles[p.one_tile >= 0 ? p.one_tile : p.units[uid].tile];
+    // the unit's view of its tile (rebuilt per unit, so that it is not live across units)
     TileRun tr;
-    if (tasks_left)
-      tile_run<LEAN>(p, t, task_fits ? image : t->image, s_pt, s_cls, tr);
-    else if (p.free_tile >= 0 && t == p.tiles + p.free_tile)
-      tile_run<LEAN>(p, t, t->image, s_pt, s_cls, tr);
+    if (p.one_tile >= 0)
+      tile_run<LEAN>(p, t, s_pt, s_cls, tr);
     else
-      tile_run<LEAN>(p, t, t->image, t->pt, t->image + t->off_cls, tr);
+      tile_run<LEAN>(p, t, t->pt, t->image + t->off_cls, tr);
     sticky_lists(t, false, 0u);  // layered units choose theirs by their activation count
     run_unit(uid, t, tr);
   }

@@ -509,9 +509,6 @@ void build_image(TileHost& t) {
   memcpy(t.image.data() + t.off_rep, t.rep.data(), t.rep.size() * 4);
   memcpy(t.image.data() + t.off_sticky, t.sticky.data(), t.sticky.size() * 4);
   memcpy(t.image.data() + t.off_cls, t.cls.data(), 256);
-  const int pcw = plan_class_words(t.ncls);
-  t.plan_bytes = (int64_t)r16(n * (t.narrow ? 8 : (pcw == 1 ? 32 : 16))) + (int64_t)r16(n * pcw * 4) +
-                 2 * (int64_t)r16(((n + 31) / 32) * 4) + 256;
 }
 
 int degree_error() {

@@ -40,7 +40,7 @@ struct TileHost {
                                      // their class masks in one 32-byte record
   int32_t inj_batch = 32;            // positions injected per worklist refill
   int32_t inj_batch0 = 32;           // the same without prefix tables (AAS scan)
-  bool global = false;               // tables read through L2, never staged in shared memory
+  bool global = false;               // CCs of all groups, no image budget
   int32_t phase = 0;                 // 0 plain, 1 activation pass, 2 layered (stickies from pass 1)
   int32_t pair = -1;                 // activation/layered tiles: index of their pair
   int32_t nact = 0;                  // activation slots (sticky states) of the pair
@@ -50,9 +50,6 @@ struct TileHost {
   std::vector<uint32_t> succ;        // nstates * 4, bit 31 = report successor
   std::vector<uint32_t> bits;        // nstates * 8 raw symbol classes
   std::vector<uint32_t> cmask;       // nstates * cw
-  int64_t plan_bytes = 0;            // the image's size for planning decisions (tile packing,
-                                     // staging): with 1, 2 or 8 mask words, as the planner was
-                                     // tuned, though the image holds ceil(classes / 32)
   std::vector<uint32_t> rep;         // ceil(nstates / 32)
   std::vector<uint32_t> sid;         // nstates: report id, group-local sid | group << 22
   std::vector<uint32_t> aas, start;
@@ -69,7 +66,7 @@ struct TableOpts {
   int precompute_cutoff = -1;
   int tile_states = 0;              // max states per tile; 0 = fill the image budget
   int64_t max_table_entries = 0;    // 0 = automatic
-  int image_budget = 128 * 1024;    // bytes of shared memory for one tile's image
+  int image_budget = 128 * 1024;    // image bytes of a tile of one group
   int unbounded_tile_states = 256;  // cap for tiles of cyclic CCs (one unit per segment)
   int64_t auto_table_bytes = 12 << 20;  // automatic depth: prefix-table bytes per tile
   int max_warmup = 2048;            // longest acyclic path that still allows chunking
@@ -81,7 +78,7 @@ struct TableOpts {
 
 constexpr int32_t kNarrowMaxStates = 32767;  // 15-bit tile-local ids
 
-// Bytes of a tile image with n states and cw class words.
+// Bytes of a tile image with n states and cw class words, for packing CCs.
 // Mask words per state in the planner's size rule (1, 2 or 8).
 inline int plan_class_words(int ncls) { return ncls <= 32 ? 1 : (ncls <= 64 ? 2 : 8); }
 

@@ -32,6 +32,6 @@ def test_auto_chunks(engine, num_seg, seg_len):
             assert np.array_equal(u["lo"][1:], u["hi"][:-1])
         longest = int((units["hi"] - units["lo"]).max())
         assert longest <= 2048
-        # one unit per warp of a full grid, or 128 positions where that is longer
-        warps = 148 * 20
+        # one unit per warp of a full grid (16 per SM), or 128 positions where that is longer
+        warps = 148 * 16
         assert longest <= max(128, -(-n // warps) + 63)
