@@ -31,17 +31,34 @@ namespace {
     }                                                                                      \
   } while (0)
 
-// Device counters of an engine: [0] raw reports, [1] unique reports, [2..3]
-// work, [5..6] the standalone sort's counts, [kRadixCount] keys left to the
-// radix pipeline after the small-set sort.
-constexpr int kNumCounters = 16;
+// Device counters of an engine (kNumCounters words, zeroed by the last kernel
+// of a match, HostOut): [0] raw reports, [1] unique reports, [2..3] work, [4]
+// error bits, [5..6] the standalone sort's counts, [kRadixCount] keys left to
+// the radix pipeline after the small-set sort, [kCursors ...] the unit cursors
+// of the three launches.
 constexpr int kDefaultQueue = 1 << 16;  // overflow-stack entries per warp
 constexpr int kRadixCount = 8;
+constexpr int kCursors = 10;
 
 int bits_for(uint64_t x) {  // bits needed to hold values < x (x >= 1)
   int b = 0;
   while (b < 64 && (x - 1) >> b) b++;
   return b;
+}
+
+// Bits [lo, lo + n) of a key.
+uint64_t bit_range(int lo, int n) { return n <= 0 ? 0ull : ((n >= 64 ? ~0ull : (1ull << n) - 1) << lo); }
+
+// The 8-bit digits that cover the bits of a key that can vary, least
+// significant first.
+std::vector<int> digits_of(uint64_t bits) {
+  std::vector<int> shifts;
+  while (bits) {
+    const int b = __builtin_ctzll(bits);
+    shifts.push_back(b);
+    bits &= ~bit_range(b, kDigitBits);
+  }
+  return shifts;
 }
 
 }  // namespace
@@ -68,6 +85,7 @@ struct ngap_tables {
   uint64_t serial = g_next_serial.fetch_add(1);
   int device = 0;
   int num_groups = 0;
+  int sid_bits = 0;  // bits of the largest group-local state id
   std::vector<TileHost> tiles;
   std::vector<TileDev> dev_desc;
   TileDev* d_tiles = nullptr;
@@ -151,12 +169,9 @@ struct ngap_engine {
   uint64_t* d_unique = nullptr;
   uint32_t* d_hist = nullptr;
   size_t hist_cap = 0;
-  // counters: [0] raw reports, [1] unique reports, [2] expanded, [3] injected
   unsigned long long* d_counters = nullptr;
-  int* d_err = nullptr;
-  unsigned int* d_unit_counter = nullptr;
-  unsigned long long* h_counters = nullptr;  // pinned mirror: [0..3] counters, [4] err,
-                                             // [kRadixCount] keys left to the radix pipeline
+  bool counters_dirty = false;  // a match was left half enqueued: zero them first
+  HostOut ho;                   // what the last kernel of a match leaves in pinned memory
   // per-warp scratch
   uint32_t* d_carry = nullptr;
   uint32_t* d_marks = nullptr;
@@ -207,8 +222,6 @@ struct ngap_engine {
     cudaFree(d_unique);
     cudaFree(d_hist);
     cudaFree(d_counters);
-    cudaFree(d_err);
-    cudaFree(d_unit_counter);
     cudaFree(d_carry);
     cudaFree(d_marks);
     cudaFree(d_ovf);
@@ -226,7 +239,9 @@ struct ngap_engine {
     for (auto& c : cap_ev)
       if (c) cudaEventDestroy(c);
     if (cap_stream) cudaStreamDestroy(cap_stream);
-    if (h_counters) cudaFreeHost(h_counters);
+    if (ho.counters) cudaFreeHost(ho.counters);
+    if (ho.reports) cudaFreeHost(ho.reports);
+    if (ho.streams) cudaFreeHost(ho.streams);
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
     if (plan_ev) cudaEventSynchronize(plan_ev);
@@ -254,6 +269,8 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
   if (rc != NGAP_OK) return rc;
   build_filters(t->tiles);
   t->num_groups = (int)g->gs.groups.size();
+  for (const GroupGraph& gg : g->gs.groups)
+    t->sid_bits = std::max(t->sid_bits, bits_for(std::max<uint64_t>(gg.attrs.size(), 1)));
   for (auto& th : t->tiles) {
     if (th.nstates >= kMaxTileStates - 1) {
       set_error("a connected component has %d states; at most %d are supported per tile",
@@ -348,13 +365,16 @@ int ngap_engine_create(int device, ngap_engine** out) {
   e->device = device;
   CUDA_TRY(cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, device));
   CUDA_TRY(cudaMalloc(&e->d_counters, kNumCounters * sizeof(unsigned long long)));
-  CUDA_TRY(cudaFuncSetAttribute(small_sort_unique<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  CUDA_TRY(cudaMemset(e->d_counters, 0, kNumCounters * sizeof(unsigned long long)));
+  CUDA_TRY(cudaFuncSetAttribute(sort_unique_cta<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSmallSortSmem));
-  CUDA_TRY(cudaFuncSetAttribute(small_sort_unique<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  CUDA_TRY(cudaFuncSetAttribute(sort_unique_cta<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSmallSortSmem));
-  CUDA_TRY(cudaMalloc(&e->d_err, sizeof(int)));
-  CUDA_TRY(cudaMalloc(&e->d_unit_counter, sizeof(unsigned int)));
-  CUDA_TRY(cudaMallocHost(&e->h_counters, kNumCounters * sizeof(unsigned long long)));
+  CUDA_TRY(cudaMallocHost(&e->ho.counters, kNumCounters * sizeof(unsigned long long)));
+  CUDA_TRY(cudaMallocHost(&e->ho.reports, kHostReports * sizeof(uint64_t)));
+  CUDA_TRY(cudaMallocHost(&e->ho.streams, kHostReports * sizeof(uint32_t)));
+  std::memset(e->ho.counters, 0, kNumCounters * sizeof(unsigned long long));
+  e->ho.d_counters = e->d_counters;
   for (auto& ev : e->ev) CUDA_TRY(cudaEventCreate(&ev));
   *out = e.release();
   return NGAP_OK;
@@ -442,7 +462,7 @@ int ensure_reports(ngap_engine* e, uint64_t cap) {
   CUDA_TRY(cudaMalloc(&e->d_tmp, cap * sizeof(uint64_t)));
   CUDA_TRY(cudaMalloc(&e->d_unique, cap * sizeof(uint64_t)));
   size_t ntiles = (cap + kSortTile - 1) / kSortTile;
-  e->hist_cap = 16 * ntiles + 16;
+  e->hist_cap = kDigits * ntiles + kDigits;
   CUDA_TRY(cudaMalloc(&e->d_hist, e->hist_cap * sizeof(uint32_t)));
   e->rep_cap = cap;
   return NGAP_OK;
@@ -746,7 +766,6 @@ int launch_grid(int64_t nunits, int grid) {
 // tiles without sticky states in the lean kernel instance; then the rest
 // (the layered tiles read what the first launch recorded).
 int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
-  mp.unit_cursor = e->d_unit_counter;
   if (e->act_entries > 0)
     CUDA_TRY(cudaMemsetAsync(e->d_act, 0xff, (size_t)e->act_entries * sizeof(uint32_t), st));
   auto run = [&](bool lean, int which) -> int {
@@ -754,7 +773,7 @@ int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
     mp.unit_begin = e->ranges.begin[which];
     mp.nunits = e->ranges.count[which];
     mp.one_tile = e->ranges.one_tile[which];
-    CUDA_TRY(cudaMemsetAsync(e->d_unit_counter, 0, sizeof(unsigned int), st));
+    mp.unit_cursor = reinterpret_cast<unsigned int*>(e->d_counters + kCursors + which);
     const int grid = launch_grid(mp.nunits, e->grid);
     if (lean)
       match_kernel<true><<<grid, kCtaThreads, smem, st>>>(mp);
@@ -831,7 +850,7 @@ int blocks_per_sm(ngap_engine* e, int smem, int* out) {
 // reports at d_out (and stream indices at d_out_stream for MODE 1).
 //   MODE 0: keys offset << 32 | id, written as id << 32 | offset;
 //   MODE 1: keys stream << sshift | offset << oshift | id (batched matching).
-// shifts: the 4-bit digits the radix pipeline sorts, least significant first.
+// shifts: the digits the radix pipeline sorts, least significant first.
 struct SortJob {
   int mode;
   uint64_t* d_in;
@@ -844,7 +863,7 @@ struct SortJob {
   unsigned long long* d_unique_n;
 };
 
-// The radix pipeline over *radix_n keys; kernels counts its launches.
+// The radix pipeline over *radix_n keys; adds its launches to *kernels.
 int radix_chain(ngap_engine* e, const SortJob& j, const unsigned long long* radix_n,
                 cudaStream_t st, int* kernels) {
   const uint32_t max_tiles = (uint32_t)((j.cap + kSortTile - 1) / kSortTile);
@@ -852,53 +871,70 @@ int radix_chain(ngap_engine* e, const SortJob& j, const unsigned long long* radi
   // ping-pong between d_in (an engine-owned buffer) and d_tmp
   uint64_t* src = j.d_in;
   uint64_t* dst = e->d_tmp;
-  int k = 0;
+  uint32_t* totals = e->d_hist + e->hist_cap - kDigits;
   for (int sh : j.shifts) {
     radix_hist<<<grid, kSortThreads, 0, st>>>(src, radix_n, j.cap, sh, e->d_hist);
-    scan_exclusive_1block<<<1, kScanThreads, 0, st>>>(e->d_hist, radix_n, j.cap, 16, nullptr);
-    radix_scatter<<<grid, kSortThreads, 0, st>>>(src, dst, radix_n, j.cap, sh, e->d_hist);
-    k += 3;
+    radix_scan<<<kDigits, kSortThreads, 0, st>>>(e->d_hist, radix_n, j.cap, totals);
+    radix_scatter<<<grid, kSortThreads, 0, st>>>(src, dst, radix_n, j.cap, sh, e->d_hist, totals);
+    *kernels += 3;
     std::swap(src, dst);
   }
   unique_count<<<grid, kSortThreads, 0, st>>>(src, radix_n, j.cap, e->d_hist);
-  scan_exclusive_1block<<<1, kScanThreads, 0, st>>>(e->d_hist, radix_n, j.cap, 1, j.d_unique_n);
+  scan_exclusive_1block<<<1, kScanThreads, 0, st>>>(e->d_hist, radix_n, j.cap, j.d_unique_n);
   if (j.mode == 0)
-    unique_write<<<grid, kSortThreads, 0, st>>>(src, radix_n, j.cap, e->d_hist, j.d_out);
+    unique_write<0><<<grid, kSortThreads, 0, st>>>(src, radix_n, j.cap, e->d_hist, j.oshift, j.sshift,
+                                                   j.d_out, nullptr);
   else
-    unique_write_fields<<<grid, kSortThreads, 0, st>>>(src, radix_n, j.cap, e->d_hist, j.oshift,
-                                                       j.sshift, j.d_out, j.d_out_stream);
-  k += 3;
-  *kernels = k;
+    unique_write<1><<<grid, kSortThreads, 0, st>>>(src, radix_n, j.cap, e->d_hist, j.oshift, j.sshift,
+                                                   j.d_out, j.d_out_stream);
+  *kernels += 3;
   CUDA_TRY(cudaGetLastError());
   return NGAP_OK;
 }
 
-void* small_kernel(int mode) {
-  return mode == 0 ? reinterpret_cast<void*>(small_sort_unique<0>)
-                   : reinterpret_cast<void*>(small_sort_unique<1>);
+// Last kernel of a match whose reports went through the radix pipeline.
+int publish(ngap_engine* e, const SortJob& j, cudaStream_t st, int* kernels) {
+  publish_results<<<1, kHostReports, 0, st>>>(e->ho, j.d_unique_n, j.d_out, j.d_out_stream);
+  *kernels += 1;
+  CUDA_TRY(cudaGetLastError());
+  return NGAP_OK;
 }
 
-// Builds the graph: the small-set kernel, then the radix pipeline in the body
-// of a conditional (IF) node whose condition the small-set kernel sets when
-// it leaves keys to the pipeline.
+// The one-CTA sort. alone: it handles any number of keys (no pipeline follows).
+int cta_sort(ngap_engine* e, const SortJob& j, bool alone, const HostOut& ho, cudaStream_t st) {
+  unsigned long long* radix_n = e->d_counters + kRadixCount;
+  const cudaGraphConditionalHandle none = 0;
+  if (j.mode == 0)
+    sort_unique_cta<0><<<1, kSmallThreads, kSmallSortSmem, st>>>(
+        j.d_in, e->d_tmp, j.d_n, j.cap, radix_n, j.d_unique_n, j.oshift, j.sshift, j.d_out,
+        j.d_out_stream, none, 0, alone, ho);
+  else
+    sort_unique_cta<1><<<1, kSmallThreads, kSmallSortSmem, st>>>(
+        j.d_in, e->d_tmp, j.d_n, j.cap, radix_n, j.d_unique_n, j.oshift, j.sshift, j.d_out,
+        j.d_out_stream, none, 0, alone, ho);
+  CUDA_TRY(cudaGetLastError());
+  e->launches++;
+  return NGAP_OK;
+}
+
+// Builds the graph: the one-CTA sort, then the radix pipeline in the body of a
+// conditional (IF) node whose condition the first kernel sets when it leaves
+// keys to the pipeline.
 int build_sort_graph(ngap_engine* e, const SortJob& j, SortGraph& sg) {
   if (!e->sort_cs) CUDA_TRY(cudaStreamCreateWithFlags(&e->sort_cs, cudaStreamNonBlocking));
   CUDA_TRY(cudaGraphCreate(&sg.g, 0));
   cudaGraphConditionalHandle h = 0;
   CUDA_TRY(cudaGraphConditionalHandleCreate(&h, sg.g, 0, cudaGraphCondAssignDefault));
   unsigned long long* radix_n = e->d_counters + kRadixCount;
-  uint64_t* d_in = j.d_in;
-  const unsigned long long* d_n = j.d_n;
-  uint64_t cap = j.cap;
-  unsigned long long* d_unique_n = j.d_unique_n;
-  int oshift = j.oshift, sshift = j.sshift;
-  uint64_t* d_out = j.d_out;
-  uint32_t* d_out_stream = j.d_out_stream;
-  int set_cond = 1;
-  void* args[] = {&d_in, &d_n, &cap, &radix_n, &d_unique_n, &oshift, &sshift, &d_out,
-                  &d_out_stream, &h, &set_cond};
+  SortJob a = j;  // kernel arguments
+  uint64_t* d_tmp = e->d_tmp;
+  int set_cond = 1, alone = 0;
+  HostOut ho = e->ho;
+  void* args[] = {&a.d_in, &d_tmp, &a.d_n, &a.cap, &radix_n, &a.d_unique_n, &a.oshift, &a.sshift,
+                  &a.d_out, &a.d_out_stream, &h, &set_cond, &alone, &ho};
   cudaKernelNodeParams kp = {};
-  kp.func = small_kernel(j.mode);
+  kp.func = j.mode == 0 ? reinterpret_cast<void*>(sort_unique_cta<0>)
+                        : reinterpret_cast<void*>(sort_unique_cta<1>);
   kp.gridDim = dim3(1);
   kp.blockDim = dim3(kSmallThreads);
   kp.sharedMemBytes = kSmallSortSmem;
@@ -915,7 +951,8 @@ int build_sort_graph(ngap_engine* e, const SortJob& j, SortGraph& sg) {
   CUDA_TRY(cudaStreamBeginCaptureToGraph(e->sort_cs, body, nullptr, nullptr, 0,
                                          cudaStreamCaptureModeThreadLocal));
   int kernels = 0;
-  const int rc = radix_chain(e, j, radix_n, e->sort_cs, &kernels);
+  int rc = radix_chain(e, j, radix_n, e->sort_cs, &kernels);
+  if (rc == NGAP_OK) rc = publish(e, j, e->sort_cs, &kernels);
   cudaGraph_t captured = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(e->sort_cs, &captured);
   if (rc != NGAP_OK) return rc;
@@ -925,11 +962,21 @@ int build_sort_graph(ngap_engine* e, const SortJob& j, SortGraph& sg) {
   return NGAP_OK;
 }
 
-// Enqueues a sort on st. Outside stream capture it replays a cached graph
-// (one launch; the radix pipeline runs only for more than kSmallSort keys);
-// inside a capture, or where graphs are unavailable, it launches the small-set
-// kernel and the pipeline, whose kernels find no keys after a small set.
-int sort_reports(ngap_engine* e, const SortJob& j, cudaStream_t st) {
+// Inputs of at most this many positions sort their reports with the one-CTA
+// kernel alone, launched directly: a launch with a conditional graph costs 7
+// us more on a B200 (29 against 22 us for an empty pipeline), and one CTA keeps
+// up with the pipeline (about 60 us) to some 30,000 reports, an eighth of the
+// positions. Longer inputs may hold millions.
+constexpr uint64_t kAloneInput = 1ull << 18;
+
+// Enqueues the sort of a match's reports on st, the match's last kernels: they
+// leave its counters and first reports for the host. For inputs beyond
+// kAloneInput, outside stream capture, it replays a cached graph (one launch; the
+// radix pipeline runs only for more than kSmallSort keys); inside a
+// capture, or where graphs are unavailable, it launches the one-CTA kernel and
+// the pipeline, whose kernels find no keys after a small set.
+int sort_reports(ngap_engine* e, const SortJob& j, uint64_t positions, cudaStream_t st) {
+  if (positions <= kAloneInput) return cta_sort(e, j, true, e->ho, st);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(st, &cs));
   if (cs == cudaStreamCaptureStatusNone && !e->sort_graph_off) {
@@ -967,45 +1014,36 @@ int sort_reports(ngap_engine* e, const SortJob& j, cudaStream_t st) {
       return NGAP_OK;
     }
   }
-  unsigned long long* radix_n = e->d_counters + kRadixCount;
-  const cudaGraphConditionalHandle none = 0;
-  const int set_cond = 0;
-  if (j.mode == 0)
-    small_sort_unique<0><<<1, kSmallThreads, kSmallSortSmem, st>>>(
-        j.d_in, j.d_n, j.cap, radix_n, j.d_unique_n, j.oshift, j.sshift, j.d_out, j.d_out_stream,
-        none, set_cond);
-  else
-    small_sort_unique<1><<<1, kSmallThreads, kSmallSortSmem, st>>>(
-        j.d_in, j.d_n, j.cap, radix_n, j.d_unique_n, j.oshift, j.sshift, j.d_out, j.d_out_stream,
-        none, set_cond);
+  int rc = cta_sort(e, j, false, HostOut(), st);
   int kernels = 0;
-  const int rc = radix_chain(e, j, radix_n, st, &kernels);
-  e->launches += 1 + kernels;
+  if (rc == NGAP_OK) rc = radix_chain(e, j, e->d_counters + kRadixCount, st, &kernels);
+  if (rc == NGAP_OK) rc = publish(e, j, st, &kernels);
+  e->launches += kernels;
   return rc;
 }
 
-// Sorts d_in[0 .. *d_n) (clamped to cap) into d_out as unique reference-encoded
-// reports; *d_unique_n receives the count. off_bits / id_bits bound the key.
-int sort_unique(ngap_engine* e, uint64_t* d_in, const unsigned long long* d_n, uint64_t cap,
-                int off_bits, int id_bits, uint64_t* d_out, unsigned long long* d_unique_n,
-                cudaStream_t st) {
-  SortJob j{0, d_in, d_n, cap, {}, 32, 64, d_out, nullptr, d_unique_n};
-  for (int b = 0; b < id_bits; b += 4) j.shifts.push_back(b);
-  for (int b = 0; b < off_bits; b += 4) j.shifts.push_back(32 + b);
-  return sort_reports(e, j, st);
+// Zeroes the counters when an earlier match was left half enqueued (otherwise
+// its last kernel did), and marks them until this match is enqueued whole.
+int begin_counters(ngap_engine* e, cudaStream_t st) {
+  if (e->counters_dirty)
+    CUDA_TRY(cudaMemsetAsync(e->d_counters, 0, kNumCounters * sizeof(unsigned long long), st));
+  e->counters_dirty = true;
+  return NGAP_OK;
 }
 
-// Batched keys stream << sshift | offset << oshift | id: radix passes over the
-// three fields, then unique reports and their stream indices.
-int sort_unique_fields(ngap_engine* e, const unsigned long long* d_n, uint64_t cap, int ibits,
-                       int oshift, int obits, int sshift, int sbits,
-                       unsigned long long* d_unique_n, cudaStream_t st) {
-  SortJob j{1, e->d_reports, d_n, cap, {}, oshift, sshift, e->d_unique, e->d_stream_ids,
-            d_unique_n};
-  for (int b = 0; b < ibits; b += 4) j.shifts.push_back(b);
-  for (int b = 0; b < obits; b += 4) j.shifts.push_back(oshift + b);
-  for (int b = 0; b < sbits; b += 4) j.shifts.push_back(sshift + b);
-  return sort_reports(e, j, st);
+// Copies the first n reports (and stream indices) of the last match to the host.
+cudaError_t copy_results(const ngap_engine* e, uint64_t n, uint64_t* reports, uint32_t* streams) {
+  if (n <= (uint64_t)kHostReports) {  // left in pinned memory by the match
+    std::memcpy(reports, e->ho.reports, n * sizeof(uint64_t));
+    if (streams) std::memcpy(streams, e->ho.streams, n * sizeof(uint32_t));
+    return cudaSuccess;
+  }
+  cudaError_t ce = cudaSetDevice(e->device);
+  if (ce == cudaSuccess)
+    ce = cudaMemcpy(reports, e->d_unique, n * sizeof(uint64_t), cudaMemcpyDeviceToHost);
+  if (ce == cudaSuccess && streams)
+    ce = cudaMemcpy(streams, e->d_stream_ids, n * sizeof(uint32_t), cudaMemcpyDeviceToHost);
+  return ce;
 }
 
 // --algorithm -> prefix depth. The blocking algorithm scans the always-active
@@ -1128,13 +1166,11 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   rc = ensure_slots(e, (size_t)full_grid * kWarpsPerCta, t->max_states, t->max_nact, kDefaultQueue);
   if (rc != NGAP_OK) return rc;
 
-  CUDA_TRY(cudaEventRecord(e->ev[0], st));
   if (input_on_device)
     CUDA_TRY(cudaMemcpyAsync(e->d_input, input, total, cudaMemcpyDeviceToDevice, st));
   else
     CUDA_TRY(cudaMemcpyAsync(e->d_input, input, total, cudaMemcpyHostToDevice, st));
-  CUDA_TRY(cudaMemsetAsync(e->d_counters, 0, 8 * sizeof(unsigned long long), st));
-  CUDA_TRY(cudaMemsetAsync(e->d_err, 0, sizeof(int), st));
+  if ((rc = begin_counters(e, st)) != NGAP_OK) return rc;
 
   MatchParams mp;
   mp.tiles = t->d_tiles;
@@ -1148,7 +1184,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   mp.rep_count = e->d_counters + 0;
   mp.reports = e->d_reports;
   mp.rep_cap = cap;
-  mp.err = e->d_err;
+  mp.err = reinterpret_cast<int*>(e->d_counters + 4);
   mp.carry = e->d_carry;
   mp.marks = e->d_marks;
   mp.ovf = e->d_ovf;
@@ -1174,18 +1210,19 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   }
   CUDA_TRY(cudaEventRecord(e->ev[2], st));
   if (!p->report_off) {
-    int off_bits = bits_for(total);
-    int id_bits = 22 + bits_for((uint64_t)std::max(t->num_groups, 1));
-    rc = sort_unique(e, e->d_reports, e->d_counters + 0, cap, off_bits, id_bits, e->d_unique,
-                     e->d_counters + 1, st);
-    if (rc != NGAP_OK) return rc;
+    const uint64_t bits = bit_range(0, t->sid_bits) |
+                          bit_range(22, bits_for((uint64_t)std::max(t->num_groups, 1))) |
+                          bit_range(32, bits_for(total));
+    const SortJob job{0,  e->d_reports, e->d_counters + 0, cap,     digits_of(bits),
+                      32, 64,           e->d_unique,       nullptr, e->d_counters + 1};
+    if ((rc = sort_reports(e, job, total, st)) != NGAP_OK) return rc;
+  } else {
+    publish_kernel<<<1, 32, 0, st>>>(e->ho);
+    CUDA_TRY(cudaGetLastError());
+    e->launches++;
   }
   CUDA_TRY(cudaEventRecord(e->ev[3], st));
-  CUDA_TRY(cudaMemcpyAsync(e->h_counters, e->d_counters, 4 * sizeof(unsigned long long),
-                           cudaMemcpyDeviceToHost, st));
-  CUDA_TRY(cudaMemcpyAsync(e->h_counters + 4, e->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CUDA_TRY(cudaMemcpyAsync(e->h_counters + kRadixCount, e->d_counters + kRadixCount,
-                           sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  e->counters_dirty = false;
   e->ran = true;
   return NGAP_OK;
 }
@@ -1199,10 +1236,10 @@ int ngap_engine_sync(ngap_engine* e) {
   CUDA_TRY(cudaStreamSynchronize(e->stream));
   CUDA_TRY(cudaEventElapsedTime(&e->match_ms, e->ev[1], e->ev[2]));
   CUDA_TRY(cudaEventElapsedTime(&e->sort_ms, e->ev[2], e->ev[3]));
-  if (e->sort_chain_pending > 0 && e->h_counters[kRadixCount] > 0)  // the radix pipeline ran
+  if (e->sort_chain_pending > 0 && e->ho.counters[kRadixCount] > 0)  // the radix pipeline ran
     e->launches += e->sort_chain_pending;
   e->sort_chain_pending = 0;
-  int err = (int)(e->h_counters[4] & 0xffffffffull);
+  int err = (int)(e->ho.counters[4] & 0xffffffffull);
   if (err & kErrTimeout) {
     set_error("a bounded device wait gave up; results are incomplete");
     return NGAP_E_TIMEOUT;
@@ -1213,7 +1250,7 @@ int ngap_engine_sync(ngap_engine* e) {
   }
   if (err & kErrResults) {
     set_error("%llu reports exceed the result capacity of %llu; results are truncated",
-              (unsigned long long)e->h_counters[0], (unsigned long long)e->rep_cap);
+              (unsigned long long)e->ho.counters[0], (unsigned long long)e->rep_cap);
     return NGAP_E_OVERFLOW_RESULTS;
   }
   return NGAP_OK;
@@ -1221,8 +1258,8 @@ int ngap_engine_sync(ngap_engine* e) {
 
 int ngap_results_count(const ngap_engine* e, uint64_t* raw, uint64_t* unique) {
   if (!e) return NGAP_E_INVALID;
-  if (raw) *raw = e->h_counters[0];
-  if (unique) *unique = e->h_counters[1];
+  if (raw) *raw = e->ho.counters[0];
+  if (unique) *unique = e->ho.counters[1];
   return NGAP_OK;
 }
 
@@ -1230,10 +1267,9 @@ const uint64_t* ngap_results_device(const ngap_engine* e) { return e ? e->d_uniq
 
 int64_t ngap_results_copy(ngap_engine* e, uint64_t* host, uint64_t cap) {
   if (!e || !host) return -1;
-  uint64_t n = std::min<uint64_t>(e->h_counters[1], cap);
+  uint64_t n = std::min<uint64_t>(e->ho.counters[1], cap);
   if (n == 0) return 0;
-  if (cudaSetDevice(e->device) != cudaSuccess) return -1;
-  cudaError_t ce = cudaMemcpy(host, e->d_unique, n * sizeof(uint64_t), cudaMemcpyDeviceToHost);
+  cudaError_t ce = copy_results(e, n, host, nullptr);
   if (ce != cudaSuccess) {
     set_error("cudaMemcpy: %s", cudaGetErrorString(ce));
     return -1;
@@ -1252,8 +1288,8 @@ int ngap_last_launches(const ngap_engine* e) { return e ? e->launches : 0; }
 
 int ngap_engine_work(const ngap_engine* e, uint64_t* expanded, uint64_t* injected) {
   if (!e) return NGAP_E_INVALID;
-  if (expanded) *expanded = e->h_counters[2];
-  if (injected) *injected = e->h_counters[3];
+  if (expanded) *expanded = e->ho.counters[2];
+  if (injected) *injected = e->ho.counters[3];
   return NGAP_OK;
 }
 
@@ -1374,7 +1410,11 @@ int ngap_reports_sort_unique(ngap_engine* e, const uint64_t* d_in, uint64_t n, u
   CUDA_TRY(cudaMemcpyAsync(e->d_counters + 5, &hn, sizeof(hn), cudaMemcpyHostToDevice, st));
   swap_halves<<<std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, 4096)), 256, 0, st>>>(e->d_reports, n);
   CUDA_TRY(cudaGetLastError());
-  rc = sort_unique(e, e->d_reports, e->d_counters + 5, n, 32, 32, d_out, e->d_counters + 6, st);
+  const SortJob job{0,  e->d_reports, e->d_counters + 5, n,       digits_of(~0ull),
+                    32, 64,           d_out,             nullptr, e->d_counters + 6};
+  int kernels = 0;
+  rc = n <= (uint64_t)kSmallSort ? cta_sort(e, job, true, HostOut(), st)
+                                 : radix_chain(e, job, job.d_n, st, &kernels);
   if (rc != NGAP_OK) return rc;
   unsigned long long un = 0;
   CUDA_TRY(cudaMemcpyAsync(&un, e->d_counters + 6, sizeof(un), cudaMemcpyDeviceToHost, st));
@@ -1394,6 +1434,7 @@ struct ngap_tableset {
   std::vector<const ngap_tables*> tables;
   std::vector<int> tile_base;  // first tile of each NFA in the combined descriptor array
   TileDev* d_tiles = nullptr;
+  int sid_bits = 0;
   int ntiles = 0, max_states = 0, max_groups = 1, max_depth = 1, device = 0;
   int max_nact = 0;
   std::vector<char> tile_lean;      // per tile of the combined array (ngap_tables::tile_lean)
@@ -1422,6 +1463,7 @@ int ngap_tableset_create(const ngap_tables* const* tables, int n, ngap_tableset*
     ts->tile_lean.insert(ts->tile_lean.end(), t->tile_lean.begin(), t->tile_lean.end());
     ts->max_states = std::max(ts->max_states, t->max_states);
     ts->max_groups = std::max(ts->max_groups, t->num_groups);
+    ts->sid_bits = std::max(ts->sid_bits, t->sid_bits);
     ts->max_nact = std::max(ts->max_nact, t->max_nact);
     for (auto& th : t->tiles) ts->max_depth = std::max(ts->max_depth, th.depth);
   }
@@ -1594,7 +1636,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   mp.rep_count = e->d_counters + 0;
   mp.reports = e->d_reports;
   mp.rep_cap = cap;
-  mp.err = e->d_err;
+  mp.err = reinterpret_cast<int*>(e->d_counters + 4);
   mp.carry = e->d_carry;
   mp.marks = e->d_marks;
   mp.ovf = e->d_ovf;
@@ -1621,23 +1663,22 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
       CUDA_TRY(cudaMemcpyAsync(e->d_input, input, input_bytes, cudaMemcpyDeviceToDevice, qs));
     else
       CUDA_TRY(cudaMemcpyAsync(e->d_input, input, input_bytes, cudaMemcpyHostToDevice, qs));
-    CUDA_TRY(cudaMemsetAsync(e->d_counters, 0, 8 * sizeof(unsigned long long), qs));
-    CUDA_TRY(cudaMemsetAsync(e->d_err, 0, sizeof(int), qs));
     int r = NGAP_OK;
     if (e->nunits > 0) {
       r = launch_plan(e, mp, smem, qs);
       if (r != NGAP_OK) return r;
     }
     if (!p->report_off) {
-      r = sort_unique_fields(e, e->d_counters + 0, cap, ibits, oshift, obits, sshift, sbits,
-                             e->d_counters + 1, qs);
-      if (r != NGAP_OK) return r;
+      const uint64_t bits = bit_range(0, ts->sid_bits) | bit_range(22, ibits - 22) |
+                            bit_range(oshift, obits) | bit_range(sshift, sbits);
+      const SortJob job{1,      e->d_reports, e->d_counters + 0, cap,             digits_of(bits),
+                        oshift, sshift,       e->d_unique,       e->d_stream_ids, e->d_counters + 1};
+      if ((r = sort_reports(e, job, input_bytes, qs)) != NGAP_OK) return r;
+    } else {
+      publish_kernel<<<1, 32, 0, qs>>>(e->ho);
+      CUDA_TRY(cudaGetLastError());
+      e->launches++;
     }
-    CUDA_TRY(cudaMemcpyAsync(e->h_counters, e->d_counters, 4 * sizeof(unsigned long long),
-                             cudaMemcpyDeviceToHost, qs));
-    CUDA_TRY(cudaMemcpyAsync(e->h_counters + 4, e->d_err, sizeof(int), cudaMemcpyDeviceToHost, qs));
-    CUDA_TRY(cudaMemcpyAsync(e->h_counters + kRadixCount, e->d_counters + kRadixCount,
-                             sizeof(unsigned long long), cudaMemcpyDeviceToHost, qs));
     return NGAP_OK;
   };
 
@@ -1645,9 +1686,10 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   e->sort_chain_pending = 0;
   if (!p->use_graph) {
     e->graph_mode = false;
-    CUDA_TRY(cudaEventRecord(e->ev[0], st));
     CUDA_TRY(cudaEventRecord(e->ev[1], st));
+    if ((rc = begin_counters(e, st)) != NGAP_OK) return rc;
     if ((rc = enqueue(st)) != NGAP_OK) return rc;
+    e->counters_dirty = false;
     CUDA_TRY(cudaEventRecord(e->ev[2], st));
     CUDA_TRY(cudaEventRecord(e->ev[3], st));
     e->ran = true;
@@ -1699,9 +1741,10 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   e->launches = e->graph_launches;
   CUDA_TRY(cudaEventRecord(e->cap_ev[0], st));  // after the caller's prior work
   CUDA_TRY(cudaStreamWaitEvent(cs, e->cap_ev[0], 0));
-  CUDA_TRY(cudaEventRecord(e->ev[0], cs));
   CUDA_TRY(cudaEventRecord(e->ev[1], cs));
+  if ((rc = begin_counters(e, cs)) != NGAP_OK) return rc;
   CUDA_TRY(cudaGraphLaunch(e->graph, cs));
+  e->counters_dirty = false;
   CUDA_TRY(cudaEventRecord(e->ev[2], cs));
   CUDA_TRY(cudaEventRecord(e->ev[3], cs));
   CUDA_TRY(cudaEventRecord(e->cap_ev[1], cs));  // the caller's later work waits for the graph
@@ -1717,13 +1760,10 @@ int ngap_batch_results(ngap_engine* e, uint64_t* reports, uint32_t* stream_ids, 
     set_error("ngap_batch_results: null argument");
     return NGAP_E_INVALID;
   }
-  const uint64_t k = std::min<uint64_t>(e->h_counters[1], cap);
+  const uint64_t k = std::min<uint64_t>(e->ho.counters[1], cap);
   *n = 0;
   if (k == 0) return NGAP_OK;
-  CUDA_TRY(cudaSetDevice(e->device));
-  CUDA_TRY(cudaMemcpy(reports, e->d_unique, k * sizeof(uint64_t), cudaMemcpyDeviceToHost));
-  if (stream_ids)
-    CUDA_TRY(cudaMemcpy(stream_ids, e->d_stream_ids, k * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+  CUDA_TRY(copy_results(e, k, reports, stream_ids));
   *n = k;
   return NGAP_OK;
 }
@@ -1751,7 +1791,7 @@ namespace {
 constexpr uint64_t kNoAllocMaxReports = 1ull << 18;  // 262,144 reports
 constexpr uint64_t kNoAllocTiles = (kNoAllocMaxReports + kSortTile - 1) / kSortTile;
 constexpr size_t kNoAllocKeyBytes = kNoAllocMaxReports * sizeof(uint64_t);
-constexpr size_t kNoAllocHistBytes = 16 * kNoAllocTiles * sizeof(uint32_t);
+constexpr size_t kNoAllocHistBytes = (kDigits * kNoAllocTiles + kDigits) * sizeof(uint32_t);
 constexpr size_t kNoAllocBytes = kNoAllocKeyBytes + kNoAllocHistBytes + 4 * sizeof(unsigned long long);
 
 static __device__ __align__(256) uint8_t g_noalloc_scratch[kNoAllocBytes];
@@ -1862,23 +1902,23 @@ extern "C" int ngap_reports_sort_unique_noalloc(const uint64_t* d_in, uint64_t n
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const uint32_t tiles = (uint32_t)((n + kSortTile - 1) / kSortTile);
   const int grid = (int)std::max<uint32_t>(1, std::min<uint32_t>(tiles, (uint32_t)sms * 8));
-  // 8 digit passes over the offset half and 8 over the id half; an even count
+  // 4 digit passes over the id half and 4 over the offset half; an even count
   // leaves the sorted keys back in the scratch buffer, d_out being the other
   // half of the ping-pong
-  const int npass = 16;
-  uint64_t* src = (npass % 2 == 0) ? keys : d_out;
-  uint64_t* dst = (npass % 2 == 0) ? d_out : keys;
+  const std::vector<int> shifts = digits_of(~0ull);
+  uint32_t* totals = hist + kDigits * kNoAllocTiles;
+  uint64_t* src = (shifts.size() % 2 == 0) ? keys : d_out;
+  uint64_t* dst = (shifts.size() % 2 == 0) ? d_out : keys;
   noalloc_prepare<<<grid, 256, 0, st>>>(d_in, n, src, counters);
-  for (int k = 0; k < npass; k++) {
-    const int sh = k < 8 ? 4 * k : 32 + 4 * (k - 8);
+  for (int sh : shifts) {
     radix_hist<<<grid, kSortThreads, 0, st>>>(src, counters, n, sh, hist);
-    scan_exclusive_1block<<<1, kScanThreads, 0, st>>>(hist, counters, n, 16, nullptr);
-    radix_scatter<<<grid, kSortThreads, 0, st>>>(src, dst, counters, n, sh, hist);
+    radix_scan<<<kDigits, kSortThreads, 0, st>>>(hist, counters, n, totals);
+    radix_scatter<<<grid, kSortThreads, 0, st>>>(src, dst, counters, n, sh, hist, totals);
     std::swap(src, dst);
   }
   unique_count<<<grid, kSortThreads, 0, st>>>(src, counters, n, hist);
-  scan_exclusive_1block<<<1, kScanThreads, 0, st>>>(hist, counters, n, 1, counters + 1);
-  unique_write<<<grid, kSortThreads, 0, st>>>(src, counters, n, hist, d_out);
+  scan_exclusive_1block<<<1, kScanThreads, 0, st>>>(hist, counters, n, counters + 1);
+  unique_write<0><<<grid, kSortThreads, 0, st>>>(src, counters, n, hist, 32, 64, d_out, nullptr);
   CUDA_TRY(cudaGetLastError());
   unsigned long long un = 0;
   CUDA_TRY(cudaMemcpyAsync(&un, counters + 1, sizeof(un), cudaMemcpyDeviceToHost, st));
