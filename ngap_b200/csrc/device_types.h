@@ -79,13 +79,16 @@ struct FilterDev {
 // matched by one warp per unit. Its hot tables form one contiguous image, read
 // in place through L1 and L2:
 //   [succ][cmask: nstates x cw x u32][rep: ceil(nstates/32) x u32][cls: 256 B]
-// succ: up to 4 tile-local successors per state; narrow tiles (< 32767
-// states) store 4 x u16 (bit 15 = report successor, 0xffff = none), wide
-// ones 4 x u32 (bit 31 = report successor, kNoSucc = none); fused wide tiles
-// (one class word) follow each state's 4 x u32 with its successors' class
-// masks (4 x u32, 0 for none), a 32-byte record. cmask: bit c of
-// word c/32 = the state accepts byte class c. cls: byte -> class id, live
-// classes first, the dead class (bytes no state accepts) last.
+// succ: a 32-byte record per state, so that an expansion is one read: up to 4
+// tile-local successors (u32, bit 31 = report successor, kNoSucc = none), then
+// for each what it accepts: its class mask in tiles of at most 32 classes (0 for
+// none), otherwise the one class it accepts, kNoClass for none or
+// kManyClasses (its mask is in cmask). cmask: bit c of word c/32 = the state
+// accepts byte class c. cls: byte -> class id, live classes first, the dead
+// class (bytes no state accepts) last.
+constexpr uint32_t kNoClass = 0xfffffffeu;
+constexpr uint32_t kManyClasses = 0xffffffffu;
+
 struct TileDev {
   int32_t group = 0;        // group of the first CC (report ids are in sid)
   int32_t nstates = 0;
@@ -96,8 +99,6 @@ struct TileDev {
   int32_t ncls = 0;         // byte classes
   int32_t cw = 8;           // class-mask words per state: ceil(classes / 32), 1..8
   int32_t nlive = 0;        // live classes: key base; class id nlive = dead
-  int32_t narrow = 1;       // 16-bit successors
-  int32_t fused = 0;        // wide, one class word: records of 2 x uint4 (successors, their masks)
   int32_t image_bytes = 0;  // multiple of 16
   int32_t off_cmask = 0, off_rep = 0, off_cls = 0;
   int32_t inj_batch = 32;   // positions injected per worklist refill (prefix tables)
@@ -112,6 +113,8 @@ struct TileDev {
   const uint32_t* sid = nullptr;    // [nstates] local -> report id (sid | group << 22)
   const uint32_t* aas = nullptr;    // [naas] local ids
   const uint32_t* start = nullptr;  // [nstart] local ids
+  int32_t run_len = 32;     // filter candidates per run
+  uint32_t rep_levels = 0;  // bit d: the depth-(d+1) table has report lists
   FilterDev filt;
   PrefixTableDev pt[kMaxDepth];
 };
@@ -132,6 +135,32 @@ struct UnitDev {
   int64_t act_row;   // phase 1 and 2 tiles: first activation slot of the unit's segment
   int32_t act_rowid; // its row (pair, segment) in the compacted activation lists
   int32_t stream;    // segment (plain matching) or stream (batched matching) index
+};
+
+// A piece of a filtered tile's work: the candidates among positions [lo, hi) of
+// a segment that ends at `end`. Reports are stored as in UnitDev.
+struct PieceDev {
+  int32_t tile;
+  uint32_t flags;     // bit0: inject start-of-data states at lo
+  uint32_t lo, hi, end;
+  uint32_t base;      // first byte of the piece's stream
+  uint64_t key_hi;
+  int64_t act_row;    // as in UnitDev
+  int32_t act_rowid;
+  int32_t pad;
+};
+
+// A run: n candidates of one piece, from cand[first], with what the piece says
+// (one read instead of two that depend on each other).
+struct alignas(16) RunDev {
+  uint32_t piece, first, n;
+  uint32_t starts;    // 1: inject the piece's start-of-data states too
+  int32_t tile;
+  uint32_t lo, end, base;
+  uint64_t key_hi;
+  int64_t act_row;
+  int32_t act_rowid;
+  int32_t pad[3];
 };
 
 }  // namespace ngap

@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -14,6 +15,7 @@
 #include "common.h"
 #include "handles.h"
 #include "match_kernel.cuh"
+#include "scan_kernel.cuh"
 #include "sort_kernels.cuh"
 #include "tables.h"
 
@@ -35,10 +37,14 @@ namespace {
 // of a match, HostOut): [0] raw reports, [1] unique reports, [2..3] work, [4]
 // error bits, [5..6] the standalone sort's counts, [kRadixCount] keys left to
 // the radix pipeline after the small-set sort, [kCursors ...] the unit cursors
-// of the three launches.
+// of the three launches, [kSliceCtl ...] the control words of the slices.
 constexpr int kDefaultQueue = 1 << 16;  // overflow-stack entries per warp
 constexpr int kRadixCount = 8;
 constexpr int kCursors = 10;
+constexpr int kSliceCtl = 16;
+constexpr int kSlotsPerSm = std::max(kWarpsPerCta, kRunWarps);  // warps with scratch of their own
+constexpr int kSliceSlots = 8;  // slices that run without zeroing control words in between
+static_assert(kSliceCtl * 8 + kSliceSlots * kCtlWords * 4 <= kNumCounters * 8, "counters");
 
 int bits_for(uint64_t x) {  // bits needed to hold values < x (x >= 1)
   int b = 0;
@@ -93,6 +99,7 @@ struct ngap_tables {
   int64_t bytes = 0;
   int32_t max_states = 0;
   std::vector<char> tile_lean;      // per tile: plain, no sticky states (the lean kernel runs it)
+  std::vector<int32_t> run_len;     // per tile: candidates per run
   std::vector<int32_t> pair_nact;  // activation slots of each (activation, layered) tile pair
   int32_t max_nact = 0;            // largest pair
 
@@ -118,16 +125,29 @@ struct UnitPlanKey {
   int64_t num_seg, seg_len;
   int is_dup, window, chunk;
   int64_t first_seg;
+  int depth;      // prefix depth of the algorithm
+  bool filtered;  // tiles with a filter may be scanned (off for the wait test hook)
   bool operator<(const UnitPlanKey& o) const {
-    return std::tie(num_seg, seg_len, is_dup, window, chunk, first_seg) <
-           std::tie(o.num_seg, o.seg_len, o.is_dup, o.window, o.chunk, o.first_seg);
+    return std::tie(num_seg, seg_len, is_dup, window, chunk, first_seg, depth, filtered) <
+           std::tie(o.num_seg, o.seg_len, o.is_dup, o.window, o.chunk, o.first_seg, o.depth,
+                    o.filtered);
   }
 };
 
-// Units of the three launches of a plan (make_units).
-struct UnitRanges {
+// Pieces scanned by one launch and matched by the next (make_slices).
+struct Slice {
+  int32_t begin, count;
+  int64_t runs;     // most runs they can give
+  bool layered;
+  int32_t one_tile; // the one tile of the pieces, or -1
+};
+
+// What the launches of a plan run: units of the three launches of
+// match_kernel (make_units) and slices of pieces (make_slices).
+struct PlanRanges {
   int32_t begin[3] = {0, 0, 0}, count[3] = {0, 0, 0};
   int32_t one_tile[3] = {-1, -1, -1};  // the one tile of a launch's units, or -1
+  std::vector<Slice> slices;
 };
 
 struct ngap_engine {
@@ -139,12 +159,18 @@ struct ngap_engine {
   size_t input_cap = 0;
   // units (cached plan for one tables object)
   uint64_t plan_tables = 0;  // serial of the tables the plain plan was made for
-  UnitPlanKey plan_key{-1, -1, -1, -1, -1, -1};
+  UnitPlanKey plan_key{-1, -1, -1, -1, -1, -1, -1, true};
   UnitDev* d_units = nullptr;
   size_t units_cap = 0;
   int32_t nunits = 0;
   int64_t longest_unit = 0;  // positions of the plan's longest unit
-  UnitRanges ranges;
+  PlanRanges ranges;
+  PieceDev* d_pieces = nullptr;  // pieces of filtered tiles (trace records follow the units')
+  size_t pieces_cap = 0;
+  uint16_t* d_cand = nullptr;    // candidates and runs of one slice
+  int64_t cand_cap = 0;
+  RunDev* d_runs = nullptr;
+  int64_t runs_cap = 0;
   // worklist traces
   bool trace = false;
   unsigned long long* d_unit_work = nullptr;
@@ -195,7 +221,7 @@ struct ngap_engine {
   // batched matching
   uint64_t batch_ts = 0;     // serial of the tableset the batched plan was made for
   std::vector<ngap_batch_stream> batch_streams;
-  int batch_window = -1, batch_chunk = -1;
+  int batch_window = -1, batch_chunk = -1, batch_depth = -1;
   uint32_t* d_stream_ids = nullptr;
   uint64_t stream_ids_cap = 0;
   cudaGraphExec_t graph = nullptr;
@@ -217,6 +243,9 @@ struct ngap_engine {
   ~ngap_engine() {
     cudaFree(d_input);
     cudaFree(d_units);
+    cudaFree(d_pieces);
+    cudaFree(d_cand);
+    cudaFree(d_runs);
     cudaFree(d_reports);
     cudaFree(d_tmp);
     cudaFree(d_unique);
@@ -250,6 +279,15 @@ struct ngap_engine {
   }
 };
 
+namespace {
+
+// Candidates per run: one injection of a warp, and no more lists than a few
+// refills of its worklist when they are long (tables of one level: hundreds
+// of states per position), so that such runs spread over the warps.
+int run_len(const TileHost& th) { return std::max(4, std::min(64, 2 * th.inj_batch)); }
+
+}  // namespace
+
 extern "C" {
 
 int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_tables** out) {
@@ -279,6 +317,7 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
     }
     t->max_states = std::max(t->max_states, th.nstates);
     t->tile_lean.push_back(th.nsticky == 0 && th.phase == 0 ? 1 : 0);
+    t->run_len.push_back(run_len(th));
     TileDev d;
     d.group = th.group;
     d.nstates = th.nstates;
@@ -289,8 +328,6 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
     d.ncls = th.ncls;
     d.cw = th.cw;
     d.nlive = th.nlive;
-    d.narrow = th.narrow ? 1 : 0;
-    d.fused = th.fused ? 1 : 0;
     d.image_bytes = (int32_t)th.image.size();
     d.off_cmask = th.off_cmask;
     d.off_rep = th.off_rep;
@@ -312,6 +349,7 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
     if ((rc = t->upload(th.sid, &d.sid)) != NGAP_OK) return rc;
     if ((rc = t->upload(th.aas, &d.aas)) != NGAP_OK) return rc;
     if ((rc = t->upload(th.start, &d.start)) != NGAP_OK) return rc;
+    d.run_len = run_len(th);
     d.filt.len = th.filt.len;
     d.filt.min_rep = th.filt.min_rep;
     d.filt.shift = th.filt.shift;
@@ -327,6 +365,7 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
       pd.hmask = ph.hmask;
       pd.cutoff = ph.cutoff;
       pd.has_reports = ph.rlist.empty() ? 0 : 1;
+      d.rep_levels |= (uint32_t)pd.has_reports << k;
       if ((rc = t->upload(ph.voff, &pd.voff)) != NGAP_OK) return rc;
       if ((rc = t->upload(ph.roff, &pd.roff)) != NGAP_OK) return rc;
       const uint32_t* slots = nullptr;
@@ -370,6 +409,10 @@ int ngap_engine_create(int device, ngap_engine** out) {
                                 kSmallSortSmem));
   CUDA_TRY(cudaFuncSetAttribute(sort_unique_cta<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSmallSortSmem));
+  CUDA_TRY(cudaFuncSetAttribute(run_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                run_smem_bytes()));
+  CUDA_TRY(cudaFuncSetAttribute(run_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                run_smem_bytes()));
   CUDA_TRY(cudaMallocHost(&e->ho.counters, kNumCounters * sizeof(unsigned long long)));
   CUDA_TRY(cudaMallocHost(&e->ho.reports, kHostReports * sizeof(uint64_t)));
   CUDA_TRY(cudaMallocHost(&e->ho.streams, kHostReports * sizeof(uint32_t)));
@@ -556,6 +599,80 @@ struct AutoChunk {
   }
 };
 
+// Length of a filtered tile's pieces: one per scan warp for short inputs, and
+// not below a scan step (256 positions); a caller's chunk length bounds it.
+int64_t piece_len(int64_t positions, int64_t warps, int64_t chunk_opt) {
+  int64_t n = ((positions + warps - 1) / warps + kScanStep - 1) / kScanStep * kScanStep;
+  if (chunk_opt > 0) n = std::min(n, chunk_opt);
+  return std::max<int64_t>(kScanStep, std::min<int64_t>(n, kPieceMax));
+}
+
+// Tiles that are scanned: acyclic ones with a filter, in plans with at least
+// kScanMin of work (scan_work). Below, a scan and its runs are two kernels whose
+// start costs more than looking every position up: an 81-byte line matches
+// in 22 us in match_kernel and 30 us scanned, 64 literals on 1 MiB in 43 and 33.
+constexpr double kScanMin = 1 << 17;
+bool is_scanned(const TileHost& th) { return th.filt.len > 0 && th.max_path >= 0; }
+
+// Positions and the states that a look-up of each would inject at prefix depth
+// `depth` (keys equally likely), with the levels that follow; layered tiles test
+// their sticky states instead.
+double scan_work(const TileHost& th, int depth, int64_t positions) {
+  if (!is_scanned(th)) return 0.0;
+  if (th.phase == 2) return (double)positions * (1 + th.nact);
+  const int d = std::max(1, std::min(depth, th.depth));
+  return (double)positions * (1 + 4 * (double)th.pt[d - 1].entries / std::pow((double)std::max(1, th.nlive), d));
+}
+
+void add_pieces(const TileHost& th, int tile, const SegSpec& s, int64_t len,
+                std::pair<int64_t, int32_t> act, std::vector<PieceDev> pieces[2]) {
+  PieceDev p{};
+  p.tile = tile;
+  p.end = (uint32_t)s.hi;
+  p.base = (uint32_t)s.base;
+  p.key_hi = s.key_hi;
+  p.act_row = act.first;
+  p.act_rowid = act.second;
+  p.pad = s.index;
+  const bool starts = s.starts && !th.start.empty();
+  for (int64_t lo = s.lo; lo < s.hi; lo += len) {
+    p.lo = (uint32_t)lo;
+    p.hi = (uint32_t)std::min(lo + len, s.hi);
+    p.flags = starts && lo == s.lo ? 1u : 0u;
+    pieces[th.phase == 2 ? 1 : 0].push_back(p);
+  }
+}
+
+// Slices of consecutive pieces whose worst case (every position a candidate)
+// fits the candidate and run buffers: pieces[0] (plain and activation tiles)
+// first, then pieces[1] (layered tiles, after the activations are known).
+constexpr int64_t kSlicePositions = 32 << 20;
+constexpr int64_t kSliceRuns = 4 << 20;
+std::vector<Slice> make_slices(const std::vector<PieceDev> pieces[2],
+                               const std::vector<int32_t>& run_len, int64_t* cands, int64_t* runs) {
+  std::vector<Slice> out;
+  *cands = *runs = 0;
+  int32_t index = 0;
+  for (int l = 0; l < 2; l++) {
+    int64_t pos = 0;
+    for (size_t i = 0; i < pieces[l].size(); i++, index++) {
+      const PieceDev& p = pieces[l][i];
+      const int64_t n = p.hi - p.lo, r = (n + run_len[p.tile] - 1) / run_len[p.tile] + 1;
+      if (i == 0 || pos + n > kSlicePositions || out.back().runs + r > kSliceRuns) {
+        out.push_back({index, 0, 0, l == 1, p.tile});
+        pos = 0;
+      }
+      if (p.tile != out.back().one_tile) out.back().one_tile = -1;
+      out.back().count++;
+      out.back().runs += r;
+      pos += n;
+      *cands = std::max(*cands, pos);
+      *runs = std::max(*runs, out.back().runs);
+    }
+  }
+  return out;
+}
+
 void add_units(const TileHost& th, int tile, const SegSpec& s, int64_t chunk,
                std::pair<int64_t, int32_t> act, std::vector<UnitDev>& pass1,
                std::vector<UnitDev>& unbounded, std::vector<UnitDev>& bounded) {
@@ -621,10 +738,10 @@ struct ActRows {
 // fewer registers spilled and a smaller code path); the rest. Within a launch the long
 // units of cyclic tiles come first. A launch whose units all belong to one
 // tile has its CTAs stage that tile's descriptors in shared memory.
-UnitRanges make_units(std::vector<UnitDev>& units, const std::vector<UnitDev>& pass1,
+PlanRanges make_units(std::vector<UnitDev>& units, const std::vector<UnitDev>& pass1,
                       const std::vector<UnitDev>& unbounded, const std::vector<UnitDev>& bounded,
                       const std::vector<char>& lean) {
-  UnitRanges r;
+  PlanRanges r;
   units.clear();
   auto append = [&](const std::vector<UnitDev>& v, int which) {
     for (const UnitDev& u : v)
@@ -648,19 +765,31 @@ UnitRanges make_units(std::vector<UnitDev>& units, const std::vector<UnitDev>& p
 }
 
 ActRows plan_units(const ngap_tables* t, const UnitPlanKey& k, int grid,
-                   std::vector<UnitDev>& units, UnitRanges& ranges) {
+                   std::vector<UnitDev>& units, std::vector<PieceDev> pieces[2], PlanRanges& ranges) {
   std::vector<UnitDev> pass1, unbounded, bounded;
   ActRows rows({t}, k.num_seg);
   AutoChunk ac;
   ac.warps = (int64_t)grid * kWarpsPerCta;
-  for (const TileHost& th : t->tiles) ac.add(th, k.num_seg * k.seg_len);
+  int64_t scanned = 0;
+  double work = 0;
+  for (const TileHost& th : t->tiles) work += scan_work(th, k.depth, k.num_seg * k.seg_len);
+  const bool scan = k.filtered && work >= kScanMin;
+  auto scans = [&](const TileHost& th) { return scan && is_scanned(th); };
+  for (const TileHost& th : t->tiles) {
+    if (scans(th)) scanned += k.num_seg * k.seg_len;
+    else ac.add(th, k.num_seg * k.seg_len);
+  }
+  const int64_t piece = piece_len(scanned, (int64_t)grid * kScanWarps, k.chunk);
   for (int ti = 0; ti < (int)t->tiles.size(); ti++) {
-    const int64_t chunk = k.chunk > 0 ? k.chunk : ac.chunk(t->tiles[ti], k.window);
+    const TileHost& th = t->tiles[ti];
+    const int64_t chunk = k.chunk > 0 ? k.chunk : ac.chunk(th, k.window);
     for (int64_t s = 0; s < k.num_seg; s++) {
       SegSpec sp{s * k.seg_len, (s + 1) * k.seg_len, k.first_seg + s == 0 || k.is_dup != 0, 0ull,
                  0, (int32_t)s};
-      add_units(t->tiles[ti], ti, sp, chunk, rows.row(0, t->tiles[ti], s), pass1, unbounded,
-                bounded);
+      if (scans(th))
+        add_pieces(th, ti, sp, piece, rows.row(0, th, s), pieces);
+      else
+        add_units(th, ti, sp, chunk, rows.row(0, th, s), pass1, unbounded, bounded);
     }
   }
   ranges = make_units(units, pass1, unbounded, bounded, t->tile_lean);
@@ -686,18 +815,75 @@ int fit_window(int window, int64_t longest) {
 int trace_buffer(ngap_engine* e, cudaStream_t st, unsigned long long** work,
                  unsigned long long** cycles) {
   *work = *cycles = nullptr;
-  if (!e->trace || e->nunits == 0) return NGAP_OK;
-  if ((size_t)e->nunits > e->unit_work_cap) {
-    const size_t cap = grown(e->unit_work_cap, (size_t)e->nunits);
+  if (!e->trace || e->h_units.empty()) return NGAP_OK;
+  if (e->h_units.size() > e->unit_work_cap) {
+    const size_t cap = grown(e->unit_work_cap, e->h_units.size());
     cudaFree(e->d_unit_work);
     e->d_unit_work = nullptr;
     e->unit_work_cap = 0;
     CUDA_TRY(cudaMalloc(&e->d_unit_work, 2 * cap * sizeof(unsigned long long)));
     e->unit_work_cap = cap;
   }
-  CUDA_TRY(cudaMemsetAsync(e->d_unit_work, 0, (size_t)e->nunits * sizeof(unsigned long long), st));
+  CUDA_TRY(cudaMemsetAsync(e->d_unit_work, 0, 2 * e->unit_work_cap * sizeof(unsigned long long), st));
   *work = e->d_unit_work;
   *cycles = e->d_unit_work + e->unit_work_cap;
+  return NGAP_OK;
+}
+
+// Device copies of a plan's units and pieces, buffers for its largest slice.
+int set_plan(ngap_engine* e, const std::vector<UnitDev>& units, const std::vector<PieceDev> pieces[2],
+             const std::vector<int32_t>& run_len, std::vector<PieceDev>& all, std::vector<Upload>& ups) {
+  all = pieces[0];
+  all.insert(all.end(), pieces[1].begin(), pieces[1].end());
+  int64_t cands = 0, runs = 0;
+  e->ranges.slices = make_slices(pieces, run_len, &cands, &runs);
+  if (units.size() > e->units_cap) {
+    const size_t cap = grown(e->units_cap, units.size());
+    cudaFree(e->d_units);
+    e->d_units = nullptr;
+    e->units_cap = 0;
+    CUDA_TRY(cudaMalloc(&e->d_units, cap * sizeof(UnitDev)));
+    e->units_cap = cap;
+  }
+  if (all.size() > e->pieces_cap) {
+    const size_t cap = grown(e->pieces_cap, all.size());
+    cudaFree(e->d_pieces);
+    e->d_pieces = nullptr;
+    e->pieces_cap = 0;
+    CUDA_TRY(cudaMalloc(&e->d_pieces, cap * sizeof(PieceDev)));
+    e->pieces_cap = cap;
+  }
+  if (cands > e->cand_cap) {
+    const int64_t cap = std::max(cands, std::min<int64_t>(grown(e->cand_cap, cands), kSlicePositions));
+    cudaFree(e->d_cand);
+    e->d_cand = nullptr;
+    e->cand_cap = 0;
+    CUDA_TRY(cudaMalloc(&e->d_cand, (size_t)cap * sizeof(uint16_t)));
+    e->cand_cap = cap;
+  }
+  if (runs > e->runs_cap) {
+    const int64_t cap = std::max(runs, std::min<int64_t>(grown(e->runs_cap, runs), kSliceRuns));
+    cudaFree(e->d_runs);
+    e->d_runs = nullptr;
+    e->runs_cap = 0;
+    CUDA_TRY(cudaMalloc(&e->d_runs, (size_t)cap * sizeof(RunDev)));
+    e->runs_cap = cap;
+  }
+  if (!units.empty()) ups.push_back({e->d_units, units.data(), units.size() * sizeof(UnitDev)});
+  if (!all.empty()) ups.push_back({e->d_pieces, all.data(), all.size() * sizeof(PieceDev)});
+  e->nunits = (int32_t)units.size();
+  e->longest_unit = longest_unit(units);
+  // host records of the traces: the units, then the pieces
+  e->h_units = units;
+  for (const PieceDev& p : all) {
+    UnitDev u{};
+    u.tile = p.tile;
+    u.lo = u.emit_lo = p.lo;
+    u.hi = p.hi;
+    u.base = p.base;
+    u.stream = p.pad;
+    e->h_units.push_back(u);
+  }
   return NGAP_OK;
 }
 
@@ -746,12 +932,20 @@ __global__ void act_compact(const int64_t* __restrict__ row_off, const int32_t* 
   const int64_t off = row_off[row];
   const int32_t n = row_n[row];
   uint32_t c = 0;
-  for (int32_t i0 = 0; i0 < n; i0 += 32) {
-    const int32_t i = i0 + lane;
-    const bool ok = i < n && act[off + i] != 0xffffffffu;
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (ok) list[off + c + __popc(m & ((1u << lane) - 1u))] = (uint32_t)i;
-    c += __popc(m);
+  for (int32_t i0 = 0; i0 < n; i0 += 256) {  // eight reads in flight per lane: the reads are the time
+    uint32_t a[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int32_t i = i0 + 32 * k + lane;
+      a[k] = i < n ? act[off + i] : 0xffffffffu;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const bool ok = a[k] != 0xffffffffu;
+      const unsigned m = __ballot_sync(0xffffffffu, ok);
+      if (ok) list[off + c + __popc(m & ((1u << lane) - 1u))] = (uint32_t)(i0 + 32 * k + lane);
+      c += __popc(m);
+    }
   }
   if (lane == 0) cnt[row] = c;
 }
@@ -765,7 +959,8 @@ int launch_grid(int64_t nunits, int grid) {
 // The matching launches of a plan: the activation tiles' work; the plain
 // tiles without sticky states in the lean kernel instance; then the rest
 // (the layered tiles read what the first launch recorded).
-int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
+int launch_plan(ngap_engine* e, MatchParams mp, const std::vector<TileDev>& tiles, int smem,
+                uint32_t readable, cudaStream_t st) {
   if (e->act_entries > 0)
     CUDA_TRY(cudaMemsetAsync(e->d_act, 0xff, (size_t)e->act_entries * sizeof(uint32_t), st));
   auto run = [&](bool lean, int which) -> int {
@@ -783,8 +978,49 @@ int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
     e->launches++;
     return NGAP_OK;
   };
+  ScanParams sp;
+  sp.tiles = mp.tiles;
+  sp.pieces = e->d_pieces;
+  sp.input = mp.input;
+  sp.readable = readable;
+  sp.cand = e->d_cand;
+  sp.runs = e->d_runs;
+  sp.act_cnt = e->d_act_cnt;
+  sp.cycles = mp.unit_cycles ? mp.unit_cycles + e->nunits : nullptr;
+  mp.piece_unit0 = e->nunits;
+  unsigned int* const ctl0 = reinterpret_cast<unsigned int*>(e->d_counters + kSliceCtl);
+  auto run_slices = [&](bool layered) -> int {
+    for (size_t i = 0; i < e->ranges.slices.size(); i++) {
+      const Slice& s = e->ranges.slices[i];
+      if (s.layered != layered) continue;
+      unsigned int* ctl = ctl0 + (i % kSliceSlots) * kCtlWords;
+      if (i >= kSliceSlots) CUDA_TRY(cudaMemsetAsync(ctl, 0, kCtlWords * sizeof(unsigned int), st));
+      sp.piece_begin = (uint32_t)s.begin;
+      sp.npieces = (uint32_t)s.count;
+      sp.ctl = ctl;
+      sp.one_tile = s.one_tile;
+      if (s.one_tile >= 0) {  // described in the parameters: no reads before the scan
+        const TileDev& td = tiles[s.one_tile];
+        sp.filt = td.filt;
+        sp.cls = td.image + td.off_cls;
+        sp.nlive = (uint32_t)td.nlive;
+        sp.run_len = td.run_len;
+        sp.phase = td.phase;
+      }
+      scan_kernel<<<launch_grid(s.count, e->grid), kScanWarps * 32, 0, st>>>(sp);
+      const int grid = launch_grid(s.runs, e->grid);
+      if (layered)
+        run_kernel<true><<<grid, kRunWarps * 32, run_smem_bytes(), st>>>(mp, e->d_cand, e->d_runs, ctl);
+      else
+        run_kernel<false><<<grid, kRunWarps * 32, run_smem_bytes(), st>>>(mp, e->d_cand, e->d_runs, ctl);
+      CUDA_TRY(cudaGetLastError());
+      e->launches += 2;
+    }
+    return NGAP_OK;
+  };
   int rc = run(false, 0);
   if (rc == NGAP_OK) rc = run(true, 1);
+  if (rc == NGAP_OK) rc = run_slices(false);
   if (rc != NGAP_OK) return rc;
   if (e->act_rows > 0) {
     act_compact<<<(e->act_rows + 7) / 8, 256, 0, st>>>(e->d_row_off, e->d_row_n, e->act_rows,
@@ -792,7 +1028,8 @@ int launch_plan(ngap_engine* e, MatchParams mp, int smem, cudaStream_t st) {
     CUDA_TRY(cudaGetLastError());
     e->launches++;
   }
-  return run(false, 2);
+  if ((rc = run(false, 2)) != NGAP_OK) return rc;
+  return run_slices(true);
 }
 
 __global__ void swap_halves(uint64_t* a, uint64_t n) {
@@ -1133,25 +1370,16 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   if (rc != NGAP_OK) return rc;
   const int full_grid = e->num_sms * bps;
   // units
-  UnitPlanKey key{p->num_seg, p->seg_len, p->is_dup ? 1 : 0, window, p->chunk, p->first_segment};
+  UnitPlanKey key{p->num_seg, p->seg_len, p->is_dup ? 1 : 0, window, p->chunk, p->first_segment,
+                  depth, e->test_skip_unit < 0};
   if (e->plan_tables != t->serial || key < e->plan_key || e->plan_key < key) {
     std::vector<UnitDev> units;
-    const ActRows rows = plan_units(t, key, full_grid, units, e->ranges);
+    std::vector<PieceDev> pieces[2], all;
+    const ActRows rows = plan_units(t, key, full_grid, units, pieces, e->ranges);
     std::vector<Upload> ups;
     if ((rc = set_act_rows(e, rows, ups)) != NGAP_OK) return rc;
-    if (units.size() > e->units_cap) {
-      const size_t cap = grown(e->units_cap, units.size());
-      cudaFree(e->d_units);
-      e->d_units = nullptr;
-      e->units_cap = 0;
-      CUDA_TRY(cudaMalloc(&e->d_units, cap * sizeof(UnitDev)));
-      e->units_cap = cap;
-    }
-    if (!units.empty()) ups.push_back({e->d_units, units.data(), units.size() * sizeof(UnitDev)});
+    if ((rc = set_plan(e, units, pieces, t->run_len, all, ups)) != NGAP_OK) return rc;
     if ((rc = upload_plan(e, st, ups)) != NGAP_OK) return rc;
-    e->nunits = (int32_t)units.size();
-    e->longest_unit = longest_unit(units);
-    e->h_units = units;
     e->plan_tables = t->serial;
     e->plan_key = key;
     e->batch_ts = 0;  // the batched plan cache no longer describes the buffers
@@ -1163,7 +1391,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   e->grid = full_grid;
   // per-warp scratch for the full grid, whatever this plan uses: a later
   // larger plan then never reallocates (cudaMalloc waits for the device)
-  rc = ensure_slots(e, (size_t)full_grid * kWarpsPerCta, t->max_states, t->max_nact, kDefaultQueue);
+  rc = ensure_slots(e, (size_t)full_grid * kSlotsPerSm, t->max_states, t->max_nact, kDefaultQueue);
   if (rc != NGAP_OK) return rc;
 
   if (input_on_device)
@@ -1204,8 +1432,8 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   if ((rc = trace_buffer(e, st, &mp.unit_work, &mp.unit_cycles)) != NGAP_OK) return rc;
   e->trace_seg_len = p->seg_len;
   CUDA_TRY(cudaEventRecord(e->ev[1], st));
-  if (e->nunits > 0) {
-    rc = launch_plan(e, mp, smem, st);
+  if (!e->h_units.empty()) {
+    rc = launch_plan(e, mp, t->dev_desc, smem, (uint32_t)((total + 15) & ~(uint64_t)15), st);
     if (rc != NGAP_OK) return rc;
   }
   CUDA_TRY(cudaEventRecord(e->ev[2], st));
@@ -1301,9 +1529,11 @@ int ngap_engine_memory(const ngap_engine* e, ngap_engine_mem* out) {
   out->input = (int64_t)e->input_cap;
   out->reports = 3 * 8 * (int64_t)e->rep_cap + 4 * (int64_t)e->hist_cap + 4 * (int64_t)e->stream_ids_cap;
   out->scratch =
-      (int64_t)e->slots * 4 * ((int64_t)e->carry_cap + e->mark_words + e->ovf_cap + 2 * e->stk_cap);
+      (int64_t)e->slots * 4 * ((int64_t)e->carry_cap + e->mark_words + e->ovf_cap + 2 * e->stk_cap) +
+      (int64_t)sizeof(uint16_t) * e->cand_cap + (int64_t)sizeof(RunDev) * e->runs_cap;
   out->plan = 8 * (int64_t)e->act_cap + 16 * (int64_t)e->rows_cap + 16 * (int64_t)e->unit_work_cap +
-              (int64_t)sizeof(UnitDev) * (int64_t)e->units_cap;
+              (int64_t)sizeof(UnitDev) * (int64_t)e->units_cap +
+              (int64_t)sizeof(PieceDev) * (int64_t)e->pieces_cap;
   return NGAP_OK;
 }
 
@@ -1338,19 +1568,19 @@ int ngap_trace_copy(ngap_engine* e, ngap_unit_trace* out, int64_t cap, int64_t* 
     return NGAP_E_INVALID;
   }
   *n = 0;
-  if (!e->trace || !e->ran || e->nunits == 0 || !e->d_unit_work) return NGAP_OK;
+  if (!e->trace || !e->ran || e->h_units.empty() || !e->d_unit_work) return NGAP_OK;
   if (!out) {  // count query
-    *n = e->nunits;
+    *n = (int64_t)e->h_units.size();
     return NGAP_OK;
   }
-  std::vector<unsigned long long> work(e->nunits), cycles(e->nunits);
+  std::vector<unsigned long long> work(e->h_units.size()), cycles(e->h_units.size());
   CUDA_TRY(cudaSetDevice(e->device));
   CUDA_TRY(cudaStreamSynchronize(e->stream));
   CUDA_TRY(cudaMemcpy(work.data(), e->d_unit_work, work.size() * sizeof(unsigned long long),
                       cudaMemcpyDeviceToHost));
   CUDA_TRY(cudaMemcpy(cycles.data(), e->d_unit_work + e->unit_work_cap,
                       cycles.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
-  const int64_t m = std::min<int64_t>(cap, e->nunits);
+  const int64_t m = std::min<int64_t>(cap, (int64_t)e->h_units.size());
   for (int64_t i = 0; i < m; i++) {
     const UnitDev& u = e->h_units[i];
     const int64_t base = e->trace_seg_len > 0 ? (int64_t)u.stream * e->trace_seg_len : u.base;
@@ -1437,7 +1667,9 @@ struct ngap_tableset {
   int sid_bits = 0;
   int ntiles = 0, max_states = 0, max_groups = 1, max_depth = 1, device = 0;
   int max_nact = 0;
-  std::vector<char> tile_lean;      // per tile of the combined array (ngap_tables::tile_lean)
+  std::vector<TileDev> tiles;       // the combined array
+  std::vector<char> tile_lean;      // per tile of it (ngap_tables::tile_lean)
+  std::vector<int32_t> run_len;     // the same
   ~ngap_tableset() { cudaFree(d_tiles); }
 };
 
@@ -1450,7 +1682,7 @@ int ngap_tableset_create(const ngap_tables* const* tables, int n, ngap_tableset*
   }
   *out = nullptr;
   std::unique_ptr<ngap_tableset> ts(new ngap_tableset());
-  std::vector<TileDev> all;
+  std::vector<TileDev>& all = ts->tiles;
   for (int i = 0; i < n; i++) {
     const ngap_tables* t = tables[i];
     if (!t || (i > 0 && t->device != tables[0]->device)) {
@@ -1461,6 +1693,7 @@ int ngap_tableset_create(const ngap_tables* const* tables, int n, ngap_tableset*
     ts->tile_base.push_back((int)all.size());
     all.insert(all.end(), t->dev_desc.begin(), t->dev_desc.end());
     ts->tile_lean.insert(ts->tile_lean.end(), t->tile_lean.begin(), t->tile_lean.end());
+    ts->run_len.insert(ts->run_len.end(), t->run_len.begin(), t->run_len.end());
     ts->max_states = std::max(ts->max_states, t->max_states);
     ts->max_groups = std::max(ts->max_groups, t->num_groups);
     ts->sid_bits = std::max(ts->sid_bits, t->sid_bits);
@@ -1566,7 +1799,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     return true;
   };
   bool replanned = false;
-  if (e->batch_ts != ts->serial || e->batch_window != window || e->batch_chunk != p->chunk ||
+  if (e->batch_ts != ts->serial || e->batch_depth != depth || e->batch_window != window || e->batch_chunk != p->chunk ||
       !same_streams() || e->plan_tables != 0) {
     std::vector<std::vector<int>> by_nfa(ts->tables.size());
     for (int i = 0; i < nstreams; i++) by_nfa[sv[i].nfa].push_back(i);
@@ -1574,44 +1807,49 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     const ActRows rows(ts->tables, nstreams);
     AutoChunk ac;
     ac.warps = (int64_t)full_grid * kWarpsPerCta;
+    int64_t scanned = 0;
+    double work = 0;
     for (const ngap_batch_stream& s : sv)
-      for (const TileHost& th : ts->tables[s.nfa]->tiles) ac.add(th, (int64_t)s.length);
+      for (const TileHost& th : ts->tables[s.nfa]->tiles) work += scan_work(th, depth, (int64_t)s.length);
+    auto scans = [&](const TileHost& th) { return work >= kScanMin && is_scanned(th); };
+    for (const ngap_batch_stream& s : sv)
+      for (const TileHost& th : ts->tables[s.nfa]->tiles) {
+        if (scans(th)) scanned += (int64_t)s.length;
+        else ac.add(th, (int64_t)s.length);
+      }
+    std::vector<PieceDev> pieces[2], all;
     for (size_t n = 0; n < ts->tables.size(); n++) {
       const ngap_tables* t = ts->tables[n];
       for (int ti = 0; ti < (int)t->tiles.size(); ti++) {
-        const int64_t auto_chunk = ac.chunk(t->tiles[ti], window);
+        const TileHost& th = t->tiles[ti];
+        const int64_t auto_chunk = ac.chunk(th, window);
         for (int si : by_nfa[n]) {
           const ngap_batch_stream& s = sv[si];
           if (s.length == 0) continue;
           SegSpec sp{(int64_t)s.offset, (int64_t)(s.offset + s.length), true,
                      (uint64_t)si << sshift, (int64_t)s.offset, si};
-          add_units(t->tiles[ti], ts->tile_base[n] + ti, sp,
-                    s.chunk > 0 ? s.chunk : (p->chunk > 0 ? p->chunk : auto_chunk),
-                    rows.row((int)n, t->tiles[ti], si), pass1, unbounded, bounded);
+          const int64_t chunk = s.chunk > 0 ? s.chunk : p->chunk;
+          if (scans(th))
+            add_pieces(th, ts->tile_base[n] + ti, sp,
+                       piece_len(scanned, (int64_t)full_grid * kScanWarps, chunk),
+                       rows.row((int)n, th, si), pieces);
+          else
+            add_units(th, ts->tile_base[n] + ti, sp, chunk > 0 ? chunk : auto_chunk,
+                      rows.row((int)n, th, si), pass1, unbounded, bounded);
         }
       }
     }
     e->ranges = make_units(units, pass1, unbounded, bounded, ts->tile_lean);
     std::vector<Upload> ups;
     if ((rc = set_act_rows(e, rows, ups)) != NGAP_OK) return rc;
-    if (units.size() > e->units_cap) {
-      const size_t cap = grown(e->units_cap, units.size());
-      cudaFree(e->d_units);
-      e->d_units = nullptr;
-      e->units_cap = 0;
-      CUDA_TRY(cudaMalloc(&e->d_units, cap * sizeof(UnitDev)));
-      e->units_cap = cap;
-    }
-    if (!units.empty()) ups.push_back({e->d_units, units.data(), units.size() * sizeof(UnitDev)});
+    if ((rc = set_plan(e, units, pieces, ts->run_len, all, ups)) != NGAP_OK) return rc;
     if ((rc = upload_plan(e, st, ups)) != NGAP_OK) return rc;
-    e->nunits = (int32_t)units.size();
-    e->longest_unit = longest_unit(units);
-    e->h_units = units;
     e->plan_tables = 0;  // the plain plan cache no longer describes the buffers
-    e->plan_key = UnitPlanKey{-1, -1, -1, -1, -1, -1};
+    e->plan_key = UnitPlanKey{-1, -1, -1, -1, -1, -1, -1, true};
     e->batch_ts = ts->serial;
     e->batch_streams = sv;
     e->batch_window = window;
+    e->batch_depth = depth;
     e->batch_chunk = p->chunk;
     replanned = true;
   }
@@ -1620,7 +1858,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     smem = cta_smem_bytes(window);
   }
   e->grid = full_grid;
-  if ((rc = ensure_slots(e, (size_t)full_grid * kWarpsPerCta, ts->max_states, ts->max_nact,
+  if ((rc = ensure_slots(e, (size_t)full_grid * kSlotsPerSm, ts->max_states, ts->max_nact,
                          p->queue_capacity > 0 ? std::max(p->queue_capacity, 1024) : kDefaultQueue)) != NGAP_OK)
     return rc;
 
@@ -1664,8 +1902,8 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     else
       CUDA_TRY(cudaMemcpyAsync(e->d_input, input, input_bytes, cudaMemcpyHostToDevice, qs));
     int r = NGAP_OK;
-    if (e->nunits > 0) {
-      r = launch_plan(e, mp, smem, qs);
+    if (!e->h_units.empty()) {
+      r = launch_plan(e, mp, ts->tiles, smem, (uint32_t)((input_bytes + 15) & ~(uint64_t)15), qs);
       if (r != NGAP_OK) return r;
     }
     if (!p->report_off) {

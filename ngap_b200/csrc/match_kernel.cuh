@@ -16,7 +16,8 @@
 //  * one warp per unit (a tile and a range of positions), taken from a global
 //    cursor, with no block-wide barrier after the start; tiles are read in
 //    place, through L1 and L2;
-//  * a look-ahead filter (FilterDev) picks the positions that need injection;
+//  * acyclic tiles with a look-ahead filter (FilterDev) are matched by another
+//    pair of kernels (scan_kernel.cuh); this one takes the rest;
 //  * per warp, in shared memory: a LIFO worklist of packed entries
 //    (state << 13 | offset in the window) whose paths are followed in
 //    registers; entries past the shared capacity spill to a per-warp global
@@ -52,10 +53,6 @@ constexpr int kReportBuf = 64;    // reports per warp buffered in shared memory
 constexpr int kInjectLow = 192;   // inject new positions while the stack holds fewer entries
 constexpr int kStickyCap = 64;    // sticky states tracked per warp (more fall back to entries)
 constexpr int kPendCap = 16;      // sticky states met while copying one injection batch
-constexpr int kScanLane = 8;      // consecutive positions a lane tests per filter scan step
-constexpr int kScanStep = 32 * kScanLane;
-constexpr int kCandLow = 64;      // the filter scans on while fewer candidates are queued
-constexpr int kCandCap = kCandLow + kScanStep;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr uint32_t kNoEntry = 0xffffffffu;  // never a valid entry: offsets stay < 8191
 constexpr uint32_t kIdMask = 0x7fffffffu;
@@ -92,6 +89,7 @@ struct MatchParams {
   int32_t stk_g_cap;        // kStickyCap
   unsigned long long* unit_work;  // [units]: entries expanded + injected per unit (tracing), or null
   unsigned long long* unit_cycles;  // [units]: SM clock cycles per unit (tracing), or null
+  int32_t piece_unit0;      // the trace record of the first piece (scan_kernel.cuh)
   int32_t unit_begin;       // units [unit_begin, unit_begin + nunits) of this launch
   int32_t nunits;
   int32_t one_tile;         // the one tile of the launch's units (descriptors staged per CTA), or -1
@@ -106,16 +104,12 @@ constexpr int32_t kWaitRounds = 1 << 24;  // default bound of an mbarrier wait
 constexpr uint32_t kNoAct = 0xffffffffu;
 
 // A window buffer: up to kMaxDepth - 1 look-behind bytes, 15 bytes of
-// alignment, W window bytes and the look-ahead bytes (one, or the filter's).
-__host__ __device__ inline int window_buf_bytes(int W) { return ((W + 64) + 15) & ~15; }
-static_assert(kMaxDepth - 1 + 15 + kMaxFilter + 15 <= 64, "window buffer slack");
-// a filter scan step may read (and ignore) up to a step and a filter past the
-// window's bytes: those are the next buffer, the reports and the scratch
-static_assert(kScanStep + kMaxFilter + 8 <= kReportBuf * 8, "filter scan over-read");
-
+// alignment, W window bytes and one look-ahead byte.
+__host__ __device__ inline int window_buf_bytes(int W) { return ((W + 48) + 15) & ~15; }
+static_assert(kMaxDepth - 1 + 15 + 1 + 15 <= 48, "window buffer slack");
 __host__ __device__ inline int warp_smem_bytes(int W) {
   return kStackCap * 4 + 2 * window_buf_bytes(W) + kReportBuf * 8 + 3 * 32 * 4 + 16 +
-         kStickyCap * 8 + kPendCap * 8 + 16 + kCandCap * 2;
+         kStickyCap * 8 + kPendCap * 8 + 16;
 }
 
 __host__ __device__ inline int cta_smem_bytes(int W) { return kWarpsPerCta * warp_smem_bytes(W); }
@@ -131,7 +125,6 @@ struct WarpSmem {
   uint32_t* pend_s;          // kPendCap sticky states met while copying a batch
   uint32_t* pend_q;
   uint32_t* pend_n;          // count (one word)
-  int16_t* cand;             // kCandCap window offsets that passed the filter
 };
 
 // Per-warp state kept in registers (uniform across the warp).
@@ -161,30 +154,23 @@ struct TileView {
   const TileDev* t;
   const PrefixTableDev* pt;  // the tile's prefix tables (shared-memory copy)
   int cw;
-  int narrow;
-  int fused;       // records of 2 x uint4: successors, then their class masks
   uint32_t nlive;  // live classes: base of the prefix-table keys
   uint32_t rep_levels;  // bit d: the depth-(d+1) table has report lists
 };
 
-// Successors of v in the 32-bit convention (bit 31 = report, kNoSucc = none).
+// State v's record: its successors and what they accept (TileDev), 32 bytes
+// in one read (two 16-byte reads take the L1 tag stage twice per lane).
+__device__ __forceinline__ void load_record(const TileView& tv, uint32_t v, uint4& sc, uint4& sm) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(sc.x), "=r"(sc.y), "=r"(sc.z), "=r"(sc.w), "=r"(sm.x), "=r"(sm.y), "=r"(sm.z), "=r"(sm.w)
+      : "l"(tv.succ + ((size_t)v << 1)));
+}
+
 __device__ __forceinline__ uint4 load_succ(const TileView& tv, uint32_t v) {
-  if (!tv.narrow) return __ldg(tv.succ + ((size_t)v << tv.fused));
-  const uint2 x = __ldg(reinterpret_cast<const uint2*>(tv.succ) + v);  // narrow tiles: 4 x u16
-  auto wide = [](uint32_t h) {
-    return h == 0xffffu ? kNoSucc : ((h & 0x7fffu) | ((h & 0x8000u) << 16));
-  };
-  return make_uint4(wide(x.x & 0xffffu), wide(x.x >> 16), wide(x.y & 0xffffu), wide(x.y >> 16));
+  return __ldg(tv.succ + ((size_t)v << 1));
 }
 
-// Fused tiles: the class masks of v's four successors (0 where none), the
-// second half of v's 32-byte record.
-__device__ __forceinline__ uint4 load_smask(const TileView& tv, uint32_t v) {
-  return __ldg(tv.succ + ((size_t)v << 1) + 1);
-}
-
-// Successor j of a state accepts class c: from the record's masks (fused
-// tiles) or from the successor's own class mask.
+// Successor u whose record word is m accepts class c.
 __device__ __forceinline__ bool succ_accepts(const TileView& tv, uint32_t u, uint32_t m, uint32_t c);
 
 // Everything about the current unit and window.
@@ -242,8 +228,8 @@ __device__ __forceinline__ bool accepts(const TileView& tv, uint32_t v, uint32_t
 }
 
 __device__ __forceinline__ bool succ_accepts(const TileView& tv, uint32_t u, uint32_t m, uint32_t c) {
-  if (tv.fused) return (m >> c) & 1u;  // m = 0 when there is no successor
-  return u != kNoSucc && accepts(tv, u & kIdMask, c);
+  if (tv.cw == 1) return (m >> c) & 1u;
+  return m == c || (m == kManyClasses && accepts(tv, u & kIdMask, c));
 }
 
 __device__ __forceinline__ bool is_report(const TileView& tv, uint32_t v) {
@@ -517,14 +503,12 @@ __device__ __forceinline__ bool register_each(const MatchParams& p, WarpSmem& ws
   return mine;
 }
 
-// Always-active states for window offsets [r0, r0 + batch) (one per lane), or
-// with CAND for the `batch` filter candidates ws.cand[r0 ...].
-template <bool CAND>
+// Always-active states for window offsets [r0, r0 + batch) (one per lane).
 __device__ __forceinline__ void inject_aas(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                            const TileView& tv, const UnitCtx& c, int lane, int r0,
                                            int batch, int depth, unsigned long long& n_injected) {
   const TileDev& t = *tv.t;
-  const int r = CAND ? (int)ws.cand[r0 + min(lane, batch - 1)] : r0 + lane;
+  const int r = r0 + lane;
   const bool valid = lane < batch && r < c.iend;
   const int64_t q = c.wb + r;
   if (depth == 0) {  // scan the always-active list
@@ -627,7 +611,7 @@ __device__ __forceinline__ void inject_aas(const MatchParams& p, WarpSmem& ws, W
     const int kk = (int)(kraw & 0xffu);
     const uint32_t v = (kraw & 0x100u) ? ws.inj[32 + l0]
                                        : __ldg(tv.pt[kk - 1].vlist + ws.inj[32 + l0] + (idx - before));
-    const uint32_t off = (uint32_t)((CAND ? (int)ws.cand[r0 + l0] : r0 + l0) + kk - 1);
+    const uint32_t off = (uint32_t)(r0 + l0 + kk - 1);
     uint32_t e = (v << kEntryPosBits) | off;
     if (tv.sticky && is_sticky(tv, v)) {  // registered after the copy instead
       const uint32_t slot = atomicAdd(ws.pend_n, 1u);
@@ -681,8 +665,7 @@ __device__ __forceinline__ void inject_key(const TileView& tv, const UnitCtx& c,
 // flight per lane. Same entries and reports as inject_aas over the two halves.
 // AHEAD (the lean kernel): after this batch's lookups, the lane's inline
 // table words of the next batch are read too, and the next call uses them.
-// CAND: the positions are the filter candidates ws.cand[r0 .. r0 + batch).
-template <bool AHEAD, bool CAND>
+template <bool AHEAD>
 __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                             const TileView& tv, const UnitCtx& c, int lane, int r0,
                                             int batch, int depth, unsigned long long& n_injected,
@@ -694,7 +677,7 @@ __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, 
   const bool read_ahead = AHEAD && ahead.r0 == r0;  // read during the last batch's expansions
 #pragma unroll
   for (int h = 0; h < 2; h++) {
-    r[h] = CAND ? (int)ws.cand[r0 + min(32 * h + lane, batch - 1)] : r0 + 32 * h + lane;
+    r[h] = r0 + 32 * h + lane;
     vb[h] = ve[h] = 0u;
     one[h] = kNoEntry;
     uint32_t key = 0u;
@@ -830,8 +813,7 @@ __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, 
       const uint32_t v = (kraw & 0x100u)
                              ? ws.inj[32 + l0]
                              : __ldg(tv.pt[kk - 1].vlist + ws.inj[32 + l0] + (idx - before));
-      const uint32_t off =
-          (uint32_t)((CAND ? (int)ws.cand[r0 + 32 * h + l0] : r0 + 32 * h + l0) + kk - 1);
+      const uint32_t off = (uint32_t)(r0 + 32 * h + l0 + kk - 1);
       store_entry(p, ws, w, base + (int)idx, (v << kEntryPosBits) | off);
     }
     base += (int)ht;
@@ -841,59 +823,13 @@ __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, 
   __syncwarp();
 }
 
-// One step of the look-ahead filter (FilterDev): tests window offsets [s0, s0 +
-// kScanStep), kScanLane consecutive ones per lane, and appends those that
-// pass to the candidate queue (n entries so far); returns the new count. s0
-// is a multiple of 8 as a shared-memory address, so positions below r0 (the
-// first to test) are masked off here.
-// What bounds it is one bitmap read per position (L2, or L1 for the small
-// bitmaps), none of which depends on another: a lane's eight are issued before
-// any is used. Measured on a B200, whole calls: 1000 25-mers on 16 MiB 691 ->
-// 308 us (kernel 598 -> 217: 4 % of the positions pass), 200 25-mers with
-// three table levels on 3 MB 79.5 -> 2.65 ms, 50 edit-distance 20-mers with
-// one level on 1 MB 20.6 -> 0.46 ms, the 32 MiB mix 3.90 -> 2.41 ms.
-__device__ __forceinline__ int filter_scan(WarpSmem& ws, const TileView& tv, const UnitCtx& c,
-                                           int lane, int s0, int r0, int n) {
-  const FilterDev& f = tv.t->filt;
-  const int len = f.len, min_rep = f.min_rep, shift = f.shift;
-  const uint32_t mul = f.mul, scale = f.scale, drop = f.drop;
-  const uint32_t* __restrict__ bits = f.bits;
-  const int o = s0 + kScanLane * lane;
-  const uint8_t* in = c.in + o;
-  uint32_t h = 0u;
-  for (int i = 0; i < len - 1; i++) h = h * mul + in[i];
-  const uint2 old = *reinterpret_cast<const uint2*>(in);  // the lane's own symbols (8-aligned)
-  uint32_t idx[kScanLane], word[kScanLane];
-  unsigned pass = 0u, test = 0u;
-#pragma unroll
-  for (int j = 0; j < kScanLane; j++) {
-    h = h * mul + in[len - 1 + j];  // a symbol enters, and the one before the lane's j-th leaves
-    if (j > 0) h -= __byte_perm(j <= 4 ? old.x : old.y, 0, 0x4440 | ((j - 1) & 3)) * drop;
-    idx[j] = (h * scale) >> shift;
-    const int r = o + j;
-    const int left = c.lim - r;  // symbols left in the unit
-    const bool in_range = r >= r0 && r < c.iend;
-    if (in_range && left >= len) test |= 1u << j;
-    else if (in_range && left >= min_rep) pass |= 1u << j;
-  }
-#pragma unroll
-  for (int j = 0; j < kScanLane; j++) word[j] = (test >> j) & 1u ? __ldg(bits + (idx[j] >> 5)) : 0u;
-#pragma unroll
-  for (int j = 0; j < kScanLane; j++) pass |= ((word[j] >> (idx[j] & 31)) & 1u) << j;
-  int total;
-  int pos = n + warp_excl<4>(__popc(pass), lane, total);
-  for (; pass; pass &= pass - 1u) ws.cand[pos++] = (int16_t)(o + __ffs(pass) - 1);
-  __syncwarp();
-  return n + total;
-}
-
 // Injection of a batch of positions: always-active states, then the sticky
 // states met while copying, then the work of every active sticky state at
 // these positions. Layered tiles (phase 2) do their sticky work separately.
 __device__ __forceinline__ void inject(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                        const TileView& tv, const UnitCtx& c, int lane, int r0,
                                        int batch, int depth, unsigned long long& n_injected) {
-  inject_aas<false>(p, ws, w, tv, c, lane, r0, batch, depth, n_injected);
+  inject_aas(p, ws, w, tv, c, lane, r0, batch, depth, n_injected);
   if (!tv.sticky || tv.t->phase == 2) return;
   __syncwarp();
   const int np = min((int)*ws.pend_n, kPendCap);
@@ -1079,66 +1015,6 @@ __device__ __forceinline__ void layered_sticky_positions(const MatchParams& p, W
   }
 }
 
-// Filtered layered tiles: the work of the segment's active sticky states (n
-// matched slots listed at act_list + row, offsets relative to base) at the m <=
-// 32 candidates ws.cand[first ...]. The filter leaves a few candidates per
-// window, so lanes hold sticky states (32 at a time, their slot, first match
-// and union mask in registers) and the candidates are visited one by one: a
-// pass over n states costs n / 32 steps per candidate, whatever m is, where
-// lanes over positions cost n steps per window. Same rule as
-// layered_sticky_positions; reporting sticky states get no filter.
-// Measured on a B200, whole calls, layered tiles without and with a filter: the
-// 32 MiB mix 2.41 -> 1.16 ms (20.8 M expansions -> 1.3 M), 512 streams against
-// eight rule sets 32.5 -> 10.8 ms, 300 dot-star regexes on 4 MB 0.80 -> 0.38.
-__device__ __forceinline__ void layered_candidates(const MatchParams& p, WarpSmem& ws, WarpRun& w,
-                                                   const TileView& tv, const UnitCtx& c, int lane,
-                                                   int first, int m, int64_t row, uint32_t n) {
-  const TileDev& t = *tv.t;
-  const int rc = lane < m ? (int)ws.cand[first + lane] : 0;
-  const uint32_t cls = lane < m ? (uint32_t)c.in[rc] : 0u;
-  uint32_t next = (uint32_t)lane < n ? __ldg(p.act_list + row + lane) : 0u;
-  for (uint32_t i0 = 0; i0 < n; i0 += 32) {
-    const uint32_t i = i0 + (uint32_t)lane;
-    const uint32_t sl = next;
-    if (i + 32 < n) next = __ldg(p.act_list + row + i + 32);
-    const uint32_t f = i < n ? __ldg(p.act + row + sl) : kNoAct;
-    const uint32_t al = i < n ? __ldg(t.act_local + sl) : 0u;
-    const uint32_t* um = t.stk_union + (size_t)sl * tv.cw;
-    const uint32_t u0 = i < n ? __ldg(um) : 0u;
-    const uint32_t u1 = i < n && tv.cw > 1 ? __ldg(um + 1) : 0u;
-    const uint32_t u2 = i < n && tv.cw > 2 ? __ldg(um + 2) : 0u;
-    for (int k = 0; k < m; k++) {
-      const int r = __shfl_sync(kFull, rc, k);
-      const uint32_t sym = __shfl_sync(kFull, cls, k);
-      const uint32_t rel = (uint32_t)(c.wb + r) - w.base;  // position in the segment
-      const uint32_t word = sym >> 5;
-      const uint32_t mask = word == 0 ? u0 : word == 1 ? u1 : word == 2 ? u2 : i < n ? __ldg(um + word) : 0u;
-      const bool hit = i < n && rel >= f && ((mask >> (sym & 31)) & 1u);
-      if (!__any_sync(kFull, hit)) continue;
-      const uint32_t on = !hit ? 0u : rel > f ? 0xfu : al >> 28;
-      uint4 su = make_uint4(kNoSucc, kNoSucc, kNoSucc, kNoSucc);
-      if (hit) su = load_succ(tv, al & kActIdMask);
-      const uint32_t us[4] = {su.x, su.y, su.z, su.w};
-      bool ok[4];
-      int cnt = 0;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        ok[j] = ((on >> j) & 1u) && us[j] != kNoSucc && accepts(tv, us[j] & kIdMask, sym);
-        cnt += ok[j];
-      }
-      report4(p, ws, w, tv, lane, ok, us, c.wb + r, r >= c.elo);
-      if (r + 1 >= c.lim) continue;  // the unit's last position: nothing to expand
-      int total;
-      int pos = w.top + warp_excl<3>(cnt, lane, total);
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (ok[j]) store_entry(p, ws, w, pos++, ((us[j] & kIdMask) << kEntryPosBits) | (uint32_t)r);
-      grow_stack(p, w, total);
-      __syncwarp();
-    }
-  }
-}
-
 // Expands the up-to-32 entries on top of the stack: one step of the worklist.
 // For tiles that register sticky states, and for --unique; the others follow
 // their paths in registers (walk_paths).
@@ -1161,8 +1037,7 @@ __device__ __forceinline__ void expand_step(const MatchParams& p, WarpSmem& ws, 
   uint4 sm = make_uint4(0u, 0u, 0u, 0u);
   uint32_t s = 0;
   if (go) {
-    sc = load_succ(tv, v);
-    if (tv.fused) sm = load_smask(tv, v);
+    load_record(tv, v, sc, sm);
     s = c.in[r + 1];
   }
   n_expanded += go;
@@ -1247,8 +1122,7 @@ __device__ __forceinline__ void walk_paths(const MatchParams& p, WarpSmem& ws, W
     uint4 sm = make_uint4(0u, 0u, 0u, 0u);
     uint32_t s = 0u;
     if (act) {
-      sc = load_succ(tv, v);
-      if (tv.fused) sm = load_smask(tv, v);
+      load_record(tv, v, sc, sm);
       s = c.in[r + 1];
     }
     n_expanded += act;
@@ -1302,8 +1176,8 @@ __device__ __forceinline__ void walk_paths(const MatchParams& p, WarpSmem& ws, W
 // A warp's view of one tile and the knobs derived from it.
 struct TileRun {
   TileView tv;
-  int depth, batch, defer, look;
-  bool layered, wide_inject, filtered;
+  int depth, batch, defer;
+  bool layered, wide_inject;
 };
 
 // Builds the view of tile t, prefix-table descriptors at pt and byte classes at
@@ -1323,11 +1197,8 @@ __device__ __forceinline__ void tile_run(const MatchParams& p, const TileDev* t,
   tv.t = t;
   tv.pt = pt;
   tv.cw = t->cw;
-  tv.narrow = t->narrow;
-  tv.fused = t->fused;
   tv.nlive = (uint32_t)t->nlive;
-  tv.rep_levels = 0u;
-  for (int d = 0; d < kMaxDepth; d++) tv.rep_levels |= (pt[d].has_reports ? 1u : 0u) << d;
+  tv.rep_levels = t->rep_levels;
   tr.depth = p.depth == 0 || t->naas == 0 ? 0 : min(p.depth, t->depth);
   tr.batch = tr.depth == 0 ? t->inj_batch0 : t->inj_batch;
   // short table lists, no sticky states: two positions per lane per injection
@@ -1338,8 +1209,6 @@ __device__ __forceinline__ void tile_run(const MatchParams& p, const TileDev* t,
   // that every position but the unit's last ones gets the full table depth.
   tr.layered = !LEAN && t->phase == 2;
   tr.defer = (tr.depth > 1 && (!tv.sticky || tr.layered)) ? tr.depth - 1 : 0;
-  tr.filtered = t->filt.len > 0;
-  tr.look = max(1, t->filt.len);
 }
 
 // Every warp takes the launch's units one by one from a global cursor, so no
@@ -1366,7 +1235,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   ws.pend_s = ws.stk_q + kStickyCap;
   ws.pend_q = ws.pend_s + kPendCap;
   ws.pend_n = ws.pend_q + kPendCap;
-  ws.cand = reinterpret_cast<int16_t*>(ws.pend_n + 4);
   if (lane == 0) *ws.pend_n = 0u;
   const int slot = blockIdx.x * kWarpsPerCta + warp;
   WarpRun w;
@@ -1391,12 +1259,12 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   bool dead = false;
   unsigned long long n_expanded = 0, n_injected = 0;
 
-  // loads window [wb, min(wb + W, hi)) plus `look` look-ahead bytes and `lb`
+  // loads window [wb, min(wb + W, hi)) plus one look-ahead byte and `lb`
   // look-behind bytes into buffer buf; returns the byte count, and in `skip`
   // the offset of wb's byte in the buffer
-  auto issue = [&](int buf, int64_t wb, int64_t hi, int lb, int look, uint32_t& skip) {
+  auto issue = [&](int buf, int64_t wb, int64_t hi, int lb, uint32_t& skip) {
     const int64_t we = min(wb + (int64_t)W, hi);
-    const int64_t end = min(we + look, hi);
+    const int64_t end = min(we + 1, hi);
     const int64_t a0 = (wb - lb) & ~(int64_t)15;
     const uint32_t bytes = (uint32_t)(((end - a0) + 15) & ~(int64_t)15);
     skip = (uint32_t)(wb - a0);
@@ -1427,7 +1295,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   auto run_unit = [&](unsigned uid, const TileDev* t, const TileRun& tr) {
     const TileView& tv = tr.tv;
     const int depth = tr.depth, batch = tr.batch, defer = tr.defer;
-    const bool layered = tr.layered, wide_inject = tr.wide_inject, filtered = tr.filtered;
+    const bool layered = tr.layered, wide_inject = tr.wide_inject;
     const UnitDev un = p.units[uid];
     const unsigned long long work0 = n_expanded + n_injected;  // per-unit trace
     if (p.unit_work && lane == 0) p.unit_cycles[uid] = clock64();  // start; the end subtracts
@@ -1438,13 +1306,12 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
     w.key_hi = un.key_hi;
     w.base = (uint32_t)un.base;
     w.act = !LEAN && t->phase == 1 ? p.act + un.act_row : nullptr;
-    const uint32_t nmatched = layered ? p.act_cnt[un.act_rowid] : 0u;
-    if (layered && !filtered) {
+    if (layered) {
       // sticky states whose first match (from the activation pass; the
       // segment's matched slots are listed at act_list) comes before the
       // unit's end: active from there on; a reporting one also reports at
       // its first match
-      const uint32_t n = nmatched;
+      const uint32_t n = p.act_cnt[un.act_rowid];
       sticky_lists(t, true, n);
       bool rep_any = false;
       for (uint32_t i0 = 0; i0 < n; i0 += 32) {
@@ -1476,12 +1343,12 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
     // nothing can become active in a layered unit without sticky states,
     // always-active states or start-of-data states at its first position
     // (such a unit runs no window: its end is moved to its start)
-    if (layered && (filtered ? nmatched == 0u : w.nstk == 0) && t->naas == 0 && !((un.flags & 1u) && t->nstart > 0))
+    if (layered && w.nstk == 0 && t->naas == 0 && !((un.flags & 1u) && t->nstart > 0))
       c.hi = un.lo;
     int cur = 0;
     uint32_t nbytes[2], skip[2];
     if (c.hi > un.lo && (int32_t)uid != p.skip_copy_unit) {
-      nbytes[0] = issue(0, un.lo, c.hi, 0, tr.look, skip[0]);
+      nbytes[0] = issue(0, un.lo, c.hi, 0, skip[0]);
     } else {  // idle, or the test hook: nothing is in flight (the hook's first wait gives up)
       nbytes[0] = 0u;
       skip[0] = 0u;
@@ -1514,8 +1381,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
       live = __any_sync(kFull, live);
       __syncwarp();
       if (we < c.hi)
-        nbytes[cur ^ 1] = issue(cur ^ 1, we, c.hi, (int)min((int64_t)defer, we - un.lo), tr.look,
-                                skip[cur ^ 1]);
+        nbytes[cur ^ 1] = issue(cur ^ 1, we, c.hi, (int)min((int64_t)defer, we - un.lo), skip[cur ^ 1]);
       c.in = ws.in[cur] + skip[cur];
       // carried states: matched at wb
       w.top = 0;
@@ -1552,46 +1418,23 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
       // the previous window (at most `defer` of them)
       // (without always-active states only plain sticky tiles have injection
       // work: their registered sticky states, batch by batch)
-      // (filtered layered tiles scan for their sticky states' successors)
-      const bool no_source = layered && filtered ? nmatched == 0u
-                                                 : t->naas == 0 && (LEAN || layered || !tv.sticky);
-      int cursor = !live || no_source ? c.iend : (int)(inj_pos - wb);
-      // filtered tiles: `cursor` is where the filter scans next (moved down to a
-      // multiple of 8 in shared memory), `first` the first position to test
-      const int first = cursor;
-      int ncand = 0;
-      if (filtered && cursor < c.iend) cursor -= (int)(smem_u32(c.in + cursor) & 7u);
+      int cursor = !live || (t->naas == 0 && (LEAN || layered || !tv.sticky))
+                       ? c.iend
+                       : (int)(inj_pos - wb);
       InjAhead ahead;  // table words of the next batch, read ahead (this window only)
       // layered tiles: next window offset of the sticky states' work
-      int scur = live && layered && !filtered && w.nstk > 0 ? 0 : c.wlen;
+      int scur = live && layered && w.nstk > 0 ? 0 : c.wlen;
       while (true) {
         // inject only when the overflow stack is empty, so that it holds at
         // most one batch's excess
         if (w.top < kInjectLow && w.ovf_n == 0) {
-          if (filtered) {
-            if (ncand < kCandLow && cursor < c.iend) {
-              ncand = filter_scan(ws, tv, c, lane, cursor, first, ncand);
-              cursor += kScanStep;
-              continue;
-            }
-            if (ncand > 0) {
-              const int m = min(ncand, !LEAN && layered ? 32 : wide_inject ? 2 * batch : batch);
-              ncand -= m;
-              if (!LEAN && layered)
-                layered_candidates(p, ws, w, tv, c, lane, ncand, m, un.act_row, nmatched);
-              else if (wide_inject)
-                inject_aas2<false, true>(p, ws, w, tv, c, lane, ncand, m, depth, n_injected, ahead);
-              else
-                inject_aas<true>(p, ws, w, tv, c, lane, ncand, m, depth, n_injected);
-              continue;
-            }
-          } else if (cursor < c.iend) {
+          if (cursor < c.iend) {
             if (wide_inject) {
-              inject_aas2<LEAN, false>(p, ws, w, tv, c, lane, cursor, 2 * batch, depth,
+              inject_aas2<LEAN>(p, ws, w, tv, c, lane, cursor, 2 * batch, depth,
                                              n_injected, ahead);
               cursor += 2 * batch;
             } else if (LEAN) {
-              inject_aas<false>(p, ws, w, tv, c, lane, cursor, batch, depth, n_injected);
+              inject_aas(p, ws, w, tv, c, lane, cursor, batch, depth, n_injected);
               cursor += batch;
             } else {
               inject(p, ws, w, tv, c, lane, cursor, batch, depth, n_injected);
@@ -1614,7 +1457,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
             __syncwarp();
             continue;
           }
-          if (cursor < c.iend || ncand > 0 || (!LEAN && scur < c.wlen)) continue;
+          if (cursor < c.iend || (!LEAN && scur < c.wlen)) continue;
           break;
         }
         // (layered tiles have no edge into a sticky state: no successor to register)

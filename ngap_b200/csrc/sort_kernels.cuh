@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kSortThreads) unique_write(
 // device-to-host copy of 64 bytes costs a call 13 us on this machine, a 64-byte
 // memset 3 us; these stores and the reset cost neither.
 constexpr int kHostReports = 1024;
-constexpr int kNumCounters = 16;
+constexpr int kNumCounters = 32;
 struct HostOut {
   unsigned long long* counters = nullptr;  // pinned, kNumCounters
   uint64_t* reports = nullptr;             // pinned, kHostReports

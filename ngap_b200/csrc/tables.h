@@ -35,9 +35,6 @@ struct TileHost {
   int32_t max_path = -1;
   int32_t num_ccs = 0;
   int32_t ncls = 0, cw = 8, nlive = 0;
-  bool narrow = true;                // 16-bit successor ids in the image
-  bool fused = false;                // wide tile of <= 32 classes: each state's successor ids and
-                                     // their class masks in one 32-byte record
   int32_t inj_batch = 32;            // positions injected per worklist refill
   int32_t inj_batch0 = 32;           // the same without prefix tables (AAS scan)
   bool global = false;               // CCs of all groups, no image budget
@@ -76,15 +73,15 @@ struct TableOpts {
   int64_t global_table_entries = 32 << 20;     // list entries per table, global tiles
 };
 
-constexpr int32_t kNarrowMaxStates = 32767;  // 15-bit tile-local ids
-
-// Bytes of a tile image with n states and cw class words, for packing CCs.
+// Size rule for packing CCs into tiles of one group: n states, cw class words
+// (8 bytes of successors per state, 16 past 32767 states; the image itself
+// holds 32-byte records).
 // Mask words per state in the planner's size rule (1, 2 or 8).
 inline int plan_class_words(int ncls) { return ncls <= 32 ? 1 : (ncls <= 64 ? 2 : 8); }
 
 inline int64_t image_bytes(int64_t n, int cw) {
   auto r16 = [](int64_t x) { return (x + 15) & ~(int64_t)15; };
-  const int64_t succ = n <= kNarrowMaxStates ? n * 8 : n * 16;
+  const int64_t succ = n <= 32767 ? n * 8 : n * 16;
   return r16(succ) + r16(n * cw * 4) + 2 * r16(((n + 31) / 32) * 4) + 256;
 }
 

@@ -5,7 +5,7 @@ random and accepted class strings through the tile's graph from the states it
 injects: a path that is alive after `len` symbols, or a report within them,
 needs its bit set, and no report may come before `min_rep` symbols.
 GPU: matches against the oracle at sizes around the filter's lengths, scan
-steps and unit ends.
+steps, pieces and segment ends.
 """
 import os
 import shutil
@@ -192,6 +192,11 @@ def test_filter_covers_every_path(checker, tmp_path, name, groups, mode):
         assert filters > 0 and clear > 0.5, r.stdout
 
 
+# inputs of 128 Ki positions and more are scanned, shorter ones looked up position
+# by position (unless their tables' lists are long)
+LENGTH = 165_000
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("name", ["hamming", "motif", "dotstar", "dense", "mixed", "wide"])
 def test_filtered_matches(engine, name):
@@ -199,20 +204,21 @@ def test_filtered_matches(engine, name):
     groups = nb.Groups(nb.Nfa.from_string(anml), group_num=2)
     rng = np.random.default_rng(17)
     alpha = W.ACGT if name in ("hamming", "motif") else W.PRINTABLE
-    gen = {"hamming": lambda: W.hamming_set(seed=3, n_patterns=30, input_len=6000, plant_every=97)[1],
-           "motif": lambda: W.hamming_set(seed=4, n_patterns=40, k=8, d=1, input_len=6000,
+    gen = {"hamming": lambda: W.hamming_set(seed=3, n_patterns=30, input_len=LENGTH, plant_every=97)[1],
+           "motif": lambda: W.hamming_set(seed=4, n_patterns=40, k=8, d=1, input_len=LENGTH,
                                           plant_every=61)[1],
-           "dotstar": lambda: W.dotstar_set(seed=6, n_patterns=60, input_len=6000, plant_every=97)[1]}
-    data = gen[name]() if name in gen else rng.choice(W.PRINTABLE[:20], size=6000).astype(np.uint8)
+           "dotstar": lambda: W.dotstar_set(seed=6, n_patterns=60, input_len=LENGTH, plant_every=97)[1]}
+    data = gen[name]() if name in gen else rng.choice(W.PRINTABLE[:20], size=LENGTH).astype(np.uint8)
     if name == "wide":
-        data = rng.choice(BYTES, size=6000, p=BYTES_LAW).astype(np.uint8)
+        data = rng.choice(BYTES, size=LENGTH, p=BYTES_LAW).astype(np.uint8)
     data = data.copy()
-    data[rng.integers(0, len(data), 40)] = rng.choice(alpha, size=40)
+    data[rng.integers(0, len(data), 800)] = rng.choice(alpha, size=800)
     data[1000:1040] = 0  # bytes no state accepts
     some = 0
     for mode, depth in (("shared", 1), ("shared", 3), ("global", -1)):
         tables = nb.Tables(groups, precompute_depth=depth, tile_mode=mode)
-        for num_seg, seg_len in ((1, 1), (3, 15), (2, 17), (1, 255), (1, 257), (2, 2065), (1, 5999)):
+        for num_seg, seg_len in ((1, 1), (3, 15), (1, 257), (2, 2065), (5003, 31), (1201, 113), (517, 257),
+                                 (38, 4099), (1, 163_841)):
             for algo, chunk, window in (("nonblockingpcgroups", 0, 0), ("nonblockingallgroups", 33, 64),
                                         ("NAPgroups", 300, 0), ("nonblockinggroups", 0, 100)):
                 got = engine.match(tables, data[:num_seg * seg_len], num_seg, seg_len, algorithm=algo,
