@@ -353,10 +353,8 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
     d.filt.len = th.filt.len;
     d.filt.min_rep = th.filt.min_rep;
     d.filt.shift = th.filt.shift;
-    d.filt.mul = th.filt.mul;
-    d.filt.scale = th.filt.scale;
     d.filt.drop = th.filt.drop;
-    if ((rc = t->upload(th.filt.bits, &d.filt.bits)) != NGAP_OK) return rc;
+    if ((rc = t->upload(th.filt.blocks, &d.filt.blocks)) != NGAP_OK) return rc;
     for (int k = 0; k < kMaxDepth; k++) {
       const PrefixTableHost& ph = th.pt[k];
       PrefixTableDev& pd = d.pt[k];

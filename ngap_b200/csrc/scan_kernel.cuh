@@ -10,7 +10,7 @@
 //    tables (or the active sticky states of a layered tile) and follows their
 //    paths in registers to their end, reading the input in place.
 // The two have opposite needs, which is why they are two kernels: the scan is
-// one bitmap read per position (a gather, which takes the L1 tag stage once per
+// one filter block read per position (a gather, which takes the L1 tag stage once per
 // lane: 32 warps with eight reads per lane in flight keep L1 84 % busy on the
 // 25-mers, 78 us for 16.8 M positions, 215 G positions/s) with few instructions;
 // runs are chains of dependent reads that want many warps and full lanes. In
@@ -118,14 +118,15 @@ __global__ void __launch_bounds__(kScanWarps * 32, 1) scan_kernel(ScanParams p) 
       __syncwarp();
       const uint8_t* in = sym + kScanLane * lane;
       uint32_t h = 0u;
-      for (int i = 0; i < f.len - 1; i++) h = h * f.mul + in[i];
-      uint32_t idx[kScanLane], word[kScanLane];
+      for (int i = 0; i < f.len - 1; i++) h = h * kFilterMul + in[i];
+      uint32_t hash[kScanLane];
+      uint2 block[kScanLane];
       unsigned found = 0u, test = 0u;
 #pragma unroll
       for (int j = 0; j < kScanLane; j++) {
-        h = h * f.mul + in[f.len - 1 + j];  // a symbol enters, and the one before the lane's j-th leaves
+        h = h * kFilterMul + in[f.len - 1 + j];  // a symbol enters, and the one before the lane's j-th leaves
         if (j > 0) h -= __byte_perm(j <= 4 ? cur.x : cur.y, 0, 0x4440 | ((j - 1) & 3)) * f.drop;
-        idx[j] = (h * f.scale) >> f.shift;
+        hash[j] = h;
         const uint32_t q = o + j;
         const int left = (int)(pc.end - q);  // symbols left in the segment
         const bool live = q >= pc.lo && q < pc.hi &&
@@ -135,9 +136,16 @@ __global__ void __launch_bounds__(kScanWarps * 32, 1) scan_kernel(ScanParams p) 
       }
 #pragma unroll
       for (int j = 0; j < kScanLane; j++)
-        word[j] = (test >> j) & 1u ? __ldg(f.bits + (idx[j] >> 5)) : 0u;
+        block[j] = (test >> j) & 1u
+                       ? __ldg(reinterpret_cast<const uint2*>(f.blocks) + ((hash[j] * kFilterBlock) >> f.shift))
+                       : make_uint2(0u, 0u);
 #pragma unroll
-      for (int j = 0; j < kScanLane; j++) found |= ((word[j] >> (idx[j] & 31)) & 1u) << j;
+      for (int j = 0; j < kScanLane; j++) {  // filter_mask's three bits, rotated to bit 0
+        const uint32_t x = (hash[j] * kFilterBits) >> 17;
+        found |= (__funnelshift_r(block[j].x, block[j].x, x) & __funnelshift_r(block[j].x, block[j].x, x >> 5) &
+                  __funnelshift_r(block[j].y, block[j].y, x >> 10) & 1u)
+                 << j;
+      }
       pass[step * 32 + lane] = (uint8_t)found;
       cur = nxt;
       __syncwarp();

@@ -834,7 +834,6 @@ std::vector<uint32_t> filter_sources(const TileHost& t) {
 
 struct FilterPlan {
   int len = 0, fbits = 0, min_rep = 0;
-  bool exact = false;
 };
 
 // Chooses how many symbols the filter looks ahead and its size from the
@@ -845,11 +844,12 @@ struct FilterPlan {
 // likely in small alphabets; over text (more than 8 classes) symbol laws are
 // skewed, and a symbol is taken to agree with probability L^-0.6 (a Zipf law
 // over 95 symbols agrees with itself with probability 0.07 = 95^-0.6).
-// Bounds: 2^28 bits (32 MB: the bitmap stays in the 126 MB L2), 32 bits per
-// key (3 % false positives), more while it fits L1 beside the kernel's shared
-// memory (kCachedBits), and kVisits steps of the walk that sets the bits.
+// Bounds: 2^28 bits (32 MB: the blocks stay in the 126 MB L2), 16 bits per key
+// (0.6 % false positives; one bit per key in 32 gave 3 %), up to 64 while it
+// fits L1 beside the kernel's shared memory (kCachedBits), and kVisits steps
+// of the walk that sets the bits.
 FilterPlan plan_filter(const TileHost& t, const std::vector<uint32_t>& src) {
-  constexpr double kVisits = 48e6, kFills = 4e6;
+  constexpr double kVisits = 80e6, kFills = 4e6;
   constexpr int kMaxBits = 28, kCachedBits = 18, kMinBits = 15;
   FilterPlan best;
   double best_est = 0.5;  // a filter that half of the positions pass saves too little
@@ -885,12 +885,12 @@ FilterPlan plan_filter(const TileHost& t, const std::vector<uint32_t>& src) {
     if (visits > kVisits || fills > kFills) break;
     pass_rep += rep * std::pow(pe, d);
     const double keys = fills + alive + rep;
-    const double space = std::pow(L, d);
-    const bool exact = space <= (double)(1u << kMaxBits) && space <= 32 * std::max(keys, 1024.0);
     int fbits = kMinBits;
-    while (fbits < kMaxBits && std::pow(2.0, fbits) < (exact ? space : 32 * keys)) fbits++;
-    while (!exact && fbits < kCachedBits && std::pow(2.0, fbits) < 512 * keys) fbits++;
-    const double fp = exact ? 0.0 : keys / std::pow(2.0, fbits);
+    while (fbits < kMaxBits && std::pow(2.0, fbits) < 16 * keys) fbits++;
+    while (fbits < kCachedBits && std::pow(2.0, fbits) < 64 * keys) fbits++;
+    const double load = keys * 64 / std::pow(2.0, fbits);  // keys per block
+    const double lo = 1 - std::exp(-load * 2 / 32), hi = 1 - std::exp(-load / 32);
+    const double fp = lo * lo * hi;
     const double est = pass_rep + alive * std::pow(pe, d) + fp;
     // a longer filter has to gain: its bits cost time to set and room in L2
     // (a candidate of a layered tile is dear: it is tested against every
@@ -899,7 +899,6 @@ FilterPlan plan_filter(const TileHost& t, const std::vector<uint32_t>& src) {
       best_est = est;
       best.len = d;
       best.fbits = fbits;
-      best.exact = exact;
     }
     if (alive <= 0) break;  // every path has reported or ended
     // next level: paths that have reported stand for all their continuations
@@ -927,17 +926,14 @@ void build_filter(TileHost& t) {
   f.len = pl.len;
   // no report within kMaxFilter symbols: more are needed than a filter looks ahead
   f.min_rep = pl.min_rep > 0 ? pl.min_rep : kMaxFilter + 1;
-  f.shift = 32 - pl.fbits;
-  f.mul = pl.exact ? (uint32_t)t.nlive : kFilterMul;
-  f.scale = pl.exact ? 1u << f.shift : kFilterScale;
+  f.shift = 32 - (pl.fbits - 6);
   f.drop = 1;
-  for (int i = 0; i < f.len; i++) f.drop *= f.mul;
-  f.bits.assign((size_t)1 << (pl.fbits > 5 ? pl.fbits - 5 : 0), 0);
+  for (int i = 0; i < f.len; i++) f.drop *= kFilterMul;
+  f.blocks.assign((size_t)1 << (pl.fbits - 6), 0);
   auto set = [&](uint32_t h) {
-    const uint32_t b = (h * f.scale) >> f.shift;
-    uint32_t* w = &f.bits[b >> 5];
-    const uint32_t m = 1u << (b & 31);
-    if (!(__atomic_load_n(w, __ATOMIC_RELAXED) & m)) __atomic_fetch_or(w, m, __ATOMIC_RELAXED);
+    uint64_t* w = &f.blocks[(h * kFilterBlock) >> f.shift];
+    const uint64_t m = filter_mask(h);
+    if ((__atomic_load_n(w, __ATOMIC_RELAXED) & m) != m) __atomic_fetch_or(w, m, __ATOMIC_RELAXED);
   };
   // class ids each state accepts, as a flat list
   std::vector<uint32_t> coff(t.nstates + 1, 0);
@@ -950,7 +946,7 @@ void build_filter(TileHost& t) {
   // every continuation (the dead class included) of a path that has reported
   std::function<void(int, uint32_t)> fill = [&](int d, uint32_t h) {
     if (d == f.len) return set(h);
-    for (int c = 0; c < t.ncls; c++) fill(d + 1, h * f.mul + (uint32_t)c);
+    for (int c = 0; c < t.ncls; c++) fill(d + 1, h * kFilterMul + (uint32_t)c);
   };
   // h: hash of the d symbols read, the last of which v matched
   std::function<void(uint32_t, int, uint32_t)> walk = [&](uint32_t v, int d, uint32_t h) {
@@ -959,7 +955,7 @@ void build_filter(TileHost& t) {
       uint32_t u = t.succ[(size_t)v * 4 + k];
       if (u == kNoSucc) continue;
       u &= 0x7fffffffu;
-      for (uint32_t i = coff[u]; i < coff[u + 1]; i++) walk(u, d + 1, h * f.mul + clist[i]);
+      for (uint32_t i = coff[u]; i < coff[u + 1]; i++) walk(u, d + 1, h * kFilterMul + clist[i]);
     }
   };
   std::atomic<size_t> next{0};

@@ -24,8 +24,8 @@ struct PrefixTableHost {
 // Host form of FilterDev.
 struct FilterHost {
   int32_t len = 0, min_rep = 1, shift = 0;
-  uint32_t mul = 0, scale = 0, drop = 0;
-  std::vector<uint32_t> bits;
+  uint32_t drop = 0;
+  std::vector<uint64_t> blocks;
 };
 
 struct TileHost {

@@ -97,9 +97,9 @@ int main(int argc, char** argv) {
       }
       need = need || !cur.empty();
       uint32_t h = 0;
-      for (int c : s) h = h * f.mul + (uint32_t)c;
-      const uint32_t b = (h * f.scale) >> f.shift;
-      const bool set = (f.bits[b >> 5] >> (b & 31)) & 1u;
+      for (int c : s) h = h * kFilterMul + (uint32_t)c;
+      const uint64_t m = filter_mask(h);
+      const bool set = (f.blocks[(h * kFilterBlock) >> f.shift] & m) == m;
       if (need && !set) return printf("tile phase %d: a needed position is filtered out\n", t.phase), 1;
       if (!(it & 1)) {
         total++;
