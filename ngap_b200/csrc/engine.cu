@@ -140,6 +140,7 @@ struct Slice {
   int64_t runs;     // most runs they can give
   bool layered;
   int32_t one_tile; // the one tile of the pieces, or -1
+  int64_t longest = 0;  // positions of the longest piece
 };
 
 // What the launches of a plan run: units of the three launches of
@@ -407,6 +408,8 @@ int ngap_engine_create(int device, ngap_engine** out) {
                                 kSmallSortSmem));
   CUDA_TRY(cudaFuncSetAttribute(sort_unique_cta<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSmallSortSmem));
+  CUDA_TRY(cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kScanWarps * kScanWarpBytes));
   CUDA_TRY(cudaFuncSetAttribute(run_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 run_smem_bytes()));
   CUDA_TRY(cudaFuncSetAttribute(run_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -598,11 +601,13 @@ struct AutoChunk {
 };
 
 // Length of a filtered tile's pieces: one per scan warp for short inputs, and
-// not below a scan step (256 positions); a caller's chunk length bounds it.
+// not below one step of a warp (256 positions); a caller's chunk length bounds it.
 int64_t piece_len(int64_t positions, int64_t warps, int64_t chunk_opt) {
-  int64_t n = ((positions + warps - 1) / warps + kScanStep - 1) / kScanStep * kScanStep;
+  int64_t n = (positions + warps - 1) / warps;
+  const int64_t step = n > kScanMinPiece ? 32 * kStripMax : kScanMinPiece;
+  n = (n + step - 1) / step * step;
   if (chunk_opt > 0) n = std::min(n, chunk_opt);
-  return std::max<int64_t>(kScanStep, std::min<int64_t>(n, kPieceMax));
+  return std::max<int64_t>(kScanMinPiece, std::min<int64_t>(n, kPieceMax));
 }
 
 // Tiles that are scanned: acyclic ones with a filter, in plans with at least
@@ -633,9 +638,11 @@ void add_pieces(const TileHost& th, int tile, const SegSpec& s, int64_t len,
   p.act_rowid = act.second;
   p.pad = s.index;
   const bool starts = s.starts && !th.start.empty();
-  for (int64_t lo = s.lo; lo < s.hi; lo += len) {
+  int64_t hi = s.lo;
+  for (int64_t lo = s.lo; lo < s.hi; lo = hi) {
+    hi = std::min((lo + len) & ~(int64_t)7, s.hi);  // later pieces start where the scan reads, at multiples of 8
     p.lo = (uint32_t)lo;
-    p.hi = (uint32_t)std::min(lo + len, s.hi);
+    p.hi = (uint32_t)hi;
     p.flags = starts && lo == s.lo ? 1u : 0u;
     pieces[th.phase == 2 ? 1 : 0].push_back(p);
   }
@@ -664,6 +671,7 @@ std::vector<Slice> make_slices(const std::vector<PieceDev> pieces[2],
       out.back().count++;
       out.back().runs += r;
       pos += n;
+      out.back().longest = std::max(out.back().longest, n);
       *cands = std::max(*cands, pos);
       *runs = std::max(*runs, out.back().runs);
     }
@@ -1005,7 +1013,9 @@ int launch_plan(ngap_engine* e, MatchParams mp, const std::vector<TileDev>& tile
         sp.run_len = td.run_len;
         sp.phase = td.phase;
       }
-      scan_kernel<<<launch_grid(s.count, e->grid), kScanWarps * 32, 0, st>>>(sp);
+      // strips of 16 where a piece fills the warp with them
+      sp.strip_bits = s.longest >= 32 * kStripMax ? 4 : 3;
+      scan_kernel<<<launch_grid(s.count, e->grid), kScanWarps * 32, kScanWarps * kScanWarpBytes, st>>>(sp);
       const int grid = launch_grid(s.runs, e->grid);
       if (layered)
         run_kernel<true><<<grid, kRunWarps * 32, run_smem_bytes(), st>>>(mp, e->d_cand, e->d_runs, ctl);

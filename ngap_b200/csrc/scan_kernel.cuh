@@ -29,9 +29,15 @@ namespace ngap {
 constexpr int kPieceMax = 4096;  // run entries pack offsets below kPieceMax + the longest path
 static_assert(kPieceMax + 2048 + kMaxDepth < kMaxWindow, "offsets fit worklist entries");
 constexpr int kScanWarps = 32;
-constexpr int kScanLane = 8;     // consecutive positions per lane and step
-constexpr int kScanStep = 32 * kScanLane;
-
+constexpr int kScanLane = 8;     // positions per lane and step: reads in flight
+constexpr int kScanMinPiece = 32 * kScanLane;
+constexpr int kStripMax = 16;    // consecutive positions per lane (a strip)
+// Per warp: class ids of 33 strips (4 bytes apart, so that lanes reading their
+// strips word by word hit 32 banks), byte classes, one bit per position.
+constexpr int kScanSymBytes = (33 * (kStripMax + 4) + 15) / 16 * 16;
+constexpr int kScanPassBytes = (kPieceMax + 32 * kStripMax) / 8;
+constexpr int kScanWarpBytes = kScanSymBytes + 256 + kScanPassBytes;
+static_assert(kScanWarpBytes % 16 == 0, "per-warp regions stay 16-byte aligned");
 // Control words of one scan and its runs (zeroed before the scan).
 enum { kCtlPieces = 0, kCtlCands = 1, kCtlRuns = 2, kCtlTaken = 3, kCtlWords = 4 };
 
@@ -50,6 +56,7 @@ struct ScanParams {
   const uint8_t* cls;
   uint32_t nlive;
   int32_t run_len, phase;
+  int32_t strip_bits;       // log2 of the positions per lane (3 or 4)
   unsigned long long* cycles;  // per piece (tracing), or null
 };
 
@@ -62,27 +69,34 @@ __device__ __forceinline__ unsigned next_index(unsigned int* counter, unsigned w
   return __shfl_sync(kFull, k, 0);
 }
 
+// The scan. A lane owns a strip of 8 or 16 consecutive positions, whose hash it
+// rolls: two words of class ids per four positions and two multiply-adds per
+// position. Longer strips have fewer instructions, but their symbols take L1 from
+// the filters: match times on a B200 with strips of 8, 16, 32 and 64: 512
+// streams 2.68, 2.60, 2.72, 3.00 ms; the 32 MiB mix 552, 519, 505, 505 us; 300
+// dot-star regexes 116, 107, 110, 118 us. (Filters of up to 64 KB copied to
+// shared memory gained the mix 1 % and nothing else: not kept.)
 __global__ void __launch_bounds__(kScanWarps * 32, 1) scan_kernel(ScanParams p) {
-  __shared__ __align__(16) uint8_t s_cls[kScanWarps][256];
-  __shared__ __align__(16) uint8_t s_sym[kScanWarps][kScanStep + 16];
-  __shared__ __align__(16) uint8_t s_pass[kScanWarps][(kPieceMax + kScanStep) / 8];
+  extern __shared__ __align__(16) uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint8_t* cls = s_cls[warp];
-  uint8_t* sym = s_sym[warp];
-  uint8_t* pass = s_pass[warp];
+  uint8_t* sym = smem_raw + warp * kScanWarpBytes;
+  uint8_t* cls = sym + kScanSymBytes;
+  uint8_t* pass = cls + 256;
   int staged = -1;  // the tile whose classes are in cls
   // eight input bytes as class ids
   auto load = [&](uint32_t at) {
     return at < p.readable ? __ldg(reinterpret_cast<const uint2*>(p.input + at)) : make_uint2(0u, 0u);
   };
-  auto classes = [&](uint2 b) {
-    uint2 c;
-    c.x = cls[b.x & 0xff] | cls[(b.x >> 8) & 0xff] << 8 | cls[(b.x >> 16) & 0xff] << 16 |
-          (uint32_t)cls[b.x >> 24] << 24;
-    c.y = cls[b.y & 0xff] | cls[(b.y >> 8) & 0xff] << 8 | cls[(b.y >> 16) & 0xff] << 16 |
-          (uint32_t)cls[b.y >> 24] << 24;
-    return c;
+  auto classes = [&](uint32_t b) {
+    return cls[b & 0xff] | cls[(b >> 8) & 0xff] << 8 | cls[(b >> 16) & 0xff] << 16 |
+           (uint32_t)cls[b >> 24] << 24;
   };
+  const int sb = p.strip_bits, strip = 1 << sb;
+  const uint32_t block_len = 32u << sb;  // positions per pass over the strips
+  // class id i of the lane's strip and the ones after it, or the word that holds ids i .. i + 3
+  const uint8_t* mine = sym + lane * (strip + 4);
+  auto at = [&](int i) { return mine + i + ((i >> sb) << 2); };
+  auto word_at = [&](int i) { return *reinterpret_cast<const uint32_t*>(at(i)); };
   // the first piece of a warp is its own number (spread over the CTAs), the
   // later ones come from a counter: short inputs start without an atomic
   unsigned k = warp * gridDim.x + blockIdx.x;
@@ -108,50 +122,72 @@ __global__ void __launch_bounds__(kScanWarps * 32, 1) scan_kernel(ScanParams p) 
       __syncwarp();
     }
     const uint32_t a0 = pc.lo & ~7u;
-    const int nsteps = (int)((pc.hi - a0 + kScanStep - 1) / kScanStep);
-    uint2 cur = classes(load(a0 + 8u * lane));
-    for (int step = 0; step < nsteps; step++) {
-      const uint32_t o = a0 + (uint32_t)(step * kScanStep + kScanLane * lane);
-      const uint2 nxt = classes(load(o + kScanStep));
-      reinterpret_cast<uint2*>(sym)[lane] = cur;
-      if (lane < 2) reinterpret_cast<uint2*>(sym + kScanStep)[lane] = nxt;
+    const int nblocks = (int)((pc.hi - a0 + block_len - 1) >> (5 + sb));
+    for (int b = 0; b < nblocks; b++) {
+      const uint32_t o = a0 + (uint32_t)b * block_len;
       __syncwarp();
-      const uint8_t* in = sym + kScanLane * lane;
-      uint32_t h = 0u;
-      for (int i = 0; i < f.len - 1; i++) h = h * kFilterMul + in[i];
-      uint32_t hash[kScanLane];
-      uint2 block[kScanLane];
-      unsigned found = 0u, test = 0u;
-#pragma unroll
-      for (int j = 0; j < kScanLane; j++) {
-        h = h * kFilterMul + in[f.len - 1 + j];  // a symbol enters, and the one before the lane's j-th leaves
-        if (j > 0) h -= __byte_perm(j <= 4 ? cur.x : cur.y, 0, 0x4440 | ((j - 1) & 3)) * f.drop;
-        hash[j] = h;
-        const uint32_t q = o + j;
-        const int left = (int)(pc.end - q);  // symbols left in the segment
-        const bool live = q >= pc.lo && q < pc.hi &&
-                          __byte_perm(j < 4 ? cur.x : cur.y, 0, 0x4440 | (j & 3)) < nlive;
-        if (live && left >= f.len) test |= 1u << j;
-        else if (live && left >= f.min_rep) found |= 1u << j;
+      for (uint32_t c = lane; c < (block_len + 16) / 8; c += 32) {
+        const uint2 in = load(o + 8 * c);
+        uint32_t* dst = reinterpret_cast<uint32_t*>(sym + 8 * c + (((8 * c) >> sb) << 2));
+        dst[0] = classes(in.x);
+        dst[1] = classes(in.y);
       }
-#pragma unroll
-      for (int j = 0; j < kScanLane; j++)
-        block[j] = (test >> j) & 1u
-                       ? __ldg(reinterpret_cast<const uint2*>(f.blocks) + ((hash[j] * kFilterBlock) >> f.shift))
-                       : make_uint2(0u, 0u);
-#pragma unroll
-      for (int j = 0; j < kScanLane; j++) {  // filter_mask's three bits, rotated to bit 0
-        const uint32_t x = (hash[j] * kFilterBits) >> 17;
-        found |= (__funnelshift_r(block[j].x, block[j].x, x) & __funnelshift_r(block[j].x, block[j].x, x >> 5) &
-                  __funnelshift_r(block[j].y, block[j].y, x >> 10) & 1u)
-                 << j;
-      }
-      pass[step * 32 + lane] = (uint8_t)found;
-      cur = nxt;
       __syncwarp();
+      const uint32_t own = o + ((uint32_t)lane << sb);  // the lane's first position
+      // whole passes inside the piece with all of the filter's symbols left need no bounds per position
+      const bool inside = o >= pc.lo && o + block_len <= pc.hi && pc.end - (o + block_len - 1) >= (uint32_t)f.len;
+      uint32_t h = 0u, left = 0u;  // left: the id that leaves before the next position
+      for (int i = 0; i < f.len - 1; i++) h = h * kFilterMul + *at(i);
+      const int w0 = (f.len - 1) & ~3, sh = ((f.len - 1) & 3) * 8;
+      uint32_t next = word_at(w0);
+      for (int i = 0; i < strip; i += kScanLane) {
+        uint32_t hash[kScanLane];
+        unsigned test = 0xffu, found = 0u;
+#pragma unroll
+        for (int g = 0; g < kScanLane / 4; g++) {
+          const uint32_t out = word_at(i + 4 * g);
+          const uint32_t w = next;
+          next = word_at(w0 + i + 4 * g + 4);
+          const uint32_t in = __funnelshift_r(w, next, sh);
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            h = h * kFilterMul + (__byte_perm(in, 0, 0x4440 | j) - left * f.drop);
+            left = __byte_perm(out, 0, 0x4440 | j);
+            hash[4 * g + j] = h;
+          }
+          // positions whose own byte no state accepts need no read
+          const uint32_t dead = nlive > 255u ? 0u : __vcmpgeu4(out, nlive * 0x01010101u) & 0x01010101u;
+          test &= ~(((dead * 0x01020408u) >> 24 & 0xfu) << (4 * g));
+        }
+        if (!inside) {
+#pragma unroll
+          for (int j = 0; j < kScanLane; j++) {
+            const uint32_t q = own + (uint32_t)(i + j);
+            const bool in_piece = q >= pc.lo && q < pc.hi;
+            const bool whole = in_piece && (int)(pc.end - q) >= f.len;
+            if (in_piece && !whole && ((test >> j) & 1u) && (int)(pc.end - q) >= f.min_rep) found |= 1u << j;
+            if (!whole) test &= ~(1u << j);
+          }
+        }
+        uint2 block[kScanLane];
+#pragma unroll
+        for (int j = 0; j < kScanLane; j++) {
+          const uint2* at = reinterpret_cast<const uint2*>(f.blocks) + ((hash[j] * kFilterBlock) >> f.shift);
+          block[j] = (test >> j) & 1u ? __ldg(at) : make_uint2(0u, 0u);
+        }
+#pragma unroll
+        for (int j = 0; j < kScanLane; j++) {  // filter_mask's three bits, rotated to bit 0
+          const uint32_t x = (hash[j] * kFilterBits) >> 17;
+          found |= (__funnelshift_r(block[j].x, block[j].x, x) & __funnelshift_r(block[j].x, block[j].x, x >> 5) &
+                    __funnelshift_r(block[j].y, block[j].y, x >> 10) & 1u)
+                   << j;
+        }
+        pass[(((uint32_t)b * block_len + ((uint32_t)lane << sb)) + (uint32_t)i) >> 3] = (uint8_t)found;
+      }
     }
+    __syncwarp();
     // the piece's candidates, in order, to the list; their runs
-    const int nwords = nsteps * (kScanStep / 32);
+    const int nwords = nblocks << sb;
     const uint32_t* words = reinterpret_cast<const uint32_t*>(pass);
     uint32_t mine = 0;
     for (int i = lane; i < nwords; i += 32) mine += __popc(words[i]);

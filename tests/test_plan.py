@@ -44,7 +44,7 @@ def test_auto_lengths(engine, num_seg, seg_len, filtered):
             assert u["lo"][0] == 0 and u["hi"][-1] == seg_len
             assert np.array_equal(u["lo"][1:], u["hi"][:-1])
         longest = int((units["hi"] - units["lo"]).max())
-        if filtered and n >= 1 << 17:  # one piece per scan warp (32 per SM), in steps of 256 positions
-            assert longest <= min(4096, max(256, -(-n // (148 * 32)) + 255))
+        if filtered and n >= 1 << 17:  # one piece per scan warp (32 per SM), in steps of 512 positions
+            assert longest <= min(4096, max(256, -(-n // (148 * 32)) + 511))
         else:  # one unit per warp (16 per SM), or 128 positions where that is longer
             assert longest <= min(2048, max(128, -(-n // (148 * 16)) + 63))
