@@ -162,6 +162,14 @@ def wide_dotstar(rng, n):
     return w.text()
 
 
+def mixed_alphabets(seed):
+    """Edit-distance rules over ACGT beside dot-star rules over text: (ANML, input)."""
+    w, rng = W.AnmlWriter("mix"), np.random.default_rng(seed)
+    _, dna = W.levenshtein_set(n_patterns=12, input_len=80_000, plant_every=997, writer=w, rng=rng)
+    _, text = W.dotstar_set(n_patterns=60, input_len=85_000, plant_every=997, writer=w, rng=rng)
+    return w.text(), np.concatenate([dna, text])
+
+
 def rule_sets():
     rng = np.random.default_rng(31)
     kw = dict(input_len=1 << 12, plant_every=1 << 8)
@@ -174,6 +182,7 @@ def rule_sets():
         "short": short_rules(rng, 12, 2, 9, W.PRINTABLE),
         "dense": short_rules(rng, 30, 1, 4, W.PRINTABLE[:20]),
         "one": short_rules(rng, 3, 1, 1, W.PRINTABLE),
+        "mix": mixed_alphabets(33)[0],
         "wide": wide_dotstar(np.random.default_rng(32), 400),
         "mixed": short_rules(rng, 60, 3, 20, W.PRINTABLE[:20]),
     }
@@ -192,13 +201,27 @@ def test_filter_covers_every_path(checker, tmp_path, name, groups, mode):
         assert filters > 0 and clear > 0.5, r.stdout
 
 
+@pytest.mark.parametrize("groups,mode", [(1, "shared"), (1, "auto")])
+def test_small_alphabets_get_their_own_tiles(built, groups, mode):
+    both = nb.Groups(nb.Nfa.from_string(mixed_alphabets(33)[0]), group_num=groups)
+    lev = W.levenshtein_set(n_patterns=12, input_len=1 << 12, plant_every=1 << 8)[0]
+    states = sum(t["num_states"] for t in nb.Groups(nb.Nfa.from_string(lev), group_num=groups).tiles())
+    tiles = both.tiles(tile_mode=mode)
+    dna = [t for t in tiles if t["phase"] == 0 and t["nlive"] == 4]
+    assert len(dna) == groups and sum(t["num_states"] for t in dna) == states
+    assert all(t["nlive"] > 8 for t in tiles if t not in dna)
+    # one alphabet alone stays one tile per group
+    alone = nb.Groups(nb.Nfa.from_string(lev), group_num=1).tiles(tile_mode="shared")
+    assert len(alone) == 1
+
+
 # inputs of 128 Ki positions and more are scanned, shorter ones looked up position
 # by position (unless their tables' lists are long)
 LENGTH = 165_000
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("name", ["hamming", "motif", "dotstar", "dense", "mixed", "wide"])
+@pytest.mark.parametrize("name", ["hamming", "motif", "dotstar", "dense", "mixed", "mix", "wide"])
 def test_filtered_matches(engine, name):
     anml = rule_sets()[name]
     groups = nb.Groups(nb.Nfa.from_string(anml), group_num=2)
@@ -207,6 +230,7 @@ def test_filtered_matches(engine, name):
     gen = {"hamming": lambda: W.hamming_set(seed=3, n_patterns=30, input_len=LENGTH, plant_every=97)[1],
            "motif": lambda: W.hamming_set(seed=4, n_patterns=40, k=8, d=1, input_len=LENGTH,
                                           plant_every=61)[1],
+           "mix": lambda: mixed_alphabets(33)[1],
            "dotstar": lambda: W.dotstar_set(seed=6, n_patterns=60, input_len=LENGTH, plant_every=97)[1]}
     data = gen[name]() if name in gen else rng.choice(W.PRINTABLE[:20], size=LENGTH).astype(np.uint8)
     if name == "wide":
