@@ -194,7 +194,9 @@ typedef struct ngap_match_params {
  * report copy: matches `input` (host or device memory, num_seg * seg_len
  * bytes) against every group and leaves the sorted, deduplicated reports on
  * the device. Asynchronous on `stream` (a cudaStream_t, NULL = default);
- * ngap_engine_sync waits and returns the run's status. */
+ * ngap_engine_sync waits and returns the run's status. `input` must stay
+ * unchanged until the match has ended on `stream`: device memory is read in
+ * place when its address and length are multiples of 16. */
 int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int input_on_device,
                const ngap_match_params* p, void* stream);
 int ngap_engine_sync(ngap_engine* e);
@@ -305,7 +307,8 @@ typedef struct ngap_batch_params {
 
 /* Matches every stream against its NFA in one persistent launch, then sorts
  * the reports by (stream, offset, id) on the device. Asynchronous on stream;
- * ngap_engine_sync waits. Offsets in the results are local to each stream. */
+ * ngap_engine_sync waits. Offsets in the results are local to each stream.
+ * `input` must stay unchanged until the match has ended, as in ngap_match. */
 int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* input,
                      uint64_t input_bytes, int input_on_device, const ngap_batch_stream* streams,
                      int nstreams, const ngap_batch_params* p, void* stream);

@@ -493,6 +493,26 @@ int upload_plan(ngap_engine* e, cudaStream_t st, const std::vector<Upload>& part
   return NGAP_OK;
 }
 
+// Whether a match reads its input where the caller has it: device memory whose
+// start and length are multiples of 16, so that the kernels' 16-byte reads and
+// bulk copies stay inside it. Otherwise it is copied into the engine's padded
+// buffer (16 MiB: 10 us of a 190 us call on a B200).
+bool input_in_place(const uint8_t* input, int on_device, uint64_t bytes) {
+  return on_device && bytes > 0 && bytes % 16 == 0 && reinterpret_cast<uintptr_t>(input) % 16 == 0;
+}
+
+// The engine's input buffer, padded for those reads.
+int ensure_input(ngap_engine* e, uint64_t bytes) {
+  const size_t need = ((bytes + 15) & ~(uint64_t)15) + 64;
+  if (need <= e->input_cap) return NGAP_OK;
+  cudaFree(e->d_input);
+  e->d_input = nullptr;
+  e->input_cap = 0;
+  CUDA_TRY(cudaMalloc(&e->d_input, need));
+  e->input_cap = need;
+  return NGAP_OK;
+}
+
 int ensure_reports(ngap_engine* e, uint64_t cap) {
   if (cap <= e->rep_cap) return NGAP_OK;
   cudaFree(e->d_reports);
@@ -1358,15 +1378,8 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   int rc = algo_config(p->algorithm, table_depth, &depth);
   if (rc != NGAP_OK) return rc;
   window = std::min(window, kMaxWindow);
-  // input: own 16-byte-aligned, padded copy
-  size_t need = ((total + 15) & ~(uint64_t)15) + 64;
-  if (need > e->input_cap) {
-    cudaFree(e->d_input);
-    e->d_input = nullptr;
-    e->input_cap = 0;
-    CUDA_TRY(cudaMalloc(&e->d_input, need));
-    e->input_cap = need;
-  }
+  const bool in_place = input_in_place(input, input_on_device, total);
+  if (!in_place && (rc = ensure_input(e, total)) != NGAP_OK) return rc;
   uint64_t cap = p->result_capacity > 0 ? p->result_capacity : 54619400ull;
   if ((rc = ensure_reports(e, cap)) != NGAP_OK) return rc;
   // shared memory: the warps' (a window too large for it is shortened)
@@ -1402,16 +1415,15 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   rc = ensure_slots(e, (size_t)full_grid * kSlotsPerSm, t->max_states, t->max_nact, kDefaultQueue);
   if (rc != NGAP_OK) return rc;
 
-  if (input_on_device)
-    CUDA_TRY(cudaMemcpyAsync(e->d_input, input, total, cudaMemcpyDeviceToDevice, st));
-  else
-    CUDA_TRY(cudaMemcpyAsync(e->d_input, input, total, cudaMemcpyHostToDevice, st));
+  if (!in_place)
+    CUDA_TRY(cudaMemcpyAsync(e->d_input, input, total,
+                             input_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
   if ((rc = begin_counters(e, st)) != NGAP_OK) return rc;
 
   MatchParams mp;
   mp.tiles = t->d_tiles;
   mp.units = e->d_units;
-  mp.input = e->d_input;
+  mp.input = in_place ? input : e->d_input;
   mp.window = window;
   mp.depth = depth;
   mp.unique = p->unique;
@@ -1779,14 +1791,8 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   if (rc != NGAP_OK) return rc;
   const int full_grid = e->num_sms * bps;
   // buffers (before any capture)
-  size_t need = ((input_bytes + 15) & ~(uint64_t)15) + 64;
-  if (need > e->input_cap) {
-    cudaFree(e->d_input);
-    e->d_input = nullptr;
-    e->input_cap = 0;
-    CUDA_TRY(cudaMalloc(&e->d_input, need));
-    e->input_cap = need;
-  }
+  const bool in_place = input_in_place(input, input_on_device, input_bytes);
+  if (!in_place && (rc = ensure_input(e, input_bytes)) != NGAP_OK) return rc;
   const uint64_t cap = p->result_capacity > 0 ? p->result_capacity : 54619400ull;
   if ((rc = ensure_reports(e, cap)) != NGAP_OK) return rc;
   if (cap > e->stream_ids_cap) {
@@ -1873,7 +1879,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   MatchParams mp;
   mp.tiles = ts->d_tiles;
   mp.units = e->d_units;
-  mp.input = e->d_input;
+  mp.input = in_place ? input : e->d_input;
   mp.window = window;
   mp.depth = depth;
   mp.unique = p->unique;
@@ -1905,10 +1911,9 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
       const int r = trace_buffer(e, qs, &mp.unit_work, &mp.unit_cycles);
       if (r != NGAP_OK) return r;
     }
-    if (input_on_device)
-      CUDA_TRY(cudaMemcpyAsync(e->d_input, input, input_bytes, cudaMemcpyDeviceToDevice, qs));
-    else
-      CUDA_TRY(cudaMemcpyAsync(e->d_input, input, input_bytes, cudaMemcpyHostToDevice, qs));
+    if (!in_place)
+      CUDA_TRY(cudaMemcpyAsync(e->d_input, input, input_bytes,
+                               input_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, qs));
     int r = NGAP_OK;
     if (!e->h_units.empty()) {
       r = launch_plan(e, mp, ts->tiles, smem, (uint32_t)((input_bytes + 15) & ~(uint64_t)15), qs);

@@ -242,6 +242,7 @@ class Engine:
         p = _lib.MatchParams(algo, num_seg, seg_len, int(is_dup), int(unique), active_threshold,
                              int(report_off), result_capacity, window, chunk, first_segment)
         if hasattr(data, "data_ptr"):
+            self._keep = data  # read where it is until the match ends
             ptr, on_dev = data.data_ptr(), int(getattr(data, "is_cuda", True))
             nbytes = data.numel() * data.element_size() if hasattr(data, "numel") else None
         else:
@@ -382,6 +383,7 @@ def batch_match_async(engine, tableset, data, offsets, lengths, nfas,
     p = _lib.BatchParams(algo, int(unique), active_threshold, int(report_off), result_capacity,
                          window, chunk, int(use_graph), int(queue_capacity))
     if hasattr(data, "data_ptr"):
+        engine._keep = data  # read where it is until the match ends
         ptr, on_dev, nbytes = data.data_ptr(), int(getattr(data, "is_cuda", True)), data.numel()
     else:
         arr = as_u8(data)
