@@ -65,7 +65,7 @@ def byte_features(data, offsets, reg_stream, reg_start, reg_len, window=ENTROPY_
     """ngap_features over the regions: [n, 258] float32 (data: host uint8 array
     or CUDA tensor)."""
     n = len(reg_stream)
-    out = np.zeros((n, _lib.FEAT_BYTES), dtype=np.float32)
+    out = np.empty((n, _lib.FEAT_BYTES), dtype=np.float32)  # every row is written
     if n == 0:
         return out
     offs = (np.asarray(offsets, dtype=np.uint64)[reg_stream] + reg_start.astype(np.uint64))
@@ -161,7 +161,10 @@ class LearnedModel:
             pass
 
     def _norm(self, x):
-        return np.ascontiguousarray((x - self.mu) / self.sd, dtype=np.float32)
+        xn = x - self.mu
+        if xn.dtype == np.float32 and np.asarray(self.sd).dtype == np.float32:
+            return np.divide(xn, self.sd, out=xn)  # in place: the same values in one array less
+        return np.ascontiguousarray(xn / self.sd, dtype=np.float32)
 
     def fit(self, x, density, epochs=60, batch=512, lr=1e-3):
         x = np.asarray(x, np.float32)
