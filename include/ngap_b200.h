@@ -106,15 +106,14 @@ typedef struct ngap_table_opts {
   int precompute_cutoff; /* --precompute-cutoff, -1 = mean list length (precompute_table.cu:171) */
   int tile_states;       /* max states per tile; 0 = automatic */
   int64_t max_table_entries; /* cap on prefix-table list entries per tile; 0 = automatic */
-  int tile_mode;         /* NGAP_TILES_*: where tiles of acyclic CCs keep their tables */
+  int tile_mode;         /* NGAP_TILES_*: how CCs are packed into tiles */
 } ngap_table_opts;
 
-/* Tile modes. Shared: every tile is sized to stage its tables in one CTA's
- * shared memory (one group per tile). Global: the acyclic CCs of all groups
- * form few large tiles read through L2, so each input position is looked up
- * once per large tile instead of once per small one. Auto picks global when
- * the acyclic CCs need more than two shared-memory tiles. Cyclic CCs always
- * use shared-memory tiles. No mode changes any report. */
+/* Tile modes. Shared: tiles of one group, packed under a size rule of 128 KB.
+ * Global: the acyclic CCs of all groups form few large tiles, so each input
+ * position is looked at once per large tile instead of once per small one.
+ * Auto picks global when the acyclic CCs need more than two tiles of that
+ * size. Cyclic CCs always use tiles of one group. No mode changes any report. */
 #define NGAP_TILES_AUTO 0
 #define NGAP_TILES_SHARED 1
 #define NGAP_TILES_GLOBAL 2
@@ -135,7 +134,7 @@ typedef struct ngap_tile_desc {
   int32_t num_states, num_ccs;
   int32_t nact;       /* sticky states of the pair (activation slots) */
   int32_t nsticky;    /* sticky states handled in the tile */
-  int32_t global;     /* 1: tables read through L2 (several groups possible) */
+  int32_t global;     /* 1: CCs of several groups possible, no size rule */
   int32_t depth;      /* prefix-table depth */
   int32_t max_path;   /* longest acyclic path (chunk warm-up + 1); -1 = cyclic */
   int32_t nlive;      /* live byte classes */
@@ -180,7 +179,8 @@ typedef struct ngap_match_params {
   int64_t seg_len;           /* bytes per segment; input holds num_seg * seg_len bytes */
   int is_dup;                /* start-of-data states in every segment (ngap_buffer.cu:479-484) */
   int unique;                /* --unique: drop duplicate worklist entries within a step */
-  int active_threshold;      /* --active-threshold: busy-lane count enabling privatization */
+  int active_threshold;      /* --active-threshold: accepted; paths are always followed in
+                                registers, whatever its value */
   int report_off;            /* --report-off: count reports only */
   uint64_t result_capacity;  /* --result-capacity */
   int window;                /* positions per worklist window; 0 = automatic */
@@ -223,8 +223,8 @@ int64_t ngap_engine_device_bytes(const ngap_engine* e);
 typedef struct ngap_engine_mem {
   int64_t input;    /* the engine's copy of the input (largest batch so far, padded) */
   int64_t reports;  /* raw and unique report buffers, sort scratch, stream ids */
-  int64_t scratch;  /* per-warp worklist scratch: overflow stacks, carry lists, bitmaps */
-  int64_t plan;     /* units, tasks, activation slots, unit traces */
+  int64_t scratch;  /* worklist scratch: overflow stacks, carry lists, bitmaps, candidates */
+  int64_t plan;     /* units, pieces, activation slots, unit traces */
 } ngap_engine_mem;
 int ngap_engine_memory(const ngap_engine* e, ngap_engine_mem* out);
 
