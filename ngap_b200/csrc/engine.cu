@@ -92,6 +92,7 @@ struct ngap_tables {
   int device = 0;
   int num_groups = 0;
   int sid_bits = 0;  // bits of the largest group-local state id
+  uint64_t report_states = 0;
   std::vector<TileHost> tiles;
   std::vector<TileDev> dev_desc;
   TileDev* d_tiles = nullptr;
@@ -308,8 +309,10 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
   if (rc != NGAP_OK) return rc;
   build_filters(t->tiles);
   t->num_groups = (int)g->gs.groups.size();
-  for (const GroupGraph& gg : g->gs.groups)
+  for (const GroupGraph& gg : g->gs.groups) {
     t->sid_bits = std::max(t->sid_bits, bits_for(std::max<uint64_t>(gg.attrs.size(), 1)));
+    for (uint8_t a : gg.attrs) t->report_states += a & 2 ? 1 : 0;
+  }
   for (auto& th : t->tiles) {
     if (th.nstates >= kMaxTileStates - 1) {
       set_error("a connected component has %d states; at most %d are supported per tile",
@@ -1227,21 +1230,22 @@ int build_sort_graph(ngap_engine* e, const SortJob& j, SortGraph& sg) {
   return NGAP_OK;
 }
 
-// Inputs of at most this many positions sort their reports with the one-CTA
-// kernel alone, launched directly: a launch with a conditional graph costs 7
-// us more on a B200 (29 against 22 us for an empty pipeline), and one CTA keeps
-// up with the pipeline (about 60 us) to some 30,000 reports, an eighth of the
-// positions. Longer inputs may hold millions.
-constexpr uint64_t kAloneInput = 1ull << 18;
+// A match whose positions times its rules' report states are at most this sorts
+// its reports with the one-CTA kernel alone, launched directly: a launch with a
+// conditional graph costs 7 us more on a B200 (29 against 22 us for an empty
+// pipeline), while one CTA keeps up with the pipeline only to some 30,000
+// reports, which larger products could exceed many times over.
+constexpr uint64_t kAloneReports = 1ull << 16;
 
 // Enqueues the sort of a match's reports on st, the match's last kernels: they
-// leave its counters and first reports for the host. For inputs beyond
-// kAloneInput, outside stream capture, it replays a cached graph (one launch; the
+// leave its counters and first reports for the host. Past
+// kAloneReports, outside stream capture, it replays a cached graph (one launch; the
 // radix pipeline runs only for more than kSmallSort keys); inside a
 // capture, or where graphs are unavailable, it launches the one-CTA kernel and
 // the pipeline, whose kernels find no keys after a small set.
-int sort_reports(ngap_engine* e, const SortJob& j, uint64_t positions, cudaStream_t st) {
-  if (positions <= kAloneInput) return cta_sort(e, j, true, e->ho, st);
+int sort_reports(ngap_engine* e, const SortJob& j, uint64_t positions, uint64_t report_states,
+                 cudaStream_t st) {
+  if (positions * report_states <= kAloneReports) return cta_sort(e, j, true, e->ho, st);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(st, &cs));
   if (cs == cudaStreamCaptureStatusNone && !e->sort_graph_off) {
@@ -1463,7 +1467,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
                           bit_range(32, bits_for(total));
     const SortJob job{0,  e->d_reports, e->d_counters + 0, cap,     digits_of(bits),
                       32, 64,           e->d_unique,       nullptr, e->d_counters + 1};
-    if ((rc = sort_reports(e, job, total, st)) != NGAP_OK) return rc;
+    if ((rc = sort_reports(e, job, total, t->report_states, st)) != NGAP_OK) return rc;
   } else {
     publish_kernel<<<1, 32, 0, st>>>(e->ho);
     CUDA_TRY(cudaGetLastError());
@@ -1685,6 +1689,7 @@ struct ngap_tableset {
   std::vector<int> tile_base;  // first tile of each NFA in the combined descriptor array
   TileDev* d_tiles = nullptr;
   int sid_bits = 0;
+  uint64_t report_states = 0;  // of the NFA that has most
   int ntiles = 0, max_states = 0, max_groups = 1, max_depth = 1, device = 0;
   int max_nact = 0;
   std::vector<TileDev> tiles;       // the combined array
@@ -1717,6 +1722,7 @@ int ngap_tableset_create(const ngap_tables* const* tables, int n, ngap_tableset*
     ts->max_states = std::max(ts->max_states, t->max_states);
     ts->max_groups = std::max(ts->max_groups, t->num_groups);
     ts->sid_bits = std::max(ts->sid_bits, t->sid_bits);
+    ts->report_states = std::max(ts->report_states, t->report_states);
     ts->max_nact = std::max(ts->max_nact, t->max_nact);
     for (auto& th : t->tiles) ts->max_depth = std::max(ts->max_depth, th.depth);
   }
@@ -1924,7 +1930,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
                             bit_range(oshift, obits) | bit_range(sshift, sbits);
       const SortJob job{1,      e->d_reports, e->d_counters + 0, cap,             digits_of(bits),
                         oshift, sshift,       e->d_unique,       e->d_stream_ids, e->d_counters + 1};
-      if ((r = sort_reports(e, job, input_bytes, qs)) != NGAP_OK) return r;
+      if ((r = sort_reports(e, job, input_bytes, ts->report_states, qs)) != NGAP_OK) return r;
     } else {
       publish_kernel<<<1, 32, 0, qs>>>(e->ho);
       CUDA_TRY(cudaGetLastError());

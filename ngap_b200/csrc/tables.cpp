@@ -844,11 +844,11 @@ std::vector<std::vector<int>> global_sets_of(const GroupSet& gs, const std::vect
 
 // The states a tile injects at a position: its always-active states, or for a
 // layered tile the successors of its sticky states. Empty when the tile gets
-// no filter: plain tiles that register sticky states while they run, layered
+// no filter: cyclic tiles (matched segment by segment), plain tiles that register sticky states while they run, layered
 // tiles whose sticky states report (at every position) or that have
 // always-active states beside them.
 std::vector<uint32_t> filter_sources(const TileHost& t) {
-  if (t.phase == kPlain && t.nsticky > 0) return {};
+  if (t.max_path < 0 || (t.phase == kPlain && t.nsticky > 0)) return {};
   if (t.phase != kLayered) return t.aas;
   if (!t.aas.empty()) return {};
   std::vector<uint32_t> src;

@@ -38,9 +38,10 @@ def expected(tables, data):
     return r[np.lexsort((r >> np.uint64(32), r & np.uint64(0xFFFFFFFF)))]
 
 
-@pytest.mark.parametrize("length", [100_000, 300_001])  # one CTA alone, or with the pipeline
+@pytest.mark.parametrize("length", [16_000, 300_001])  # one CTA alone, or with the pipeline
 @pytest.mark.parametrize("hits", [0, 1, 31, 512, 1023, 1024, 1025, 4097, 8190, 8192, 8194, 70_000])
 def test_match_reports(engine, rules, one, length, hits):
+    hits = min(hits, length)
     rng = np.random.default_rng(hits + length)
     data = np.full(length, ord("x"), np.uint8)
     at = rng.choice(length, size=hits, replace=False)
