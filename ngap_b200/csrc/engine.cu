@@ -504,6 +504,10 @@ bool input_in_place(const uint8_t* input, int on_device, uint64_t bytes) {
   return on_device && bytes > 0 && bytes % 16 == 0 && reinterpret_cast<uintptr_t>(input) % 16 == 0;
 }
 
+// Last input byte that the scan may read. (A count would not fit: the 16-byte
+// units of an input just below 4 GiB end at 2^32.)
+uint32_t last_readable(uint64_t bytes) { return (uint32_t)((bytes - 1) | 15u); }
+
 // The engine's input buffer, padded for those reads.
 int ensure_input(ngap_engine* e, uint64_t bytes) {
   const size_t need = ((bytes + 15) & ~(uint64_t)15) + 64;
@@ -989,7 +993,7 @@ int launch_grid(int64_t nunits, int grid) {
 // tiles without sticky states in the lean kernel instance; then the rest
 // (the layered tiles read what the first launch recorded).
 int launch_plan(ngap_engine* e, MatchParams mp, const std::vector<TileDev>& tiles, int smem,
-                uint32_t readable, cudaStream_t st) {
+                uint32_t last, cudaStream_t st) {
   if (e->act_entries > 0)
     CUDA_TRY(cudaMemsetAsync(e->d_act, 0xff, (size_t)e->act_entries * sizeof(uint32_t), st));
   auto run = [&](bool lean, int which) -> int {
@@ -1011,7 +1015,7 @@ int launch_plan(ngap_engine* e, MatchParams mp, const std::vector<TileDev>& tile
   sp.tiles = mp.tiles;
   sp.pieces = e->d_pieces;
   sp.input = mp.input;
-  sp.readable = readable;
+  sp.last = last;
   sp.cand = e->d_cand;
   sp.runs = e->d_runs;
   sp.act_cnt = e->d_act_cnt;
@@ -1457,7 +1461,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   e->trace_seg_len = p->seg_len;
   CUDA_TRY(cudaEventRecord(e->ev[1], st));
   if (!e->h_units.empty()) {
-    rc = launch_plan(e, mp, t->dev_desc, smem, (uint32_t)((total + 15) & ~(uint64_t)15), st);
+    rc = launch_plan(e, mp, t->dev_desc, smem, last_readable(total), st);
     if (rc != NGAP_OK) return rc;
   }
   CUDA_TRY(cudaEventRecord(e->ev[2], st));
@@ -1922,7 +1926,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
                                input_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, qs));
     int r = NGAP_OK;
     if (!e->h_units.empty()) {
-      r = launch_plan(e, mp, ts->tiles, smem, (uint32_t)((input_bytes + 15) & ~(uint64_t)15), qs);
+      r = launch_plan(e, mp, ts->tiles, smem, last_readable(input_bytes), qs);
       if (r != NGAP_OK) return r;
     }
     if (!p->report_off) {

@@ -46,7 +46,7 @@ struct ScanParams {
   const PieceDev* pieces;
   uint32_t piece_begin, npieces;
   const uint8_t* input;     // 16-byte aligned
-  uint32_t readable;        // bytes of input that may be read (a multiple of 16)
+  uint32_t last;            // last byte of input that may be read (15 modulo 16)
   uint16_t* cand;           // candidates: offsets in their piece
   RunDev* runs;
   unsigned int* ctl;
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 1) scan_kernel(ScanParams p) 
   int staged = -1;  // the tile whose classes are in cls
   // eight input bytes as class ids
   auto load = [&](uint32_t at) {
-    return at < p.readable ? __ldg(reinterpret_cast<const uint2*>(p.input + at)) : make_uint2(0u, 0u);
+    return at <= p.last ? __ldg(reinterpret_cast<const uint2*>(p.input + at)) : make_uint2(0u, 0u);
   };
   auto classes = [&](uint32_t b) {
     return cls[b & 0xff] | cls[(b >> 8) & 0xff] << 8 | cls[(b >> 16) & 0xff] << 16 |
@@ -135,7 +135,9 @@ __global__ void __launch_bounds__(kScanWarps * 32, 1) scan_kernel(ScanParams p) 
       __syncwarp();
       const uint32_t own = o + ((uint32_t)lane << sb);  // the lane's first position
       // whole passes inside the piece with all of the filter's symbols left need no bounds per position
-      const bool inside = o >= pc.lo && o + block_len <= pc.hi && pc.end - (o + block_len - 1) >= (uint32_t)f.len;
+      // (the sum in 64 bits: inputs reach to 4 GiB)
+      const bool inside = o >= pc.lo && (uint64_t)o + block_len <= pc.hi &&
+                          pc.end - (o + block_len - 1) >= (uint32_t)f.len;
       uint32_t h = 0u, left = 0u;  // left: the id that leaves before the next position
       for (int i = 0; i < f.len - 1; i++) h = h * kFilterMul + *at(i);
       const int w0 = (f.len - 1) & ~3, sh = ((f.len - 1) & 3) * 8;
@@ -164,8 +166,8 @@ __global__ void __launch_bounds__(kScanWarps * 32, 1) scan_kernel(ScanParams p) 
           for (int j = 0; j < kScanLane; j++) {
             const uint32_t q = own + (uint32_t)(i + j);
             const bool in_piece = q >= pc.lo && q < pc.hi;
-            const bool whole = in_piece && (int)(pc.end - q) >= f.len;
-            if (in_piece && !whole && ((test >> j) & 1u) && (int)(pc.end - q) >= f.min_rep) found |= 1u << j;
+            const bool whole = in_piece && pc.end - q >= (uint32_t)f.len;
+            if (in_piece && !whole && ((test >> j) & 1u) && pc.end - q >= (uint32_t)f.min_rep) found |= 1u << j;
             if (!whole) test &= ~(1u << j);
           }
         }

@@ -34,3 +34,24 @@ def test_device_input(engine, start, length):
     engine.sync()
     assert np.array_equal(engine.results(), want)
     del junk
+
+
+@pytest.mark.parametrize("length", [2**31 + 4099, 2**32 - 16, 2**32 - 1])
+def test_largest_input(built, length):
+    """Segments past 2 GiB and up to the end of the 32-bit offsets: text planted
+    at both ends, across a piece's and a scan launch's edges and past 2 GiB
+    gives the oracle's reports of it, moved to its place."""
+    import torch
+    anml, text = W.literal_set(seed=6, n_patterns=20, input_len=600, plant_every=40)
+    groups = nb.Groups(nb.Nfa.from_string(anml), group_num=1)
+    tables = nb.Tables(groups, precompute_depth=2)
+    found, _ = oracle.match(groups.views(), text, 1, len(text))
+    assert len(found) > 0
+    buf = torch.zeros(length, dtype=torch.uint8, device="cuda")
+    places = [0, 4096 * 3 - 300, (32 << 20) - 300, 2**31 + 7, length - len(text)]
+    for at in places:
+        buf[at:at + len(text)] = torch.from_numpy(text)
+    want = np.sort(np.concatenate([found + np.uint64(at) for at in places]))
+    engine = nb.Engine(0)
+    got = engine.match(tables, buf, 1, length)
+    assert np.array_equal(np.sort(got), want)
