@@ -515,7 +515,7 @@ __device__ __forceinline__ void walk_run(const MatchParams& p, WarpSmem& ws, War
   }
 }
 
-// Warps of a CTA: 32 of 64 registers (8 bytes spilled) rather than 16 of 122,
+// Warps of a CTA: 32 of 64 registers (the plain instance spills 120 bytes) rather than 16 of 122,
 // because runs wait for reads most of the time. Match times on a B200 with 16,
 // 20, 24 and 32: 1000 25-mers 194, 181, 174, 160 us; 200 25-mers with three table
 // levels 625, 546, 468, 394; the 32 MiB mix 639, 619, 607, 599.
