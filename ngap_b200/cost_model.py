@@ -163,8 +163,11 @@ class LearnedModel:
     def _norm(self, x):
         xn = x - self.mu
         if xn.dtype == np.float32 and np.asarray(self.sd).dtype == np.float32:
-            return np.divide(xn, self.sd, out=xn)  # in place: the same values in one array less
-        return np.ascontiguousarray(xn / self.sd, dtype=np.float32)
+            xn = np.divide(xn, self.sd, out=xn)  # in place: the same values in one array less
+        else:
+            xn = xn / self.sd
+        # rows one after another, whatever the strides of x (x - mu keeps their order)
+        return np.ascontiguousarray(xn, dtype=np.float32)
 
     def fit(self, x, density, epochs=60, batch=512, lr=1e-3):
         x = np.asarray(x, np.float32)

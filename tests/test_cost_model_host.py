@@ -40,6 +40,24 @@ def test_static_and_mean_models():
     assert np.allclose(cm.relative_error(np.array([1.0, 0.0]), np.array([2.0, 0.01])), [0.5, 0.2])
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("order", ["C", "F", "strided", "reversed"])
+def test_standardised_rows_are_contiguous(order, dtype):
+    """LearnedModel hands the library the address of its standardised features:
+    they lie row by row whatever the strides of x."""
+    rng = np.random.default_rng(4)
+    x = rng.standard_normal((37, 11)).astype(dtype)
+    given = {"C": x, "F": np.asfortranarray(x), "strided": np.repeat(x, 2, axis=1)[:, ::2],
+             "reversed": x[::-1, ::-1].copy()[::-1, ::-1]}[order]
+    assert np.array_equal(given, x)
+    m = cm.LearnedModel.__new__(cm.LearnedModel)  # no library handle
+    m.mu = rng.standard_normal(11).astype(np.float32)
+    m.sd = rng.uniform(0.5, 2.0, 11).astype(np.float32)
+    got = m._norm(given)
+    assert got.dtype == np.float32 and got.flags.c_contiguous
+    assert np.array_equal(got, ((x - m.mu) / m.sd).astype(np.float32))
+
+
 def test_host_features_definition():
     rng = np.random.default_rng(0)
     for L in (1, 700, 1024, 5000, 16384):
