@@ -20,6 +20,8 @@
 #include <vector>
 
 #include "common.h"
+#include "context.h"
+#include "kept_block.h"
 
 namespace {
 
@@ -350,37 +352,24 @@ struct ngap_mlp {
 namespace {
 
 // Device memory of ngap_features. A call has waited for its stream when it
-// returns, so each host thread keeps its last block (at most kFeatKeep bytes,
-// freed when the thread ends) instead of allocating three and freeing them,
+// returns, so each host thread keeps its last block of a context (at most kFeatKeep
+// bytes, freed when the thread ends) instead of allocating three and freeing them,
 // which waits for the whole device, on every call (4095 regions of 64 MB: 1.46 ->
 // 0.6 ms a call on a B200).
 constexpr size_t kFeatKeep = 32 << 20;
-struct FeatureSpace {
-  void* ptr = nullptr;
-  size_t cap = 0;
-  int device = -1;
-  cudaError_t reserve(size_t bytes) {
-    int dev = 0;
-    cudaError_t ce = cudaGetDevice(&dev);
-    if (ce != cudaSuccess || (dev == device && bytes <= cap)) return ce;
-    release();
-    if ((ce = cudaMalloc(&ptr, bytes)) != cudaSuccess) {
-      ptr = nullptr;
-      return ce;
-    }
-    cap = bytes;
-    device = dev;
-    return ce;
+struct CudaApi {
+  uint64_t context() { return ngap::current_context_id(); }
+  void init() { cudaFree(nullptr); }
+  int device() {
+    int d = -1;
+    cudaGetDevice(&d);
+    return d;
   }
-  void release() {
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    cap = 0;
-    device = -1;
-  }
-  ~FeatureSpace() { release(); }
+  void set_device(int d) { cudaSetDevice(d); }
+  int alloc(void** p, size_t bytes) { return (int)cudaMalloc(p, bytes); }
+  void free(void* p) { cudaFree(p); }
 };
-thread_local FeatureSpace t_feature_space;
+thread_local ngap::KeptBlocks<CudaApi> t_feature_space;
 
 }  // namespace
 
@@ -403,12 +392,12 @@ int ngap_features(const uint8_t* data, uint64_t bytes, int on_device, const uint
   const size_t off_len = (size_t)n * sizeof(uint64_t), off_out = 2 * off_len;
   const size_t out_bytes = (size_t)n * NGAP_FEAT_BYTES * sizeof(float);
   const size_t off_data = (off_out + out_bytes + 15) & ~(size_t)15;
-  FeatureSpace big;  // beyond what the thread keeps
   const size_t need = off_data + (on_device ? 0 : (size_t)bytes);
-  FeatureSpace& ws = need <= kFeatKeep ? t_feature_space : big;
-  cudaError_t ce = ws.reserve(need);
+  void* block = nullptr;
+  bool mine = false;
+  cudaError_t ce = (cudaError_t)t_feature_space.reserve(need, kFeatKeep, &block, &mine);
   if (ce == cudaSuccess) {
-    uint8_t* base = static_cast<uint8_t*>(ws.ptr);
+    uint8_t* base = static_cast<uint8_t*>(block);
     const uint8_t* d_data = on_device ? data : base + off_data;
     uint64_t* d_off = reinterpret_cast<uint64_t*>(base);
     uint64_t* d_len = reinterpret_cast<uint64_t*>(base + off_len);
@@ -422,8 +411,9 @@ int ngap_features(const uint8_t* data, uint64_t bytes, int on_device, const uint
       ce = cudaGetLastError();
     }
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, st);
-    const cudaError_t se = cudaStreamSynchronize(st);  // the space is free again
+    const cudaError_t se = cudaStreamSynchronize(st);  // the block is free again
     if (ce == cudaSuccess) ce = se;
+    if (mine) cudaFree(block);
   }
   if (ce != cudaSuccess) {
     ngap::set_error("ngap_features: %s", cudaGetErrorString(ce));

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "common.h"
+#include "context.h"
 #include "handles.h"
 #include "match_kernel.cuh"
 #include "scan_kernel.cuh"
@@ -2060,25 +2061,7 @@ static __device__ __align__(256) uint8_t g_noalloc_scratch[kNoAllocBytes];
 std::mutex g_noalloc_mu;
 constexpr int kNoAllocMaxDevices = 64;
 uint8_t* g_noalloc_addr[kNoAllocMaxDevices] = {};
-void* g_noalloc_ctx[kNoAllocMaxDevices] = {};  // context the address belongs to
-
-// The calling thread's current CUDA context (driver cuCtxGetCurrent, reached
-// through the runtime's entry-point lookup so that the library does not link
-// the driver library), or nullptr when it cannot be read.
-void* current_context() {
-  using Fn = int (*)(void**);
-  static Fn fn = []() -> Fn {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<Fn>(f);
-  }();
-  void* ctx = nullptr;
-  if (!fn || fn(&ctx) != 0) return nullptr;
-  return ctx;
-}
+uint64_t g_noalloc_ctx[kNoAllocMaxDevices] = {};  // context the address belongs to
 
 // Device address of the scratch array on the current device. In host code
 // g_noalloc_scratch names a host-side stand-in, not device memory, so the
@@ -2093,7 +2076,7 @@ int noalloc_scratch(int dev, uint8_t** out) {
     return NGAP_E_INVALID;
   }
   std::lock_guard<std::mutex> lk(g_noalloc_mu);
-  void* ctx = current_context();
+  const uint64_t ctx = current_context_id();
   if (!g_noalloc_addr[dev] || !ctx || ctx != g_noalloc_ctx[dev]) {
     void* p = nullptr;
     cudaError_t ce = cudaGetSymbolAddress(&p, g_noalloc_scratch);
@@ -2104,7 +2087,7 @@ int noalloc_scratch(int dev, uint8_t** out) {
     }
     g_noalloc_addr[dev] = static_cast<uint8_t*>(p);
     // the runtime may have made the primary context current just now
-    g_noalloc_ctx[dev] = ctx ? ctx : current_context();
+    g_noalloc_ctx[dev] = ctx ? ctx : current_context_id();
   }
   *out = g_noalloc_addr[dev];
   return NGAP_OK;
