@@ -195,8 +195,9 @@ typedef struct ngap_match_params {
  * bytes) against every group and leaves the sorted, deduplicated reports on
  * the device. Asynchronous on `stream` (a cudaStream_t, NULL = default);
  * ngap_engine_sync waits and returns the run's status. `input` must stay
- * unchanged until the match has ended on `stream`: device memory is read in
- * place when its address and length are multiples of 16. */
+ * unchanged until the match has ended on `stream`: device memory of the
+ * engine's GPU is read in place when its address and length are multiples of
+ * 16; memory of another GPU is copied. */
 int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int input_on_device,
                const ngap_match_params* p, void* stream);
 int ngap_engine_sync(ngap_engine* e);

@@ -16,6 +16,7 @@
 #include "context.h"
 #include "handles.h"
 #include "match_kernel.cuh"
+#include "plan_rules.h"
 #include "scan_kernel.cuh"
 #include "sort_kernels.cuh"
 #include "tables.h"
@@ -497,12 +498,21 @@ int upload_plan(ngap_engine* e, cudaStream_t st, const std::vector<Upload>& part
   return NGAP_OK;
 }
 
-// Whether a match reads its input where the caller has it: device memory whose
-// start and length are multiples of 16, so that the kernels' 16-byte reads and
-// bulk copies stay inside it. Otherwise it is copied into the engine's padded
-// buffer (16 MiB: 10 us of a 190 us call on a B200).
-bool input_in_place(const uint8_t* input, int on_device, uint64_t bytes) {
-  return on_device && bytes > 0 && bytes % 16 == 0 && reinterpret_cast<uintptr_t>(input) % 16 == 0;
+// Whether a match reads its input where the caller has it: device memory of
+// this GPU whose start and length are multiples of 16. Otherwise it is copied into
+// the engine's padded buffer (16 MiB: 10 us of a 190 us call on a B200).
+bool input_in_place(const ngap_engine* e, const uint8_t* input, int on_device, uint64_t bytes) {
+  return reads_in_place(input, on_device != 0, bytes, e->device, [](const void* p) {
+    InputMemory m;
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) {
+      m.device = a.type == cudaMemoryTypeDevice;
+      m.owner = a.device;
+    } else {
+      cudaGetLastError();  // an address the runtime does not know is copied
+    }
+    return m;
+  });
 }
 
 // Last input byte that the scan may read. (A count would not fit: the 16-byte
@@ -1387,7 +1397,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   int rc = algo_config(p->algorithm, table_depth, &depth);
   if (rc != NGAP_OK) return rc;
   window = std::min(window, kMaxWindow);
-  const bool in_place = input_in_place(input, input_on_device, total);
+  const bool in_place = input_in_place(e, input, input_on_device, total);
   if (!in_place && (rc = ensure_input(e, total)) != NGAP_OK) return rc;
   uint64_t cap = p->result_capacity > 0 ? p->result_capacity : 54619400ull;
   if ((rc = ensure_reports(e, cap)) != NGAP_OK) return rc;
@@ -1802,7 +1812,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   if (rc != NGAP_OK) return rc;
   const int full_grid = e->num_sms * bps;
   // buffers (before any capture)
-  const bool in_place = input_in_place(input, input_on_device, input_bytes);
+  const bool in_place = input_in_place(e, input, input_on_device, input_bytes);
   if (!in_place && (rc = ensure_input(e, input_bytes)) != NGAP_OK) return rc;
   const uint64_t cap = p->result_capacity > 0 ? p->result_capacity : 54619400ull;
   if ((rc = ensure_reports(e, cap)) != NGAP_OK) return rc;
@@ -1968,7 +1978,8 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   }
   cudaStream_t cs = e->cap_stream;
   std::vector<uint64_t> key = {ts->serial, (uint64_t)(uintptr_t)input, input_bytes,
-                               (uint64_t)input_on_device, (uint64_t)p->algorithm,
+                               (uint64_t)input_on_device, (uint64_t)in_place,
+                               (uint64_t)p->algorithm,
                                (uint64_t)p->unique, (uint64_t)p->active_threshold,
                                (uint64_t)p->report_off, cap, (uint64_t)window, (uint64_t)p->chunk,
                                (uint64_t)e->trace, (uint64_t)e->ovf_cap};
