@@ -230,6 +230,7 @@ struct ngap_engine {
   uint64_t stream_ids_cap = 0;
   cudaGraphExec_t graph = nullptr;
   std::vector<uint64_t> graph_key;
+  uint64_t buffers = 0;  // counts allocations of device buffers: a captured batch holds their addresses
   bool graph_mode = false;
   int graph_launches = 0;
   cudaStream_t cap_stream = nullptr;  // capture/replay stream of the batched graph
@@ -523,6 +524,7 @@ uint32_t last_readable(uint64_t bytes) { return (uint32_t)((bytes - 1) | 15u); }
 int ensure_input(ngap_engine* e, uint64_t bytes) {
   const size_t need = ((bytes + 15) & ~(uint64_t)15) + 64;
   if (need <= e->input_cap) return NGAP_OK;
+  e->buffers++;
   cudaFree(e->d_input);
   e->d_input = nullptr;
   e->input_cap = 0;
@@ -533,6 +535,7 @@ int ensure_input(ngap_engine* e, uint64_t bytes) {
 
 int ensure_reports(ngap_engine* e, uint64_t cap) {
   if (cap <= e->rep_cap) return NGAP_OK;
+  e->buffers++;
   cudaFree(e->d_reports);
   cudaFree(e->d_tmp);
   cudaFree(e->d_unique);
@@ -564,6 +567,7 @@ int ensure_slots(ngap_engine* e, size_t slots, int max_states, int max_nact, int
   }
   const int stk_cap = max_nact > kStickyCap ? max_nact : 0;
   if (slots <= e->slots && stk_cap > e->stk_cap) {  // only the sticky lists grow
+    e->buffers++;
     cudaFree(e->d_stk);
     e->d_stk = nullptr;
     e->stk_cap = 0;
@@ -571,6 +575,7 @@ int ensure_slots(ngap_engine* e, size_t slots, int max_states, int max_nact, int
     e->stk_cap = stk_cap;
   }
   if (slots <= e->slots && carry_cap <= e->carry_cap && mark_words <= e->mark_words) return NGAP_OK;
+  e->buffers++;
   cudaFree(e->d_carry);
   cudaFree(e->d_marks);
   cudaFree(e->d_ovf);
@@ -861,6 +866,7 @@ int trace_buffer(ngap_engine* e, cudaStream_t st, unsigned long long** work,
   *work = *cycles = nullptr;
   if (!e->trace || e->h_units.empty()) return NGAP_OK;
   if (e->h_units.size() > e->unit_work_cap) {
+    e->buffers++;
     const size_t cap = grown(e->unit_work_cap, e->h_units.size());
     cudaFree(e->d_unit_work);
     e->d_unit_work = nullptr;
@@ -882,6 +888,7 @@ int set_plan(ngap_engine* e, const std::vector<UnitDev>& units, const std::vecto
   int64_t cands = 0, runs = 0;
   e->ranges.slices = make_slices(pieces, run_len, &cands, &runs);
   if (units.size() > e->units_cap) {
+    e->buffers++;
     const size_t cap = grown(e->units_cap, units.size());
     cudaFree(e->d_units);
     e->d_units = nullptr;
@@ -890,6 +897,7 @@ int set_plan(ngap_engine* e, const std::vector<UnitDev>& units, const std::vecto
     e->units_cap = cap;
   }
   if (all.size() > e->pieces_cap) {
+    e->buffers++;
     const size_t cap = grown(e->pieces_cap, all.size());
     cudaFree(e->d_pieces);
     e->d_pieces = nullptr;
@@ -898,6 +906,7 @@ int set_plan(ngap_engine* e, const std::vector<UnitDev>& units, const std::vecto
     e->pieces_cap = cap;
   }
   if (cands > e->cand_cap) {
+    e->buffers++;
     const int64_t cap = std::max(cands, std::min<int64_t>(grown(e->cand_cap, cands), kSlicePositions));
     cudaFree(e->d_cand);
     e->d_cand = nullptr;
@@ -906,6 +915,7 @@ int set_plan(ngap_engine* e, const std::vector<UnitDev>& units, const std::vecto
     e->cand_cap = cap;
   }
   if (runs > e->runs_cap) {
+    e->buffers++;
     const int64_t cap = std::max(runs, std::min<int64_t>(grown(e->runs_cap, runs), kSliceRuns));
     cudaFree(e->d_runs);
     e->d_runs = nullptr;
@@ -936,6 +946,7 @@ int set_act_rows(ngap_engine* e, const ActRows& rows, std::vector<Upload>& ups) 
   e->act_entries = rows.total;
   e->act_rows = (int32_t)rows.row_off.size();
   if (e->act_entries > e->act_cap) {
+    e->buffers++;
     const int64_t cap = grown(e->act_cap, e->act_entries);
     cudaFree(e->d_act);
     cudaFree(e->d_act_list);
@@ -946,6 +957,7 @@ int set_act_rows(ngap_engine* e, const ActRows& rows, std::vector<Upload>& ups) 
     e->act_cap = cap;
   }
   if (e->act_rows > e->rows_cap) {
+    e->buffers++;
     const int32_t cap = grown(e->rows_cap, e->act_rows);
     cudaFree(e->d_row_off);
     cudaFree(e->d_row_n);
@@ -1817,6 +1829,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   const uint64_t cap = p->result_capacity > 0 ? p->result_capacity : 54619400ull;
   if ((rc = ensure_reports(e, cap)) != NGAP_OK) return rc;
   if (cap > e->stream_ids_cap) {
+    e->buffers++;
     cudaFree(e->d_stream_ids);
     e->d_stream_ids = nullptr;
     e->stream_ids_cap = 0;
@@ -1982,7 +1995,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
                                (uint64_t)p->algorithm,
                                (uint64_t)p->unique, (uint64_t)p->active_threshold,
                                (uint64_t)p->report_off, cap, (uint64_t)window, (uint64_t)p->chunk,
-                               (uint64_t)e->trace, (uint64_t)e->ovf_cap};
+                               (uint64_t)e->trace, (uint64_t)e->ovf_cap, e->buffers};
   if (replanned || !e->graph || key != e->graph_key) {
     if (e->graph) {
       cudaGraphExecDestroy(e->graph);
