@@ -880,6 +880,15 @@ int trace_buffer(ngap_engine* e, cudaStream_t st, unsigned long long** work,
   return NGAP_OK;
 }
 
+// Drops the cached plan before another one is made: a plan that cannot be
+// finished (an allocation fails) leaves neither the old one, whose buffers may be
+// gone, nor half of its own. The next match plans again.
+void forget_plan(ngap_engine* e) {
+  e->plan_tables = 0;
+  e->plan_key = UnitPlanKey{-1, -1, -1, -1, -1, -1, -1, true};
+  e->batch_ts = 0;
+}
+
 // Device copies of a plan's units and pieces, buffers for its largest slice.
 int set_plan(ngap_engine* e, const std::vector<UnitDev>& units, const std::vector<PieceDev> pieces[2],
              const std::vector<int32_t>& run_len, std::vector<PieceDev>& all, std::vector<Upload>& ups) {
@@ -1425,6 +1434,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   UnitPlanKey key{p->num_seg, p->seg_len, p->is_dup ? 1 : 0, window, p->chunk, p->first_segment,
                   depth, e->test_skip_unit < 0};
   if (e->plan_tables != t->serial || key < e->plan_key || e->plan_key < key) {
+    forget_plan(e);
     std::vector<UnitDev> units;
     std::vector<PieceDev> pieces[2], all;
     const ActRows rows = plan_units(t, key, full_grid, units, pieces, e->ranges);
@@ -1434,7 +1444,6 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
     if ((rc = upload_plan(e, st, ups)) != NGAP_OK) return rc;
     e->plan_tables = t->serial;
     e->plan_key = key;
-    e->batch_ts = 0;  // the batched plan cache no longer describes the buffers
   }
   if (p->window <= 0) {
     window = fit_window(window, e->longest_unit);
@@ -1849,6 +1858,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   bool replanned = false;
   if (e->batch_ts != ts->serial || e->batch_depth != depth || e->batch_window != window || e->batch_chunk != p->chunk ||
       !same_streams() || e->plan_tables != 0) {
+    forget_plan(e);
     std::vector<std::vector<int>> by_nfa(ts->tables.size());
     for (int i = 0; i < nstreams; i++) by_nfa[sv[i].nfa].push_back(i);
     std::vector<UnitDev> pass1, unbounded, bounded, units;
@@ -1892,8 +1902,6 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     if ((rc = set_act_rows(e, rows, ups)) != NGAP_OK) return rc;
     if ((rc = set_plan(e, units, pieces, ts->run_len, all, ups)) != NGAP_OK) return rc;
     if ((rc = upload_plan(e, st, ups)) != NGAP_OK) return rc;
-    e->plan_tables = 0;  // the plain plan cache no longer describes the buffers
-    e->plan_key = UnitPlanKey{-1, -1, -1, -1, -1, -1, -1, true};
     e->batch_ts = ts->serial;
     e->batch_streams = sv;
     e->batch_window = window;

@@ -1,0 +1,133 @@
+"""The host side of a match on the CPU, against a stand-in for the CUDA runtime
+(fake_cudart.c): what is launched and uploaded after an allocation has failed,
+and after buffers have moved. Each check runs in a process of its own."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+PRELUDE = r"""
+import ctypes
+import numpy as np
+import ngap_b200 as nb
+from ngap_b200 import workloads as W
+from ngap_b200._lib import lib
+
+fake = ctypes.CDLL(None)
+size = lambda name: ctypes.c_size_t.in_dll(fake, name)
+count = lambda name: ctypes.c_long.in_dll(fake, name).value
+
+
+def log(f, *a, **kw):
+    "Launches and asynchronous copies of one call."
+    fake.fake_reset()
+    f(*a, **kw)
+    return (ctypes.c_char * (1 << 20)).in_dll(fake, "fake_log").value.decode().split(";")[:-1]
+
+
+def fails(f, *a, **kw):
+    try:
+        f(*a, **kw)
+    except nb.NgapError as ex:
+        assert ex.status == 5 and "out of memory" in str(ex), ex
+        return
+    raise AssertionError("the allocation did not fail")
+
+
+def tables(text, depth=2, groups=1):
+    return nb.Tables(nb.Groups(nb.Nfa.from_string(text), group_num=groups), precompute_depth=depth)
+
+
+CAP = 4096
+"""
+
+
+@pytest.fixture(scope="module")
+def run(built, tmp_path_factory):
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    if shutil.which("gcc") is None or not os.path.exists(os.path.join(cuda, "include", "cuda_runtime_api.h")):
+        pytest.skip("no C compiler or CUDA headers")
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    subprocess.run(["gcc", "-O1", "-shared", "-fPIC", "-I", os.path.join(cuda, "include"),
+                    os.path.join(ROOT, "tests", "fake_cudart.c"), "-o", so], check=True)
+
+    def go(body):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + body + "\nprint('ok')"], cwd=ROOT, timeout=300,
+                           env=dict(os.environ, LD_PRELOAD=so), capture_output=True, text=True)
+        assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
+    return go
+
+
+FAILED_PLAN = r"""
+text, _ = W.literal_set(seed=5, n_patterns=20, input_len=1000, plant_every=100)
+t = tables(text)
+ts = nb.TableSet([t])
+short, long = np.zeros(3000, np.uint8), np.zeros(9_000_000, np.uint8)
+
+
+def plain(e, data):
+    e.match_async(t, data, 1, len(data), result_capacity=CAP)
+
+
+def batch(e, data):
+    n = len(data) // 3
+    nb.batch_match_async(e, ts, data, [0, n, 2 * n], [n, n, n], [0, 0, 0], result_capacity=CAP)
+
+
+for first in (plain, batch):
+    for other in (plain, batch):
+        e = nb.Engine(0)
+        want = log(first, e, short)
+        assert any("match_kernel" in x for x in want) and not any("scan_kernel" in x for x in want)
+        again = log(first, e, short)  # the plan is kept: nothing to upload but the input
+        assert len(again) < len(want)
+        # the longer plan's candidate list (2 bytes a position) cannot be had
+        # (the input is copied into a buffer of half that size)
+        size("fake_fail_at").value = 2 * len(long) - 4096
+        fails(other, e, long)
+        size("fake_fail_at").value = 0
+        # the first call again: its own units are uploaded and launched, not the other plan's
+        assert log(first, e, short) == want
+        # and the longer input goes through once there is room
+        assert any("scan_kernel" in x for x in log(other, e, long))
+        assert log(first, e, short) == want
+"""
+
+
+def test_failed_plan_is_forgotten(run):
+    run(FAILED_PLAN)
+
+
+CAPTURE = r"""
+text, _ = W.literal_set(seed=5, n_patterns=20, input_len=1000, plant_every=100)
+ts = nb.TableSet([tables(text)])
+data = np.zeros(1 << 20, np.uint8)
+e = nb.Engine(0)
+
+
+def batch():
+    nb.batch_match_async(e, ts, data, [0, 1000], [1000, 500000], [0, 0], use_graph=True, result_capacity=CAP)
+
+
+batch()
+n = count("fake_instantiated")
+batch()
+assert count("fake_instantiated") == n  # replayed
+keys = ctypes.c_void_p()
+assert fake.cudaMalloc(ctypes.byref(keys), ctypes.c_size_t(64 * CAP)) == 0
+held = e.memory()["reports"]
+e.sort_unique_device(keys.value, 8 * CAP, keys.value)
+assert e.memory()["reports"] > held  # the report buffers are others now
+batch()
+assert count("fake_instantiated") == n + 1  # captured again
+batch()
+assert count("fake_instantiated") == n + 1
+"""
+
+
+def test_capture_follows_the_buffers(run):
+    run(CAPTURE)
