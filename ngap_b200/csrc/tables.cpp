@@ -771,30 +771,75 @@ std::array<uint32_t, 8> alphabet_of(const GroupGraph& g, const CcInfo& c) {
   return alpha;
 }
 
-// Splits CCs that would share a tile: those of one small alphabet (say ACGT, at
-// most kSmallAlphabet symbols shared by at least kSmallAlphabetCcs CCs) get sets
-// of their own where there are others too, the others come last. In a tile with
-// text rules their keys would be base-95 numbers, whose tables and filter
+// Splits CCs that would share a tile: those over one small alphabet (say ACGT: at
+// most kSmallAlphabet symbols, CCs that use only some of them included) get a
+// set of their own where there are others too, the others come last. In a tile
+// with text rules their keys would be base-95 numbers, whose tables and filter
 // reach 4 and 8 symbols instead of 12 and 16 (100 edit-distance and 400 dot-star
-// rules, match times on a B200: 520 KB 602 -> 68 us, 1000 bytes 546 -> 71 us).
+// rules, match times on a B200: 520 KB 602 -> 68 us, 1000 bytes 546 -> 71 us). But every
+// tile is one more scan of the input, so a set has at least kSmallAlphabetCcs
+// CCs and one in kSmallAlphabetShare of the states: short words have small
+// alphabets too, hundreds of different ones (10,000 words: 148 sets without the
+// share, none with it).
 constexpr int kSmallAlphabet = 8;
 constexpr size_t kSmallAlphabetCcs = 4;
+constexpr int64_t kSmallAlphabetShare = 8;
 std::vector<std::vector<int>> by_alphabet(const GroupSet& gs, const std::vector<CcInfo>& ccs,
                                           const std::vector<int>& set) {
-  std::map<std::array<uint32_t, 8>, std::vector<int>> small;
-  std::vector<int> others;
-  for (int i : set) {
-    const std::array<uint32_t, 8> alpha = alphabet_of(gs.groups[ccs[i].group], ccs[i]);
+  using Alphabet = std::array<uint32_t, 8>;
+  struct Small {
+    std::vector<int> ccs;
+    int64_t states = 0;
+  };
+  auto symbols = [](const Alphabet& a) {
     int n = 0;
-    for (uint32_t w : alpha) n += __builtin_popcount(w);
-    if (n <= kSmallAlphabet) small[alpha].push_back(i);
-    else others.push_back(i);
+    for (uint32_t w : a) n += __builtin_popcount(w);
+    return n;
+  };
+  std::map<Alphabet, Small> small;
+  std::vector<int> others;
+  Alphabet whole{};
+  int64_t states = 0;
+  for (int i : set) {
+    const Alphabet alpha = alphabet_of(gs.groups[ccs[i].group], ccs[i]);
+    for (int w = 0; w < 8; w++) whole[w] |= alpha[w];
+    states += ccs[i].end - ccs[i].begin;
+    if (symbols(alpha) > kSmallAlphabet) {
+      others.push_back(i);
+      continue;
+    }
+    Small& s = small[alpha];
+    s.ccs.push_back(i);
+    s.states += ccs[i].end - ccs[i].begin;
   }
+  if (small.empty() || symbols(whole) <= kSmallAlphabet) return {set};
+  auto subset = [](const Alphabet& a, const Alphabet& b) {
+    for (int w = 0; w < 8; w++)
+      if (a[w] & ~b[w]) return false;
+    return true;
+  };
+  // the alphabets with most states first, each with what is left of its subsets;
+  // fewer than kSmallAlphabetShare of them can have their share
+  std::vector<std::map<Alphabet, Small>::iterator> order;
+  for (auto it = small.begin(); it != small.end(); ++it) order.push_back(it);
+  std::stable_sort(order.begin(), order.end(),
+                   [](const auto& a, const auto& b) { return a->second.states > b->second.states; });
   std::vector<std::vector<int>> out;
-  for (auto& kv : small) {
-    if (kv.second.size() >= kSmallAlphabetCcs) out.push_back(kv.second);
-    else others.insert(others.end(), kv.second.begin(), kv.second.end());
+  for (size_t k = 0; k < order.size() && (int64_t)k < 4 * kSmallAlphabetShare; k++) {
+    if (order[k]->second.ccs.empty()) continue;
+    Small all;
+    for (const auto& it : order)
+      if (subset(it->first, order[k]->first)) {
+        all.ccs.insert(all.ccs.end(), it->second.ccs.begin(), it->second.ccs.end());
+        all.states += it->second.states;
+      }
+    if (all.ccs.size() < kSmallAlphabetCcs || all.states * kSmallAlphabetShare < states) continue;
+    for (const auto& it : order)
+      if (subset(it->first, order[k]->first)) it->second = Small();
+    std::sort(all.ccs.begin(), all.ccs.end());
+    out.push_back(all.ccs);
   }
+  for (auto& kv : small) others.insert(others.end(), kv.second.ccs.begin(), kv.second.ccs.end());
   std::sort(others.begin(), others.end());
   if (!others.empty()) out.push_back(others);
   return out;
