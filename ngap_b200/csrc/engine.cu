@@ -1479,6 +1479,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   mp.carry_cap = e->carry_cap;
   mp.mark_words = e->mark_words;
   mp.ovf_cap = e->ovf_cap;
+  mp.mark_inject = (kStackCap + e->ovf_cap) / 4;
   mp.work = e->d_counters + 2;
   mp.act = e->d_act;
   mp.act_list = e->d_act_list;
@@ -1937,6 +1938,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   mp.carry_cap = e->carry_cap;
   mp.mark_words = e->mark_words;
   mp.ovf_cap = e->ovf_cap;
+  mp.mark_inject = (kStackCap + e->ovf_cap) / 4;
   mp.work = e->d_counters + 2;
   mp.act = e->d_act;
   mp.act_list = e->d_act_list;

@@ -80,6 +80,7 @@ struct MatchParams {
   uint32_t* marks;          // [slots][mark_words]
   uint32_t* ovf;            // [slots][ovf_cap]
   int32_t carry_cap, mark_words, ovf_cap;
+  int32_t mark_inject;      // entries of a run's worklist at which its injection waits
   unsigned long long* work; // [0] entries expanded, [1] entries injected
   uint32_t* act;            // activation slots (first match of sticky states, offset in the
                             // segment; 0xffffffff = none)

@@ -247,16 +247,34 @@ struct RunCtx {
 
 __device__ __forceinline__ uint32_t symbol(const RunCtx& c, int r) { return __ldg(c.cls + __ldg(c.in + r)); }
 
+// What a run puts on its worklist before it follows the paths. Positions that
+// pass a filter are the ones with long lists, and 32 of them are injected at once,
+// so that a batch's lists can be many times what the worklist holds (32 URLs
+// against 4000 rules on "http://www.": 128,000 entries). An injection therefore
+// stops near mark_inject entries, a quarter of the worklist; the paths are
+// followed, and it goes on from `resume` (0: all is done). Lists of up to that many
+// entries, nearly all, are injected in one go as before.
+__device__ __forceinline__ int held(const WarpRun& w) { return w.top + w.ovf_n; }
+static_assert((kStackCap + 1024) / 4 >= kInjectLow + 4 * 32, "short lists always fit");
+
 // Injects the states a tile has always active at the piece's offset r of each
-// lane (valid lanes): as inject_aas, without a window to clamp to.
+// lane (valid lanes): as inject_aas, without a window to clamp to. resume: index
+// into the always-active list (depth 0) or into the lanes' lists one after another.
 __device__ __forceinline__ void inject_run(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                            const TileView& tv, const RunCtx& c, int lane, bool valid,
-                                           int r, int depth, unsigned long long& n_injected) {
+                                           int r, int depth, uint32_t& resume,
+                                           unsigned long long& n_injected) {
   const TileDev& t = *tv.t;
   const uint32_t q = c.lo + (uint32_t)r;
+  const uint32_t from = resume;
+  resume = 0;
   if (depth == 0) {  // scan the always-active list
     const uint32_t s = valid ? symbol(c, r) : 0u;
-    for (int i = 0; i < t.naas; i++) {
+    for (int i = (int)from; i < t.naas; i++) {
+      if (held(w) > p.mark_inject - 32) {
+        resume = (uint32_t)i;
+        return;
+      }
       const uint32_t a = __ldg(t.aas + i);
       const bool ok = valid && accepts(tv, a, s);
       const bool rep = ok && is_report(tv, a);
@@ -305,7 +323,7 @@ __device__ __forceinline__ void inject_run(const MatchParams& p, WarpSmem& ws, W
     uint32_t rb, re;
     pt_find(deep, key, true, false, vb, ve, rb, re, one);
   }
-  if (tv.rep_levels) {  // reports of the first k symbols, level by level
+  if (tv.rep_levels && from == 0) {  // reports of the first k symbols, level by level
     uint32_t kk = 0;
 #pragma unroll
     for (int d = 0; d < kMaxDepth; d++) {
@@ -327,14 +345,14 @@ __device__ __forceinline__ void inject_run(const MatchParams& p, WarpSmem& ws, W
   }
   // entries at the segment's last position have nothing to expand
   const uint32_t len = use && r + k < c.lim ? (ve - vb) + (one != kNoEntry ? 1u : 0u) : 0u;
-  n_injected += len;
+  if (from == 0) n_injected += len;
   uint32_t incl = len;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t y = __shfl_up_sync(kFull, incl, o);
     if (lane >= o) incl += y;
   }
-  const uint32_t total = __shfl_sync(kFull, incl, 31);
+  uint32_t total = __shfl_sync(kFull, incl, 31);
   if (total == 0) return;
   const uint32_t off = (uint32_t)(r + k - 1);
   if (__reduce_max_sync(kFull, len) <= 4u) {  // short lists: every lane copies its own
@@ -350,7 +368,10 @@ __device__ __forceinline__ void inject_run(const MatchParams& p, WarpSmem& ws, W
     ws.inj[32 + lane] = one != kNoEntry ? one : vb;  // a lone state itself, or where the list starts
     ws.inj[64 + lane] = off | (uint32_t)(k > 0 ? k : 1) << 16 | (one != kNoEntry ? 0x1000000u : 0u);
     __syncwarp();
-    for (uint32_t i = lane; i < total; i += 32) {
+    const uint32_t all = total;
+    total = min(all, from + (uint32_t)(p.mark_inject - held(w)));  // what there is room for
+    if (total < all) resume = total;
+    for (uint32_t i = from + lane; i < total; i += 32) {
       int l0 = 0, l1 = 31;
       while (l0 < l1) {  // first lane whose inclusive prefix exceeds i
         const int m = (l0 + l1) >> 1;
@@ -361,8 +382,9 @@ __device__ __forceinline__ void inject_run(const MatchParams& p, WarpSmem& ws, W
       const uint32_t x = ws.inj[64 + l0];
       const uint32_t v = x >> 24 ? ws.inj[32 + l0]
                                  : __ldg(tv.pt[((x >> 16) & 0xffu) - 1].vlist + ws.inj[32 + l0] + (i - before));
-      store_entry(p, ws, w, w.top + (int)i, (v << kEntryPosBits) | (x & 0xffffu));
+      store_entry(p, ws, w, w.top + (int)(i - from), (v << kEntryPosBits) | (x & 0xffffu));
     }
+    total -= from;
   }
   grow_stack(p, w, (int)total);
   __syncwarp();
@@ -370,11 +392,19 @@ __device__ __forceinline__ void inject_run(const MatchParams& p, WarpSmem& ws, W
 
 // Start-of-data states at the piece's first position (ngap_buffer.cu:613-631),
 // except sticky ones of layered tiles (registered from the activation pass).
+// resume: index into the start-of-data list.
 __device__ __forceinline__ void inject_starts(const MatchParams& p, WarpSmem& ws, WarpRun& w,
-                                              const TileView& tv, const RunCtx& c, int lane) {
+                                              const TileView& tv, const RunCtx& c, int lane,
+                                              uint32_t& resume) {
   const TileDev& t = *tv.t;
   const uint32_t s0 = symbol(c, 0);
-  for (int i0 = 0; i0 < t.nstart; i0 += 32) {
+  int i0 = (int)resume;
+  resume = 0;
+  for (; i0 < t.nstart; i0 += 32) {
+    if (held(w) > p.mark_inject - 32) {
+      resume = (uint32_t)i0;
+      return;
+    }
     const int i = i0 + lane;
     const uint32_t v = i < t.nstart ? __ldg(t.start + i) : 0u;
     const bool ok = i < t.nstart && accepts(tv, v, s0);
@@ -389,17 +419,21 @@ __device__ __forceinline__ void inject_starts(const MatchParams& p, WarpSmem& ws
 // filter leaves few positions, so lanes hold sticky states (32 at a time, their
 // slot, first match and union mask in registers) and the candidates are
 // visited one by one: a pass over n states costs n / 32 steps per candidate. Same
-// rule as layered_sticky_positions; reporting sticky states get no filter.
+// rule as layered_sticky_positions; reporting sticky states get no filter. resume:
+// the first of 32 sticky states + the candidate.
 // Measured on a B200, whole calls, layered tiles without and with a filter: the
 // 32 MiB mix 2.41 -> 1.16 ms (20.8 M expansions -> 1.3 M), 512 streams against
 // eight rule sets 32.5 -> 10.8 ms, 300 dot-star regexes on 4 MB 0.80 -> 0.38.
 __device__ __forceinline__ void layered_run(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                             const TileView& tv, const RunCtx& c, int lane, int rc,
-                                            int m, int64_t row, uint32_t n) {
+                                            int m, int64_t row, uint32_t n, uint32_t& resume) {
   const TileDev& t = *tv.t;
   const uint32_t cls = lane < m ? symbol(c, rc) : 0u;
-  uint32_t next = (uint32_t)lane < n ? __ldg(p.act_list + row + lane) : 0u;
-  for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+  uint32_t i0 = resume & ~31u;
+  int k = (int)(resume & 31u);
+  resume = 0;
+  uint32_t next = i0 + (uint32_t)lane < n ? __ldg(p.act_list + row + i0 + lane) : 0u;
+  for (; i0 < n; i0 += 32, k = 0) {
     const uint32_t i = i0 + (uint32_t)lane;
     const uint32_t sl = next;
     if (i + 32 < n) next = __ldg(p.act_list + row + i + 32);
@@ -409,7 +443,7 @@ __device__ __forceinline__ void layered_run(const MatchParams& p, WarpSmem& ws, 
     const uint32_t u0 = i < n ? __ldg(um) : 0u;
     const uint32_t u1 = i < n && tv.cw > 1 ? __ldg(um + 1) : 0u;
     const uint32_t u2 = i < n && tv.cw > 2 ? __ldg(um + 2) : 0u;
-    for (int k = 0; k < m; k++) {
+    for (; k < m; k++) {
       const int r = __shfl_sync(kFull, rc, k);
       const uint32_t sym = __shfl_sync(kFull, cls, k);
       const uint32_t rel = c.lo + (uint32_t)r - w.base;  // position in the segment
@@ -437,6 +471,10 @@ __device__ __forceinline__ void layered_run(const MatchParams& p, WarpSmem& ws, 
         if (ok[j]) store_entry(p, ws, w, pos++, ((us[j] & kIdMask) << kEntryPosBits) | (uint32_t)r);
       grow_stack(p, w, total);
       __syncwarp();
+      if (held(w) > p.mark_inject - 4 * 32) {
+        resume = k + 1 < m ? i0 + (uint32_t)k + 1u : i0 + 32 < n ? i0 + 32 : 0u;
+        if (resume) return;
+      }
     }
   }
 }
@@ -564,19 +602,26 @@ __global__ void __launch_bounds__(kRunWarps * 32, 1) run_kernel(MatchParams p, c
     w.act = !LAYERED && t->phase == 1 ? p.act + run.act_row : nullptr;
     TileRun tr;
     tile_run<!LAYERED>(p, t, t->pt, cls, tr);
-    if (run.starts) inject_starts(p, ws, w, tr.tv, c, lane);
     const int batch = LAYERED ? 32 : min(tr.batch, 32);
     const uint32_t active = LAYERED ? p.act_cnt[run.act_rowid] : 0u;
-    for (uint32_t c0 = 0; c0 < run.n; c0 += batch) {
-      const int m = (int)min((uint32_t)batch, run.n - c0);
-      const int r = lane < m ? (int)__ldg(cand + run.first + c0 + lane) : 0;
-      if (LAYERED)
-        layered_run(p, ws, w, tr.tv, c, lane, r, m, run.act_row, active);
-      else
-        inject_run(p, ws, w, tr.tv, c, lane, lane < m, r, tr.depth, n_injected);
-      if (w.top >= kInjectLow || w.ovf_n > 0) walk_run(p, ws, w, tr.tv, c, lane, n_expanded);
+    bool starts = run.starts != 0u;
+    uint32_t c0 = 0, resume = 0;
+    while (starts || c0 < run.n) {
+      if (starts) {
+        inject_starts(p, ws, w, tr.tv, c, lane, resume);
+        starts = resume != 0u;
+      } else {
+        const int m = (int)min((uint32_t)batch, run.n - c0);
+        const int r = lane < m ? (int)__ldg(cand + run.first + c0 + lane) : 0;
+        if (LAYERED)
+          layered_run(p, ws, w, tr.tv, c, lane, r, m, run.act_row, active, resume);
+        else
+          inject_run(p, ws, w, tr.tv, c, lane, lane < m, r, tr.depth, resume, n_injected);
+        if (resume == 0u) c0 += batch;
+      }
+      // the paths: when the worklist is full enough, and at the end
+      if (held(w) >= (starts || c0 < run.n ? kInjectLow : 1)) walk_run(p, ws, w, tr.tv, c, lane, n_expanded);
     }
-    if (w.top > 0 || w.ovf_n > 0) walk_run(p, ws, w, tr.tv, c, lane, n_expanded);
     if (p.unit_work) {  // work of the run's piece (all lanes)
       unsigned long long d = n_expanded + n_injected - work0;
 #pragma unroll
