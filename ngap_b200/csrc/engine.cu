@@ -41,6 +41,8 @@ namespace {
 // the radix pipeline after the small-set sort, [kCursors ...] the unit cursors
 // of the three launches, [kSliceCtl ...] the control words of the slices.
 constexpr int kDefaultQueue = 1 << 16;  // overflow-stack entries per warp
+constexpr int kQueueSpare = 128;  // more of them: a worklist holds the caller's capacity and 512 entries
+static_assert(kStackCap + kQueueSpare == 512, "512 entries, in shared memory or beyond it");
 constexpr int kRadixCount = 8;
 constexpr int kCursors = 10;
 constexpr int kSliceCtl = 16;
@@ -553,7 +555,8 @@ int ensure_reports(ngap_engine* e, uint64_t cap) {
   return NGAP_OK;
 }
 
-int ensure_slots(ngap_engine* e, size_t slots, int max_states, int max_nact, int ovf_cap) {
+int ensure_slots(ngap_engine* e, size_t slots, int max_states, int max_nact, int queue) {
+  int ovf_cap = queue + kQueueSpare;
   int carry_cap = std::max(max_states, 32);
   int mark_words = (max_states + 31) / 32 + 1;
   // the overflow stacks only grow: a request for fewer entries than held
@@ -1026,6 +1029,15 @@ int launch_grid(int64_t nunits, int grid) {
 // (the layered tiles read what the first launch recorded).
 int launch_plan(ngap_engine* e, MatchParams mp, const std::vector<TileDev>& tiles, int smem,
                 uint32_t last, cudaStream_t st) {
+  auto set_marks = [](MatchParams& m, int longest) {
+    const WorklistMarks k = worklist_marks(kStackCap + m.ovf_cap, longest);
+    m.mark_inject = k.inject;
+    m.mark_walk = k.walk;
+    m.mark_single = k.single;
+  };
+  set_marks(mp, mp.window);
+  MatchParams rp = mp;  // the runs': no windows, paths to their end
+  set_marks(rp, kMaxRunPath);
   if (e->act_entries > 0)
     CUDA_TRY(cudaMemsetAsync(e->d_act, 0xff, (size_t)e->act_entries * sizeof(uint32_t), st));
   auto run = [&](bool lean, int which) -> int {
@@ -1052,7 +1064,7 @@ int launch_plan(ngap_engine* e, MatchParams mp, const std::vector<TileDev>& tile
   sp.runs = e->d_runs;
   sp.act_cnt = e->d_act_cnt;
   sp.cycles = mp.unit_cycles ? mp.unit_cycles + e->nunits : nullptr;
-  mp.piece_unit0 = e->nunits;
+  rp.piece_unit0 = e->nunits;
   unsigned int* const ctl0 = reinterpret_cast<unsigned int*>(e->d_counters + kSliceCtl);
   auto run_slices = [&](bool layered) -> int {
     for (size_t i = 0; i < e->ranges.slices.size(); i++) {
@@ -1077,9 +1089,9 @@ int launch_plan(ngap_engine* e, MatchParams mp, const std::vector<TileDev>& tile
       scan_kernel<<<launch_grid(s.count, e->grid), kScanWarps * 32, kScanWarps * kScanWarpBytes, st>>>(sp);
       const int grid = launch_grid(s.runs, e->grid);
       if (layered)
-        run_kernel<true><<<grid, kRunWarps * 32, run_smem_bytes(), st>>>(mp, e->d_cand, e->d_runs, ctl);
+        run_kernel<true><<<grid, kRunWarps * 32, run_smem_bytes(), st>>>(rp, e->d_cand, e->d_runs, ctl);
       else
-        run_kernel<false><<<grid, kRunWarps * 32, run_smem_bytes(), st>>>(mp, e->d_cand, e->d_runs, ctl);
+        run_kernel<false><<<grid, kRunWarps * 32, run_smem_bytes(), st>>>(rp, e->d_cand, e->d_runs, ctl);
       CUDA_TRY(cudaGetLastError());
       e->launches += 2;
     }
@@ -1479,7 +1491,6 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   mp.carry_cap = e->carry_cap;
   mp.mark_words = e->mark_words;
   mp.ovf_cap = e->ovf_cap;
-  mp.mark_inject = (kStackCap + e->ovf_cap) / 4;
   mp.work = e->d_counters + 2;
   mp.act = e->d_act;
   mp.act_list = e->d_act_list;
@@ -1938,7 +1949,6 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   mp.carry_cap = e->carry_cap;
   mp.mark_words = e->mark_words;
   mp.ovf_cap = e->ovf_cap;
-  mp.mark_inject = (kStackCap + e->ovf_cap) / 4;
   mp.work = e->d_counters + 2;
   mp.act = e->d_act;
   mp.act_list = e->d_act_list;

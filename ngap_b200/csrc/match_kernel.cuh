@@ -80,7 +80,7 @@ struct MatchParams {
   uint32_t* marks;          // [slots][mark_words]
   uint32_t* ovf;            // [slots][ovf_cap]
   int32_t carry_cap, mark_words, ovf_cap;
-  int32_t mark_inject;      // entries of a run's worklist at which its injection waits
+  int32_t mark_inject, mark_walk, mark_single;  // worklist_marks
   unsigned long long* work; // [0] entries expanded, [1] entries injected
   uint32_t* act;            // activation slots (first match of sticky states, offset in the
                             // segment; 0xffffffff = none)
@@ -297,6 +297,25 @@ __device__ __forceinline__ void store_entry(const MatchParams& p, WarpSmem& ws, 
     if (j < p.ovf_cap) w.ovf[j] = e;
     else atomicOr(p.err, kErrQueue);
   }
+}
+
+// Entries on a warp's worklist.
+__device__ __forceinline__ int held(const WarpRun& w) { return w.top + w.ovf_n; }
+
+// How full a worklist of `all` entries may be before its warp works in another
+// way: mark_inject, at which a run's injection waits (scan_kernel.cuh); mark_walk,
+// above which paths are not followed in registers (32 of them leave up to three
+// entries each at every symbol, which nobody takes while they last) but the 32
+// entries on top are expanded at a time, short-lived ones with the others;
+// mark_single, above which the top entry alone is, depth first: three more
+// entries a symbol at most, for which `longest` symbols' room is left where there
+// is that much. Few matches come near any of them.
+struct WorklistMarks {
+  int32_t inject, walk, single;
+};
+__host__ __device__ inline WorklistMarks worklist_marks(int all, int longest) {
+  const int room = 3 * longest + 5 * 32;
+  return {all / 4, all / 2, all - (all / 4 < room ? all / 4 : room)};
 }
 
 __device__ __forceinline__ void grow_stack(const MatchParams& p, WarpRun& w, int cnt) {
@@ -1017,12 +1036,12 @@ __device__ __forceinline__ void layered_sticky_positions(const MatchParams& p, W
 }
 
 // Expands the up-to-32 entries on top of the stack: one step of the worklist.
-// For tiles that register sticky states, and for --unique; the others follow
-// their paths in registers (walk_paths).
+// For tiles that register sticky states, for --unique and for worklists past
+// mark_walk; otherwise paths are followed in registers (walk_paths).
 __device__ __forceinline__ void expand_step(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                             const TileView& tv, const UnitCtx& c, int lane,
                                             int cursor, unsigned long long& n_expanded) {
-  const int n = min(w.top, 32);
+  const int n = min(w.top, held(w) > p.mark_single ? 1 : 32);
   uint32_t e = lane < n ? ws.stack[w.top - 1 - lane] : kNoEntry;
   w.top -= n;
   __syncwarp();
@@ -1107,6 +1126,10 @@ __device__ __forceinline__ void walk_paths(const MatchParams& p, WarpSmem& ws, W
   bool act = false;
   unsigned live = 0u;
   while (true) {
+    if (held(w) > p.mark_walk) {  // back to the worklist: expand_step goes on
+      push_entry(p, ws, w, lane, act, (v << kEntryPosBits) | (uint32_t)r);
+      return;
+    }
     if (w.top > 0 && __popc(live) <= 16) {  // idle lanes take the entries on top of the stack
       const int n = min(w.top, 32 - __popc(live));
       const int k = __popc(~live & lanemask_lt(lane));
@@ -1462,7 +1485,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
           break;
         }
         // (layered tiles have no edge into a sticky state: no successor to register)
-        if ((LEAN || !tv.sticky || layered) && !p.unique)
+        if ((LEAN || !tv.sticky || layered) && !p.unique && held(w) <= p.mark_walk)
           walk_paths(p, ws, w, tv, c, lane, n_expanded);
         else
           expand_step(p, ws, w, tv, c, lane, cursor, n_expanded);

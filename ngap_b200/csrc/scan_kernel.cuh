@@ -26,8 +26,9 @@
 
 namespace ngap {
 
+constexpr int kMaxRunPath = 2048;  // states of the longest path of an acyclic tile (TableOpts::max_warmup)
 constexpr int kPieceMax = 4096;  // run entries pack offsets below kPieceMax + the longest path
-static_assert(kPieceMax + 2048 + kMaxDepth < kMaxWindow, "offsets fit worklist entries");
+static_assert(kPieceMax + kMaxRunPath + kMaxDepth < kMaxWindow, "offsets fit worklist entries");
 constexpr int kScanWarps = 32;
 constexpr int kScanLane = 8;     // positions per lane and step: reads in flight
 constexpr int kScanMinPiece = 32 * kScanLane;
@@ -254,8 +255,16 @@ __device__ __forceinline__ uint32_t symbol(const RunCtx& c, int r) { return __ld
 // stops near mark_inject entries, a quarter of the worklist; the paths are
 // followed, and it goes on from `resume` (0: all is done). Lists of up to that many
 // entries, nearly all, are injected in one go as before.
-__device__ __forceinline__ int held(const WarpRun& w) { return w.top + w.ovf_n; }
 static_assert((kStackCap + 1024) / 4 >= kInjectLow + 4 * 32, "short lists always fit");
+
+// Entries from the overflow stack to the empty shared one.
+__device__ __forceinline__ void refill_stack(WarpSmem& ws, WarpRun& w, int lane) {
+  const int m = min(w.ovf_n, kStackCap);
+  for (int i = lane; i < m; i += 32) ws.stack[i] = w.ovf[w.ovf_n - m + i];
+  w.ovf_n -= m;
+  w.top = m;
+  __syncwarp();
+}
 
 // Injects the states a tile has always active at the piece's offset r of each
 // lane (valid lanes): as inject_aas, without a window to clamp to. resume: index
@@ -479,6 +488,46 @@ __device__ __forceinline__ void layered_run(const MatchParams& p, WarpSmem& ws, 
   }
 }
 
+// One step of a run's worklist past mark_walk: expand_step without windows.
+__device__ __forceinline__ void step_run(const MatchParams& p, WarpSmem& ws, WarpRun& w,
+                                         const TileView& tv, const RunCtx& c, int lane,
+                                         unsigned long long& n_expanded) {
+  if (w.top == 0) refill_stack(ws, w, lane);
+  const int n = min(w.top, held(w) > p.mark_single ? 1 : 32);
+  const uint32_t e = lane < n ? ws.stack[w.top - 1 - lane] : 0u;
+  w.top -= n;
+  __syncwarp();
+  const uint32_t v = e >> kEntryPosBits;
+  const int r = (int)(e & ((1u << kEntryPosBits) - 1));
+  const bool go = lane < n && r + 1 < c.lim;
+  uint4 sc = make_uint4(kNoSucc, kNoSucc, kNoSucc, kNoSucc);
+  uint4 sm = make_uint4(0u, 0u, 0u, 0u);
+  uint32_t s = 0u;
+  if (go) {
+    load_record(tv, v, sc, sm);
+    s = symbol(c, r + 1);
+  }
+  n_expanded += go;
+  const uint32_t u[4] = {sc.x, sc.y, sc.z, sc.w};
+  const uint32_t um[4] = {sm.x, sm.y, sm.z, sm.w};
+  bool ok[4];
+  int cnt = 0;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    ok[j] = go && succ_accepts(tv, u[j], um[j], s);
+    cnt += ok[j];
+  }
+  report4(p, ws, w, tv, lane, ok, u, (int64_t)c.lo + r + 1, true);
+  const int more = go && r + 2 < c.lim ? cnt : 0;  // the successors have a next symbol
+  int total;
+  int pos = w.top + warp_excl<3>(more, lane, total);
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+    if (more && ok[j]) store_entry(p, ws, w, pos++, ((u[j] & kIdMask) << kEntryPosBits) | (uint32_t)(r + 1));
+  grow_stack(p, w, total);
+  __syncwarp();
+}
+
 // Follows every path on the stack to its end: walk_paths without windows (no
 // state is carried over).
 __device__ __forceinline__ void walk_run(const MatchParams& p, WarpSmem& ws, WarpRun& w,
@@ -489,13 +538,13 @@ __device__ __forceinline__ void walk_run(const MatchParams& p, WarpSmem& ws, War
   bool act = false;
   unsigned live = 0u;
   while (true) {
-    if (w.top == 0 && w.ovf_n > 0 && __popc(live) <= 16) {  // refill from the overflow stack
-      const int m = min(w.ovf_n, kStackCap);
-      for (int i = lane; i < m; i += 32) ws.stack[i] = w.ovf[w.ovf_n - m + i];
-      w.ovf_n -= m;
-      w.top = m;
-      __syncwarp();
+    if (held(w) > p.mark_walk) {  // all paths back to the worklist until it is half as full
+      push_entry(p, ws, w, lane, act, (v << kEntryPosBits) | (uint32_t)r);
+      act = false;
+      live = 0u;
+      while (held(w) > p.mark_inject) step_run(p, ws, w, tv, c, lane, n_expanded);
     }
+    if (w.top == 0 && w.ovf_n > 0 && __popc(live) <= 16) refill_stack(ws, w, lane);
     if (w.top > 0 && __popc(live) <= 16) {  // idle lanes take the entries on top of the stack
       const int n = min(w.top, 32 - __popc(live));
       const int k = __popc(~live & lanemask_lt(lane));

@@ -105,3 +105,35 @@ def test_shared_prefix_with_automatic_worklists(engine):
     for _ in range(2):
         got = engine.match(nb.Tables(groups, precompute_depth=-1), data, 1, len(data))
         assert len(want) >= 15_000 and np.array_equal(got, want)
+
+
+def side_paths(rules, length):
+    """h a a a ...: every symbol matches the next state and three that end there."""
+    w = W.AnmlWriter("side")
+    for n in range(rules):
+        for i in range(length):
+            w.ste(f"p{n}_{i}", b"h" if i == 0 else b"a", [f"p{n}_{i + 1}"] + [f"d{n}_{i}_{k}" for k in range(3)]
+                  if i + 1 < length else [], start="all-input" if i == 0 else None, report=i + 1 == length)
+        for i in range(3 * length - 3):
+            w.ste(f"d{n}_{i // 3}_{i % 3}", b"a", [])
+    return nb.Groups(nb.Nfa.from_string(w.text()), group_num=1)
+
+
+@pytest.mark.parametrize("size", [20_000, 160_000])  # looked up position by position, and scanned
+@pytest.mark.parametrize("length", [60, 400, 2047])
+@pytest.mark.parametrize("algorithm", ["nonblockingallgroups", "NAPgroups"])
+def test_side_paths(built, size, length, algorithm):
+    """Long paths that leave three short ones at every symbol: 32 of them
+    followed side by side leave 96 entries a symbol, which wait for the paths' end."""
+    groups = side_paths(40 if length < 1000 else 10, length)
+    data = np.resize(np.frombuffer(b"h" + b"a" * (length - 1 if length > 1000 else length + 5), np.uint8), size)
+    check(groups, data, QUEUE, algorithm)
+
+
+def test_side_paths_with_automatic_worklists(engine):
+    groups = side_paths(40, 1400)
+    tables = nb.Tables(groups, precompute_depth=-1)
+    for size in (30_000, 160_000):
+        data = np.resize(np.frombuffer(b"h" + b"a" * 1500, np.uint8), size)
+        want, _ = oracle.match(groups.views(), data, 1, len(data))
+        assert len(want) > 0 and np.array_equal(engine.match(tables, data, 1, len(data)), want)
