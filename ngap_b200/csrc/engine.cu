@@ -418,10 +418,9 @@ int ngap_engine_create(int device, ngap_engine** out) {
                                 kSmallSortSmem));
   CUDA_TRY(cudaFuncSetAttribute(scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kScanWarps * kScanWarpBytes));
-  CUDA_TRY(cudaFuncSetAttribute(run_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                run_smem_bytes()));
-  CUDA_TRY(cudaFuncSetAttribute(run_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                run_smem_bytes()));
+  for (auto kernel : {run_kernel<false, false>, run_kernel<false, true>, run_kernel<true, false>,
+                      run_kernel<true, true>})
+    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, run_smem_bytes()));
   CUDA_TRY(cudaMallocHost(&e->ho.counters, kNumCounters * sizeof(unsigned long long)));
   CUDA_TRY(cudaMallocHost(&e->ho.reports, kHostReports * sizeof(uint64_t)));
   CUDA_TRY(cudaMallocHost(&e->ho.streams, kHostReports * sizeof(uint32_t)));
@@ -1088,10 +1087,9 @@ int launch_plan(ngap_engine* e, MatchParams mp, const std::vector<TileDev>& tile
       sp.strip_bits = s.longest >= 32 * kStripMax ? 4 : 3;
       scan_kernel<<<launch_grid(s.count, e->grid), kScanWarps * 32, kScanWarps * kScanWarpBytes, st>>>(sp);
       const int grid = launch_grid(s.runs, e->grid);
-      if (layered)
-        run_kernel<true><<<grid, kRunWarps * 32, run_smem_bytes(), st>>>(rp, e->d_cand, e->d_runs, ctl);
-      else
-        run_kernel<false><<<grid, kRunWarps * 32, run_smem_bytes(), st>>>(rp, e->d_cand, e->d_runs, ctl);
+      const auto kernel = layered ? (mp.unique ? run_kernel<true, true> : run_kernel<true, false>)
+                                  : (mp.unique ? run_kernel<false, true> : run_kernel<false, false>);
+      kernel<<<grid, kRunWarps * 32, run_smem_bytes(), st>>>(rp, e->d_cand, e->d_runs, ctl);
       CUDA_TRY(cudaGetLastError());
       e->launches += 2;
     }

@@ -488,18 +488,24 @@ __device__ __forceinline__ void layered_run(const MatchParams& p, WarpSmem& ws, 
   }
 }
 
-// One step of a run's worklist past mark_walk: expand_step without windows.
+// One step of a run's worklist past mark_walk, or with --unique: expand_step without windows.
+template <bool UNIQUE>
 __device__ __forceinline__ void step_run(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                          const TileView& tv, const RunCtx& c, int lane,
                                          unsigned long long& n_expanded) {
   if (w.top == 0) refill_stack(ws, w, lane);
   const int n = min(w.top, held(w) > p.mark_single ? 1 : 32);
-  const uint32_t e = lane < n ? ws.stack[w.top - 1 - lane] : 0u;
+  const uint32_t e = lane < n ? ws.stack[w.top - 1 - lane] : kNoEntry;
   w.top -= n;
   __syncwarp();
+  bool go = lane < n;
+  if (UNIQUE) {  // identical entries once (every lane votes; those without an entry hold kNoEntry)
+    const unsigned same = __match_any_sync(kFull, e);
+    go = go && __ffs(same) - 1 == lane;
+  }
   const uint32_t v = e >> kEntryPosBits;
   const int r = (int)(e & ((1u << kEntryPosBits) - 1));
-  const bool go = lane < n && r + 1 < c.lim;
+  go = go && r + 1 < c.lim;
   uint4 sc = make_uint4(kNoSucc, kNoSucc, kNoSucc, kNoSucc);
   uint4 sm = make_uint4(0u, 0u, 0u, 0u);
   uint32_t s = 0u;
@@ -542,7 +548,7 @@ __device__ __forceinline__ void walk_run(const MatchParams& p, WarpSmem& ws, War
       push_entry(p, ws, w, lane, act, (v << kEntryPosBits) | (uint32_t)r);
       act = false;
       live = 0u;
-      while (held(w) > p.mark_inject) step_run(p, ws, w, tv, c, lane, n_expanded);
+      while (held(w) > p.mark_inject) step_run<false>(p, ws, w, tv, c, lane, n_expanded);
     }
     if (w.top == 0 && w.ovf_n > 0 && __popc(live) <= 16) refill_stack(ws, w, lane);
     if (w.top > 0 && __popc(live) <= 16) {  // idle lanes take the entries on top of the stack
@@ -613,8 +619,10 @@ constexpr int kRunWarpBytes = kStackCap * 4 + kReportBuf * 8 + 3 * 32 * 4;
 static_assert(kRunWarpBytes % 16 == 0, "per-warp regions stay 16-byte aligned");
 __host__ __device__ inline int run_smem_bytes() { return kRunWarps * kRunWarpBytes; }
 
-// One warp per run. LAYERED: the runs' tiles are layered tiles.
-template <bool LAYERED>
+// One warp per run. LAYERED: the runs' tiles are layered tiles. UNIQUE: step by
+// step, dropping duplicate entries of a step (--unique): paths that meet in a state
+// at the same symbol are then followed once, as match_kernel does.
+template <bool LAYERED, bool UNIQUE>
 __global__ void __launch_bounds__(kRunWarps * 32, 1) run_kernel(MatchParams p, const uint16_t* cand,
                                                                const RunDev* runs, unsigned int* ctl) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -669,7 +677,11 @@ __global__ void __launch_bounds__(kRunWarps * 32, 1) run_kernel(MatchParams p, c
         if (resume == 0u) c0 += batch;
       }
       // the paths: when the worklist is full enough, and at the end
-      if (held(w) >= (starts || c0 < run.n ? kInjectLow : 1)) walk_run(p, ws, w, tr.tv, c, lane, n_expanded);
+      if (held(w) < (starts || c0 < run.n ? kInjectLow : 1)) continue;
+      if (UNIQUE)
+        while (held(w) > 0) step_run<true>(p, ws, w, tr.tv, c, lane, n_expanded);
+      else
+        walk_run(p, ws, w, tr.tv, c, lane, n_expanded);
     }
     if (p.unit_work) {  // work of the run's piece (all lanes)
       unsigned long long d = n_expanded + n_injected - work0;
