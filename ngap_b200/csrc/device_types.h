@@ -124,10 +124,23 @@ struct TileDev {
   const uint32_t* aas = nullptr;    // [naas] local ids
   const uint32_t* start = nullptr;  // [nstart] local ids
   int32_t run_len = 32;     // filter candidates per run
+  int32_t one_by_one = 0;   // blocking algorithm: windows of one position (many_paths)
   uint32_t rep_levels = 0;  // bit d: the depth-(d+1) table has report lists
   FilterDev filt;
   PrefixTableDev pt[kMaxDepth];
 };
+
+// Whether so many paths can end in one state at one position that following them one
+// by one is out of bounds: `most` of them, infinite in a cyclic tile. The blocking
+// algorithm, which looks at a state once a position, then works in windows of
+// one position, whose states are carried to the next without duplicates;
+// elsewhere it takes whole windows (algo_config). The line: edit-distance rules
+// (two edits in 20 symbols: at most 466 paths) are far better off in whole windows,
+// where few of those paths are ever alive (50 rules on 1 MiB: 318 ms in windows of
+// one position, 0.33 ms scanned on a B200); a bound far above theirs says that
+// paths multiply.
+constexpr double kManyPaths = 1024;
+inline bool many_paths(double most) { return !(most <= kManyPaths); }
 
 // A unit of work: one tile over input positions [lo, hi); reports are kept for
 // positions >= emit_lo (the positions before are warm-up of a chunk). A report

@@ -131,11 +131,12 @@ struct UnitPlanKey {
   int is_dup, window, chunk;
   int64_t first_seg;
   int depth;      // prefix depth of the algorithm
+  bool blocking;
   bool filtered;  // tiles with a filter may be scanned (off for the wait test hook)
   bool operator<(const UnitPlanKey& o) const {
-    return std::tie(num_seg, seg_len, is_dup, window, chunk, first_seg, depth, filtered) <
+    return std::tie(num_seg, seg_len, is_dup, window, chunk, first_seg, depth, blocking, filtered) <
            std::tie(o.num_seg, o.seg_len, o.is_dup, o.window, o.chunk, o.first_seg, o.depth,
-                    o.filtered);
+                    o.blocking, o.filtered);
   }
 };
 
@@ -165,7 +166,7 @@ struct ngap_engine {
   size_t input_cap = 0;
   // units (cached plan for one tables object)
   uint64_t plan_tables = 0;  // serial of the tables the plain plan was made for
-  UnitPlanKey plan_key{-1, -1, -1, -1, -1, -1, -1, true};
+  UnitPlanKey plan_key{-1, -1, -1, -1, -1, -1, -1, false, true};
   UnitDev* d_units = nullptr;
   size_t units_cap = 0;
   int32_t nunits = 0;
@@ -228,6 +229,7 @@ struct ngap_engine {
   uint64_t batch_ts = 0;     // serial of the tableset the batched plan was made for
   std::vector<ngap_batch_stream> batch_streams;
   int batch_window = -1, batch_chunk = -1, batch_depth = -1;
+  bool batch_blocking = false;
   uint32_t* d_stream_ids = nullptr;
   uint64_t stream_ids_cap = 0;
   cudaGraphExec_t graph = nullptr;
@@ -319,6 +321,7 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
     for (uint8_t a : gg.attrs) t->report_states += a & 2 ? 1 : 0;
   }
   for (auto& th : t->tiles) {
+    count_paths(th);
     if (th.nstates >= kMaxTileStates - 1) {
       set_error("a connected component has %d states; at most %d are supported per tile",
                 th.nstates, kMaxTileStates - 2);
@@ -359,6 +362,7 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
     if ((rc = t->upload(th.aas, &d.aas)) != NGAP_OK) return rc;
     if ((rc = t->upload(th.start, &d.start)) != NGAP_OK) return rc;
     d.run_len = run_len(th);
+    d.one_by_one = many_paths(th.max_paths) ? 1 : 0;
     d.filt.len = th.filt.len;
     d.filt.min_rep = th.filt.min_rep;
     d.filt.shift = th.filt.shift;
@@ -660,13 +664,15 @@ int64_t piece_len(int64_t positions, int64_t warps, int64_t chunk_opt) {
 // start costs more than looking every position up: an 81-byte line matches
 // in 22 us in match_kernel and 30 us scanned, 64 literals on 1 MiB in 43 and 33.
 constexpr double kScanMin = 1 << 17;
-bool is_scanned(const TileHost& th) { return th.filt.len > 0 && th.max_path >= 0; }
+bool is_scanned(const TileHost& th, bool blocking) {
+  return th.filt.len > 0 && th.max_path >= 0 && !(blocking && many_paths(th.max_paths));
+}
 
 // Positions and the states that a look-up of each would inject at prefix depth
 // `depth` (keys equally likely), with the levels that follow; layered tiles test
 // their sticky states instead.
-double scan_work(const TileHost& th, int depth, int64_t positions) {
-  if (!is_scanned(th)) return 0.0;
+double scan_work(const TileHost& th, int depth, bool blocking, int64_t positions) {
+  if (!is_scanned(th, blocking)) return 0.0;
   if (th.phase == 2) return (double)positions * (1 + th.nact);
   const int d = std::max(1, std::min(depth, th.depth));
   return (double)positions * (1 + 4 * (double)th.pt[d - 1].entries / std::pow((double)std::max(1, th.nlive), d));
@@ -823,9 +829,9 @@ ActRows plan_units(const ngap_tables* t, const UnitPlanKey& k, int grid,
   ac.warps = (int64_t)grid * kWarpsPerCta;
   int64_t scanned = 0;
   double work = 0;
-  for (const TileHost& th : t->tiles) work += scan_work(th, k.depth, k.num_seg * k.seg_len);
+  for (const TileHost& th : t->tiles) work += scan_work(th, k.depth, k.blocking, k.num_seg * k.seg_len);
   const bool scan = k.filtered && work >= kScanMin;
-  auto scans = [&](const TileHost& th) { return scan && is_scanned(th); };
+  auto scans = [&](const TileHost& th) { return scan && is_scanned(th, k.blocking); };
   for (const TileHost& th : t->tiles) {
     if (scans(th)) scanned += k.num_seg * k.seg_len;
     else ac.add(th, k.num_seg * k.seg_len);
@@ -887,7 +893,7 @@ int trace_buffer(ngap_engine* e, cudaStream_t st, unsigned long long** work,
 // gone, nor half of its own. The next match plans again.
 void forget_plan(ngap_engine* e) {
   e->plan_tables = 0;
-  e->plan_key = UnitPlanKey{-1, -1, -1, -1, -1, -1, -1, true};
+  e->plan_key = UnitPlanKey{-1, -1, -1, -1, -1, -1, -1, false, true};
   e->batch_ts = 0;
 }
 
@@ -1364,7 +1370,9 @@ cudaError_t copy_results(const ngap_engine* e, uint64_t n, uint64_t* reports, ui
 // --algorithm -> prefix depth. The blocking algorithm scans the always-active
 // list like NAP, over whole windows: windows of one position cost a TMA copy
 // and a wait per position and tile (64 literals in ten groups on 1 MiB: 9466 us
-// on a B200, 85 us with windows of 2048). R1, R2 and all ask for
+// on a B200, 85 us with windows of 2048). Within a window it follows paths, not
+// states: tiles in which many paths can meet (cyclic ones, above all, where they
+// would double at every symbol) keep windows of one position. R1, R2 and all ask for
 // privatization, which the kernel does for every algorithm (walk_paths).
 int algo_config(int algo, int table_depth, int* depth) {
   switch (algo) {
@@ -1427,6 +1435,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   for (auto& th : t->tiles) table_depth = std::max(table_depth, th.depth);
   int rc = algo_config(p->algorithm, table_depth, &depth);
   if (rc != NGAP_OK) return rc;
+  const bool blocking = p->algorithm == NGAP_ALGO_BLOCKING;
   window = std::min(window, kMaxWindow);
   const bool in_place = input_in_place(e, input, input_on_device, total);
   if (!in_place && (rc = ensure_input(e, total)) != NGAP_OK) return rc;
@@ -1442,7 +1451,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   const int full_grid = e->num_sms * bps;
   // units
   UnitPlanKey key{p->num_seg, p->seg_len, p->is_dup ? 1 : 0, window, p->chunk, p->first_segment,
-                  depth, e->test_skip_unit < 0};
+                  depth, blocking, e->test_skip_unit < 0};
   if (e->plan_tables != t->serial || key < e->plan_key || e->plan_key < key) {
     forget_plan(e);
     std::vector<UnitDev> units;
@@ -1476,6 +1485,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   mp.input = in_place ? input : e->d_input;
   mp.window = window;
   mp.depth = depth;
+  mp.blocking = blocking;
   mp.unique = p->unique;
   mp.report_off = p->report_off;
   mp.off_shift = 32;
@@ -1834,6 +1844,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   int depth = 1, window = p->window > 0 ? p->window : 2048;
   int rc = algo_config(p->algorithm, ts->max_depth, &depth);
   if (rc != NGAP_OK) return rc;
+  const bool blocking = p->algorithm == NGAP_ALGO_BLOCKING;
   window = std::min(window, kMaxWindow);
   while (window > 64 && cta_smem_bytes(window) > 227 * 1024 - 1024) window /= 2;
   int smem = cta_smem_bytes(window);
@@ -1866,7 +1877,8 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     return true;
   };
   bool replanned = false;
-  if (e->batch_ts != ts->serial || e->batch_depth != depth || e->batch_window != window || e->batch_chunk != p->chunk ||
+  if (e->batch_ts != ts->serial || e->batch_depth != depth ||
+      e->batch_blocking != blocking || e->batch_window != window || e->batch_chunk != p->chunk ||
       !same_streams() || e->plan_tables != 0) {
     forget_plan(e);
     std::vector<std::vector<int>> by_nfa(ts->tables.size());
@@ -1878,8 +1890,8 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     int64_t scanned = 0;
     double work = 0;
     for (const ngap_batch_stream& s : sv)
-      for (const TileHost& th : ts->tables[s.nfa]->tiles) work += scan_work(th, depth, (int64_t)s.length);
-    auto scans = [&](const TileHost& th) { return work >= kScanMin && is_scanned(th); };
+      for (const TileHost& th : ts->tables[s.nfa]->tiles) work += scan_work(th, depth, blocking, (int64_t)s.length);
+    auto scans = [&](const TileHost& th) { return work >= kScanMin && is_scanned(th, blocking); };
     for (const ngap_batch_stream& s : sv)
       for (const TileHost& th : ts->tables[s.nfa]->tiles) {
         if (scans(th)) scanned += (int64_t)s.length;
@@ -1916,6 +1928,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     e->batch_streams = sv;
     e->batch_window = window;
     e->batch_depth = depth;
+    e->batch_blocking = blocking;
     e->batch_chunk = p->chunk;
     replanned = true;
   }
@@ -1934,6 +1947,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   mp.input = in_place ? input : e->d_input;
   mp.window = window;
   mp.depth = depth;
+  mp.blocking = blocking;
   mp.unique = p->unique;
   mp.report_off = p->report_off;
   mp.off_shift = oshift;

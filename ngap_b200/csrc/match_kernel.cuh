@@ -69,6 +69,7 @@ struct MatchParams {
   const uint8_t* input;     // 16-byte aligned, readable up to round_up(len, 16)
   int32_t window;           // W <= kMaxWindow
   int32_t depth;            // 0: scan the AAS list; >= 1: tables up to min(depth, tile.depth)
+  int32_t blocking;         // blocking algorithm: tiles marked one_by_one get windows of one position
   int32_t unique;
   int32_t report_off;
   int32_t off_shift;        // bit position of the offset in report keys (32 when not batched)
@@ -303,8 +304,8 @@ __device__ __forceinline__ void store_entry(const MatchParams& p, WarpSmem& ws, 
 __device__ __forceinline__ int held(const WarpRun& w) { return w.top + w.ovf_n; }
 
 // How full a worklist of `all` entries may be before its warp works in another
-// way: mark_inject, at which a run's injection waits (scan_kernel.cuh); mark_walk,
-// above which paths are not followed in registers (32 of them leave up to three
+// way: mark_inject, at which a run's injection waits (scan_kernel.cuh), and here
+// that of the always-active list; mark_walk, above which paths are not followed in registers (32 of them leave up to three
 // entries each at every symbol, which nobody takes while they last) but the 32
 // entries on top are expanded at a time, short-lived ones with the others;
 // mark_single, above which the top entry alone is, depth first: three more
@@ -523,17 +524,26 @@ __device__ __forceinline__ bool register_each(const MatchParams& p, WarpSmem& ws
   return mine;
 }
 
-// Always-active states for window offsets [r0, r0 + batch) (one per lane).
+// Always-active states for window offsets [r0, r0 + batch) (one per lane). resume:
+// index into the always-active list (depth 0) at which the last call stopped, its
+// worklist near mark_inject; 0 when it is through.
 __device__ __forceinline__ void inject_aas(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                            const TileView& tv, const UnitCtx& c, int lane, int r0,
-                                           int batch, int depth, unsigned long long& n_injected) {
+                                           int batch, int depth, int& resume,
+                                           unsigned long long& n_injected) {
   const TileDev& t = *tv.t;
   const int r = r0 + lane;
   const bool valid = lane < batch && r < c.iend;
   const int64_t q = c.wb + r;
   if (depth == 0) {  // scan the always-active list
     const uint32_t s = valid ? c.in[r] : 0u;
-    for (int i = 0; i < t.naas; i++) {
+    int i = resume;
+    resume = 0;
+    for (; i < t.naas; i++) {
+      if (held(w) > p.mark_inject - 32) {
+        resume = i;
+        return;
+      }
       const uint32_t a = __ldg(t.aas + i);
       const bool ok = valid && accepts(tv, a, s);
       const bool rep = ok && is_report(tv, a) && q >= c.emit_lo;
@@ -848,9 +858,10 @@ __device__ __forceinline__ void inject_aas2(const MatchParams& p, WarpSmem& ws, 
 // these positions. Layered tiles (phase 2) do their sticky work separately.
 __device__ __forceinline__ void inject(const MatchParams& p, WarpSmem& ws, WarpRun& w,
                                        const TileView& tv, const UnitCtx& c, int lane, int r0,
-                                       int batch, int depth, unsigned long long& n_injected) {
-  inject_aas(p, ws, w, tv, c, lane, r0, batch, depth, n_injected);
-  if (!tv.sticky || tv.t->phase == 2) return;
+                                       int batch, int depth, int& resume,
+                                       unsigned long long& n_injected) {
+  inject_aas(p, ws, w, tv, c, lane, r0, batch, depth, resume, n_injected);
+  if (resume || !tv.sticky || tv.t->phase == 2) return;
   __syncwarp();
   const int np = min((int)*ws.pend_n, kPendCap);
   for (int i = 0; i < np; i++) {
@@ -1245,13 +1256,12 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   __shared__ __align__(16) PrefixTableDev s_pt[kMaxDepth];
   __shared__ __align__(16) uint8_t s_cls[256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int W = p.window;
-  uint8_t* base = smem_raw + (size_t)warp * warp_smem_bytes(W);
+  uint8_t* base = smem_raw + (size_t)warp * warp_smem_bytes(p.window);
   WarpSmem ws;
   ws.stack = reinterpret_cast<uint32_t*>(base);
   ws.in[0] = base + kStackCap * 4;
-  ws.in[1] = ws.in[0] + window_buf_bytes(W);
-  ws.rbuf = reinterpret_cast<unsigned long long*>(ws.in[1] + window_buf_bytes(W));
+  ws.in[1] = ws.in[0] + window_buf_bytes(p.window);
+  ws.rbuf = reinterpret_cast<unsigned long long*>(ws.in[1] + window_buf_bytes(p.window));
   ws.inj = reinterpret_cast<uint32_t*>(ws.rbuf + kReportBuf);
   ws.bar = reinterpret_cast<uint64_t*>(ws.inj + 3 * 32);
   ws.stk_s = reinterpret_cast<uint32_t*>(ws.bar + 2);
@@ -1286,7 +1296,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
   // loads window [wb, min(wb + W, hi)) plus one look-ahead byte and `lb`
   // look-behind bytes into buffer buf; returns the byte count, and in `skip`
   // the offset of wb's byte in the buffer
-  auto issue = [&](int buf, int64_t wb, int64_t hi, int lb, uint32_t& skip) {
+  auto issue = [&](int buf, int64_t wb, int W, int64_t hi, int lb, uint32_t& skip) {
     const int64_t we = min(wb + (int64_t)W, hi);
     const int64_t end = min(we + 1, hi);
     const int64_t a0 = (wb - lb) & ~(int64_t)15;
@@ -1320,6 +1330,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
     const TileView& tv = tr.tv;
     const int depth = tr.depth, batch = tr.batch, defer = tr.defer;
     const bool layered = tr.layered, wide_inject = tr.wide_inject;
+    const int W = p.blocking && t->one_by_one ? 1 : p.window;
     const UnitDev un = p.units[uid];
     const unsigned long long work0 = n_expanded + n_injected;  // per-unit trace
     if (p.unit_work && lane == 0) p.unit_cycles[uid] = clock64();  // start; the end subtracts
@@ -1372,7 +1383,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
     int cur = 0;
     uint32_t nbytes[2], skip[2];
     if (c.hi > un.lo && (int32_t)uid != p.skip_copy_unit) {
-      nbytes[0] = issue(0, un.lo, c.hi, 0, skip[0]);
+      nbytes[0] = issue(0, un.lo, W, c.hi, 0, skip[0]);
     } else {  // idle, or the test hook: nothing is in flight (the hook's first wait gives up)
       nbytes[0] = 0u;
       skip[0] = 0u;
@@ -1405,7 +1416,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
       live = __any_sync(kFull, live);
       __syncwarp();
       if (we < c.hi)
-        nbytes[cur ^ 1] = issue(cur ^ 1, we, c.hi, (int)min((int64_t)defer, we - un.lo), skip[cur ^ 1]);
+        nbytes[cur ^ 1] = issue(cur ^ 1, we, W, c.hi, (int)min((int64_t)defer, we - un.lo), skip[cur ^ 1]);
       c.in = ws.in[cur] + skip[cur];
       // carried states: matched at wb
       w.top = 0;
@@ -1445,6 +1456,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
       int cursor = !live || (t->naas == 0 && (LEAN || layered || !tv.sticky))
                        ? c.iend
                        : (int)(inj_pos - wb);
+      int resume = 0;  // the always-active list of an injection that waits (inject_aas)
       InjAhead ahead;  // table words of the next batch, read ahead (this window only)
       // layered tiles: next window offset of the sticky states' work
       int scur = live && layered && w.nstk > 0 ? 0 : c.wlen;
@@ -1458,11 +1470,11 @@ __global__ void __launch_bounds__(kCtaThreads, 1) match_kernel(MatchParams p) {
                                              n_injected, ahead);
               cursor += 2 * batch;
             } else if (LEAN) {
-              inject_aas(p, ws, w, tv, c, lane, cursor, batch, depth, n_injected);
-              cursor += batch;
+              inject_aas(p, ws, w, tv, c, lane, cursor, batch, depth, resume, n_injected);
+              cursor += resume ? 0 : batch;
             } else {
-              inject(p, ws, w, tv, c, lane, cursor, batch, depth, n_injected);
-              cursor += batch;
+              inject(p, ws, w, tv, c, lane, cursor, batch, depth, resume, n_injected);
+              cursor += resume ? 0 : batch;
             }
             continue;
           }

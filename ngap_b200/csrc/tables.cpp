@@ -34,6 +34,7 @@
 #include <cmath>
 #include <cstring>
 #include <functional>
+#include <limits>
 #include <map>
 #include <numeric>
 #include <thread>
@@ -1050,6 +1051,60 @@ void build_filter(TileHost& t) {
 }
 
 }  // namespace
+
+// A path is a sequence of states that match consecutive symbols, from one that
+// needs no predecessor. paths(v): how many can end in v at one position of one
+// input, at most: those that start there, and for a class c of the symbol before,
+// all paths of the predecessors that accept c (predecessors of disjoint classes, such as
+// a pattern's symbol and its mismatch, are never matched together).
+void count_paths(TileHost& t) {
+  const double kMany = std::numeric_limits<double>::infinity();
+  t.max_paths = t.report_paths = kMany;
+  if (t.max_path < 0 || (t.phase == kPlain && t.nsticky > 0)) return;
+  const size_t n = (size_t)t.nstates;
+  std::vector<uint32_t> off(n + 1, 0), pred;
+  auto each_edge = [&](auto f) {
+    for (size_t v = 0; v < n; v++)
+      for (int k = 0; k < 4; k++)
+        if (t.succ[v * 4 + k] != kNoSucc) f((uint32_t)v, t.succ[v * 4 + k] & 0x7fffffffu);
+  };
+  each_edge([&](uint32_t, uint32_t u) { off[u + 1]++; });
+  for (size_t v = 0; v < n; v++) off[v + 1] += off[v];
+  pred.resize(off[n]);
+  std::vector<uint32_t> at(off.begin(), off.end() - 1), left(n);
+  each_edge([&](uint32_t v, uint32_t u) { pred[at[u]++] = v; });
+  std::vector<double> paths(n, 0.0);
+  for (uint32_t v : t.aas) paths[v] = 1;
+  for (uint32_t v : t.start) paths[v] = 1;
+  for (uint32_t a : t.act_local)
+    if (t.phase == kLayered) paths[a & kActIdMask] = 1;  // an active sticky state, at every position
+  std::vector<uint32_t> order;
+  for (size_t v = 0; v < n; v++)
+    if ((left[v] = off[v + 1] - off[v]) == 0) order.push_back((uint32_t)v);
+  double most = 0, reports = 0;
+  std::vector<double> by_class(t.nlive + 1);
+  for (size_t i = 0; i < order.size(); i++) {
+    const uint32_t v = order[i];
+    if (off[v + 1] - off[v] == 1) {
+      paths[v] += paths[pred[off[v]]];
+    } else if (off[v + 1] > off[v]) {
+      std::fill(by_class.begin(), by_class.end(), 0.0);
+      for (uint32_t k = off[v]; k < off[v + 1]; k++)
+        for (int c = 0; c < t.nlive; c++)
+          if (accepts_cls(t, pred[k], c)) by_class[c] += paths[pred[k]];
+      paths[v] += *std::max_element(by_class.begin(), by_class.end());
+    }
+    most = std::max(most, paths[v]);
+    if (is_report(t, v)) reports += paths[v];
+    for (int k = 0; k < 4; k++) {
+      const uint32_t u = t.succ[(size_t)v * 4 + k];
+      if (u != kNoSucc && --left[u & 0x7fffffffu] == 0) order.push_back(u & 0x7fffffffu);
+    }
+  }
+  if (order.size() < n) return;  // a cycle: no bound
+  t.max_paths = most;
+  t.report_paths = t.phase == kActivation ? 0 : reports;  // activation tiles report nothing
+}
 
 void build_filters(std::vector<TileHost>& tiles) {
   for (TileHost& t : tiles) build_filter(t);

@@ -56,6 +56,8 @@ struct TileHost {
   int32_t off_cmask = 0, off_rep = 0, off_sticky = 0, off_cls = 0;
   PrefixTableHost pt[kMaxDepth];
   FilterHost filt;
+  double max_paths = 0;              // most paths that end in one state at one position (count_paths)
+  double report_paths = 0;           // the same, added up over the report states
 };
 
 struct TableOpts {
@@ -90,6 +92,9 @@ int build_tiles(const GroupSet& gs, const TableOpts& opts, std::vector<TileHost>
 
 // Builds the look-ahead filter of every tile that gains from one.
 void build_filters(std::vector<TileHost>& tiles);
+
+// Fills in max_paths and report_paths (infinite for cyclic tiles).
+void count_paths(TileHost& t);
 
 // Checks the public table options (NULL = the defaults) and converts them;
 // `fn` names the entry point in the error message. *device gets the device.
