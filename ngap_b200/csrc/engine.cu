@@ -46,7 +46,14 @@ static_assert(kStackCap + kQueueSpare == 512, "512 entries, in shared memory or 
 constexpr int kRadixCount = 8;
 constexpr int kCursors = 10;
 constexpr int kSliceCtl = 16;
-constexpr int kSlotsPerSm = std::max(kWarpsPerCta, kRunWarps);  // warps with scratch of their own
+static_assert(kRunWarps % kWarpsPerCta == 0, "the runs' warps share what match_kernel's have");
+
+// Overflow-stack entries of a run's warp, where a warp of match_kernel has ovf_cap.
+// There are twice as many, so that equal shares would need twice the memory
+// (1.24 GB on 148 SMs at the default capacity, 0.62 GB with halves); they inject no
+// more than a quarter of their worklist at a time (mark_inject) and work depth
+// first past half of it, which bounds what they need. Small capacities are kept whole.
+int run_queue(int ovf_cap) { return std::max(ovf_cap / 2, std::min(ovf_cap, 8192 + kQueueSpare)); }
 constexpr int kSliceSlots = 8;  // slices that run without zeroing control words in between
 static_assert(kSliceCtl * 8 + kSliceSlots * kCtlWords * 4 <= kNumCounters * 8, "counters");
 
@@ -210,6 +217,7 @@ struct ngap_engine {
   uint32_t* d_marks = nullptr;
   uint32_t* d_ovf = nullptr;
   size_t slots = 0;
+  size_t ovf_words = 0;
   int carry_cap = 0, mark_words = 0, ovf_cap = 0;
   int max_smem_set = -1;
   int bps_smem = -1, bps_val = 0;  // resident CTAs per SM at the last shared-memory size
@@ -558,10 +566,14 @@ int ensure_reports(ngap_engine* e, uint64_t cap) {
   return NGAP_OK;
 }
 
-int ensure_slots(ngap_engine* e, size_t slots, int max_states, int max_nact, int queue) {
+// Scratch of the resident warps of `ctas` CTAs: carry lists, bitmaps and sticky
+// lists for the warps of match_kernel, worklists for those and for the runs' warps,
+// which use the same memory in turn (run_queue).
+int ensure_slots(ngap_engine* e, size_t ctas, int max_states, int max_nact, int queue) {
   int ovf_cap = queue + kQueueSpare;
   int carry_cap = std::max(max_states, 32);
   int mark_words = (max_states + 31) / 32 + 1;
+  size_t slots = ctas * kWarpsPerCta;
   // the overflow stacks only grow: a request for fewer entries than held
   // keeps them (more room changes no result, while reallocating would
   // cudaFree, which waits for every stream of the device)
@@ -588,6 +600,7 @@ int ensure_slots(ngap_engine* e, size_t slots, int max_states, int max_nact, int
   cudaFree(e->d_stk);
   e->d_carry = e->d_marks = e->d_ovf = e->d_stk = nullptr;
   e->stk_cap = 0;
+  e->ovf_words = 0;
   slots = std::max(slots, e->slots);
   e->slots = 0;
   if (stk_cap > 0) {
@@ -597,7 +610,9 @@ int ensure_slots(ngap_engine* e, size_t slots, int max_states, int max_nact, int
   CUDA_TRY(cudaMalloc(&e->d_carry, slots * (size_t)carry_cap * sizeof(uint32_t)));
   CUDA_TRY(cudaMalloc(&e->d_marks, slots * (size_t)mark_words * sizeof(uint32_t)));
   CUDA_TRY(cudaMemset(e->d_marks, 0, slots * (size_t)mark_words * sizeof(uint32_t)));
-  CUDA_TRY(cudaMalloc(&e->d_ovf, slots * (size_t)ovf_cap * sizeof(uint32_t)));
+  const size_t words = slots * std::max<size_t>(ovf_cap, (size_t)run_queue(ovf_cap) * kRunWarps / kWarpsPerCta);
+  CUDA_TRY(cudaMalloc(&e->d_ovf, words * sizeof(uint32_t)));
+  e->ovf_words = words;
   e->slots = slots;
   e->carry_cap = carry_cap;
   e->mark_words = mark_words;
@@ -1042,6 +1057,7 @@ int launch_plan(ngap_engine* e, MatchParams mp, const std::vector<TileDev>& tile
   };
   set_marks(mp, mp.window);
   MatchParams rp = mp;  // the runs': no windows, paths to their end
+  rp.ovf_cap = run_queue(mp.ovf_cap);
   set_marks(rp, kMaxRunPath);
   if (e->act_entries > 0)
     CUDA_TRY(cudaMemsetAsync(e->d_act, 0xff, (size_t)e->act_entries * sizeof(uint32_t), st));
@@ -1471,7 +1487,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
   e->grid = full_grid;
   // per-warp scratch for the full grid, whatever this plan uses: a later
   // larger plan then never reallocates (cudaMalloc waits for the device)
-  rc = ensure_slots(e, (size_t)full_grid * kSlotsPerSm, t->max_states, t->max_nact, kDefaultQueue);
+  rc = ensure_slots(e, (size_t)full_grid, t->max_states, t->max_nact, kDefaultQueue);
   if (rc != NGAP_OK) return rc;
 
   if (!in_place)
@@ -1609,7 +1625,7 @@ int ngap_engine_memory(const ngap_engine* e, ngap_engine_mem* out) {
   out->input = (int64_t)e->input_cap;
   out->reports = 3 * 8 * (int64_t)e->rep_cap + 4 * (int64_t)e->hist_cap + 4 * (int64_t)e->stream_ids_cap;
   out->scratch =
-      (int64_t)e->slots * 4 * ((int64_t)e->carry_cap + e->mark_words + e->ovf_cap + 2 * e->stk_cap) +
+      (int64_t)e->slots * 4 * ((int64_t)e->carry_cap + e->mark_words + 2 * e->stk_cap) + 4 * (int64_t)e->ovf_words +
       (int64_t)sizeof(uint16_t) * e->cand_cap + (int64_t)sizeof(RunDev) * e->runs_cap;
   out->plan = 8 * (int64_t)e->act_cap + 16 * (int64_t)e->rows_cap + 16 * (int64_t)e->unit_work_cap +
               (int64_t)sizeof(UnitDev) * (int64_t)e->units_cap +
@@ -1937,7 +1953,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     smem = cta_smem_bytes(window);
   }
   e->grid = full_grid;
-  if ((rc = ensure_slots(e, (size_t)full_grid * kSlotsPerSm, ts->max_states, ts->max_nact,
+  if ((rc = ensure_slots(e, (size_t)full_grid, ts->max_states, ts->max_nact,
                          p->queue_capacity > 0 ? std::max(p->queue_capacity, 1024) : kDefaultQueue)) != NGAP_OK)
     return rc;
 

@@ -131,3 +131,27 @@ assert count("fake_instantiated") == n + 1
 
 def test_capture_follows_the_buffers(run):
     run(CAPTURE)
+
+
+SCRATCH = r"""
+text, _ = W.literal_set(seed=5, n_patterns=200, input_len=1000, plant_every=100)
+t = tables(text)
+ts = nb.TableSet([t])
+states = t.stats()["states"]
+data = np.zeros(300_000, np.uint8)
+SMS = 148
+for queue in (0, 1024, 4096, 16384, 65536):
+    e = nb.Engine(0)
+    nb.batch_match_async(e, ts, data, [0], [len(data)], [0], result_capacity=CAP, queue_capacity=queue)
+    slices = 2 * len(data) + 64 * (len(data) // 4 + 2 * len(data) // 249)  # candidates and runs
+    # 16 warps with a worklist of the capacity and lists of every state
+    per_warp = 4 * (max(queue or 65536, 1024) + 128 + states + states // 32 + 2)
+    small = 32 if queue and queue < 16384 else 16  # small worklists are held whole by 32 warps
+    assert e.memory()["scratch"] <= SMS * (16 * per_warp + 4 * (small - 16) * (queue + 128)) + slices
+    if not 0 < queue < 16384:  # no more than 20 warps an SM took
+        assert e.memory()["scratch"] - slices <= SMS * 20 * 4 * ((queue or 65536) + states + states // 32 + 2)
+"""
+
+
+def test_scratch_of_the_resident_warps(run):
+    run(SCRATCH)
