@@ -147,15 +147,6 @@ struct UnitPlanKey {
   }
 };
 
-// Pieces scanned by one launch and matched by the next (make_slices).
-struct Slice {
-  int32_t begin, count;
-  int64_t runs;     // most runs they can give
-  bool layered;
-  int32_t one_tile; // the one tile of the pieces, or -1
-  int64_t longest = 0;  // positions of the longest piece
-};
-
 // What the launches of a plan run: units of the three launches of
 // match_kernel (make_units) and slices of pieces (make_slices).
 struct PlanRanges {
@@ -650,6 +641,7 @@ int launch_of(const TileHost& th) {
 // of four batches 748, 809, 1090, 1484 us; 1000 25-mers on 16 MiB (more units
 // than warps at any of them) 895, 405, 258, 260 us.
 struct AutoChunk {
+  static constexpr int64_t kShortest = 1024;  // unless that gives fewer units than warps
   int64_t positions[3] = {0, 0, 0};  // of bounded tiles, per launch
   int64_t warps = 1;
   void add(const TileHost& th, int64_t len) {
@@ -664,21 +656,10 @@ struct AutoChunk {
   }
 };
 
-// Length of a filtered tile's pieces: one per scan warp for short inputs, and
-// not below one step of a warp (256 positions); a caller's chunk length bounds it.
-int64_t piece_len(int64_t positions, int64_t warps, int64_t chunk_opt) {
-  int64_t n = (positions + warps - 1) / warps;
-  const int64_t step = n > kScanMinPiece ? 32 * kStripMax : kScanMinPiece;
-  n = (n + step - 1) / step * step;
-  if (chunk_opt > 0) n = std::min(n, chunk_opt);
-  return std::max<int64_t>(kScanMinPiece, std::min<int64_t>(n, kPieceMax));
-}
-
 // Tiles that are scanned: acyclic ones with a filter, in plans with at least
 // kScanMin of work (scan_work). Below, a scan and its runs are two kernels whose
 // start costs more than looking every position up: an 81-byte line matches
 // in 22 us in match_kernel and 30 us scanned, 64 literals on 1 MiB in 43 and 33.
-constexpr double kScanMin = 1 << 17;
 bool is_scanned(const TileHost& th, bool blocking) {
   return th.filt.len > 0 && th.max_path >= 0 && !(blocking && many_paths(th.max_paths));
 }
@@ -712,37 +693,6 @@ void add_pieces(const TileHost& th, int tile, const SegSpec& s, int64_t len,
     p.flags = starts && lo == s.lo ? 1u : 0u;
     pieces[th.phase == 2 ? 1 : 0].push_back(p);
   }
-}
-
-// Slices of consecutive pieces whose worst case (every position a candidate)
-// fits the candidate and run buffers: pieces[0] (plain and activation tiles)
-// first, then pieces[1] (layered tiles, after the activations are known).
-constexpr int64_t kSlicePositions = 32 << 20;
-constexpr int64_t kSliceRuns = 4 << 20;
-std::vector<Slice> make_slices(const std::vector<PieceDev> pieces[2],
-                               const std::vector<int32_t>& run_len, int64_t* cands, int64_t* runs) {
-  std::vector<Slice> out;
-  *cands = *runs = 0;
-  int32_t index = 0;
-  for (int l = 0; l < 2; l++) {
-    int64_t pos = 0;
-    for (size_t i = 0; i < pieces[l].size(); i++, index++) {
-      const PieceDev& p = pieces[l][i];
-      const int64_t n = p.hi - p.lo, r = (n + run_len[p.tile] - 1) / run_len[p.tile] + 1;
-      if (i == 0 || pos + n > kSlicePositions || out.back().runs + r > kSliceRuns) {
-        out.push_back({index, 0, 0, l == 1, p.tile});
-        pos = 0;
-      }
-      if (p.tile != out.back().one_tile) out.back().one_tile = -1;
-      out.back().count++;
-      out.back().runs += r;
-      pos += n;
-      out.back().longest = std::max(out.back().longest, n);
-      *cands = std::max(*cands, pos);
-      *runs = std::max(*runs, out.back().runs);
-    }
-  }
-  return out;
 }
 
 void add_units(const TileHost& th, int tile, const SegSpec& s, int64_t chunk,
@@ -912,25 +862,31 @@ void forget_plan(ngap_engine* e) {
   e->batch_ts = 0;
 }
 
-// Device copies of a plan's units and pieces, buffers for its largest slice.
+// Device copies of a plan's units and pieces, and buffers for its largest slice;
+// as large as `room` asks for where that is more.
 int set_plan(ngap_engine* e, const std::vector<UnitDev>& units, const std::vector<PieceDev> pieces[2],
-             const std::vector<int32_t>& run_len, std::vector<PieceDev>& all, std::vector<Upload>& ups) {
+             const std::vector<int32_t>& run_len, const PlanRoom& room, std::vector<PieceDev>& all,
+             std::vector<Upload>& ups) {
   all = pieces[0];
   all.insert(all.end(), pieces[1].begin(), pieces[1].end());
   int64_t cands = 0, runs = 0;
   e->ranges.slices = make_slices(pieces, run_len, &cands, &runs);
-  if (units.size() > e->units_cap) {
+  cands = std::max(cands, room.cands);
+  runs = std::max(runs, room.runs);
+  const size_t nunits = std::max(units.size(), (size_t)room.units);
+  const size_t npieces = std::max(all.size(), (size_t)room.pieces);
+  if (nunits > e->units_cap) {
     e->buffers++;
-    const size_t cap = grown(e->units_cap, units.size());
+    const size_t cap = grown(e->units_cap, nunits);
     cudaFree(e->d_units);
     e->d_units = nullptr;
     e->units_cap = 0;
     CUDA_TRY(cudaMalloc(&e->d_units, cap * sizeof(UnitDev)));
     e->units_cap = cap;
   }
-  if (all.size() > e->pieces_cap) {
+  if (npieces > e->pieces_cap) {
     e->buffers++;
-    const size_t cap = grown(e->pieces_cap, all.size());
+    const size_t cap = grown(e->pieces_cap, npieces);
     cudaFree(e->d_pieces);
     e->d_pieces = nullptr;
     e->pieces_cap = 0;
@@ -1475,7 +1431,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
     const ActRows rows = plan_units(t, key, full_grid, units, pieces, e->ranges);
     std::vector<Upload> ups;
     if ((rc = set_act_rows(e, rows, ups)) != NGAP_OK) return rc;
-    if ((rc = set_plan(e, units, pieces, t->run_len, all, ups)) != NGAP_OK) return rc;
+    if ((rc = set_plan(e, units, pieces, t->run_len, PlanRoom(), all, ups)) != NGAP_OK) return rc;
     if ((rc = upload_plan(e, st, ups)) != NGAP_OK) return rc;
     e->plan_tables = t->serial;
     e->plan_key = key;
@@ -1764,6 +1720,7 @@ struct ngap_tableset {
   uint64_t report_states = 0;  // of the NFA that has most
   int ntiles = 0, max_states = 0, max_groups = 1, max_depth = 1, device = 0;
   int max_nact = 0;
+  BatchShape shape;                 // of its NFAs
   std::vector<TileDev> tiles;       // the combined array
   std::vector<char> tile_lean;      // per tile of it (ngap_tables::tile_lean)
   std::vector<int32_t> run_len;     // the same
@@ -1796,7 +1753,16 @@ int ngap_tableset_create(const ngap_tables* const* tables, int n, ngap_tableset*
     ts->sid_bits = std::max(ts->sid_bits, t->sid_bits);
     ts->report_states = std::max(ts->report_states, t->report_states);
     ts->max_nact = std::max(ts->max_nact, t->max_nact);
-    for (auto& th : t->tiles) ts->max_depth = std::max(ts->max_depth, th.depth);
+    int64_t scanned = 0;
+    for (auto& th : t->tiles) {
+      ts->max_depth = std::max(ts->max_depth, th.depth);
+      scanned += is_scanned(th, false);
+    }
+    BatchShape& sh = ts->shape;
+    sh.tiles = std::max(sh.tiles, (int64_t)t->tiles.size());
+    sh.scanned = std::max(sh.scanned, scanned);
+    sh.plain = std::max(sh.plain, (int64_t)t->tiles.size() - scanned);
+    for (int32_t n : t->run_len) sh.run_len = std::min<int64_t>(sh.run_len, n);
   }
   ts->device = tables[0]->device;
   ts->ntiles = (int)all.size();
@@ -1938,7 +1904,17 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     e->ranges = make_units(units, pass1, unbounded, bounded, ts->tile_lean);
     std::vector<Upload> ups;
     if ((rc = set_act_rows(e, rows, ups)) != NGAP_OK) return rc;
-    if ((rc = set_plan(e, units, pieces, ts->run_len, all, ups)) != NGAP_OK) return rc;
+    BatchShape shape = ts->shape;
+    shape.streams = nstreams;
+    shape.chunk = AutoChunk::kShortest;
+    for (const ngap_batch_stream& s : sv) {
+      const int64_t chunk = s.chunk > 0 ? s.chunk : p->chunk;
+      shape.positions += (int64_t)s.length;
+      shape.chunk = std::min<int64_t>(shape.chunk, chunk > 0 ? chunk : AutoChunk::kShortest);
+    }
+    shape.warps = (int64_t)full_grid * kScanWarps;
+    if (blocking) shape.plain = shape.tiles;  // tiles with a filter may be units too
+    if ((rc = set_plan(e, units, pieces, ts->run_len, plan_room(shape), all, ups)) != NGAP_OK) return rc;
     if ((rc = upload_plan(e, st, ups)) != NGAP_OK) return rc;
     e->batch_ts = ts->serial;
     e->batch_streams = sv;

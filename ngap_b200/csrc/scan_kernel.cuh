@@ -23,16 +23,14 @@
 #pragma once
 
 #include "match_kernel.cuh"
+#include "slices.h"
 
 namespace ngap {
 
 constexpr int kMaxRunPath = 2048;  // states of the longest path of an acyclic tile (TableOpts::max_warmup)
-constexpr int kPieceMax = 4096;  // run entries pack offsets below kPieceMax + the longest path
+// run entries pack offsets below kPieceMax (slices.h) + the longest path
 static_assert(kPieceMax + kMaxRunPath + kMaxDepth < kMaxWindow, "offsets fit worklist entries");
 constexpr int kScanWarps = 32;
-constexpr int kScanLane = 8;     // positions per lane and step: reads in flight
-constexpr int kScanMinPiece = 32 * kScanLane;
-constexpr int kStripMax = 16;    // consecutive positions per lane (a strip)
 // Per warp: class ids of 33 strips (4 bytes apart, so that lanes reading their
 // strips word by word hit 32 banks), byte classes, one bit per position.
 constexpr int kScanSymBytes = (33 * (kStripMax + 4) + 15) / 16 * 16;

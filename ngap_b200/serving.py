@@ -220,14 +220,16 @@ class Server:
     the budget. Each engine's buffers (an input copy of max_batch_bytes,
     report buffers for `rep_cap` reports, per-warp overflow stacks) are
     allocated by a one-stream warm-up batch at construction, so they are
-    counted from the start and never grow while serving; a budget that
+    counted from the start and never grow while serving, whichever NFAs the
+    later batches name (a batch reserves room for any mix of its size: units,
+    pieces, candidates and runs, at most 320 MB of the latter two); a budget that
     cannot hold the tables and those buffers raises ValueError. A request that
     can never be admitted (longer than max_batch_bytes, or needing more than
     the budget leaves with every engine as it is) is rejected at arrival:
     its `error` is set and it gets no reports.
     """
 
-    UNIT_BYTES = 80  # device bytes of a unit record plus its share of a task record
+    UNIT_BYTES = 80  # device bytes of a unit record (64) or a piece record (48), and some slack
 
     def __init__(self, tableset, predictor=None, rho_ref=2.0, slots=2, budget=1 << 30,
                  max_batch_bytes=64 << 20, device=0, queue_capacity=0,
@@ -271,7 +273,10 @@ class Server:
         big.chunk = lo
         k = self.max_requests
         each = max(1, max_batch_bytes // k)
-        many = [Request(-2 - i, i % len(tiles), np.zeros(each, np.uint8), 0.0) for i in range(k)]
+        # together exactly as long as the longest batch: what it reserves is then the most
+        last = max(each, max_batch_bytes - each * (k - 1))
+        many = [Request(-2 - i, i % len(tiles), np.zeros(each if i + 1 < k else last, np.uint8), 0.0)
+                for i in range(k)]
         for r in many:
             r.chunk = lo
         for sl in self.slots:

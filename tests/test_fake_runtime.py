@@ -155,3 +155,56 @@ for queue in (0, 1024, 4096, 16384, 65536):
 
 def test_scratch_of_the_resident_warps(run):
     run(SCRATCH)
+
+
+RESERVE = r"""
+rng = np.random.default_rng(5)
+dense = W.AnmlWriter("dense")  # most positions report: no filter
+dense.ste("a", W.PRINTABLE[:60], ["b"], start="all-input", report=True)
+dense.ste("b", W.PRINTABLE[:60], report=True)
+loop = W.AnmlWriter("loop")    # cyclic
+loop.ste("x", b"x", ["y"], start="all-input")
+loop.ste("y", b"y", ["y", "z"])
+loop.ste("z", b"z", report=True)
+long = [bytes(rng.integers(97, 123, 8).astype(np.uint8)) for _ in range(3000)]
+lists = W.AnmlWriter("lists")  # long lists in shallow tables: the shortest runs
+for n, word in enumerate(long):
+    for i, c in enumerate(word):
+        lists.ste(f"r{n}_{i}", [ord("h") if i == 0 else c], [f"r{n}_{i + 1}"] if i < 7 else [],
+                  start="all-input" if i == 0 else None, report=i == 7)
+texts = [W.literal_set(seed=5, n_patterns=20, input_len=1000, plant_every=100)[0], dense.text(), loop.text(),
+         W.dotstar_set(seed=6, n_patterns=40, input_len=1000, plant_every=100)[0], lists.text()]
+ts = nb.TableSet([tables(t, depth=1, groups=3) for t in texts])
+N = len(texts)
+CHUNK, MOST, REQUESTS = 256, 3_000_001, 40
+data = np.zeros(MOST, np.uint8)
+
+
+def batch(e, lens, nfas, chunk):
+    offs = np.concatenate([[0], np.cumsum(lens)[:-1]])
+    nb.batch_match_async(e, ts, data[:int(sum(lens))], offs, lens, nfas, chunks=np.full(len(lens), chunk),
+                         result_capacity=CAP, algorithm=algorithm)
+    e.sync()
+
+
+for algorithm in ("nonblockingpcgroups", "NAPgroups", "blockinggroups"):
+    for lo, hi in ((CHUNK, 2048), (0, 0)):  # chunks chosen per request, or automatic
+        e = nb.Engine(0)
+        batch(e, [MOST], [0], lo)            # as a server warms up: one request, then the most
+        each = MOST // REQUESTS
+        batch(e, [each] * (REQUESTS - 1) + [MOST - each * (REQUESTS - 1)], np.arange(REQUESTS) % N, lo)
+        held = e.memory()
+        assert held["scratch"] > 0 and held["plan"] > 0
+        for nfa in list(range(N)) + [-1] * 10:
+            for size in (MOST, MOST // 7, 5000, 40):
+                k = int(rng.integers(1, REQUESTS + 1)) if nfa < 0 else (1 if size == MOST // 7 else REQUESTS)
+                cuts = np.sort(rng.integers(0, size + 1, k - 1))
+                lens = np.diff(np.concatenate([[0], cuts, [size]]))
+                nfas = rng.integers(0, N, k) if nfa < 0 else np.full(k, nfa)
+                batch(e, lens, nfas, int(rng.integers(lo, hi + 1)))
+                assert e.memory() == held, (algorithm, lo, nfa, size, k, held, e.memory())
+"""
+
+
+def test_batches_of_other_rules_allocate_nothing(run):
+    run(RESERVE)
