@@ -103,7 +103,7 @@ struct ngap_tables {
   int device = 0;
   int num_groups = 0;
   int sid_bits = 0;  // bits of the largest group-local state id
-  uint64_t report_states = 0;
+  double report_paths = 0;  // most reports a position can give, duplicates included
   std::vector<TileHost> tiles;
   std::vector<TileDev> dev_desc;
   TileDev* d_tiles = nullptr;
@@ -317,10 +317,10 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
   t->num_groups = (int)g->gs.groups.size();
   for (const GroupGraph& gg : g->gs.groups) {
     t->sid_bits = std::max(t->sid_bits, bits_for(std::max<uint64_t>(gg.attrs.size(), 1)));
-    for (uint8_t a : gg.attrs) t->report_states += a & 2 ? 1 : 0;
   }
   for (auto& th : t->tiles) {
     count_paths(th);
+    t->report_paths += th.report_paths;
     if (th.nstates >= kMaxTileStates - 1) {
       set_error("a connected component has %d states; at most %d are supported per tile",
                 th.nstates, kMaxTileStates - 2);
@@ -1254,12 +1254,13 @@ int build_sort_graph(ngap_engine* e, const SortJob& j, SortGraph& sg) {
   return NGAP_OK;
 }
 
-// A match whose positions times its rules' report states are at most this sorts
-// its reports with the one-CTA kernel alone, launched directly: a launch with a
-// conditional graph costs 7 us more on a B200 (29 against 22 us for an empty
-// pipeline), while one CTA keeps up with the pipeline only to some 30,000
-// reports, which larger products could exceed many times over.
-constexpr uint64_t kAloneReports = 1ull << 16;
+// A match that can give at most so many reports (positions times the paths that end
+// in report states, TileHost::report_paths, since a report that several paths lead
+// to is emitted several times) sorts them with the one-CTA kernel alone, launched
+// directly: a launch with a conditional graph costs 7 us more on a B200 (29 against
+// 22 us for an empty pipeline), while one CTA keeps up with the pipeline only to
+// some 30,000 reports, which larger bounds could exceed many times over.
+constexpr double kAloneReports = 1 << 16;
 
 // Enqueues the sort of a match's reports on st, the match's last kernels: they
 // leave its counters and first reports for the host. Past
@@ -1267,9 +1268,8 @@ constexpr uint64_t kAloneReports = 1ull << 16;
 // radix pipeline runs only for more than kSmallSort keys); inside a
 // capture, or where graphs are unavailable, it launches the one-CTA kernel and
 // the pipeline, whose kernels find no keys after a small set.
-int sort_reports(ngap_engine* e, const SortJob& j, uint64_t positions, uint64_t report_states,
-                 cudaStream_t st) {
-  if (positions * report_states <= kAloneReports) return cta_sort(e, j, true, e->ho, st);
+int sort_reports(ngap_engine* e, const SortJob& j, double most_reports, cudaStream_t st) {
+  if (most_reports <= kAloneReports) return cta_sort(e, j, true, e->ho, st);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(st, &cs));
   if (cs == cudaStreamCaptureStatusNone && !e->sort_graph_off) {
@@ -1495,7 +1495,7 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
                           bit_range(32, bits_for(total));
     const SortJob job{0,  e->d_reports, e->d_counters + 0, cap,     digits_of(bits),
                       32, 64,           e->d_unique,       nullptr, e->d_counters + 1};
-    if ((rc = sort_reports(e, job, total, t->report_states, st)) != NGAP_OK) return rc;
+    if ((rc = sort_reports(e, job, (double)total * t->report_paths, st)) != NGAP_OK) return rc;
   } else {
     publish_kernel<<<1, 32, 0, st>>>(e->ho);
     CUDA_TRY(cudaGetLastError());
@@ -1717,7 +1717,6 @@ struct ngap_tableset {
   std::vector<int> tile_base;  // first tile of each NFA in the combined descriptor array
   TileDev* d_tiles = nullptr;
   int sid_bits = 0;
-  uint64_t report_states = 0;  // of the NFA that has most
   int ntiles = 0, max_states = 0, max_groups = 1, max_depth = 1, device = 0;
   int max_nact = 0;
   BatchShape shape;                 // of its NFAs
@@ -1751,7 +1750,6 @@ int ngap_tableset_create(const ngap_tables* const* tables, int n, ngap_tableset*
     ts->max_states = std::max(ts->max_states, t->max_states);
     ts->max_groups = std::max(ts->max_groups, t->num_groups);
     ts->sid_bits = std::max(ts->sid_bits, t->sid_bits);
-    ts->report_states = std::max(ts->report_states, t->report_states);
     ts->max_nact = std::max(ts->max_nact, t->max_nact);
     int64_t scanned = 0;
     for (auto& th : t->tiles) {
@@ -1964,6 +1962,10 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   mp.skip_copy_unit = -1;
   e->trace_seg_len = 0;
 
+  double most_reports = 0;  // streams may share bytes of the input
+  for (const ngap_batch_stream& s : sv)
+    if (s.length > 0) most_reports += (double)s.length * ts->tables[s.nfa]->report_paths;
+
   auto enqueue = [&](cudaStream_t qs) -> int {
     if (e->trace) {
       const int r = trace_buffer(e, qs, &mp.unit_work, &mp.unit_cycles);
@@ -1982,7 +1984,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
                             bit_range(oshift, obits) | bit_range(sshift, sbits);
       const SortJob job{1,      e->d_reports, e->d_counters + 0, cap,             digits_of(bits),
                         oshift, sshift,       e->d_unique,       e->d_stream_ids, e->d_counters + 1};
-      if ((r = sort_reports(e, job, input_bytes, ts->report_states, qs)) != NGAP_OK) return r;
+      if ((r = sort_reports(e, job, most_reports, qs)) != NGAP_OK) return r;
     } else {
       publish_kernel<<<1, 32, 0, qs>>>(e->ho);
       CUDA_TRY(cudaGetLastError());

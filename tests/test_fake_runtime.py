@@ -208,3 +208,52 @@ for algorithm in ("nonblockingpcgroups", "NAPgroups", "blockinggroups"):
 
 def test_batches_of_other_rules_allocate_nothing(run):
     run(RESERVE)
+
+
+SORTS = r"""
+# which sort a match ends with: the one-CTA kernel alone, or the graph with the pipeline
+words, _ = W.literal_set(seed=5, n_patterns=6, input_len=1000, plant_every=100)
+forks = W.AnmlWriter("forks")  # 2^9 paths to the end of a (b|b) c (b|b) c ...
+for i in range(9):
+    forks.ste(f"a{i}", b"a" if i == 0 else b"c", [f"b{i}", f"e{i}"], start="all-input" if i == 0 else None)
+    for x in "be":
+        forks.ste(f"{x}{i}", b"b", [f"a{i + 1}"])
+forks.ste("a9", b"c", [], report=True)
+loop = W.AnmlWriter("loop")
+loop.ste("h", b"h", ["x", "y"], start="all-input")
+for c in "xy":
+    loop.ste(c, b"a", ["x", "y", "z"])
+loop.ste("z", b"z", [], report=True)
+t = [tables(x, depth=1) for x in (words, forks.text(), loop.text())]
+ts = nb.TableSet(t)
+data = np.zeros(4000, np.uint8)
+e = nb.Engine(0)
+
+
+def alone(f, *a, **kw):
+    out = log(f, *a, **kw)
+    graph, cta = any(x.startswith("graph") for x in out), any("sort_unique_cta" in x for x in out)
+    assert graph != cta, out
+    return cta
+
+
+def plain(k, n):
+    return alone(e.match_async, t[k], data, 1, n, result_capacity=CAP)
+
+
+def batch(nfas, offs, lens):
+    return alone(nb.batch_match_async, e, ts, data, offs, lens, nfas, result_capacity=CAP)
+
+
+assert plain(0, 4000) and plain(0, 100)          # 4000 positions, one path to each of 6 reports
+assert plain(1, 128) and not plain(1, 129)       # 512 paths to one report: 65,536 reports at most
+assert not plain(2, 1)                           # cyclic: no bound
+assert batch([0, 0], [0, 2000], [2000, 2000])
+assert not batch([0] * 30, [0] * 30, [4000] * 30)  # streams over the same bytes
+assert batch([0] * 30, [0] * 30, [40] * 30)
+assert batch([0, 1, 2], [0, 1000, 1100], [1000, 100, 0]) and not batch([0, 1], [0, 1000], [1000, 300])
+"""
+
+
+def test_sorts_by_the_reports_that_can_come(run):
+    run(SORTS)
