@@ -232,10 +232,12 @@ bool dump_reports(const std::string& path, const std::vector<uint64_t>& v) {
 
 // --tuning (ngap.cu:1995-2056): the reference reruns the whole input over a
 // grid of its knobs (fetch size x AAS interval x active threshold) and keeps
-// the fastest run that validates. The knobs here are the engine's: window,
-// chunk length and, for the privatizing algorithms, the active threshold. A
-// candidate counts only when its reports equal the first candidate's. The
-// best choice is written back into mp for the run that follows.
+// the fastest run that validates. The knobs here are the engine's, window and
+// chunk length; for the privatizing algorithms the active threshold is run
+// through its grid as well, though paths are followed in registers whatever
+// it is: the threshold that is printed in the end is one of equals. A candidate
+// counts only when its reports equal the first candidate's. The best choice is
+// written back into mp for the run that follows.
 bool tune(ngap_engine* eng, const ngap_tables* tables, const std::vector<uint8_t>& ss,
           uint64_t total, ngap_match_params& mp) {
   const bool priv = mp.algorithm == NGAP_ALGO_NONBLOCKING_R1 ||

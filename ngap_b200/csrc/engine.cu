@@ -2019,7 +2019,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   std::vector<uint64_t> key = {ts->serial, (uint64_t)(uintptr_t)input, input_bytes,
                                (uint64_t)input_on_device, (uint64_t)in_place,
                                (uint64_t)p->algorithm,
-                               (uint64_t)p->unique, (uint64_t)p->active_threshold,
+                               (uint64_t)p->unique,
                                (uint64_t)p->report_off, cap, (uint64_t)window, (uint64_t)p->chunk,
                                (uint64_t)e->trace, (uint64_t)e->ovf_cap, e->buffers};
   if (replanned || !e->graph || key != e->graph_key) {

@@ -109,8 +109,8 @@ data = np.zeros(1 << 20, np.uint8)
 e = nb.Engine(0)
 
 
-def batch():
-    nb.batch_match_async(e, ts, data, [0, 1000], [1000, 500000], [0, 0], use_graph=True, result_capacity=CAP)
+def batch(**kw):
+    nb.batch_match_async(e, ts, data, [0, 1000], [1000, 500000], [0, 0], use_graph=True, result_capacity=CAP, **kw)
 
 
 batch()
@@ -126,6 +126,10 @@ batch()
 assert count("fake_instantiated") == n + 1  # captured again
 batch()
 assert count("fake_instantiated") == n + 1
+batch(active_threshold=3)  # no kernel reads it
+assert count("fake_instantiated") == n + 1
+batch(unique=True)
+assert count("fake_instantiated") == n + 2
 """
 
 
