@@ -230,6 +230,7 @@ class Engine:
         check(lib().ngap_engine_create(device, ctypes.byref(h)))
         self._h = h
         self.device = device
+        self._keep = None  # input of the match in flight
 
     def match_async(self, tables, data, num_seg, seg_len, algorithm="nonblockingallgroups",
                     is_dup=False, unique=False, active_threshold=20, report_off=False,
@@ -259,7 +260,10 @@ class Engine:
 
     def sync(self):
         """Waits for the engine's last match; raises NgapError on its status."""
-        return check(lib().ngap_engine_sync(self._h))
+        try:
+            return check(lib().ngap_engine_sync(self._h))
+        finally:
+            self._keep = None  # the match has ended: its input is the caller's alone again
 
     def set_trace(self, enable=True):
         """Records per-unit worklist work in the following matches."""

@@ -261,3 +261,40 @@ assert batch([0, 1, 2], [0, 1000, 1100], [1000, 100, 0]) and not batch([0, 1], [
 
 def test_sorts_by_the_reports_that_can_come(run):
     run(SORTS)
+
+
+KEEP = r"""
+import weakref
+
+
+class Tensor:  # a device tensor
+    is_cuda = True
+
+    def __init__(self, n):
+        self.p = ctypes.c_void_p()
+        assert fake.cudaMalloc(ctypes.byref(self.p), ctypes.c_size_t(n)) == 0
+        self.n = n
+
+    data_ptr = lambda self: self.p.value
+    numel = lambda self: self.n
+    element_size = lambda self: 1
+
+
+text, _ = W.literal_set(seed=5, n_patterns=20, input_len=1000, plant_every=100)
+t = tables(text)
+ts = nb.TableSet([t])
+e = nb.Engine(0)
+for start in (lambda x: e.match_async(t, x, 1, 4096, result_capacity=CAP),
+              lambda x: nb.batch_match_async(e, ts, x, [0], [4096], [0], result_capacity=CAP)):
+    x = Tensor(4096)
+    alive = weakref.ref(x)
+    start(x)
+    del x
+    assert alive() is not None  # read in place: kept while the match runs
+    e.sync()
+    assert alive() is None      # and no longer
+"""
+
+
+def test_input_is_kept_until_the_match_has_ended(run):
+    run(KEEP)
