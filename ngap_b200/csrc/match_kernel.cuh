@@ -524,6 +524,21 @@ __device__ __forceinline__ bool register_each(const MatchParams& p, WarpSmem& ws
   return mine;
 }
 
+// Which of the always-active states i0 .. i0 + kAasStep - 1 accept class s (valid
+// lanes); their ids to a. One vote then covers the step: nearly all of a long list
+// matches nowhere in a batch.
+constexpr int kAasStep = 4;
+__device__ __forceinline__ uint32_t aas_step(const TileView& tv, int i0, uint32_t s, bool valid,
+                                             uint32_t a[kAasStep]) {
+  const TileDev& t = *tv.t;
+  uint32_t ok = 0u;
+#pragma unroll
+  for (int j = 0; j < kAasStep; j++) a[j] = __ldg(t.aas + min(i0 + j, t.naas - 1));
+#pragma unroll
+  for (int j = 0; j < kAasStep; j++) ok |= (valid && i0 + j < t.naas && accepts(tv, a[j], s) ? 1u : 0u) << j;
+  return ok;
+}
+
 // Always-active states for window offsets [r0, r0 + batch) (one per lane). resume:
 // index into the always-active list (depth 0) at which the last call stopped, its
 // worklist near mark_inject; 0 when it is through.
@@ -537,19 +552,24 @@ __device__ __forceinline__ void inject_aas(const MatchParams& p, WarpSmem& ws, W
   const int64_t q = c.wb + r;
   if (depth == 0) {  // scan the always-active list
     const uint32_t s = valid ? c.in[r] : 0u;
-    int i = resume;
+    int i0 = resume;
     resume = 0;
-    for (; i < t.naas; i++) {
-      if (held(w) > p.mark_inject - 32) {
-        resume = i;
+    for (; i0 < t.naas; i0 += kAasStep) {
+      if (held(w) > p.mark_inject - 32 * kAasStep) {
+        resume = i0;
         return;
       }
-      const uint32_t a = __ldg(t.aas + i);
-      const bool ok = valid && accepts(tv, a, s);
-      const bool rep = ok && is_report(tv, a) && q >= c.emit_lo;
-      emit_report(p, ws, w, lane, rep, rep ? (__ldg(t.sid + a)) : 0u, (uint32_t)q);
-      push_entry(p, ws, w, lane, ok && q + 1 < c.hi, (a << kEntryPosBits) | (uint32_t)r);
-      n_injected += ok;
+      uint32_t a[kAasStep];
+      const uint32_t ok = aas_step(tv, i0, s, valid, a);
+      if (!__any_sync(kFull, ok != 0u)) continue;
+#pragma unroll
+      for (int j = 0; j < kAasStep; j++) {
+        const bool hit = (ok >> j) & 1u;
+        const bool rep = hit && is_report(tv, a[j]) && q >= c.emit_lo;
+        emit_report(p, ws, w, lane, rep, rep ? (__ldg(t.sid + a[j])) : 0u, (uint32_t)q);
+        push_entry(p, ws, w, lane, hit && q + 1 < c.hi, (a[j] << kEntryPosBits) | (uint32_t)r);
+      }
+      n_injected += __popc(ok);
     }
     return;
   }

@@ -253,7 +253,7 @@ __device__ __forceinline__ uint32_t symbol(const RunCtx& c, int r) { return __ld
 // stops near mark_inject entries, a quarter of the worklist; the paths are
 // followed, and it goes on from `resume` (0: all is done). Lists of up to that many
 // entries, nearly all, are injected in one go as before.
-static_assert((kStackCap + 1024) / 4 >= kInjectLow + 4 * 32, "short lists always fit");
+static_assert((512 + 1024) / 4 >= kInjectLow + 4 * 32, "short lists always fit");
 
 // Entries from the overflow stack to the empty shared one.
 __device__ __forceinline__ void refill_stack(WarpSmem& ws, WarpRun& w, int lane) {
@@ -277,17 +277,22 @@ __device__ __forceinline__ void inject_run(const MatchParams& p, WarpSmem& ws, W
   resume = 0;
   if (depth == 0) {  // scan the always-active list
     const uint32_t s = valid ? symbol(c, r) : 0u;
-    for (int i = (int)from; i < t.naas; i++) {
-      if (held(w) > p.mark_inject - 32) {
-        resume = (uint32_t)i;
+    for (int i0 = (int)from; i0 < t.naas; i0 += kAasStep) {
+      if (held(w) > p.mark_inject - 32 * kAasStep) {
+        resume = (uint32_t)i0;
         return;
       }
-      const uint32_t a = __ldg(t.aas + i);
-      const bool ok = valid && accepts(tv, a, s);
-      const bool rep = ok && is_report(tv, a);
-      emit_report(p, ws, w, lane, rep, rep ? __ldg(t.sid + a) : 0u, q);
-      push_entry(p, ws, w, lane, ok && r + 1 < c.lim, (a << kEntryPosBits) | (uint32_t)r);
-      n_injected += ok;
+      uint32_t a[kAasStep];
+      const uint32_t ok = aas_step(tv, i0, s, valid, a);
+      if (!__any_sync(kFull, ok != 0u)) continue;
+#pragma unroll
+      for (int j = 0; j < kAasStep; j++) {
+        const bool hit = (ok >> j) & 1u;
+        const bool rep = hit && is_report(tv, a[j]);
+        emit_report(p, ws, w, lane, rep, rep ? __ldg(t.sid + a[j]) : 0u, q);
+        push_entry(p, ws, w, lane, hit && r + 1 < c.lim, (a[j] << kEntryPosBits) | (uint32_t)r);
+      }
+      n_injected += __popc(ok);
     }
     return;
   }
