@@ -1157,10 +1157,6 @@ __device__ __forceinline__ void walk_paths(const MatchParams& p, WarpSmem& ws, W
   bool act = false;
   unsigned live = 0u;
   while (true) {
-    if (held(w) > p.mark_walk) {  // back to the worklist: expand_step goes on
-      push_entry(p, ws, w, lane, act, (v << kEntryPosBits) | (uint32_t)r);
-      return;
-    }
     if (w.top > 0 && __popc(live) <= 16) {  // idle lanes take the entries on top of the stack
       const int n = min(w.top, 32 - __popc(live));
       const int k = __popc(~live & lanemask_lt(lane));
@@ -1224,6 +1220,10 @@ __device__ __forceinline__ void walk_paths(const MatchParams& p, WarpSmem& ws, W
     v = follow;
     r++;
     live = __ballot_sync(kFull, act);
+    if ((events & 4u) && held(w) > p.mark_walk) {  // back to the worklist: expand_step goes on
+      push_entry(p, ws, w, lane, act, (v << kEntryPosBits) | (uint32_t)r);
+      return;
+    }
     if (live == 0u && w.top == 0) return;
   }
 }

@@ -547,12 +547,6 @@ __device__ __forceinline__ void walk_run(const MatchParams& p, WarpSmem& ws, War
   bool act = false;
   unsigned live = 0u;
   while (true) {
-    if (held(w) > p.mark_walk) {  // all paths back to the worklist until it is half as full
-      push_entry(p, ws, w, lane, act, (v << kEntryPosBits) | (uint32_t)r);
-      act = false;
-      live = 0u;
-      while (held(w) > p.mark_inject) step_run<false>(p, ws, w, tv, c, lane, n_expanded);
-    }
     if (w.top == 0 && w.ovf_n > 0 && __popc(live) <= 16) refill_stack(ws, w, lane);
     if (w.top > 0 && __popc(live) <= 16) {  // idle lanes take the entries on top of the stack
       const int n = min(w.top, 32 - __popc(live));
@@ -607,6 +601,14 @@ __device__ __forceinline__ void walk_run(const MatchParams& p, WarpSmem& ws, War
     v = follow;
     r++;
     live = __ballot_sync(kFull, act);
+    // the worklist has grown past mark_walk (injections end far below it): all
+    // paths back to it, and steps until it is half as full
+    if ((events & 2u) && held(w) > p.mark_walk) {
+      push_entry(p, ws, w, lane, act, (v << kEntryPosBits) | (uint32_t)r);
+      act = false;
+      live = 0u;
+      while (held(w) > p.mark_inject) step_run<false>(p, ws, w, tv, c, lane, n_expanded);
+    }
     if (live == 0u && w.top == 0 && w.ovf_n == 0) return;
   }
 }
