@@ -94,8 +94,13 @@ def load_peaks():
     return 6650.0, "fallback"
 
 
+# of one match: filtered tiles are scanned and their candidates run, the rest is
+# matched in windows
+MATCH_KERNELS = "scan_kernel + run_kernel + match_kernel"
+
+
 def profiled(workload, num_seg):
-    """ncu figures of the matching kernel (DRAM and L2 bytes per launch, L2
+    """ncu figures of the matching kernels (DRAM and L2 bytes per launch, L2
     throughput) from the committed summary of the same workload and segment
     count, or None."""
     p = os.path.join(ROOT, "profiles", "match_kernel_traffic.json")
@@ -560,15 +565,17 @@ def run_plain(args, warmup, rank, world, local_rank, dist):
         line["parity_vs_oracle"] = par
     if algo_cmp is not None:
         line["algorithms"] = algo_cmp
-    # roofline of the matching kernel: bytes this design must move per launch
-    # (every input byte, table byte and raw report once) over its CUDA-event
-    # time; the measured DRAM and L2 bytes of the same launch from ncu; and
-    # the reference's worklist formulation for comparison
-    alg = n_in + tables.device_bytes + 8 * raw
+    # roofline of the matching kernels: bytes that a match must move (every
+    # input byte read and every raw report written once; tables and filters may stay
+    # in L2, and most of their bytes are never read) over their CUDA-event time;
+    # the measured DRAM and L2 bytes of the same kernels from ncu; and the
+    # reference's worklist formulation for comparison
+    alg = n_in + 8 * raw
     roof = {"bound": "hbm", "unit": "GB/s", "peak": peak, "peak_source": peak_kind,
-            "kernel": "match_kernel", "kernel_ms": mk,
+            "kernel": MATCH_KERNELS, "kernel_ms": mk,
             "algorithmic_bytes": alg,
-            "algorithmic_def": "input bytes + table bytes + 8 B per raw report, per launch",
+            "algorithmic_def": "input bytes + 8 B per raw report, per match",
+            "table_bytes": tables.device_bytes,
             "achieved": alg / (mk / 1e3) / 1e9}
     roof["frac"] = roof["achieved"] / peak
     prof = profiled(args.workload, num_seg)
@@ -751,11 +758,11 @@ def batched_part(args, warmup, suite, local_rank, steps):
         out["parity_vs_oracle"] = par
     peak, peak_kind = load_peaks()
     mk = float(np.mean(match_ms))
-    tb = sum(t.device_bytes for t in s.tables)
-    alg = s.total + tb + 8 * raw
+    alg = s.total + 8 * raw
     out["roofline"] = {"bound": "hbm", "unit": "GB/s", "peak": peak, "peak_source": peak_kind,
-                       "kernel": "match_kernel", "kernel_ms": mk, "algorithmic_bytes": alg,
-                       "algorithmic_def": "input bytes + table bytes + 8 B per raw report",
+                       "kernel": MATCH_KERNELS, "kernel_ms": mk, "algorithmic_bytes": alg,
+                       "algorithmic_def": "input bytes + 8 B per raw report",
+                       "table_bytes": sum(t.device_bytes for t in s.tables),
                        "achieved": alg / (mk / 1e3) / 1e9,
                        "frac": alg / (mk / 1e3) / 1e9 / peak}
     prof = profiled("batched_suite", len(s.offsets))

@@ -67,7 +67,8 @@ __host__ __device__ inline uint32_t prefix_hash(uint32_t key) {
 // edit-distance 20-mers 175 -> 134, 1000 25-mers 156 -> 131 (4 % -> 1 % of the
 // positions pass), the 32 MiB mix 616 -> 548, 512 streams 3.02 -> 2.66 ms.
 constexpr int kMaxFilter = 16;       // most symbols a filter looks ahead
-constexpr uint32_t kFilterMul = 0x9E3779B1u;  // odd multipliers
+// odd multipliers: the first prime of xxHash32 and the two of MurmurHash3's 32-bit finalizer
+constexpr uint32_t kFilterMul = 0x9E3779B1u;
 constexpr uint32_t kFilterBlock = 0x85EBCA6Bu;
 constexpr uint32_t kFilterBits = 0xC2B2AE35u;
 

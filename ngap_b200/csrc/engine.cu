@@ -1801,9 +1801,9 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   const int ibits = 22 + bits_for((uint64_t)std::max(ts->max_groups, 1));
   int obits = bits_for(max_len);
   int sbits = bits_for((uint64_t)nstreams);
-  // field widths rounded up to the radix digit (4 bits) when the key still
-  // fits: the same number of radix passes and far fewer distinct layouts, so
-  // that the sort's CUDA graph (keyed by the layout) is reused across batches
+  // field widths rounded up to multiples of 4 bits when the key still fits: at
+  // most one more 8-bit digit and far fewer distinct layouts, so that the sort's
+  // CUDA graph (keyed by the layout) is reused across batches
   // of other lengths and stream counts instead of being captured again
   if (ibits + ((obits + 3) & ~3) + ((sbits + 3) & ~3) <= 64) {
     obits = (obits + 3) & ~3;

@@ -148,13 +148,13 @@ struct WarpRun {
 
 // The tile a warp works on.
 struct TileView {
-  const uint4* succ;    // wide tiles
+  const uint4* succ;    // state records (TileDev)
   const uint32_t* cmask;
   const uint32_t* rep;
   const uint32_t* sticky;  // sticky-state bitmap, nullptr when the tile has none
   const uint8_t* cls;
   const TileDev* t;
-  const PrefixTableDev* pt;  // the tile's prefix tables (shared-memory copy)
+  const PrefixTableDev* pt;  // the tile's prefix tables (a shared-memory copy in one-tile launches)
   int cw;
   uint32_t nlive;  // live classes: base of the prefix-table keys
   uint32_t rep_levels;  // bit d: the depth-(d+1) table has report lists

@@ -1,7 +1,7 @@
-// Tiles, byte classes, shared-memory images and prefix-memoization tables.
+// Tiles, byte classes, tile images, look-ahead filters and prefix-memoization tables.
 //
-// A tile is a set of whole CCs: of one group for shared-memory tiles, of any
-// groups for global tiles. CCs never share states or edges, so the way CCs
+// A tile is a set of whole CCs: of one group under a size rule, or of any groups
+// (global tiles). CCs never share states or edges, so the way CCs
 // are packed into tiles changes no report: every state keeps its report id
 // (group-local sid | group << 22, TileHost::sid). Two facts about the graph
 // are used:
@@ -706,7 +706,7 @@ bool emit_tile(const GroupSet& gs, const std::vector<CcInfo>& ccs, bool global, 
 }
 
 // Packs CCs into tiles in order: a tile is closed when the next CC would pass
-// `max_states` or, for shared-memory tiles, the image budget. Layered CCs are
+// `max_states` or, for tiles of one group, the size rule. Layered CCs are
 // packed into pairs of tiles (activation, layered) over the same CCs.
 class TilePacker {
  public:
@@ -848,8 +848,8 @@ std::vector<std::vector<int>> by_alphabet(const GroupSet& gs, const std::vector<
 
 // CC indices of one kind -> the sets that become global tiles. Clusters by
 // alphabet (the bytes any state of the CC accepts) with at most 32 byte
-// classes become global when they would need more than two shared-memory
-// tiles; the remaining CCs of the kind form one more global set when they too
+// classes become global when they would need more than two tiles of one
+// group's size; the remaining CCs of the kind form one more global set when they too
 // would need more than two.
 std::vector<std::vector<int>> global_sets_of(const GroupSet& gs, const std::vector<CcInfo>& ccs,
                                              const std::vector<int>& kind, const TableOpts& opts) {
@@ -1138,8 +1138,8 @@ int build_tiles(const GroupSet& gs, const TableOpts& opts, std::vector<TileHost>
     }
   }
   // Global tiles (tile_mode 2: every acyclic or layered CC; 0: the sets
-  // global_sets_of picks); everything else, other cyclic CCs included, uses
-  // shared-memory tiles of one group.
+  // global_sets_of picks); everything else, other cyclic CCs included, goes into
+  // tiles of one group.
   std::vector<char> in_global(ccs.size(), 0);
   std::vector<std::vector<int>> gsets[2];
   if (opts.tile_mode == 2) {

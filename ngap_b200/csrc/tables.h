@@ -1,5 +1,5 @@
 // Host-side construction of the matching tables: tiles of CCs, their byte
-// classes, shared-memory images and prefix-memoization tables.
+// classes, images, look-ahead filters and prefix-memoization tables.
 #pragma once
 
 #include <vector>
@@ -63,21 +63,22 @@ struct TileHost {
 struct TableOpts {
   int precompute_depth = 0;
   int precompute_cutoff = -1;
-  int tile_states = 0;              // max states per tile; 0 = fill the image budget
+  int tile_states = 0;              // max states per tile; 0 = fill the size rule
   int64_t max_table_entries = 0;    // 0 = automatic
-  int image_budget = 128 * 1024;    // image bytes of a tile of one group
+  int image_budget = 128 * 1024;    // size rule of a tile of one group (image_bytes)
   int unbounded_tile_states = 256;  // cap for tiles of cyclic CCs (one unit per segment)
   int64_t auto_table_bytes = 12 << 20;  // automatic depth: prefix-table bytes per tile
   int max_warmup = 2048;            // longest acyclic path that still allows chunking
-  int tile_mode = 0;                // 0 automatic, 1 shared-memory tiles, 2 global tiles
+  int tile_mode = 0;                // 0 automatic, 1 tiles of one group, 2 global tiles
   bool layered = true;              // chunk CCs that are cyclic only through sticky self-loops
   int64_t auto_global_table_bytes = 192 << 20;  // automatic depth, global tiles
   int64_t global_table_entries = 32 << 20;     // list entries per table, global tiles
 };
 
 // Size rule for packing CCs into tiles of one group: n states, cw class words
-// (8 bytes of successors per state, 16 past 32767 states; the image itself
-// holds 32-byte records).
+// (8 bytes of successors per state, 16 past 32767 states). It was made for images
+// staged in shared memory and is kept as the unit of packing; images are read in
+// place and hold 32-byte records.
 // Mask words per state in the planner's size rule (1, 2 or 8).
 inline int plan_class_words(int ncls) { return ncls <= 32 ? 1 : (ncls <= 64 ? 2 : 8); }
 
