@@ -300,8 +300,9 @@ typedef struct ngap_batch_params {
   int chunk;                /* 0 = automatic */
   int use_graph;            /* capture the pipeline in a CUDA graph; replay it while the
                                tableset, streams, parameters and input pointer repeat */
-  int queue_capacity;       /* overflow-stack entries per warp (>= 1024); 0 = 65536. An
-                               engine keeps the largest capacity it has held (a smaller
+  int queue_capacity;       /* overflow-stack entries per warp (>= 1024); 0 = 65536. (The
+                               warps that follow a scan's candidates have half as many
+                               past 8192: they need less.) An engine keeps the largest capacity it has held (a smaller
                                request runs with that one). A run that needs more fails
                                with NGAP_E_OVERFLOW_QUEUE */
 } ngap_batch_params;

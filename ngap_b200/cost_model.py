@@ -16,7 +16,7 @@ from the longest prefix-table list (kernel_ngap_OA.cu:180-194). Here:
   longest and mean list, expected list length per position);
 * StaticModel is the fallback: the tables' expected list length per position
   (all keys equally likely), doubled for the expansions that follow each
-  injected state; it never looks at the input. NfaMeanModel is a calibrated
+  state; it never looks at the input, nor at the filters. NfaMeanModel is a calibrated
   baseline: the mean traced density of each NFA. LearnedModel is the 2 x 64
   MLP of ngap_mlp_* (FP32 training, BF16 or FP32 inference) on the log of the
   density;
@@ -108,9 +108,11 @@ def relative_error(pred, true, floor=0.05):
 
 
 class StaticModel:
-    """Density from the tables alone: expected states injected per position
+    """Density from the tables alone: expected list length per position
     (deepest prefix table, keys equally likely), times two for the
-    expansions that follow them."""
+    expansions that follow them. It does not know the look-ahead filters, which
+    keep most of these lists from being injected: for filtered rules it is an
+    upper estimate."""
     name = "static"
 
     def __init__(self, stats_per_nfa):
