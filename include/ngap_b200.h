@@ -302,9 +302,10 @@ typedef struct ngap_batch_params {
                                tableset, streams, parameters and input pointer repeat */
   int queue_capacity;       /* overflow-stack entries per warp (>= 1024); 0 = 65536. (The
                                warps that follow a scan's candidates have half as many
-                               past 8192: they need less.) An engine keeps the largest capacity it has held (a smaller
-                               request runs with that one). A run that needs more fails
-                               with NGAP_E_OVERFLOW_QUEUE */
+                               past 8192: they need less.) An engine keeps the largest
+                               capacity it has held (a smaller request runs with that
+                               one). A run that needs more fails with
+                               NGAP_E_OVERFLOW_QUEUE */
 } ngap_batch_params;
 
 /* Matches every stream against its NFA in one persistent launch, then sorts
