@@ -80,6 +80,23 @@ std::vector<int> digits_of(uint64_t bits) {
 
 }  // namespace
 
+// One sort of report keys: d_in[0 .. *d_n) (clamped to cap) into unique
+// reports at d_out (and stream indices at d_out_stream for MODE 1).
+//   MODE 0: keys offset << 32 | id, written as id << 32 | offset;
+//   MODE 1: keys stream << sshift | offset << oshift | id (batched matching).
+// shifts: the digits the radix pipeline sorts, least significant first.
+struct SortJob {
+  int mode;
+  uint64_t* d_in;
+  const unsigned long long* d_n;
+  uint64_t cap;
+  std::vector<int> shifts;
+  int oshift, sshift;
+  uint64_t* d_out;
+  uint32_t* d_out_stream;
+  unsigned long long* d_unique_n;
+};
+
 // A report sort captured as a CUDA graph (see sort_reports).
 struct SortGraph {
   std::vector<uint64_t> key;
@@ -103,6 +120,7 @@ struct ngap_tables {
   int device = 0;
   int num_groups = 0;
   int sid_bits = 0;  // bits of the largest group-local state id
+  uint64_t report_states = 0;
   double report_paths = 0;  // most reports a position can give, duplicates included
   std::vector<TileHost> tiles;
   std::vector<TileDev> dev_desc;
@@ -243,6 +261,8 @@ struct ngap_engine {
   cudaStream_t sort_cs = nullptr;     // capture stream of those graphs
   bool sort_graph_off = false;
   int sort_chain_pending = 0;         // pipeline kernels of the last graph sort, if it ran
+  bool sort_open = false;             // the last sort may have left keys to the pipeline (finish_sort)
+  SortJob sort_job;                   // that sort
   // test hook for the bounded device wait (ngap_engine_test_wait_timeout): armed for the
   // next ngap_match only
   int32_t test_skip_unit = -1;
@@ -317,6 +337,7 @@ int ngap_tables_build(const ngap_groups* g, const ngap_table_opts* opts, ngap_ta
   t->num_groups = (int)g->gs.groups.size();
   for (const GroupGraph& gg : g->gs.groups) {
     t->sid_bits = std::max(t->sid_bits, bits_for(std::max<uint64_t>(gg.attrs.size(), 1)));
+    for (uint8_t a : gg.attrs) t->report_states += a & 2 ? 1 : 0;
   }
   for (auto& th : t->tiles) {
     count_paths(th);
@@ -1138,23 +1159,6 @@ int blocks_per_sm(ngap_engine* e, int smem, int* out) {
   return NGAP_OK;
 }
 
-// One sort of report keys: d_in[0 .. *d_n) (clamped to cap) into unique
-// reports at d_out (and stream indices at d_out_stream for MODE 1).
-//   MODE 0: keys offset << 32 | id, written as id << 32 | offset;
-//   MODE 1: keys stream << sshift | offset << oshift | id (batched matching).
-// shifts: the digits the radix pipeline sorts, least significant first.
-struct SortJob {
-  int mode;
-  uint64_t* d_in;
-  const unsigned long long* d_n;
-  uint64_t cap;
-  std::vector<int> shifts;
-  int oshift, sshift;
-  uint64_t* d_out;
-  uint32_t* d_out_stream;
-  unsigned long long* d_unique_n;
-};
-
 // The radix pipeline over *radix_n keys; adds its launches to *kernels.
 int radix_chain(ngap_engine* e, const SortJob& j, const unsigned long long* radix_n,
                 cudaStream_t st, int* kernels) {
@@ -1192,18 +1196,18 @@ int publish(ngap_engine* e, const SortJob& j, cudaStream_t st, int* kernels) {
   return NGAP_OK;
 }
 
-// The one-CTA sort. alone: it handles any number of keys (no pipeline follows).
-int cta_sort(ngap_engine* e, const SortJob& j, bool alone, const HostOut& ho, cudaStream_t st) {
+// The one-CTA sort of at most `most` keys.
+int cta_sort(ngap_engine* e, const SortJob& j, uint64_t most, const HostOut& ho, cudaStream_t st) {
   unsigned long long* radix_n = e->d_counters + kRadixCount;
   const cudaGraphConditionalHandle none = 0;
   if (j.mode == 0)
     sort_unique_cta<0><<<1, kSmallThreads, kSmallSortSmem, st>>>(
         j.d_in, e->d_tmp, j.d_n, j.cap, radix_n, j.d_unique_n, j.oshift, j.sshift, j.d_out,
-        j.d_out_stream, none, 0, alone, ho);
+        j.d_out_stream, none, 0, most, ho);
   else
     sort_unique_cta<1><<<1, kSmallThreads, kSmallSortSmem, st>>>(
         j.d_in, e->d_tmp, j.d_n, j.cap, radix_n, j.d_unique_n, j.oshift, j.sshift, j.d_out,
-        j.d_out_stream, none, 0, alone, ho);
+        j.d_out_stream, none, 0, most, ho);
   CUDA_TRY(cudaGetLastError());
   e->launches++;
   return NGAP_OK;
@@ -1220,10 +1224,11 @@ int build_sort_graph(ngap_engine* e, const SortJob& j, SortGraph& sg) {
   unsigned long long* radix_n = e->d_counters + kRadixCount;
   SortJob a = j;  // kernel arguments
   uint64_t* d_tmp = e->d_tmp;
-  int set_cond = 1, alone = 0;
+  int set_cond = 1;
+  uint64_t most = kSmallSort;
   HostOut ho = e->ho;
   void* args[] = {&a.d_in, &d_tmp, &a.d_n, &a.cap, &radix_n, &a.d_unique_n, &a.oshift, &a.sshift,
-                  &a.d_out, &a.d_out_stream, &h, &set_cond, &alone, &ho};
+                  &a.d_out, &a.d_out_stream, &h, &set_cond, &most, &ho};
   cudaKernelNodeParams kp = {};
   kp.func = j.mode == 0 ? reinterpret_cast<void*>(sort_unique_cta<0>)
                         : reinterpret_cast<void*>(sort_unique_cta<1>);
@@ -1254,13 +1259,42 @@ int build_sort_graph(ngap_engine* e, const SortJob& j, SortGraph& sg) {
   return NGAP_OK;
 }
 
-// A match that can give at most so many reports (positions times the paths that end
-// in report states, TileHost::report_paths, since a report that several paths lead
-// to is emitted several times) sorts them with the one-CTA kernel alone, launched
-// directly: a launch with a conditional graph costs 7 us more on a B200 (29 against
-// 22 us for an empty pipeline), while one CTA keeps up with the pipeline only to
-// some 30,000 reports, which larger bounds could exceed many times over.
-constexpr double kAloneReports = 1 << 16;
+// A match whose positions times its rules' report states are at most this sorts
+// its reports with the one-CTA kernel, launched directly: a launch with a conditional
+// graph costs 7 us more on a B200 (29 against 22 us for an empty pipeline), while
+// one CTA keeps up with the pipeline only to some 30,000 reports. More keys than
+// this can come all the same where several paths lead to a report, each of which
+// emits it; the kernel then leaves them, and ngap_engine_sync launches the pipeline.
+constexpr uint64_t kAloneReports = 1ull << 16;
+
+// How many reports a match can give: without duplicates, and with them (positions
+// times the paths that end in report states, TileHost::report_paths).
+struct MostReports {
+  double unique = 0, all = 0;
+  void add(const ngap_tables* t, uint64_t positions) {
+    if (positions == 0) return;
+    unique += (double)positions * (double)t->report_states;
+    all += (double)positions * t->report_paths;
+  }
+};
+
+// Launches the pipeline for keys that the one-CTA kernel left, the match having ended
+// on e->stream, and waits for it.
+int finish_sort(ngap_engine* e) {
+  if (!e->sort_open) return NGAP_OK;
+  e->sort_open = false;
+  if (e->ho.counters[kRadixCount] > 0) {
+    int kernels = 0;
+    int rc = radix_chain(e, e->sort_job, e->d_counters + kRadixCount, e->stream, &kernels);
+    if (rc == NGAP_OK) rc = publish(e, e->sort_job, e->stream, &kernels);
+    if (rc != NGAP_OK) return rc;
+    e->launches += kernels;
+    CUDA_TRY(cudaEventRecord(e->ev[3], e->stream));
+    CUDA_TRY(cudaStreamSynchronize(e->stream));
+  }
+  e->counters_dirty = false;  // by whichever kernel came last
+  return NGAP_OK;
+}
 
 // Enqueues the sort of a match's reports on st, the match's last kernels: they
 // leave its counters and first reports for the host. Past
@@ -1268,10 +1302,16 @@ constexpr double kAloneReports = 1 << 16;
 // radix pipeline runs only for more than kSmallSort keys); inside a
 // capture, or where graphs are unavailable, it launches the one-CTA kernel and
 // the pipeline, whose kernels find no keys after a small set.
-int sort_reports(ngap_engine* e, const SortJob& j, double most_reports, cudaStream_t st) {
-  if (most_reports <= kAloneReports) return cta_sort(e, j, true, e->ho, st);
+int sort_reports(ngap_engine* e, const SortJob& j, const MostReports& most, cudaStream_t st) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(st, &cs));
+  if (cs == cudaStreamCaptureStatusNone && std::min(most.unique, most.all) <= kAloneReports) {
+    e->sort_open = true;
+    e->sort_job = j;
+    return cta_sort(e, j, kAloneReports, e->ho, st);
+  }
+  if (cs != cudaStreamCaptureStatusNone && most.all <= kAloneReports)  // nobody would finish it
+    return cta_sort(e, j, ~0ull, e->ho, st);
   if (cs == cudaStreamCaptureStatusNone && !e->sort_graph_off) {
     std::vector<uint64_t> key = {(uint64_t)j.mode,   (uint64_t)(uintptr_t)j.d_in,
                                  (uint64_t)(uintptr_t)j.d_n, j.cap,
@@ -1307,7 +1347,7 @@ int sort_reports(ngap_engine* e, const SortJob& j, double most_reports, cudaStre
       return NGAP_OK;
     }
   }
-  int rc = cta_sort(e, j, false, HostOut(), st);
+  int rc = cta_sort(e, j, kSmallSort, HostOut(), st);
   int kernels = 0;
   if (rc == NGAP_OK) rc = radix_chain(e, j, e->d_counters + kRadixCount, st, &kernels);
   if (rc == NGAP_OK) rc = publish(e, j, st, &kernels);
@@ -1321,6 +1361,7 @@ int begin_counters(ngap_engine* e, cudaStream_t st) {
   if (e->counters_dirty)
     CUDA_TRY(cudaMemsetAsync(e->d_counters, 0, kNumCounters * sizeof(unsigned long long), st));
   e->counters_dirty = true;
+  e->sort_open = false;
   return NGAP_OK;
 }
 
@@ -1495,14 +1536,16 @@ int ngap_match(ngap_engine* e, const ngap_tables* t, const uint8_t* input, int i
                           bit_range(32, bits_for(total));
     const SortJob job{0,  e->d_reports, e->d_counters + 0, cap,     digits_of(bits),
                       32, 64,           e->d_unique,       nullptr, e->d_counters + 1};
-    if ((rc = sort_reports(e, job, (double)total * t->report_paths, st)) != NGAP_OK) return rc;
+    MostReports most;
+    most.add(t, total);
+    if ((rc = sort_reports(e, job, most, st)) != NGAP_OK) return rc;
   } else {
     publish_kernel<<<1, 32, 0, st>>>(e->ho);
     CUDA_TRY(cudaGetLastError());
     e->launches++;
   }
   CUDA_TRY(cudaEventRecord(e->ev[3], st));
-  e->counters_dirty = false;
+  e->counters_dirty = e->sort_open;
   e->ran = true;
   return NGAP_OK;
 }
@@ -1514,6 +1557,8 @@ int ngap_engine_sync(ngap_engine* e) {
   }
   CUDA_TRY(cudaSetDevice(e->device));
   CUDA_TRY(cudaStreamSynchronize(e->stream));
+  const int rc = finish_sort(e);
+  if (rc != NGAP_OK) return rc;
   CUDA_TRY(cudaEventElapsedTime(&e->match_ms, e->ev[1], e->ev[2]));
   CUDA_TRY(cudaEventElapsedTime(&e->sort_ms, e->ev[2], e->ev[3]));
   if (e->sort_chain_pending > 0 && e->ho.counters[kRadixCount] > 0)  // the radix pipeline ran
@@ -1683,8 +1728,12 @@ int ngap_reports_sort_unique(ngap_engine* e, const uint64_t* d_in, uint64_t n, u
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   *n_out = 0;
   if (n == 0) return NGAP_OK;
-  int rc = ensure_reports(e, n);
-  if (rc != NGAP_OK) return rc;
+  int rc = NGAP_OK;
+  if (e->ran && e->sort_open) {  // the last match's reports are in the buffers used below
+    CUDA_TRY(cudaStreamSynchronize(e->stream));
+    if ((rc = finish_sort(e)) != NGAP_OK) return rc;
+  }
+  if ((rc = ensure_reports(e, n)) != NGAP_OK) return rc;
   // input arrives in the reference encoding (id << 32 | offset): swap halves
   // into sort keys in the engine's report buffer
   CUDA_TRY(cudaMemcpyAsync(e->d_reports, d_in, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
@@ -1695,7 +1744,7 @@ int ngap_reports_sort_unique(ngap_engine* e, const uint64_t* d_in, uint64_t n, u
   const SortJob job{0,  e->d_reports, e->d_counters + 5, n,       digits_of(~0ull),
                     32, 64,           d_out,             nullptr, e->d_counters + 6};
   int kernels = 0;
-  rc = n <= (uint64_t)kSmallSort ? cta_sort(e, job, true, HostOut(), st)
+  rc = n <= (uint64_t)kSmallSort ? cta_sort(e, job, kSmallSort, HostOut(), st)
                                  : radix_chain(e, job, job.d_n, st, &kernels);
   if (rc != NGAP_OK) return rc;
   unsigned long long un = 0;
@@ -1962,9 +2011,8 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
   mp.skip_copy_unit = -1;
   e->trace_seg_len = 0;
 
-  double most_reports = 0;  // streams may share bytes of the input
-  for (const ngap_batch_stream& s : sv)
-    if (s.length > 0) most_reports += (double)s.length * ts->tables[s.nfa]->report_paths;
+  MostReports most;  // streams may share bytes of the input
+  for (const ngap_batch_stream& s : sv) most.add(ts->tables[s.nfa], s.length);
 
   auto enqueue = [&](cudaStream_t qs) -> int {
     if (e->trace) {
@@ -1984,7 +2032,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
                             bit_range(oshift, obits) | bit_range(sshift, sbits);
       const SortJob job{1,      e->d_reports, e->d_counters + 0, cap,             digits_of(bits),
                         oshift, sshift,       e->d_unique,       e->d_stream_ids, e->d_counters + 1};
-      if ((r = sort_reports(e, job, most_reports, qs)) != NGAP_OK) return r;
+      if ((r = sort_reports(e, job, most, qs)) != NGAP_OK) return r;
     } else {
       publish_kernel<<<1, 32, 0, qs>>>(e->ho);
       CUDA_TRY(cudaGetLastError());
@@ -2000,7 +2048,7 @@ int ngap_batch_match(ngap_engine* e, const ngap_tableset* ts, const uint8_t* inp
     CUDA_TRY(cudaEventRecord(e->ev[1], st));
     if ((rc = begin_counters(e, st)) != NGAP_OK) return rc;
     if ((rc = enqueue(st)) != NGAP_OK) return rc;
-    e->counters_dirty = false;
+    e->counters_dirty = e->sort_open;
     CUDA_TRY(cudaEventRecord(e->ev[2], st));
     CUDA_TRY(cudaEventRecord(e->ev[3], st));
     e->ran = true;

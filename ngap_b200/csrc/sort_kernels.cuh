@@ -347,13 +347,14 @@ __global__ void __launch_bounds__(kHostReports) publish_results(HostOut ho,
 
 // One CTA sorts and deduplicates: up to kBitonic keys with a bitonic network, up
 // to kSmallSort with radix passes between two shared-memory buffers (only
-// over the digits that vary), and, where `alone` says that no pipeline
-// follows, any number with the same passes between d_in and tmp in global
-// memory. It then writes the unique reports like unique_write. It stores in *radix_n the key count the radix
+// over the digits that vary), and up to `most`, where that is larger, with the same
+// passes between d_in and tmp in global memory. It then writes the unique
+// reports like unique_write. It stores in *radix_n the key count the radix
 // pipeline still has to sort: 0 when the keys were handled here (the
 // pipeline's kernels then find no tiles), n otherwise; launched from a graph, it
 // also sets the condition of the conditional node that holds the pipeline.
-// ho.counters != nullptr: it publishes when it handled the keys.
+// ho.counters != nullptr: it publishes when it handled the keys; otherwise it
+// copies the counters out and leaves them to the pipeline.
 constexpr int kSmallSort = 8192;
 constexpr int kBitonic = 1024;
 constexpr int kSmallThreads = 1024;
@@ -445,18 +446,22 @@ __global__ void __launch_bounds__(kSmallThreads) sort_unique_cta(
     uint64_t* keys, uint64_t* tmp, const unsigned long long* d_n, uint64_t cap,
     unsigned long long* radix_n, unsigned long long* d_unique_n, int oshift, int sshift,
     uint64_t* __restrict__ out, uint32_t* __restrict__ out_stream, cudaGraphConditionalHandle cond,
-    int set_cond, int alone, HostOut ho) {
+    int set_cond, uint64_t most, HostOut ho) {
   extern __shared__ __align__(16) uint64_t sk[];
   __shared__ uint32_t wsum[kDigits], first[kDigits];
   __shared__ unsigned long long s_vary;
   const uint64_t n = dev_count(d_n, cap);
-  const bool big = n > (uint64_t)kSmallSort && !alone;
+  const bool big = n > most;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   if (t == 0) {
     *radix_n = big ? n : 0ull;
     if (set_cond) cudaGraphSetConditional(cond, big ? 1u : 0u);  // graph launches only
   }
-  if (big) return;
+  if (big) {
+    __syncthreads();
+    if (ho.counters && t < kNumCounters) ho.counters[t] = __ldcg(ho.d_counters + t);
+    return;
+  }
   const uint64_t* src = sk;
   if (n <= (uint64_t)kBitonic) {
     const uint32_t nn = (uint32_t)n;

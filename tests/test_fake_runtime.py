@@ -249,13 +249,26 @@ def batch(nfas, offs, lens):
     return alone(nb.batch_match_async, e, ts, data, offs, lens, nfas, result_capacity=CAP)
 
 
-assert plain(0, 4000) and plain(0, 100)          # 4000 positions, one path to each of 6 reports
-assert plain(1, 128) and not plain(1, 129)       # 512 paths to one report: 65,536 reports at most
-assert not plain(2, 1)                           # cyclic: no bound
+assert plain(0, 4000) and plain(0, 100)          # 4000 positions, 6 reports
+assert plain(1, 4000) and plain(2, 4000)         # one report (however many paths lead to it)
+big = np.zeros(70_000, np.uint8)
+assert alone(e.match_async, t[1], big, 1, 65_536, result_capacity=CAP)
+assert not alone(e.match_async, t[1], big, 1, 65_537, result_capacity=CAP)
 assert batch([0, 0], [0, 2000], [2000, 2000])
 assert not batch([0] * 30, [0] * 30, [4000] * 30)  # streams over the same bytes
 assert batch([0] * 30, [0] * 30, [40] * 30)
-assert batch([0, 1, 2], [0, 1000, 1100], [1000, 100, 0]) and not batch([0, 1], [0, 1000], [1000, 300])
+assert batch([0, 1, 2], [0, 1000, 1100], [1000, 100, 0])
+
+
+def captured(nfas, offs, lens):
+    "In a capture nobody would finish a sort that left keys: the pipeline is there unless duplicates are bounded too."
+    out = log(nb.batch_match_async, e, ts, data, offs, lens, nfas, result_capacity=CAP, use_graph=True)
+    return not any("radix_scatter" in x for x in out)
+
+
+assert captured([0, 0], [0, 2000], [2000, 2000])
+assert captured([1], [0], [128]) and not captured([1], [0], [129])  # 512 paths to one report
+assert not captured([2], [0], [1])                                  # cyclic: no bound
 """
 
 
