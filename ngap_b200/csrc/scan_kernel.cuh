@@ -666,6 +666,12 @@ __global__ void __launch_bounds__(kRunWarps * 32, 1) run_kernel(MatchParams p, c
     tile_run<!LAYERED>(p, t, t->pt, cls, tr);
     const int batch = LAYERED ? 32 : min(tr.batch, 32);
     const uint32_t active = LAYERED ? p.act_cnt[run.act_rowid] : 0u;
+    auto follow = [&]() {  // every path on the worklist to its end
+      if (UNIQUE)
+        while (held(w) > 0) step_run<true>(p, ws, w, tr.tv, c, lane, n_expanded);
+      else
+        walk_run(p, ws, w, tr.tv, c, lane, n_expanded);
+    };
     bool starts = run.starts != 0u;
     uint32_t c0 = 0, resume = 0;
     while (starts || c0 < run.n) {
@@ -681,13 +687,9 @@ __global__ void __launch_bounds__(kRunWarps * 32, 1) run_kernel(MatchParams p, c
           inject_run(p, ws, w, tr.tv, c, lane, lane < m, r, tr.depth, resume, n_injected);
         if (resume == 0u) c0 += batch;
       }
-      // the paths: when the worklist is full enough, and at the end
-      if (held(w) < (starts || c0 < run.n ? kInjectLow : 1)) continue;
-      if (UNIQUE)
-        while (held(w) > 0) step_run<true>(p, ws, w, tr.tv, c, lane, n_expanded);
-      else
-        walk_run(p, ws, w, tr.tv, c, lane, n_expanded);
+      if (held(w) >= kInjectLow) follow();
     }
+    if (held(w) > 0) follow();
     if (p.unit_work) {  // work of the run's piece (all lanes)
       unsigned long long d = n_expanded + n_injected - work0;
 #pragma unroll
