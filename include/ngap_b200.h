@@ -194,7 +194,9 @@ typedef struct ngap_match_params {
  * report copy: matches `input` (host or device memory, num_seg * seg_len
  * bytes) against every group and leaves the sorted, deduplicated reports on
  * the device. Asynchronous on `stream` (a cudaStream_t, NULL = default);
- * ngap_engine_sync waits and returns the run's status. `input` must stay
+ * ngap_engine_sync waits and returns the run's status; results are valid after
+ * it, not after a wait for the stream alone (it finishes the report sort where
+ * duplicates left it far more keys than reports could be). `input` must stay
  * unchanged until the match has ended on `stream`: device memory of the
  * engine's GPU is read in place when its address and length are multiples of
  * 16; memory of another GPU is copied. */
