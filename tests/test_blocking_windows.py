@@ -155,6 +155,25 @@ def test_blocking_follows_states(engine, size, rules):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("size", [5_000, 200_000])
+def test_blocking_reports_few_duplicates(engine, size):
+    """Forks followed in whole windows: 2^8 paths, two states before the report."""
+    groups = nb.Groups(nb.Nfa.from_string(forks(8)), group_num=1)
+    data = np.full(size, ord("x"), np.uint8)
+    word = np.frombuffer(b"a" + b"bc" * 8, np.uint8)
+    for at in range(50, size - 50, 997):
+        data[at:at + len(word)] = word
+    want, _ = oracle.match(groups.views(), data, 1, size)
+    tables = nb.Tables(groups, precompute_depth=1)
+    cap = 2 * len(want)
+    assert np.array_equal(engine.match(tables, data, 1, size, algorithm="blockinggroups", result_capacity=cap), want)
+    nb.batch_match_async(engine, nb.TableSet([tables]), data, [0], [size], [0], algorithm="blockinggroups",
+                         result_capacity=cap)
+    engine.sync()
+    assert np.array_equal(nb.batch_results(engine)[0], want)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("algorithm", ["blockinggroups", "NAPgroups"])
 @pytest.mark.parametrize("size", [3_000, 150_000])
 def test_many_always_active_states_of_one_symbol(built, algorithm, size):
